@@ -92,6 +92,51 @@ def test_gemm_f32(M, N, K):
     assert torch.equal(one[0], got[0])
 
 
+@pytest.mark.parametrize("K", [63, 64, 65, 1023, 1024, 1028, 3100])
+def test_gemm_f32_rows_agree_across_kernels(K):
+    """The few-row kernels (1, 2, 4, 8 and 16 rows), the tile kernel (more) and both ways of loading sum in one order: a row
+    is the same to the last bit whatever the batch.  Bound: K FMAs in slices of 64, so below K/64 + 64 roundings of 2^-24
+    relative to sum |a w| < K * 4 sigma, far below 1e-5 of the largest result."""
+    ops = _ops("float32")
+    g = torch.Generator().manual_seed(14)
+    a, w = torch.randn(130, K, generator=g).cuda(), torch.randn(203, K, generator=g).cuda()
+    whole = ops.linear(a, w)
+    assert _err(whole, (a.double() @ w.double().T).float()) < 1e-5
+    for M in (1, 2, 3, 4, 7, 8, 9, 16, 17, 64, 65):
+        assert torch.equal(ops.linear(a[:M].contiguous(), w), whole[:M]), M
+    shifted = torch.empty(203 * K + 1, device="cuda")[1:].view(203, K).copy_(w)      # rows that no 16-byte load can take
+    assert torch.equal(ops.linear(a[:5].contiguous(), shifted), whole[:5]) and torch.equal(ops.linear(a, shifted), whole)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("n_heads,n_kv,d", [(16, 2, 64), (22, 2, 40), (8, 8, 37), (16, 1, 200), (4, 2, 96)])
+def test_attention_generic_shares_of_keys(dtype, n_heads, n_kv, d):
+    """Key counts around the pieces of 32 and the turns of the warps, groups that fill a block of heads and groups that do
+    not, head sizes that no 16-byte load can take; a row does not depend on the batch."""
+    ops = _ops(dtype)
+    lens = [1, 31, 33, 64, 257, 300]
+    cache, slots = _paged_setup(ops, lens, n_kv, d, 0, dtype)
+    lane, T = cache.lane(0), sum(lens)
+    qkv = torch.randn(T, (n_heads + 2 * n_kv) * d, generator=torch.Generator().manual_seed(15)).to(DT[dtype]).cuda()
+    positions = torch.cat([torch.arange(n) for n in lens]).int().cuda()
+    token_seq = torch.cat([torch.full((n,), i) for i, n in enumerate(lens)]).int().cuda()
+    sl = torch.tensor(slots, dtype=torch.int32).cuda()
+    q = ops.rope_store(qkv, n_heads, n_kv, d, positions, token_seq, sl, lane.page_table, lane.k, lane.v, None, 1.0, 0)
+    rows = qkv.float().cpu().view(T, n_heads + 2 * n_kv, d)
+    scale = 1 / math.sqrt(d)
+    for window in (0, 45):
+        out = ops.attention_generic(q, lane.k, lane.v, positions, token_seq, sl, lane.page_table, n_kv, scale, window=window)
+        o = 0
+        for n in lens:
+            want = plain.dense_attention(rows[o:o + n, :n_heads], rows[o:o + n, n_heads:n_heads + n_kv],
+                                         rows[o:o + n, n_heads + n_kv:], scale, window=window).reshape(n, -1)
+            assert _err(out[o:o + n], want) < KTOL[dtype], (n, window)
+            o += n
+        last = ops.attention_generic(q[-1:].contiguous(), lane.k, lane.v, positions[-1:].contiguous(), token_seq[-1:].contiguous(),
+                                     sl, lane.page_table, n_kv, scale, window=window)
+        assert torch.equal(last[0], out[-1])
+
+
 def test_linear_bf16():
     ops = _ops("bfloat16")
     g = torch.Generator().manual_seed(5)
