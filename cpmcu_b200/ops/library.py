@@ -114,7 +114,7 @@ _SIGNATURES = {
     "cpm_moe_route": [_P, c_int, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, _P, c_int, c_int, c_int,
                       c_float, _P],
     "cpm_moe_group": [_P, c_int, c_int, _P, _P, _P],
-    "cpm_moe_expert_product": [_P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, _P, c_float, c_float, c_float, c_int,
+    "cpm_moe_expert_product": [_P, _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, _P, c_float, c_float, c_float, c_int,
                                _P],
     "cpm_moe_pair_product": [_P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, _P, c_float, c_float, c_float, _P],
     "cpm_moe_combine": [_P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, _P],
@@ -172,6 +172,8 @@ def load() -> ctypes.CDLL:
             lib.cpm_set_decode_early(int(os.environ["CPMCU_DECODE_EARLY"]))
         lib.cpm_gemm_tcgen05_error.argtypes = []
         lib.cpm_gemm_tcgen05_error.restype = c_int
+        lib.cpm_moe_tcgen05_error.argtypes = []
+        lib.cpm_moe_tcgen05_error.restype = c_int
         lib.cpm_attention_tcgen05_error.argtypes = []
         lib.cpm_attention_tcgen05_error.restype = c_int
         lib.cpm_select_blocks_scratch_floats.argtypes = [c_int, c_int, c_int, c_int]

@@ -916,13 +916,17 @@ class Ops:
         """Error code the tcgen05 attention kernel recorded since the last call (0 = none); synchronises."""
         return int(self.lib.cpm_attention_tcgen05_error())
 
+    def moe_tcgen05_error(self) -> int:
+        """Error code the tcgen05 kernel of the experts' products recorded since the last call (0 = none); synchronises."""
+        return int(self.lib.cpm_moe_tcgen05_error())
+
     def raise_on_kernel_error(self) -> None:
         """The tcgen05 kernels bound every wait and record a code instead of hanging; this turns a recorded
         code into an exception.  It synchronises the device: call it where the host waits anyway."""
-        gemm, attn = self.tcgen05_error(), self.attention_tcgen05_error()
-        if gemm or attn:
+        gemm, attn, moe = self.tcgen05_error(), self.attention_tcgen05_error(), self.moe_tcgen05_error()
+        if gemm or attn or moe:
             raise RuntimeError(f"a tcgen05 kernel gave up waiting on a barrier (product: code {gemm}, attention: code "
-                               f"{attn}); the results of this step are not valid")
+                               f"{attn}, experts: code {moe}); the results of this step are not valid")
         self.raise_on_bounds_error()
         arena = self.workspace.persistent.arena if self.workspace is not None else None
         if arena is not None and arena.guards:
@@ -1463,9 +1467,8 @@ class Ops:
         pairs = n * top
         h = self.empty(pairs, ff)
         y = self.empty(pairs, hidden)
-        if (self.code == BF16 and pairs <= self.MOE_PAIRWISE_MAX_PAIRS and hidden % 8 == 0 and ff % 8 == 0
-                and hidden <= 12288 and ff <= 12288):
-            # few pairs (a decode step): every pair streams its expert's weights, no grouping
+        if self.code == BF16 and pairs <= min(self.MOE_PAIRWISE_MAX_PAIRS, 8192) and hidden % 8 == 0 and ff % 8 == 0:
+            # few pairs (a decode step): every chosen expert's weights are streamed once, no grouping
             check(self.lib.cpm_moe_pair_product(_ptr(x), _ptr(first), _ptr(second), _ptr(h), _ptr(chosen), pairs, top, ff, hidden, mode,
                                                 _ptr(input_scale), *lims, self._stream()), "moe gate/up product by pair")
             check(self.lib.cpm_moe_pair_product(_ptr(h), _ptr(w_down), None, _ptr(y), _ptr(chosen), pairs, top, hidden, ff, 0,
@@ -1474,9 +1477,10 @@ class Ops:
         offsets = self.empty(E + 1, dtype=torch.int32)
         order = self.empty(pairs, dtype=torch.int32)
         check(self.lib.cpm_moe_group(_ptr(chosen), pairs, E, _ptr(offsets), _ptr(order), self._stream()), "moe_group")
-        check(self.lib.cpm_moe_expert_product(_ptr(x), _ptr(first), _ptr(second), _ptr(h), _ptr(offsets), _ptr(order), pairs, E, top,
+        # (y holds the tokens' rows in expert order until the down product writes it)
+        check(self.lib.cpm_moe_expert_product(_ptr(x), _ptr(first), _ptr(second), _ptr(h), _ptr(offsets), _ptr(order), _ptr(y), pairs, E, top,
                                               ff, hidden, mode, _ptr(input_scale), *lims, self.code, self._stream()), "moe gate/up product")
-        check(self.lib.cpm_moe_expert_product(_ptr(h), _ptr(w_down), None, _ptr(y), _ptr(offsets), _ptr(order), pairs, E, top,
+        check(self.lib.cpm_moe_expert_product(_ptr(h), _ptr(w_down), None, _ptr(y), _ptr(offsets), _ptr(order), None, pairs, E, top,
                                               hidden, ff, 0, None, 0.0, 0.0, 0.0, self.code, self._stream()), "moe down product")
         return y
 

@@ -855,3 +855,53 @@ def test_decode_attention_with_rotation_inside(n_heads, n_kv, d):
     r3 = three.float().cpu().view(3, -1, d)
     ref = plain.dense_attention(r3[:, :n_heads], r3[:, n_heads:n_heads + n_kv], r3[:, n_heads + n_kv:], scale)[-1].reshape(-1)
     assert _err(got[0], ref) < KTOL["bfloat16"]
+
+
+@pytest.mark.parametrize("E,top,W,ff,n,skew", [
+    (64, 6, 256, 768, 700, False),     # one chunk an expert, whole feature tiles
+    (4, 2, 136, 72, 700, True),        # chunks of more than 256 pairs, a ragged last slice of K, an expert nobody chose
+    (512, 3, 64, 136, 65, False),      # the most experts, most of one pair or none
+    (3, 1, 8, 12, 600, False),         # a row shorter than a slice, rows that are no whole 16-byte pieces
+    (8, 4, 200, 40, 24, False),        # the most pairs of the kernel for few
+    (8, 4, 200, 40, 25, False),        # one more: tiles
+    (2, 1, 72, 264, 33, False),        # more pairs of one expert than the eight columns of an instruction
+])
+@pytest.mark.parametrize("mode", ["silu", "relu2", "bounded"])
+def test_expert_products_by_tiles_and_for_few(E, top, W, ff, n, skew, mode):
+    """Both kernels of the experts' products against the formulas in 64 bits.  Each output is rounded to bf16 twice (the gated
+    value, then the down product), relative to the largest value: two times 2^-9 and the sums' spread, within KTOL."""
+    ops = _ops("bfloat16")
+    g = torch.Generator().manual_seed(E * 1000 + n)
+    x = torch.randn(n, W, generator=g).bfloat16()
+    wg, wu = ((torch.randn(E, ff, W, generator=g) * W ** -0.5).bfloat16() for _ in range(2))
+    wd = (torch.randn(E, W, ff, generator=g) * ff ** -0.5).bfloat16()
+    usable = E - 1 if skew else E
+    prefer = torch.rand(n, usable, generator=g) + (torch.arange(usable) == 0) * (0.9 if skew else 0.0)
+    chosen = prefer.topk(top).indices.int()
+    scale = torch.rand(n, top, generator=g) + 0.5
+    clamp = (1.5, 1.702, 1.0) if mode == "bounded" else None
+    xd, got = x.cuda().double(), None
+    up = torch.einsum("nw,efw->nef", xd, wu.cuda().double())
+    if mode == "relu2":
+        got = ops.moe_experts(x.cuda(), chosen.cuda(), None, wu.cuda(), wd.cuda(), input_scale=scale.cuda())
+    else:
+        got = ops.moe_experts(x.cuda(), chosen.cuda(), wg.cuda(), wu.cuda(), wd.cuda(), clamp=clamp)
+        gate = torch.einsum("nw,efw->nef", xd, wg.cuda().double())
+    rows, idx = torch.arange(n).cuda()[:, None], chosen.long().cuda()
+    u = up[rows, idx]
+    if mode == "relu2":
+        h = torch.relu(u * scale.cuda().double()[..., None]) ** 2
+    elif mode == "silu":
+        h = torch.nn.functional.silu(gate[rows, idx]) * u
+    else:
+        a, b = gate[rows, idx].clamp(max=1.5), u.clamp(-1.5, 1.5)
+        h = a * torch.sigmoid(1.702 * a) * (b + 1.0)
+    want = torch.einsum("ntf,ntwf->ntw", h, wd.cuda().double()[idx]) if E * W * ff * n < 1 << 28 else \
+        torch.stack([torch.einsum("tf,twf->tw", h[t], wd.cuda()[idx[t]].double()) for t in range(n)])
+    assert _err(got.view(n, top, W), want) < KTOL["bfloat16"]
+    assert ops.moe_tcgen05_error() == 0
+    weights = torch.rand(n, top, generator=g)
+    shared = torch.randn(n, W, generator=g).bfloat16()
+    out = ops.moe_combine(got, weights.cuda(), shared.cuda(), weights[:, 0].contiguous().cuda())
+    total = (got.view(n, top, W).double() * weights.cuda().double()[..., None]).sum(1) + weights[:, :1].cuda().double() * shared.cuda().double()
+    assert _err(out, total) < 2.0 ** -8                            # one rounding to bf16
