@@ -266,9 +266,98 @@ head_project_kernel(const In* __restrict__ in, const Wt* __restrict__ w, Out* __
     }
 }
 
+// The same product for the bf16 matrices of a decode step (N a multiple of 8, so that a row's pieces of 8 columns are 16 bytes):
+// TOK tokens x one head x 32 columns a block, a thread 8 columns of every 64th row.  The first eight rows of a
+// thread, all of them at ranks up to 512, are asked for before the kernel ahead is waited for (no kernel writes weights),
+// so that what is left behind the wait is one trip for the inputs, the sums and two reductions.  Bound by that chain of latencies: 2.4 MB of
+// matrices are read in less than a microsecond.  One column a thread, in rounds of sixteen rows behind the wait, took 21 us a launch in a
+// decode step of 8 tokens (16 heads, 512 -> 128) and 8.4 us (128 -> 512).
+template <int TOK, typename In, typename Out>
+__global__ void __launch_bounds__(256)
+head_project_few_kernel(const In* __restrict__ in, const bf16* __restrict__ w, Out* __restrict__ out, int n_tokens, int n_heads, int K, int N) {
+    extern __shared__ __align__(16) float hf_smem[];                 // [K][TOK] inputs
+    __shared__ float red[8][TOK][32];
+    constexpr int kAhead = 8;
+    const int h = blockIdx.y, t0 = blockIdx.x * TOK, nt = min(TOK, n_tokens - t0);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n = blockIdx.z * 32 + 8 * (threadIdx.x & 3), kp = threadIdx.x >> 2;
+    const bf16* wh = w + (int64_t)h * K * N + (n < N ? n : 0);       // columns past N: the row's first, never stored
+    uint4 ahead[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+        const int k = kp + 64 * u;
+        ahead[u] = k < K ? __ldg(reinterpret_cast<const uint4*>(wh + (int64_t)k * N)) : make_uint4(0, 0, 0, 0);
+    }
+    pdl_launch_dependents();
+    pdl_wait();
+    for (int k = threadIdx.x; k < K; k += 256)
+#pragma unroll
+        for (int tt = 0; tt < TOK; ++tt) hf_smem[k * TOK + tt] = tt < nt ? to_f32(in[((int64_t)(t0 + tt) * n_heads + h) * K + k]) : 0.f;
+    __syncthreads();
+    float acc[8 * TOK];                                                // [column][token]
+#pragma unroll
+    for (int i = 0; i < 8 * TOK; ++i) acc[i] = 0.f;
+    auto add = [&](const uint4& raw, int k) {
+        float x[TOK];
+#pragma unroll
+        for (int tt = 0; tt < TOK; ++tt) x[tt] = hf_smem[k * TOK + tt];
+        const __nv_bfloat162* pr = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float2 f = __bfloat1622float2(pr[i]);
+#pragma unroll
+            for (int tt = 0; tt < TOK; ++tt) {
+                acc[2 * i * TOK + tt] = fmaf(x[tt], f.x, acc[2 * i * TOK + tt]);
+                acc[(2 * i + 1) * TOK + tt] = fmaf(x[tt], f.y, acc[(2 * i + 1) * TOK + tt]);
+            }
+        }
+    };
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u)
+        if (kp + 64 * u < K) add(ahead[u], kp + 64 * u);
+#pragma unroll 4
+    for (int k = kp + 64 * kAhead; k < K; k += 64) add(__ldg(reinterpret_cast<const uint4*>(wh + (int64_t)k * N)), k);
+    // the warp's eight partial sums of a column: lanes trade halves, so that each ends up with one column's tokens
+#pragma unroll
+    for (int step = 0; step < 3; ++step) {
+        const int mask = 16 >> step, half = (4 * TOK) >> step;
+        const bool upper = lane & mask;
+#pragma unroll
+        for (int i = 0; i < half; ++i) {
+            const float give = upper ? acc[i] : acc[i + half], keep = upper ? acc[i + half] : acc[i];
+            acc[i] = keep + __shfl_xor_sync(0xffffffffu, give, mask);
+        }
+    }
+    const int col = 8 * (lane & 3) + ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
+#pragma unroll
+    for (int tt = 0; tt < TOK; ++tt) red[warp][tt][col] = acc[tt];
+    __syncthreads();
+    const int c = threadIdx.x & 31, tt = threadIdx.x >> 5, nn = blockIdx.z * 32 + c;
+    if (tt < nt && nn < N) {
+        float sum = 0.f;
+#pragma unroll
+        for (int v = 0; v < 8; ++v) sum += red[v][tt][c];
+        out[((int64_t)(t0 + tt) * n_heads + h) * N + nn] = from_f32<Out>(sum);
+    }
+}
+
+template <int TOK, typename In, typename Out>
+static int launch_head_project_few(const void* in, const void* w, void* out, int n_tokens, int n_heads, int K, int N, cudaStream_t stream) {
+    cpm_launch(kLaunchProduct, head_project_few_kernel<TOK, In, Out>, dim3((n_tokens + TOK - 1) / TOK, n_heads, (N + 31) / 32), dim3(256),
+               (size_t)K * TOK * sizeof(float), stream, (const In*)in, (const bf16*)w, (Out*)out, n_tokens, n_heads, K, N);
+    return launch_status();
+}
+
 template <typename In, typename Wt, typename Out>
 static int launch_head_project(const void* in, const void* w, void* out, int n_tokens, int n_heads, int K, int N,
                                cudaStream_t stream) {
+    // (what the inputs take of shared memory is kept to what a launch has without asking)
+    if (sizeof(Wt) == 2 && N % 8 == 0 && ((uintptr_t)w & 15) == 0 && (size_t)K * 8 * sizeof(float) <= 36 * 1024) {
+        if (n_tokens == 1) return launch_head_project_few<1, In, Out>(in, w, out, n_tokens, n_heads, K, N, stream);
+        if (n_tokens == 2) return launch_head_project_few<2, In, Out>(in, w, out, n_tokens, n_heads, K, N, stream);
+        if (n_tokens <= 4) return launch_head_project_few<4, In, Out>(in, w, out, n_tokens, n_heads, K, N, stream);
+        return launch_head_project_few<8, In, Out>(in, w, out, n_tokens, n_heads, K, N, stream);
+    }
     const size_t smem = (size_t)kProjectTokens * (K + kProjectParts * kProjectCols) * sizeof(float);
     auto kern = head_project_kernel<In, Wt, Out>;
     if (smem > 227 * 1024) return CPM_BAD_ARGUMENT;
@@ -678,10 +767,12 @@ latent_attention_mma_kernel(const float* __restrict__ q, const bf16* __restrict_
     }
 }
 
-// One block per (token, head group, row of the tile): the shares' weights are worked out once, then the threads add up
-// the shares' columns.
-__global__ void latent_attention_merge_kernel(const float* __restrict__ scratch, void* __restrict__ out_any, int out_bf16, int n_heads,
-                                              int rank, int n_splits) {
+// One block per (token, head group, row of the tile): the weights of the shares that had keys are worked out once, then a thread
+// adds up two columns of all of them, sixteen shares in flight.  Bound by the latency of two dependent trips to L2 (one column at a
+// time in rounds of eight shares, empty ones too: 14.5 us a launch for 8 tokens of 16 heads, rank 512, 32 shares).
+__global__ void __launch_bounds__(288)
+latent_attention_merge_kernel(const float* __restrict__ scratch, void* __restrict__ out_any, int out_bf16, const int* __restrict__ positions,
+                              int window, int n_heads, int rank, int n_splits) {
     __shared__ float weight[64];
     __shared__ float inv_l;
     pdl_launch_dependents();
@@ -689,37 +780,52 @@ __global__ void latent_attention_merge_kernel(const float* __restrict__ scratch,
     const int t = blockIdx.x, hg = blockIdx.y, r = blockIdx.z;
     const int h = hg * kMmaRows + r;
     if (h >= n_heads) return;
+    // the shares that had keys come first (the same arithmetic as in the kernel that wrote them)
+    const int p = positions[t];
+    const int lo = window > 0 ? max(0, p - window + 1) : 0;
+    const int tiles = (p + 1 - lo + kMmaKeys - 1) / kMmaKeys, per = (tiles + n_splits - 1) / n_splits;
+    const int used = (tiles + per - 1) / per;
     const float* base = scratch + (((int64_t)t * gridDim.y + hg) * n_splits * kMmaRows + r) * (rank + 2);
     const int64_t share = (int64_t)kMmaRows * (rank + 2);
     if (threadIdx.x < 32) {
-        float mx = -INFINITY;
-        for (int s = threadIdx.x; s < n_splits; s += 32) mx = fmaxf(mx, base[s * share + rank]);
+        float ms[2], ls[2], mx = -INFINITY;                          // at most 64 shares
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int s = threadIdx.x + 32 * i;
+            ms[i] = s < used ? base[s * share + rank] : -INFINITY;
+            ls[i] = s < used ? base[s * share + rank + 1] : 0.f;
+            mx = fmaxf(mx, ms[i]);
+        }
         mx = warp_max(mx);
         float l = 0.f;
-        for (int s = threadIdx.x; s < n_splits; s += 32) {
-            const float ms = base[s * share + rank];
-            const float w = ms == -INFINITY ? 0.f : exp2f(ms - mx);      // the shares' maxima are base-2 logarithms
-            weight[s] = w;
-            l = fmaf(base[s * share + rank + 1], w, l);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const float w = ms[i] == -INFINITY ? 0.f : exp2f(ms[i] - mx);      // the shares' maxima are base-2 logarithms
+            weight[threadIdx.x + 32 * i] = w;
+            l = fmaf(ls[i], w, l);
         }
         l = warp_sum(l);
         if (threadIdx.x == 0) inv_l = l > 0.f ? 1.f / l : 0.f;
     }
     __syncthreads();
     const int64_t o = ((int64_t)t * n_heads + h) * rank;
-    for (int c = threadIdx.x; c < rank; c += blockDim.x) {
-        float acc = 0.f;
-        for (int s0 = 0; s0 < n_splits; s0 += 8) {
-            float v[8];
+    for (int c = 2 * threadIdx.x; c < rank; c += 2 * blockDim.x) {       // the rank is even, a share's row 8-byte aligned
+        float2 acc = make_float2(0.f, 0.f);
+        for (int s0 = 0; s0 < used; s0 += 16) {
+            float2 v[16];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) v[u] = s0 + u < n_splits ? base[(s0 + u) * share + c] : 0.f;
+            for (int u = 0; u < 16; ++u) v[u] = s0 + u < used ? *reinterpret_cast<const float2*>(base + (s0 + u) * share + c) : make_float2(0.f, 0.f);
 #pragma unroll
-            for (int u = 0; u < 8; ++u)
-                if (s0 + u < n_splits) acc = fmaf(v[u], weight[s0 + u], acc);
+            for (int u = 0; u < 16; ++u)
+                if (s0 + u < used) {
+                    acc.x = fmaf(v[u].x, weight[s0 + u], acc.x);
+                    acc.y = fmaf(v[u].y, weight[s0 + u], acc.y);
+                }
         }
-        const float res = acc * inv_l;
-        if (out_bf16) static_cast<bf16*>(out_any)[o + c] = __float2bfloat16_rn(res);
-        else static_cast<float*>(out_any)[o + c] = res;
+        acc.x *= inv_l;
+        acc.y *= inv_l;
+        if (out_bf16) *reinterpret_cast<uint32_t*>(static_cast<bf16*>(out_any) + o + c) = pack_bf16(acc.x, acc.y);
+        else *reinterpret_cast<float2*>(static_cast<float*>(out_any) + o + c) = acc;
     }
 }
 
@@ -748,8 +854,8 @@ static int launch_latent_mma(const float* q, const void* cache, void* out, int o
     cpm_launch(kLaunchAttention, kern, grid, 128, smem, stream, q, (const bf16*)cache, out, out_bf16, scratch, positions, token_seq, slots,
                page_table, max_pages, window, n_heads, rank, scale, n_splits);
     if (n_splits > 1)
-        cpm_launch(kLaunchCombine, latent_attention_merge_kernel, dim3(n_tokens, groups, kMmaRows), 128, 0, stream, (const float*)scratch, out,
-                   out_bf16, n_heads, rank, n_splits);
+        cpm_launch(kLaunchCombine, latent_attention_merge_kernel, dim3(n_tokens, groups, kMmaRows), rank > 512 ? 288 : rank > 256 ? 256 : 128, 0, stream,
+                   (const float*)scratch, out, out_bf16, positions, window, n_heads, rank, n_splits);
     return launch_status();
 }
 

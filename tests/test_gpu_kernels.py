@@ -905,3 +905,18 @@ def test_expert_products_by_tiles_and_for_few(E, top, W, ff, n, skew, mode):
     out = ops.moe_combine(got, weights.cuda(), shared.cuda(), weights[:, 0].contiguous().cuda())
     total = (got.view(n, top, W).double() * weights.cuda().double()[..., None]).sum(1) + weights[:, :1].cuda().double() * shared.cuda().double()
     assert _err(out, total) < 2.0 ** -8                            # one rounding to bf16
+
+
+@pytest.mark.parametrize("K,N", [(1, 8), (63, 40), (513, 128), (576, 136), (1151, 24)])
+@pytest.mark.parametrize("n", [1, 2, 3, 8, 9])
+def test_head_project_of_few_tokens(K, N, n):
+    """The per-head maps of a decode step: sums shorter and longer than what is asked for ahead, ragged columns, every number of
+    tokens a block takes, from and to both types; 64-bit products.  fp32 results: sums of K products in another order."""
+    ops = _ops("bfloat16")
+    H = 3
+    g = torch.Generator().manual_seed(K * 31 + N + n)
+    w = (torch.randn(H, K, N, generator=g) * K ** -0.5).bfloat16().cuda()
+    for x in (torch.randn(n, H, K, generator=g).cuda(), torch.randn(n, H, K, generator=g).bfloat16().cuda()):
+        want = torch.einsum("thk,hkn->thn", x.double(), w.double())
+        assert _err(ops.head_project(x, w, H, out_f32=True), want) < 2e-6
+        assert _err(ops.head_project(x, w, H, out_f32=False), want) < 2.0 ** -8
