@@ -342,43 +342,131 @@ __device__ __forceinline__ void put_new_token(unsigned char* stage, const bf16* 
     }
 }
 
+// How a decode step's pages are shared out.  The sequences of a batch differ in length, and a step ends with its slowest block, so
+// they are cut into shares of one size: the smallest ``pages`` a share (from ``least`` on) with which all sequences together
+// need at most ``budget`` shares, each sequence at most kMaxShares.  Every block works that out from the lengths, before it
+// waits for the kernel ahead.  (An equal number of shares a sequence: 64 sequences of 500 to 8000 tokens, 2 kv heads of 64, took 29.9 us
+// a layer, as long as one SM needs for the longest sequence; 8 of 513 to 4085 tokens, 2 kv heads of 128, 8.5 us.)
+constexpr int kMaxShares = 32;
+struct DecodeShare { int seq, index, count, pages; };      // share ``index`` of the ``count`` of sequence ``seq``; seq -1: none
+
+// Where that is not worth its search, a sequence's pages are cut into n_splits shares, less where they do not fill them: at head
+// size 128 with one block an SM and several shares a sequence, the search (about a microsecond where the block cannot start before
+// the kernel ahead ends) ate what it gave (8 sequences of 513 to 4085 tokens: 28.3 ms for eight steps of the 8B sizes against 27.3).
+__host__ __device__ constexpr bool decode_by_size(int d, int n_splits) { return n_splits > 1 && (d == 64 || n_splits <= 2); }
+__device__ __forceinline__ DecodeShare equal_decode_share(const int* __restrict__ kv_len, int seq, int index, int n_splits) {
+    const int pages = max(1, (__ldg(kv_len + seq) + kPageTokens - 1) / kPageTokens), per = (pages + n_splits - 1) / n_splits;
+    DecodeShare s{seq, index, (pages + per - 1) / per, per};
+    if (index >= s.count) s.seq = -1;
+    return s;
+}
+
+__device__ __forceinline__ int pages_of_sequence(const int* __restrict__ kv_len, int b) {
+    return max(1, (__ldg(kv_len + b) + kPageTokens - 1) / kPageTokens);
+}
+
+// Pages a share; a warp's work.
+__device__ __forceinline__ int decode_share_pages(const int* __restrict__ kv_len, int n, int budget, int least, int lane) {
+    auto pages_of = [&](int b) { return pages_of_sequence(kv_len, b); };
+    int total = 0, longest = 0;
+    for (int b = lane; b < n; b += 32) {
+        const int p = pages_of(b);
+        total += p;
+        longest = max(longest, p);
+    }
+    total = __reduce_add_sync(0xffffffffu, total);
+    longest = __reduce_max_sync(0xffffffffu, longest);
+    auto shares = [&](int pages) {
+        int c = 0;
+        for (int b = lane; b < n; b += 32) c += (pages_of(b) + pages - 1) / pages;
+        return __reduce_add_sync(0xffffffffu, c);
+    };
+    int lo = max(least, max((total + budget - 1) / budget, (longest + kMaxShares - 1) / kMaxShares));
+    if (shares(lo) > budget) {                             // (one share a sequence always fits: budget >= n)
+        int hi = budget > n ? min(longest, (total + budget - n - 1) / (budget - n)) : longest;
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (shares(mid) > budget) lo = mid; else hi = mid;
+        }
+        lo = hi;
+    }
+    return lo;
+}
+
+__device__ __forceinline__ DecodeShare find_decode_share(const int* __restrict__ kv_len, int n, int budget, int least, int x, int lane) {
+    const int lo = decode_share_pages(kv_len, n, budget, least, lane);
+    DecodeShare s{-1, 0, 0, lo};
+    int before = 0;
+    for (int b0 = 0; b0 < n; b0 += 32) {
+        const int b = b0 + lane, own = b < n ? (pages_of_sequence(kv_len, b) + lo - 1) / lo : 0;
+        int upto = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += v;
+        }
+        const unsigned past = __ballot_sync(0xffffffffu, x < before + upto);
+        if (past) {
+            const int src = __ffs(past) - 1;
+            s.seq = b0 + src;
+            s.count = __shfl_sync(0xffffffffu, own, src);
+            s.index = x - (before + __shfl_sync(0xffffffffu, upto, src) - s.count);
+            return s;
+        }
+        before += __shfl_sync(0xffffffffu, upto, 31);
+    }
+    return s;
+}
+
+// Warps of a decode block: three fill an SM's shared memory at head size 128; at head size 64 they fill half of it, and two blocks
+// an SM overlap one's start and merge with the other's pages.
+template <int D> struct DecodeBlock {
+    static constexpr int kWarps = D == 64 ? 3 : DecodeSmem<D>::kWarps;
+    static constexpr int kPerSm = D == 64 ? 2 : 1;
+    static constexpr int kSmem = kWarps * kDecodeStages * DecodeSmem<D>::kStageBytes;
+};
+
 template <int D>
-__global__ void __launch_bounds__(DecodeSmem<D>::kWarps * 32, 1)
+__global__ void __launch_bounds__(DecodeBlock<D>::kWarps * 32, DecodeBlock<D>::kPerSm)
 decode_attention_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_cache, const bf16* __restrict__ v_cache,
                         const int* __restrict__ kv_len, const int* __restrict__ slots,
                         const int* __restrict__ page_table, int max_pages, float* __restrict__ part_o,
-                        float* __restrict__ part_ml, bf16* __restrict__ out, int n_heads, int n_kv, int m_tiles,
-                        int n_splits, float scale_log2, DecodeRope rope, int v_shift, int v_runs) {
-    // A block takes one share of a sequence's pages; its warps take every third page of the
-    // share and merge their results in shared memory before anything is written.  With one share
-    // per sequence the block writes the final result to ``out`` itself and no combine kernel follows.
+                        float* __restrict__ part_ml, int* __restrict__ arrivals, bf16* __restrict__ out, int n_seqs, int n_heads,
+                        int n_kv, int m_tiles, int n_splits, float scale_log2, DecodeRope rope, int v_shift, int v_runs) {
+    // A block takes one share of a sequence's pages (n_splits 1: all of them); its warps take every kWarps-th page of the
+    // share and merge their results in shared memory before anything is written.  Where a sequence is one share
+    // the block writes the final result to ``out`` itself; else, with ``arrivals`` (a zeroed counter per sequence and head tile,
+    // left zeroed), the block that finishes last adds up the shares, and without, a kernel behind this one.
+    constexpr int kWarps = DecodeBlock<D>::kWarps;
     using S = DecodeSmem<D>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    __shared__ float sm_m[DecodeSmem<D>::kWarps][16], sm_l[DecodeSmem<D>::kWarps][16];
+    __shared__ float sm_m[kWarps][16], sm_l[kWarps][16];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int split = blockIdx.x;
     // v_runs > 1: the grid's z axis holds v_runs runs over the same sequences, run r with the values shifted by r heads;
     // bv is the row of the output (run-major), b the sequence
-    const int kvh = blockIdx.y / m_tiles, mt = blockIdx.y % m_tiles, bv = blockIdx.z;
-    const int n_real = v_runs > 1 ? (int)gridDim.z / v_runs : (int)gridDim.z;
-    const int b = bv % n_real;
-    if (v_runs > 1) v_shift = bv / n_real;
+    const int kvh = blockIdx.y / m_tiles, mt = blockIdx.y % m_tiles;
+    if (v_runs > 1) v_shift = blockIdx.z;
     const int group = n_heads / n_kv;
     const int j = lane & 3, g = lane >> 2;
     pdl_launch_dependents();
     // Lengths, slots, page numbers and every page but the sequence's last were written by earlier steps (or by the
     // host before this one): they are read, and the first pages asked for, before this kernel waits for the
     // one ahead of it, which writes only the step's own token (into the last page) and q.
+    const DecodeShare share = decode_by_size(D, n_splits) ? find_decode_share(kv_len, n_seqs, n_seqs * n_splits, kWarps, blockIdx.x, lane)
+                                                          : equal_decode_share(kv_len, blockIdx.x / n_splits, blockIdx.x % n_splits, n_splits);
+    const int b = share.seq;
+    if (b < 0) return;
+    const int bv = blockIdx.z * n_seqs + b;
     const int len = kv_len[b];
     const int n_pages = (len + kPageTokens - 1) / kPageTokens;
-    const int per = (n_pages + n_splits - 1) / n_splits;
-    const int p0 = split * per, p1 = min(n_pages, p0 + per);
+    const int per = share.pages;
+    const int p0 = share.index * per, p1 = min(n_pages, p0 + per);
     const int* pages = page_table + (int64_t)slots[b] * max_pages;
     const uint32_t my_stages = (uint32_t)__cvta_generic_to_shared(smem_raw) + warp * kDecodeStages * S::kStageBytes;
     const int64_t page_elems = (int64_t)n_kv * kPageTokens * D;
 
     auto issue = [&](int k) {           // the warp's k-th page into stage k % kDecodeStages
-        const int p = p0 + warp + k * DecodeSmem<D>::kWarps;
+        const int p = p0 + warp + k * kWarps;
         if (p < p1) {
             const int64_t base = (int64_t)CPM_PAGE(pages, p, max_pages) * page_elems + (int64_t)kvh * kPageTokens * D;
             // v_shift: the values come from key-value head (kvh + v_shift) mod n_kv (0: the keys' own head)
@@ -388,10 +476,26 @@ decode_attention_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_c
         cp_async_commit();
     };
     // the warp whose first two pages include the last page waits first (its copies must stay in order)
-    const bool early = rope.early && p0 + warp != n_pages - 1 && p0 + warp + DecodeSmem<D>::kWarps != n_pages - 1;
+    const bool early = rope.early && p0 + warp != n_pages - 1 && p0 + warp + kWarps != n_pages - 1;
     if (early) {
         issue(0);
         issue(1);
+    }
+    // the step's angles need the position alone: they are worked out before the wait too
+    constexpr int kTurned = (D == 64 || D == 128) ? D / 64 : 1;
+    float cs[kTurned][8], sn[kTurned][8];
+    if constexpr (D == 64 || D == 128) {
+        if (rope.qkv && rope.inv_freq) {
+            // this thread's dims 32w + 8j .. + 7 of the first half pair with the same dims of fragment w + D/64
+#pragma unroll
+            for (int w = 0; w < D / 64; ++w)
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    sincosf((float)(len - 1) * rope.inv_freq[32 * w + 8 * j + e], &sn[w][e], &cs[w][e]);
+                    cs[w][e] *= rope.magnitude;
+                    sn[w][e] *= rope.magnitude;
+                }
+        }
     }
     pdl_wait();
     if (!early) {
@@ -413,25 +517,17 @@ decode_attention_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_c
     }
     if constexpr (D == 64 || D == 128) {
         if (rope.qkv && rope.inv_freq) {
-            // this thread's dims 32w + 8j .. + 7 of the first half pair with the same dims of fragment w + D/64
 #pragma unroll
             for (int w = 0; w < D / 64; ++w) {
-                float cs[8], sn[8];
-#pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                    sincosf((float)(len - 1) * rope.inv_freq[32 * w + 8 * j + e], &sn[e], &cs[e]);
-                    cs[e] *= rope.magnitude;
-                    sn[e] *= rope.magnitude;
-                }
-                rotate8(qf[0][w], qf[0][w + D / 64], cs, sn);
-                rotate8(qf[1][w], qf[1][w + D / 64], cs, sn);
+                rotate8(qf[0][w], qf[0][w + D / 64], cs[w], sn[w]);
+                rotate8(qf[1][w], qf[1][w + D / 64], cs[w], sn[w]);
             }
         }
     }
-    for (int k = 0; p0 + warp + k * DecodeSmem<D>::kWarps < p1; ++k) {
+    for (int k = 0; p0 + warp + k * kWarps < p1; ++k) {
         cp_async_wait<kDecodeStages - 1>();
         __syncwarp();
-        const int p = p0 + warp + k * DecodeSmem<D>::kWarps;
+        const int p = p0 + warp + k * kWarps;
         if constexpr (D == 64 || D == 128) {
             if (rope.qkv && rope.write_cache && p == n_pages - 1) {
                 // the step's own token is not in the cache yet: this warp holds its page and puts it there
@@ -469,22 +565,22 @@ decode_attention_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_c
         sm_l[warp][g + 8] = st.l[1];
     }
     __syncthreads();
-    const int64_t unit = (((int64_t)bv * n_kv + kvh) * m_tiles + mt) * n_splits + split;
+    const int64_t unit = ((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
     float* po = part_o + unit * 16 * D;
-    for (int i = threadIdx.x; i < 16 * D; i += DecodeSmem<D>::kWarps * 32) {
+    for (int i = threadIdx.x; i < 16 * D; i += kWarps * 32) {
         const int row = i / D, c = i - row * D;
         float mx = -INFINITY;
 #pragma unroll
-        for (int w = 0; w < DecodeSmem<D>::kWarps; ++w) mx = fmaxf(mx, sm_m[w][row]);
+        for (int w = 0; w < kWarps; ++w) mx = fmaxf(mx, sm_m[w][row]);
         const float use = mx == -INFINITY ? 0.f : mx;
         float o = 0.f, l = 0.f;
 #pragma unroll
-        for (int w = 0; w < DecodeSmem<D>::kWarps; ++w) {
+        for (int w = 0; w < kWarps; ++w) {
             const float f = exp2f(sm_m[w][row] - use);
             o += sm_o[(w * 16 + row) * kLd + c] * f;
             l += sm_l[w][row] * f;
         }
-        if (n_splits == 1) {
+        if (share.count == 1) {
             const int local = mt * 16 + row;
             if (local < group)
                 out[((int64_t)bv * n_heads + kvh * group + local) * D + c] = __float2bfloat16_rn(l > 0.f ? o / l : 0.f);
@@ -496,35 +592,136 @@ decode_attention_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_c
             part_ml[unit * 32 + 2 * row + 1] = l;
         }
     }
+    if (share.count == 1 || arrivals == nullptr) return;
+    // ---- the last of a sequence's blocks adds up the shares ----
+    __threadfence();
+    __syncthreads();
+    int* last = reinterpret_cast<int*>(sm_l);                          // (its sums have been used)
+    if (threadIdx.x == 0) {
+        int* counter = arrivals + ((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * n_seqs + b;
+        const bool mine = atomicAdd(counter, 1) == share.count - 1;
+        if (mine) *counter = 0;
+        *last = mine;
+    }
+    __syncthreads();
+    if (!*last) return;
+    __threadfence();
+    float* weight = reinterpret_cast<float*>(smem_raw);                // [count][16]: a share's part in a row's result
+    float* ml = weight + kMaxShares * 16;                              // [count][32]
+    const int64_t first = unit - share.index;
+    const int rows = min(16, group - mt * 16);
+    for (int i = threadIdx.x; i < share.count * 32; i += kWarps * 32) ml[i] = __ldcg(part_ml + first * 32 + i);
+    __syncthreads();
+    for (int i = threadIdx.x; i < share.count * 16; i += kWarps * 32) {
+        const int row = i & 15, s = i >> 4;
+        float mx = -INFINITY, l = 0.f;
+        for (int k = 0; k < share.count; ++k) mx = fmaxf(mx, ml[k * 32 + 2 * row]);
+        const float use = mx == -INFINITY ? 0.f : mx;
+        for (int k = 0; k < share.count; ++k) l = fmaf(ml[k * 32 + 2 * row + 1], exp2f(ml[k * 32 + 2 * row] - use), l);
+        weight[i] = l > 0.f ? exp2f(ml[s * 32 + 2 * row] - use) / l : 0.f;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < rows * (D / 4); i += kWarps * 32) {
+        const int row = i / (D / 4), c = (i % (D / 4)) * 4;
+        const float* src = part_o + (first * 16 + row) * D + c;
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int s0 = 0; s0 < share.count; s0 += 8) {                  // eight shares in flight
+            float4 o[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                o[u] = s0 + u < share.count ? __ldcg(reinterpret_cast<const float4*>(src + (s0 + u) * 16 * D)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const float w = s0 + u < share.count ? weight[(s0 + u) * 16 + row] : 0.f;
+                acc.x = fmaf(o[u].x, w, acc.x);
+                acc.y = fmaf(o[u].y, w, acc.y);
+                acc.z = fmaf(o[u].z, w, acc.z);
+                acc.w = fmaf(o[u].w, w, acc.w);
+            }
+        }
+        store4(out + ((int64_t)bv * n_heads + kvh * group + mt * 16 + row) * D + c, acc);
+    }
 }
 
-// out[b, h, :] = sum_s o_s * 2^(m_s - M) / sum_s l_s * 2^(m_s - M)
-__global__ void combine_splits_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
-                                      bf16* __restrict__ out, int n_heads, int n_kv, int m_tiles, int n_splits,
-                                      int D) {
-    pdl_launch_dependents();
+// out[b, h, :] = sum_s o_s * 2^(m_s - M) / sum_s l_s * 2^(m_s - M), one warp a row and head.  kv_len: the sequences were cut as the decode
+// kernel does it (those of one share are written already); null: n_splits shares each.  Rows are runs x n_seqs.  Bound by the
+// latency of its loads: the statistics and the first eight shares' sums are on their way together.
+template <int D>
+__global__ void __launch_bounds__(128)
+combine_shares_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml, const int* __restrict__ kv_len,
+                      bf16* __restrict__ out, int n_seqs, int n_heads, int n_kv, int m_tiles, int n_splits) {
+    constexpr int kCols = D / 4, kRowsAtOnce = 32 / kCols;         // a lane holds four columns; small heads: several shares at a time
     pdl_wait();
-    const int h = blockIdx.x, b = blockIdx.y;
-    const int group = n_heads / n_kv;
-    const int kvh = h / group, local = h % group;
-    const int mt = local / 16, row = local % 16;
-    const int64_t unit0 = (((int64_t)b * n_kv + kvh) * m_tiles + mt) * n_splits;
-    float mx = -INFINITY;
-    for (int s = 0; s < n_splits; ++s) mx = fmaxf(mx, part_ml[(unit0 + s) * 32 + 2 * row]);
-    float denom = 0.f;
-    for (int s = 0; s < n_splits; ++s) {
-        const float m = part_ml[(unit0 + s) * 32 + 2 * row];
-        if (m != -INFINITY) denom += part_ml[(unit0 + s) * 32 + 2 * row + 1] * exp2f(m - mx);
-    }
-    const float inv = denom > 0.f ? 1.f / denom : 0.f;
-    for (int c = threadIdx.x; c < D; c += blockDim.x) {
-        float acc = 0.f;
-        for (int s = 0; s < n_splits; ++s) {
-            const float m = part_ml[(unit0 + s) * 32 + 2 * row];
-            if (m != -INFINITY) acc += part_o[((unit0 + s) * 16 + row) * D + c] * exp2f(m - mx);
+    const int h = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31, row = blockIdx.y;
+    if (h >= n_heads) return;
+    const int group = n_heads / n_kv, kvh = h / group, local = h % group;
+    const int unit = kvh * m_tiles + local / 16, units = n_kv * m_tiles, r = local % 16;
+    const int b = row % n_seqs;
+    int count = n_splits;
+    int64_t first = ((int64_t)row * units + unit) * n_splits;
+    if (kv_len != nullptr) {
+        int before = b * n_splits;
+        if (decode_by_size(D, n_splits)) {
+            const int pages = decode_share_pages(kv_len, n_seqs, n_seqs * n_splits, DecodeBlock<D>::kWarps, lane);
+            count = (pages_of_sequence(kv_len, b) + pages - 1) / pages;
+            before = 0;
+            for (int i = lane; i < b; i += 32) before += (pages_of_sequence(kv_len, i) + pages - 1) / pages;
+            before = __reduce_add_sync(0xffffffffu, before);
+        } else {
+            count = equal_decode_share(kv_len, b, 0, n_splits).count;
         }
-        out[((int64_t)b * n_heads + h) * D + c] = __float2bfloat16_rn(acc * inv);
+        if (count == 1) return;
+        first = ((int64_t)(row / n_seqs) * units + unit) * n_seqs * n_splits + before;
     }
+    const float* ml = part_ml + first * 32 + 2 * r;
+    const int c = (lane % kCols) * 4, sub = lane / kCols;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    float denom = 0.f, mx = -INFINITY;
+    for (int s0 = 0; s0 < count; s0 += 32) {
+        const int here = min(32, count - s0);
+        const float2 v = lane < here ? *reinterpret_cast<const float2*>(ml + (s0 + lane) * 32) : make_float2(-INFINITY, 0.f);
+        const float* src = part_o + ((first + s0) * 16 + r) * D + c;
+        float w = 0.f;
+        for (int s = 0; s < here; s += 8 * kRowsAtOnce) {
+            float4 o[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const int at = s + u * kRowsAtOnce + sub;
+                o[u] = sub < kRowsAtOnce && at < here ? *reinterpret_cast<const float4*>(src + (int64_t)at * 16 * D) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+            if (s == 0) {                                              // these 32 shares' maximum joins the ones before
+                const float m = fmaxf(mx, warp_max(v.x)), use = m == -INFINITY ? 0.f : m, old = exp2f(mx - use);
+                acc.x *= old;
+                acc.y *= old;
+                acc.z *= old;
+                acc.w *= old;
+                w = exp2f(v.x - use);
+                denom = denom * old + v.y * w;
+                mx = m;
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const int at = s + u * kRowsAtOnce + sub;
+                const float ws = __shfl_sync(0xffffffffu, w, min(at, 31));
+                if (at < here && ws != 0.f) {
+                    acc.x = fmaf(o[u].x, ws, acc.x);
+                    acc.y = fmaf(o[u].y, ws, acc.y);
+                    acc.z = fmaf(o[u].z, ws, acc.z);
+                    acc.w = fmaf(o[u].w, ws, acc.w);
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int o = kCols; o < 32 && kRowsAtOnce > 1; o <<= 1) {
+        acc.x += __shfl_xor_sync(0xffffffffu, acc.x, o);
+        acc.y += __shfl_xor_sync(0xffffffffu, acc.y, o);
+        acc.z += __shfl_xor_sync(0xffffffffu, acc.z, o);
+        acc.w += __shfl_xor_sync(0xffffffffu, acc.w, o);
+    }
+    denom = warp_sum(denom);
+    const float inv = denom > 0.f ? 1.f / denom : 0.f;
+    if (sub == 0) store4(out + ((int64_t)row * n_heads + h) * D + c, make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv));
 }
 
 // Floats of scratch the decode kernels need for these sizes.
@@ -533,44 +730,49 @@ CPM_API int64_t cpm_decode_attention_scratch_floats(int n_seqs, int n_heads, int
     return (int64_t)n_seqs * n_kv * m_tiles * n_splits * (16 * d + 32);
 }
 
+// Blocks of the decode kernel an SM holds.
+CPM_API int cpm_decode_attention_blocks_per_sm(int d) { return d == 64 ? DecodeBlock<64>::kPerSm : 1; }
+
 template <int D>
 static int launch_decode(const void* q, const void* k_cache, const void* v_cache, void* out, const int* kv_len,
                          const int* slots, const int* page_table, int max_pages, float* scratch, int n_seqs,
-                         int n_heads, int n_kv, int n_splits, float scale, cudaStream_t stream,
+                         int n_heads, int n_kv, int n_splits, float scale, int* arrivals, cudaStream_t stream,
                          DecodeRope rope = DecodeRope{nullptr, nullptr, 1.f, 0, nullptr, nullptr, 0}, int v_shift = 0,
                          int v_runs = 1) {
     const int m_tiles = (n_heads / n_kv + 15) / 16;
-    const int n_rows = n_seqs * (v_runs > 1 ? v_runs : 1);       // rows of the output: sequences, or runs x sequences
-    if (n_rows > 65535) return CPM_BAD_ARGUMENT;
+    const int runs = v_runs > 1 ? v_runs : 1, n_rows = n_seqs * runs;       // rows of the output: runs x sequences
+    if (n_rows > 65535 || n_kv * m_tiles > 65535) return CPM_BAD_ARGUMENT;
+    const int64_t shares = (int64_t)n_seqs * n_splits;
+    if (shares > 0x7fffffff) return CPM_BAD_ARGUMENT;
     float* part_o = scratch;
-    float* part_ml = scratch + (int64_t)n_rows * n_kv * m_tiles * n_splits * 16 * D;
-    dim3 grid(n_splits, n_kv * m_tiles, n_rows);
+    float* part_ml = scratch + shares * runs * n_kv * m_tiles * 16 * D;
     auto kern = decode_attention_kernel<D>;
     rope.early = g_decode_early;
-    constexpr int smem = DecodeSmem<D>::kTotal;
+    constexpr int smem = DecodeBlock<D>::kSmem;
     static bool configured[kMaxDevices] = {};            // per kernel and per device
     if (int st = ensure_dynamic_smem(kern, smem, configured)) return st;
-    cpm_launch(kLaunchAttention, kern, grid, DecodeSmem<D>::kWarps * 32, smem, stream, (const bf16*)q, (const bf16*)k_cache, (const bf16*)v_cache,
-               kv_len, slots, page_table, max_pages, part_o, part_ml, (bf16*)out, n_heads, n_kv, m_tiles, n_splits,
-               scale * 1.4426950408889634f, rope, v_shift, v_runs);
-    if (n_splits > 1)
-        cpm_launch(kLaunchCombine, combine_splits_kernel, dim3(n_heads, n_rows), D >= 128 ? 128 : 64, 0, stream, (const float*)part_o,
-                   (const float*)part_ml, (bf16*)out, n_heads, n_kv, m_tiles, n_splits, (int)D);
+    cpm_launch(kLaunchAttention, kern, dim3((unsigned)shares, n_kv * m_tiles, runs), DecodeBlock<D>::kWarps * 32, smem, stream, (const bf16*)q,
+               (const bf16*)k_cache, (const bf16*)v_cache, kv_len, slots, page_table, max_pages, part_o, part_ml, arrivals, (bf16*)out,
+               n_seqs, n_heads, n_kv, m_tiles, n_splits, scale * 1.4426950408889634f, rope, v_shift, runs);
+    if (n_splits > 1 && arrivals == nullptr)
+        cpm_launch(kLaunchCombine, combine_shares_kernel<D>, dim3((n_heads + 3) / 4, n_rows), 128, 0, stream, (const float*)part_o,
+                   (const float*)part_ml, kv_len, (bf16*)out, n_seqs, n_heads, n_kv, m_tiles, n_splits);
     return launch_status();
 }
 
-// q [n_seqs, heads, d] bf16, one token per sequence; out [n_seqs, heads, d] bf16.
+// q [n_seqs, heads, d] bf16, one token per sequence; out [n_seqs, heads, d] bf16.  arrivals: null, or n_seqs * n_kv * ceil(group / 16) (times
+// the runs) counters that are zero, are zero again when the kernel ends, and belong to no other kernel meanwhile.
 CPM_API int cpm_decode_attention_bf16(const void* q, const void* k_cache, const void* v_cache, void* out,
                                       const int* kv_len, const int* slots, const int* page_table, int max_pages,
                                       float* scratch, int n_seqs, int n_heads, int n_kv, int d, int n_splits,
-                                      float scale, cudaStream_t stream) {
+                                      float scale, int* arrivals, cudaStream_t stream) {
     if (n_seqs <= 0) return CPM_OK;
     if (n_kv <= 0 || n_heads % n_kv || n_splits < 1 || n_seqs > 65535 || !scratch) return CPM_BAD_ARGUMENT;
     switch (d) {
-        case 32: return launch_decode<32>(q, k_cache, v_cache, out, kv_len, slots, page_table, max_pages, scratch, n_seqs, n_heads, n_kv, n_splits, scale, stream);
-        case 64: return launch_decode<64>(q, k_cache, v_cache, out, kv_len, slots, page_table, max_pages, scratch, n_seqs, n_heads, n_kv, n_splits, scale, stream);
-        case 96: return launch_decode<96>(q, k_cache, v_cache, out, kv_len, slots, page_table, max_pages, scratch, n_seqs, n_heads, n_kv, n_splits, scale, stream);
-        case 128: return launch_decode<128>(q, k_cache, v_cache, out, kv_len, slots, page_table, max_pages, scratch, n_seqs, n_heads, n_kv, n_splits, scale, stream);
+        case 32: return launch_decode<32>(q, k_cache, v_cache, out, kv_len, slots, page_table, max_pages, scratch, n_seqs, n_heads, n_kv, n_splits, scale, arrivals, stream);
+        case 64: return launch_decode<64>(q, k_cache, v_cache, out, kv_len, slots, page_table, max_pages, scratch, n_seqs, n_heads, n_kv, n_splits, scale, arrivals, stream);
+        case 96: return launch_decode<96>(q, k_cache, v_cache, out, kv_len, slots, page_table, max_pages, scratch, n_seqs, n_heads, n_kv, n_splits, scale, arrivals, stream);
+        case 128: return launch_decode<128>(q, k_cache, v_cache, out, kv_len, slots, page_table, max_pages, scratch, n_seqs, n_heads, n_kv, n_splits, scale, arrivals, stream);
         default: return CPM_BAD_ARGUMENT;
     }
 }
@@ -580,7 +782,7 @@ CPM_API int cpm_decode_attention_bf16(const void* q, const void* k_cache, const 
 CPM_API int cpm_decode_attention_bf16_vshift(const void* q, const void* k_cache, const void* v_cache, void* out,
                                              const int* kv_len, const int* slots, const int* page_table, int max_pages,
                                              float* scratch, int n_seqs, int n_heads, int n_kv, int d, int n_splits,
-                                             float scale, int v_shift, int v_runs, cudaStream_t stream) {
+                                             float scale, int v_shift, int v_runs, int* arrivals, cudaStream_t stream) {
     // v_runs > 1: one launch does runs 0 .. v_runs - 1 (v_shift is then not used); out is [v_runs, n_seqs, heads, d] and
     // scratch holds cpm_decode_attention_scratch_floats(v_runs * n_seqs, ...) floats
     if (n_seqs <= 0) return CPM_OK;
@@ -589,10 +791,10 @@ CPM_API int cpm_decode_attention_bf16_vshift(const void* q, const void* k_cache,
         return CPM_BAD_ARGUMENT;
     const DecodeRope none{nullptr, nullptr, 1.f, 0, nullptr, nullptr, 0};
     switch (d) {
-        case 32: return launch_decode<32>(q, k_cache, v_cache, out, kv_len, slots, page_table, max_pages, scratch, n_seqs, n_heads, n_kv, n_splits, scale, stream, none, v_shift, v_runs);
-        case 64: return launch_decode<64>(q, k_cache, v_cache, out, kv_len, slots, page_table, max_pages, scratch, n_seqs, n_heads, n_kv, n_splits, scale, stream, none, v_shift, v_runs);
-        case 96: return launch_decode<96>(q, k_cache, v_cache, out, kv_len, slots, page_table, max_pages, scratch, n_seqs, n_heads, n_kv, n_splits, scale, stream, none, v_shift, v_runs);
-        case 128: return launch_decode<128>(q, k_cache, v_cache, out, kv_len, slots, page_table, max_pages, scratch, n_seqs, n_heads, n_kv, n_splits, scale, stream, none, v_shift, v_runs);
+        case 32: return launch_decode<32>(q, k_cache, v_cache, out, kv_len, slots, page_table, max_pages, scratch, n_seqs, n_heads, n_kv, n_splits, scale, arrivals, stream, none, v_shift, v_runs);
+        case 64: return launch_decode<64>(q, k_cache, v_cache, out, kv_len, slots, page_table, max_pages, scratch, n_seqs, n_heads, n_kv, n_splits, scale, arrivals, stream, none, v_shift, v_runs);
+        case 96: return launch_decode<96>(q, k_cache, v_cache, out, kv_len, slots, page_table, max_pages, scratch, n_seqs, n_heads, n_kv, n_splits, scale, arrivals, stream, none, v_shift, v_runs);
+        case 128: return launch_decode<128>(q, k_cache, v_cache, out, kv_len, slots, page_table, max_pages, scratch, n_seqs, n_heads, n_kv, n_splits, scale, arrivals, stream, none, v_shift, v_runs);
         default: return CPM_BAD_ARGUMENT;
     }
 }
@@ -604,13 +806,13 @@ CPM_API int cpm_decode_attention_rope_bf16(const void* qkv, void* k_cache, void*
                                            const int* kv_len, const int* slots, const int* page_table, int max_pages,
                                            float* scratch, int n_seqs, int n_heads, int n_kv, int d, int n_splits,
                                            float scale, const float* inv_freq, float magnitude, int write_cache,
-                                           cudaStream_t stream) {
+                                           int* arrivals, cudaStream_t stream) {
     if (n_seqs <= 0) return CPM_OK;
     if (n_kv <= 0 || n_heads % n_kv || n_splits < 1 || n_seqs > 65535 || !scratch || !qkv) return CPM_BAD_ARGUMENT;
     const DecodeRope rope{(const bf16*)qkv, inv_freq, magnitude, write_cache, (bf16*)k_cache, (bf16*)v_cache, 0};
     switch (d) {
-        case 64: return launch_decode<64>(nullptr, k_cache, v_cache, out, kv_len, slots, page_table, max_pages, scratch, n_seqs, n_heads, n_kv, n_splits, scale, stream, rope);
-        case 128: return launch_decode<128>(nullptr, k_cache, v_cache, out, kv_len, slots, page_table, max_pages, scratch, n_seqs, n_heads, n_kv, n_splits, scale, stream, rope);
+        case 64: return launch_decode<64>(nullptr, k_cache, v_cache, out, kv_len, slots, page_table, max_pages, scratch, n_seqs, n_heads, n_kv, n_splits, scale, arrivals, stream, rope);
+        case 128: return launch_decode<128>(nullptr, k_cache, v_cache, out, kv_len, slots, page_table, max_pages, scratch, n_seqs, n_heads, n_kv, n_splits, scale, arrivals, stream, rope);
         default: return CPM_BAD_ARGUMENT;
     }
 }
@@ -971,8 +1173,8 @@ static int launch_listed(const void* q, const void* k_cache, const void* v_cache
                (const bf16*)k_cache, (const bf16*)v_cache, (bf16*)out, positions, token_seq, slots, page_table, max_pages,
                block_list, list_cap, n_heads, n_kv, m_tiles, scale * 1.4426950408889634f, part_o, part_ml, n_splits);
     if (n_splits > 1)
-        combine_splits_kernel<<<dim3(n_heads, n_tokens), D >= 128 ? 128 : 64, 0, stream>>>(part_o, part_ml, (bf16*)out, n_heads,
-                                                                                    n_kv, m_tiles, n_splits, D);
+        combine_shares_kernel<D><<<dim3((n_heads + 3) / 4, n_tokens), 128, 0, stream>>>(part_o, part_ml, nullptr, (bf16*)out, n_tokens,
+                                                                                        n_heads, n_kv, m_tiles, n_splits);
     return launch_status();
 }
 
@@ -1197,7 +1399,7 @@ int cpm_decode_attention_bf16_static(const void* q, const void* k_cache, const v
     const int status = static_scratch_for_current_device(&scratch, error_text, error_text_len);
     if (status != CPM_OK) return status;
     return cpm_decode_attention_bf16(q, k_cache, v_cache, out, kv_len, slots, page_table, max_pages, scratch, n_seqs,
-                                     n_heads, n_kv, d, n_splits, scale, stream);
+                                     n_heads, n_kv, d, n_splits, scale, nullptr, stream);
 }
 
 CPM_BOUNDS_TU(attention_bf16)

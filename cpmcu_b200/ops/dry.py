@@ -27,6 +27,10 @@ class _NoLibrary:
         return n_seqs * n_kv * ((n_heads // n_kv + 15) // 16) * n_splits * (16 * d + 32)
 
     @staticmethod
+    def cpm_decode_attention_blocks_per_sm(d):
+        return 2 if d == 64 else 1
+
+    @staticmethod
     def cpm_select_blocks_scratch_floats(n_tokens, n_kv, max_entries, n_slices):
         return n_tokens * n_kv * (max_entries * 16 + n_slices * 32)
 
@@ -68,6 +72,7 @@ class DryOps(Ops):
         self.lib = _NoLibrary()
         self.element_size = 4 if dtype == torch.float32 else 2
         self.sm_count = sm_count
+        self.arrivals = None
         self.use_tcgen05 = self.use_tcgen05_attention = self.use_tcgen05_listed = self.use_tcgen05_sink = True
         self.tcgen05_pair = False
         arena = Arena(None, None)

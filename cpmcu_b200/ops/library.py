@@ -37,9 +37,9 @@ _SIGNATURES = {
     "cpm_select_blocks": [_P, _P, _P, _P, _P, _P, c_int, _P, c_int, c_int, c_int, c_int, c_int, c_float, c_int,
                           c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P, c_int, _P],
     "cpm_advance_decode": [_P, _P, _P, _P, _P, _P, c_int, _P],
-    "cpm_decode_attention_bf16": [_P, _P, _P, _P, _P, _P, _P, c_int, _P, c_int, c_int, c_int, c_int, c_int, c_float, _P],
+    "cpm_decode_attention_bf16": [_P, _P, _P, _P, _P, _P, _P, c_int, _P, c_int, c_int, c_int, c_int, c_int, c_float, _P, _P],
     "cpm_decode_attention_rope_bf16": [_P, _P, _P, _P, _P, _P, _P, c_int, _P, c_int, c_int, c_int, c_int, c_int, c_float,
-                                       _P, c_float, c_int, _P],
+                                       _P, c_float, c_int, _P, _P],
     "cpm_prefill_attention_bf16": [_P, _P, _P, _P, _P, _P, c_int, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_float,
                                    _P],
     "cpm_listed_attention_bf16": [_P, _P, _P, _P, _P, _P, _P, _P, c_int, _P, c_int, c_int, c_int, c_int, c_int, c_float, _P,
@@ -104,7 +104,7 @@ _SIGNATURES = {
     "cpm_scale_heads_bf16": [_P, _P, _P, c_int, c_int, c_int, _P],
     "cpm_talk_mix_bf16": [_P, _P, _P, c_int, c_int, c_int, c_int, _P],
     "cpm_decode_attention_bf16_vshift": [_P, _P, _P, _P, _P, _P, _P, c_int, _P, c_int, c_int, c_int, c_int, c_int, c_float, c_int,
-                                         c_int, _P],
+                                         c_int, _P, _P],
     "cpm_prefill_attention_bf16_vshift": [_P, _P, _P, _P, _P, _P, c_int, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_float,
                                           c_int, _P],
     "cpm_prefill_attention_tcgen05_vshift": [_P, _P, _P, _P, _P, _P, c_int, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int,
@@ -184,6 +184,8 @@ def load() -> ctypes.CDLL:
         lib.cpm_listed_tile_error.restype = c_int
         lib.cpm_listed_attention_tcgen05_max_pages.argtypes = []
         lib.cpm_listed_attention_tcgen05_max_pages.restype = c_int
+        lib.cpm_decode_attention_blocks_per_sm.argtypes = [c_int]
+        lib.cpm_decode_attention_blocks_per_sm.restype = c_int
         lib.cpm_decode_attention_scratch_floats.argtypes = [c_int, c_int, c_int, c_int, c_int]
         lib.cpm_decode_attention_scratch_floats.restype = c_int64
         lib.cpm_latent_attention_scratch_floats.argtypes = [c_int, c_int, c_int, c_int]

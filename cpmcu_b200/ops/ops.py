@@ -66,6 +66,8 @@ class Ops:
         self.tcgen05_pair = os.environ.get("CPMCU_TCGEN05_PAIR", "0") == "1"      # pairs of blocks on 256-row tiles
         self.workspace = None       # cpmcu_b200.memory.Workspace: where a step's intermediates live (None: torch's allocator)
         self.weights = None         # cpmcu_b200.memory.Region that holds the weights (None: torch's allocator)
+        # counters of the decode attention's blocks (see _arrivals): zero between launches
+        self.arrivals = torch.zeros(16384, dtype=torch.int32, device=self.device)
 
     _stream = staticmethod(_current_stream)
 
@@ -785,12 +787,27 @@ class Ops:
                                           _ptr(live), ids.numel(), self._stream()), "advance_decode")
 
     # ---- bf16 tensor-core attention ----
-    def decode_splits(self, n_seqs: int, n_heads: int, n_kv: int) -> int:
-        """How many shares a sequence's pages are cut into: the decode attention kernel holds one
-        block per SM (its page buffers fill the shared memory), so aim at one wave of blocks."""
+    def decode_splits(self, n_seqs: int, n_heads: int, n_kv: int, d: int = 0) -> int:
+        """How many shares a sequence's pages are cut into, on average (the decode attention gives long sequences more): the
+        kernel holds one block per SM (its page buffers fill the shared memory; with ``d`` the number the decode kernel
+        holds at that head size), so aim at one wave of blocks, but where one wave is about one share a sequence at
+        two, so that there are shares to give to the long ones."""
         m_tiles = (n_heads // n_kv + 15) // 16
         units = max(1, n_seqs * n_kv * m_tiles)
-        return max(1, min(self.MAX_DECODE_SPLITS, self.sm_count // units))
+        room = self.sm_count * (self.lib.cpm_decode_attention_blocks_per_sm(d) if d else 1)
+        wave = max(1, min(self.MAX_DECODE_SPLITS, room // units))
+        return min(2, 2 * room // units) if d and wave == 1 and 2 * room >= 2 * units else wave
+
+    def _arrivals(self, rows: int, n_heads: int, n_kv: int, d: int) -> Optional[torch.Tensor]:
+        """Counters with which the decode attention's blocks find out which of them is the last of its sequence and adds up
+        the shares, so that no kernel for that has to follow (it cost 3.4 us a layer at one sequence, 4.5 us at eight).
+        Launches that share them must follow one another: they are given only where a workspace is attached, whose memory
+        asks for the same; elsewhere, or with more rows than there are counters, the shares are added up by a kernel of its own.
+        So they are at head sizes above 64, where a block's three warps take longer for 16 rows of the shares than that kernel
+        (8 sequences of the 8B sizes: 29.3 against 28.3 ms for eight steps)."""
+        if d > 64 or self.workspace is None or self.arrivals is None or rows * n_kv * ((n_heads // n_kv + 15) // 16) > self.arrivals.numel():
+            return None
+        return self.arrivals
 
     def decode_attention(self, q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, kv_len: torch.Tensor,
                          slots: torch.Tensor, page_table: torch.Tensor, n_kv: int, scale: float,
@@ -803,23 +820,24 @@ class Ops:
         n, n_heads, d = q.shape
         rows = n * max(1, int(v_runs))
         if n_splits is None:
-            n_splits = self.decode_splits(rows, n_heads, n_kv)
+            n_splits = self.decode_splits(rows, n_heads, n_kv, d)
         floats = self.lib.cpm_decode_attention_scratch_floats(rows, n_heads, n_kv, d, n_splits)
         scratch = self.empty(floats, dtype=torch.float32)
+        arrivals = self._arrivals(rows, n_heads, n_kv, d)
         if out is None:
             out = self.empty(rows, n_heads * d) if v_runs <= 1 else self.empty(v_runs, n, n_heads * d)
         if v_shift or v_runs > 1:
             check(self.lib.cpm_decode_attention_bf16_vshift(_ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(out), _ptr(kv_len),
                                                             _ptr(slots), _ptr(page_table), page_table.shape[1], _ptr(scratch),
                                                             n, n_heads, n_kv, d, n_splits, float(scale), int(v_shift),
-                                                            max(1, int(v_runs)), self._stream()),
+                                                            max(1, int(v_runs)), _ptr(arrivals), self._stream()),
                   f"decode attention (head_dim {d}, values shifted)")
         else:
             check(self.lib.cpm_decode_attention_bf16(_ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(out), _ptr(kv_len),
                                                      _ptr(slots), _ptr(page_table), page_table.shape[1], _ptr(scratch),
-                                                     n, n_heads, n_kv, d, n_splits, float(scale), self._stream()),
+                                                     n, n_heads, n_kv, d, n_splits, float(scale), _ptr(arrivals), self._stream()),
                   f"decode attention (head_dim {d})")
-        if n_splits > 1:
+        if n_splits > 1 and arrivals is None:
             LAUNCHES_EXTRA[0] += 1       # the launcher starts two kernels: the shares, then their combination
         return out
 
@@ -851,16 +869,17 @@ class Ops:
             if inv_freq.numel() != d // 2:
                 raise ValueError("inv_freq needs head_dim/2 entries")
         if n_splits is None:
-            n_splits = self.decode_splits(n, n_heads, n_kv)
+            n_splits = self.decode_splits(n, n_heads, n_kv, d)
         floats = self.lib.cpm_decode_attention_scratch_floats(n, n_heads, n_kv, d, n_splits)
         scratch = self.empty(floats, dtype=torch.float32)
         out = self.empty(n, n_heads * d)
+        arrivals = self._arrivals(n, n_heads, n_kv, d)
         check(self.lib.cpm_decode_attention_rope_bf16(_ptr(qkv), _ptr(lane.k), _ptr(lane.v), _ptr(out), _ptr(kv_len),
                                                       _ptr(slots), _ptr(lane.page_table), lane.page_table.shape[1],
                                                       _ptr(scratch), n, n_heads, n_kv, d, n_splits, float(scale),
                                                       _ptr(inv_freq), float(magnitude), 1 if write_cache else 0,
-                                                      self._stream()), f"decode attention with rotation (head_dim {d})")
-        if n_splits > 1:
+                                                      _ptr(arrivals), self._stream()), f"decode attention with rotation (head_dim {d})")
+        if n_splits > 1 and arrivals is None:
             LAUNCHES_EXTRA[0] += 1
         return out
 

@@ -920,3 +920,41 @@ def test_head_project_of_few_tokens(K, N, n):
         want = torch.einsum("thk,hkn->thn", x.double(), w.double())
         assert _err(ops.head_project(x, w, H, out_f32=True), want) < 2e-6
         assert _err(ops.head_project(x, w, H, out_f32=False), want) < 2.0 ** -8
+
+
+@pytest.mark.parametrize("n_heads,n_kv,d", [(16, 2, 64), (4, 2, 128), (40, 2, 32), (3, 3, 96)])
+@pytest.mark.parametrize("lens", [[1], [3000], [64, 65, 1, 2111, 700, 129], [1 + 17 * i % 900 for i in range(150)], [2500] + [5] * 33])
+def test_decode_attention_shares_of_ragged_batches(n_heads, n_kv, d, lens):
+    """Sequences cut into shares of one size, added up by the last block and by a kernel of its own, against one share a sequence
+    and against fp32 torch on the longest: one sequence, more sequences than a warp, lengths at the edges of a page."""
+    from cpmcu_b200.cache import Cache
+    from cpmcu_b200.parts.base import CacheNeeds
+
+    ops = _ops("bfloat16")
+    n, g = len(lens), torch.Generator().manual_seed(sum(lens))
+    c = Cache([CacheNeeds(kv_heads=n_kv, head_dim=d)], max_tokens=sum(64 * ((m + 63) // 64) for m in lens), dtype=torch.bfloat16,
+              device="cuda:0", n_slots=n)
+    slots = c.open_sequences(n)
+    for s, m in zip(slots, lens):
+        c.reserve(s, m)
+    c.sync()
+    lane = c.lane(0)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32).cuda()
+    rows = torch.randn(sum(lens), (n_heads + 2 * n_kv) * d, generator=g).bfloat16()
+    ops.rope_store(rows.cuda(), n_heads, n_kv, d, torch.cat([torch.arange(m) for m in lens]).int().cuda(),
+                   torch.cat([torch.full((m,), i) for i, m in enumerate(lens)]).int().cuda(), i32(slots), lane.page_table, lane.k, lane.v,
+                   None, 1.0, 0)
+    q = torch.randn(n, n_heads, d, generator=g).bfloat16().cuda()
+    run = lambda splits: ops.decode_attention(q, lane.k, lane.v, i32(lens), i32(slots), lane.page_table, n_kv, d ** -0.5, n_splits=splits)
+    want = run(1)
+    i = max(range(n), key=lambda j: lens[j])
+    own = rows[sum(lens[:i]):sum(lens[:i + 1])].float().view(lens[i], -1, d)
+    ref = plain.dense_attention(torch.cat([torch.zeros(lens[i] - 1, n_heads, d), q[i:i + 1].float().cpu()]), own[:, n_heads:n_heads + n_kv],
+                                own[:, n_heads + n_kv:], d ** -0.5)[-1].reshape(-1)
+    for splits in (None, 2, 5):
+        assert _err(run(splits), want) < KTOL["bfloat16"]
+    ops._arrivals = lambda *a: ops.arrivals
+    for splits in (None, 2, 5, None):
+        got = run(splits)
+        assert _err(got, want) < KTOL["bfloat16"] and _err(got[i], ref) < KTOL["bfloat16"]
+        assert not ops.arrivals.any()
