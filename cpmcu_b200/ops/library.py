@@ -81,7 +81,7 @@ _SIGNATURES = {
     "cpm_hyper_step": [_P, _P, _P, _P, _P, _P, c_float, _P, _P, c_int, c_int, c_int, c_int, _P],
     "cpm_hyper_fan_out": [_P, _P, c_int, c_int, c_int, _P],
     "cpm_linear_recurrence": [_P, _P, c_int64, _P, c_int64, _P, c_int64, c_int, _P, c_int64, _P, _P, _P, _P, _P, c_int, c_int,
-                              c_int, c_int, c_int, c_float, _P],
+                              c_int, c_int, c_int, c_float, c_int, _P],
     "cpm_conv_prepare": [_P, c_int64, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int,
                          c_int, c_int, c_int, c_int, c_float, _P],
     "cpm_sigmoid_power": [_P, _P, c_float, c_int, c_int, _P],

@@ -1019,7 +1019,8 @@ class Ops:
         check(self.lib.cpm_linear_recurrence(_ptr(q), _ptr(k), q.stride(0), _ptr(v), v.stride(0), _ptr(decay), decay.stride(0),
                                              1 if vector else 0, _ptr(beta), beta.stride(0) if beta is not None else 0,
                                              _ptr(state), _ptr(ctx.positions), _ptr(ctx.cu_q), _ptr(ctx.slot_dev), _ptr(out),
-                                             ctx.n_seqs, heads, qk_heads, d, dv, float(q_scale), self._stream()),
+                                             ctx.n_seqs, heads, qk_heads, d, dv, float(q_scale),
+                                             1 if ctx.is_decode and n == ctx.n_seqs else 0, self._stream()),
               f"linear_recurrence ({heads} heads, {d} x {dv})")
         return out
 

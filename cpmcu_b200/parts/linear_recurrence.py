@@ -245,7 +245,10 @@ class LightningAttention(_MatrixStateMixer):
         self.w_in = self.ops.keep(torch.cat([tensors[n[x]] for x in ("q", "k", "v", "g")], dim=0).contiguous())
         self.w_o = self.ops.keep(tensors[n["o"]].contiguous())
         self.w_norm = self._keep32(tensors[n["norm"]])
-        self.decay = self.ops.keep(torch.tensor(self.decay_values, dtype=torch.float32, device=self.w_norm.device))
+        a = torch.tensor(self.decay_values, dtype=torch.float64)
+        self.decay = self.ops.keep(a.float().to(self.w_norm.device).contiguous())
+        powers = a[:, None] ** torch.arange(QUERY_TILE_TOKENS + 1, dtype=torch.float64)[None, :]       # formed once, in 64-bit
+        self.powers = self.ops.keep(powers.float().to(self.w_norm.device).contiguous())
 
     def weight_bytes(self) -> int:
         return sum(t.numel() * t.element_size() for t in (self.w_in, self.w_o, self.w_norm))
@@ -259,8 +262,12 @@ class LightningAttention(_MatrixStateMixer):
         ops.silu_columns(proj, 2 * H * d + H * dv)
         q, k = proj[:, :H * d], proj[:, H * d:2 * H * d]
         v, g = proj[:, 2 * H * d:2 * H * d + H * dv], proj[:, 2 * H * d + H * dv:]
-        decay = self.decay.unsqueeze(0).expand(ctx.n_tokens, H)             # the same row for every token (stride 0)
-        o = ops.linear_recurrence(ctx, q, k, v, decay, None, lane.state["matrix_state"], H, H, d, dv, self.q_scale)
+        if self.q_scale == 1.0 and ops.retention_tiles_ok(ctx, d, dv):
+            # a prompt: by tiles of 64 tokens, as the retention's (16 heads of 64 x 128, 2,048 tokens: 359 us token by token)
+            o = ops.retention_tiles(ctx, q, k, v, None, self.powers, lane.state["matrix_state"], H, d, dv)
+        else:
+            decay = self.decay.unsqueeze(0).expand(ctx.n_tokens, H)         # the same row for every token (stride 0)
+            o = ops.linear_recurrence(ctx, q, k, v, decay, None, lane.state["matrix_state"], H, H, d, dv, self.q_scale)
         return ops.linear(ops.gated_group_norm(o, g, self.w_norm, self.eps, self.group, self.gate), self.w_o)
 
 

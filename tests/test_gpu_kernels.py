@@ -862,8 +862,9 @@ def test_decode_attention_with_rotation_inside(n_heads, n_kv, d):
     (4, 2, 136, 72, 700, True),        # chunks of more than 256 pairs, a ragged last slice of K, an expert nobody chose
     (512, 3, 64, 136, 65, False),      # the most experts, most of one pair or none
     (3, 1, 8, 12, 600, False),         # a row shorter than a slice, rows that are no whole 16-byte pieces
-    (8, 4, 200, 40, 24, False),        # the most pairs of the kernel for few
-    (8, 4, 200, 40, 25, False),        # one more: tiles
+    (8, 4, 200, 40, 40, False),        # the most pairs of the kernel for few
+    (8, 4, 200, 40, 41, False),        # more: tiles
+    (16, 4, 2048, 768, 7, False),      # sums of many slices
     (2, 1, 72, 264, 33, False),        # more pairs of one expert than the eight columns of an instruction
 ])
 @pytest.mark.parametrize("mode", ["silu", "relu2", "bounded"])
@@ -958,3 +959,41 @@ def test_decode_attention_shares_of_ragged_batches(n_heads, n_kv, d, lens):
         got = run(splits)
         assert _err(got, want) < KTOL["bfloat16"] and _err(got[i], ref) < KTOL["bfloat16"]
         assert not ops.arrivals.any()
+
+
+@pytest.mark.parametrize("H,G,d,dv", [(1, 1, 1, 4), (6, 3, 31, 36), (4, 4, 64, 128), (2, 1, 100, 64), (3, 3, 256, 8), (2, 2, 128, 6)])
+@pytest.mark.parametrize("delta,vector", [(False, False), (False, True), (True, False), (True, True)])
+def test_recurrence_of_one_token_a_sequence(H, G, d, dv, delta, vector):
+    """A decode step of the matrix state (and, at a value size that is no multiple of 4, the walk in its place) against the
+    formulas in 64 bits: operands that are slices of wider rows, a fresh sequence over a dirty slot, slots out of order."""
+    from types import SimpleNamespace
+
+    ops = _ops("float32")
+    n, g = 3, torch.Generator().manual_seed(H * 100 + d + dv)
+    wide = torch.randn(n, 2 * G * d + H * dv + 4, generator=g)
+    q, k, v = wide[:, :G * d], wide[:, G * d:2 * G * d] * d ** -0.5, wide[:, 2 * G * d:2 * G * d + H * dv]
+    wide[:, G * d:2 * G * d] = k
+    pad = (-2 * G * d) % 4                                       # the values begin on a 16-byte boundary
+    dev = torch.zeros(n, 2 * G * d + pad + H * dv + (-H * dv) % 4 + 4 * ((2 * G * d + pad) % 4 == 0)).cuda()
+    dev[:, :2 * G * d] = wide[:, :2 * G * d].cuda()
+    dev[:, 2 * G * d + pad:2 * G * d + pad + H * dv] = v.cuda()
+    decay = torch.rand(n, H * (d if vector else 1), generator=g) * 0.5 + 0.5
+    beta = torch.rand(n, H, generator=g) if delta else None
+    state = torch.randn(5, H, d, dv, generator=g)
+    slots, positions = [4, 0, 2], [7, 0, 3]
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32).cuda()
+    ctx = SimpleNamespace(positions=i32(positions), cu_q=i32([0, 1, 2, 3]), slot_dev=i32(slots), n_seqs=n, is_decode=True)
+    st = state.cuda()
+    got = ops.linear_recurrence(ctx, dev[:, :G * d], dev[:, G * d:2 * G * d], dev[:, 2 * G * d + pad:2 * G * d + pad + H * dv], decay.cuda(),
+                                None if beta is None else beta.cuda(), st, H, G, d, dv, 0.7, vector_decay=vector)
+    want, after = torch.zeros(n, H, dv, dtype=torch.float64), state.double().clone()
+    for i in range(n):
+        for h in range(H):
+            a = decay[i].double().view(H, -1)[h][:, None]
+            S = (torch.zeros(d, dv, dtype=torch.float64) if positions[i] == 0 else state[slots[i], h].double()) * a
+            kk, qq, u = (x[i].double().view(-1, w)[y] for x, w, y in ((k, d, h // (H // G)), (q, d, h // (H // G)), (v, dv, h)))
+            if delta:
+                u = beta[i, h].double() * (u - S.T @ kk)
+            S = S + kk[:, None] * u[None]
+            want[i, h], after[slots[i], h] = 0.7 * (S.T @ qq), S
+    assert _err(got, want) < KTOL["float32"] and _err(st, after) < KTOL["float32"]
