@@ -197,28 +197,48 @@ __global__ void scale_heads_kernel(const bf16* __restrict__ q, const float* __re
         out[t * n_heads * d + i] = __float2bfloat16_rn(__bfloat162float(q[t * n_heads * d + i]) * temp[i / d]);
 }
 
-// parts [n_kv][tokens][heads][d] (run s at parts[s]) -> out [tokens][heads][d]
-__global__ void talk_mix_kernel(const bf16* __restrict__ parts, const float* __restrict__ talk, bf16* __restrict__ out,
-                                int64_t n_tokens, int n_heads, int n_kv, int d) {
-    extern __shared__ float mix_smem[];          // [n_kv][heads][d] of this token, then talk [heads][heads]
-    float* tk = mix_smem + n_kv * n_heads * d;
+// parts [n_kv][tokens][heads][d] (run s at parts[s]) -> out [tokens][heads][d].  A thread forms VEC neighbouring channels of one
+// receiving head; its loads, one a giving head, depend on nothing but each other's addresses and are in flight eight at a time (staging a
+// token's runs in shared memory first, one channel a load, took 12.8 us a launch for 16 tokens of 16 heads of 64).
+template <int VEC>
+__global__ void __launch_bounds__(128)
+talk_mix_kernel(const bf16* __restrict__ parts, const float* __restrict__ talk, bf16* __restrict__ out, int64_t n_tokens, int n_heads, int n_kv,
+                int d) {
+    extern __shared__ float tk[];                // talk [heads][heads]
     pdl_launch_dependents();
     for (int i = threadIdx.x; i < n_heads * n_heads; i += blockDim.x) tk[i] = talk[i];
     pdl_wait();
-    const int64_t t = blockIdx.x;
-    const int row = n_heads * d;
-    for (int i = threadIdx.x; i < n_kv * row; i += blockDim.x)
-        mix_smem[i] = __bfloat162float(parts[((int64_t)(i / row) * n_tokens + t) * row + i % row]);
     __syncthreads();
-    const int rep = n_heads / n_kv;
-    for (int i = threadIdx.x; i < row; i += blockDim.x) {
-        const int h = i / d, c = i % d;
-        float acc = 0.f;
-        for (int g = 0; g < n_heads; ++g) {
-            const int s = (h / rep - g / rep + n_kv) % n_kv;          // the run in which head g saw the values of h's head
-            acc = fmaf(tk[h * n_heads + g], mix_smem[(s * n_heads + g) * d + c], acc);
+    const int64_t t = blockIdx.x;
+    const int row = n_heads * d, rep = n_heads / n_kv, i = (blockIdx.y * 128 + threadIdx.x) * VEC;
+    if (i >= row) return;
+    const int h = i / d, c = i % d;
+    const float* weights = tk + h * n_heads;
+    float acc[VEC] = {};
+#pragma unroll 8
+    for (int g = 0; g < n_heads; ++g) {
+        const int s = (h / rep - g / rep + n_kv) % n_kv;          // the run in which head g saw the values of h's head
+        const bf16* src = parts + ((int64_t)s * n_tokens + t) * row + (int64_t)g * d + c;
+        const float w = weights[g];
+        if (VEC == 8) {
+            const uint4 raw = *reinterpret_cast<const uint4*>(src);
+            const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float2 f = __bfloat1622float2(p[e]);
+                acc[(2 * e) % VEC] = fmaf(w, f.x, acc[(2 * e) % VEC]);
+                acc[(2 * e + 1) % VEC] = fmaf(w, f.y, acc[(2 * e + 1) % VEC]);
+            }
+        } else {
+            acc[0] = fmaf(w, __bfloat162float(*src), acc[0]);
         }
-        out[t * row + i] = __float2bfloat16_rn(acc);
+    }
+    bf16* dst = out + t * row + i;
+    if (VEC == 8) {
+        store4(dst, make_float4(acc[0], acc[1 % VEC], acc[2 % VEC], acc[3 % VEC]));
+        store4(dst + 4, make_float4(acc[4 % VEC], acc[5 % VEC], acc[6 % VEC], acc[7 % VEC]));
+    } else {
+        *dst = __float2bfloat16_rn(acc[0]);
     }
 }
 
@@ -229,20 +249,22 @@ CPM_API int cpm_scale_heads_bf16(const void* q, const float* temp, void* out, in
     return launch_status();
 }
 
-static bool g_mix_smem_done[kMaxDevices];
-
 CPM_API int cpm_talk_mix_bf16(const void* parts, const float* talk, void* out, int n_tokens, int n_heads, int n_kv, int d,
                               cudaStream_t stream) {
     if (n_tokens <= 0) return CPM_OK;
     if (n_heads < 1 || n_kv < 1 || n_heads % n_kv) return CPM_BAD_ARGUMENT;
-    const size_t smem = (size_t)(n_kv * n_heads * d + n_heads * n_heads) * sizeof(float);
+    const size_t smem = (size_t)n_heads * n_heads * sizeof(float);
     if (smem > 200 * 1024) return CPM_BAD_ARGUMENT;
+    const int vec = d % 8 == 0 && !(((uintptr_t)parts | (uintptr_t)out) & 15) ? 8 : 1;
+    const dim3 grid(n_tokens, (n_heads * d / vec + 127) / 128);
+    if (grid.y > 65535) return CPM_BAD_ARGUMENT;
+    auto kern = vec == 8 ? talk_mix_kernel<8> : talk_mix_kernel<1>;
+    static bool configured[2][kMaxDevices] = {};
     if (smem > 48 * 1024) {
-        const int e = ensure_dynamic_smem(talk_mix_kernel, 200 * 1024, g_mix_smem_done);
+        const int e = ensure_dynamic_smem(kern, 200 * 1024, configured[vec == 8]);
         if (e != CPM_OK) return e;
     }
-    cpm_launch(kLaunchCombine, talk_mix_kernel, dim3(n_tokens), dim3(256), smem, stream, (const bf16*)parts, talk, (bf16*)out,
-               (int64_t)n_tokens, n_heads, n_kv, d);
+    cpm_launch(kLaunchNorm, kern, grid, dim3(128), smem, stream, (const bf16*)parts, talk, (bf16*)out, (int64_t)n_tokens, n_heads, n_kv, d);
     return launch_status();
 }
 
