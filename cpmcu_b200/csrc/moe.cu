@@ -369,8 +369,10 @@ moe_tile_kernel(const T* __restrict__ A, const T* __restrict__ B0, const T* __re
 // accumulation), the weights its 16 rows, straight from memory in 16-byte loads; the 8 warps take turns at 32-wide slices of K
 // and meet in shared memory.  A weight row of another pair with the same expert costs a column that is there anyway.
 // Bound by the weights' way from memory.  Before, every pair was a matrix-vector product of its own over an input row in
-// shared memory, whose reads met eight to a bank: 16 tokens of 4 choices among 32 experts of 512 x 1024 took 25.4 us for gate
-// and up and 17.9 us for down, 4 tokens of 6 choices among 64 experts of 768 x 2048 27.9 and 17.6 us.
+// shared memory, whose reads met eight to a bank: in decode steps 16 tokens of 4 choices among 32 experts of 512 x 1024 took 25.4 us for
+// gate and up and 17.9 us for down, now 14.5 and 8.7; 4 tokens of 6 choices among 64 experts of 768 x 2048 27.9 and 17.6 us, now 22.4 and
+// 14.6.  Four blocks an SM, two slices of K a warp in flight, hide a block's start and its sums behind the others' loads (two blocks of
+// four slices: 20.0 and 12.2 us at the first of these sizes).
 constexpr int kFewRows = 32;
 
 __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
@@ -387,7 +389,7 @@ __device__ __forceinline__ uint4 load_once(const bf16* p) {
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(256, 4)
 moe_few_pairs_kernel(const bf16* __restrict__ A, const bf16* __restrict__ B0, const bf16* __restrict__ B1, bf16* __restrict__ C,
                      const int* __restrict__ chosen, int n_pairs, int top, int N, int K, const float* __restrict__ in_scale, GluClamp clamp) {
     constexpr bool GATED = MODE == 1 || MODE == 3, BY_TOKEN = MODE != 0;
@@ -436,7 +438,7 @@ moe_few_pairs_kernel(const bf16* __restrict__ A, const bf16* __restrict__ B0, co
         const int mine = same[min(c0 + g, count - 1)];
         const bf16* x = A + (int64_t)(BY_TOKEN ? mine / top : mine) * K + 8 * j;
         float acc[2][4] = {};
-#pragma unroll 4
+#pragma unroll 2
         for (int s = warp; s < slices; s += 8) {
             uint4 a[4] = {}, b = make_uint4(0, 0, 0, 0);
             if (32 * s + 8 * j < K) {                          // K is a multiple of 8: a lane's piece is whole or absent

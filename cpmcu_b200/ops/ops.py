@@ -1458,7 +1458,10 @@ class Ops:
               f"moe_route ({n_experts} experts, top {top})")
         return chosen, weights, gate
 
-    MOE_PAIRWISE_MAX_PAIRS = int(os.environ.get("CPMCU_MOE_PAIRWISE_MAX", "96"))     # up to here a pair streams its expert alone
+    # Up to here the chosen experts are streamed without grouping.  Both kernels' products of a layer, inputs cold: 64 experts of
+    # 768 x 2048, 6 choices: 96 pairs 95 against 129 us by tiles, 198 pairs 126 against 137, 384 pairs 191 against 142; 32 of 512 x 1024, 4 choices:
+    # 96 pairs 34 against 46, 192 pairs 50 against 46.
+    MOE_PAIRWISE_MAX_PAIRS = int(os.environ.get("CPMCU_MOE_PAIRWISE_MAX", "160"))
 
     def moe_experts(self, x: torch.Tensor, chosen: torch.Tensor, w_gate: Optional[torch.Tensor], w_up: torch.Tensor,
                     w_down: torch.Tensor, input_scale: Optional[torch.Tensor] = None,
