@@ -12,15 +12,21 @@
 //   up to 16 rows (decode): bound by streaming the weights; a block owns 8 weight rows, a thread one slice of one of them for
 //     all token rows.  Weight pieces of 1,024 columns come by 16-byte cp.async three stages deep, each slice padded by four
 //     floats so that the 16-byte reads of a quarter warp (8 rows) fall into 8 different bank groups.
-//   more rows: 64 x 64 tiles, 128 threads with 8 x 4 outputs each.  Both operands stay K-major in shared memory as they lie
-//     in global memory (rows padded to 36 floats: conflict-free 16-byte reads along K, no transposition), 32 columns a stage,
-//     three stages by cp.async.  12 shared reads of 16 bytes per 128 FMAs a thread.
+//   more rows: tiles of 64, 80 or 96 rows times 64 columns, one block of four groups of 64 threads an SM.  A group sums every fourth
+//     slice of the whole tile, a thread 8, 10 or 12 rows of 8 columns: a shared read of 16 bytes takes an SM as long as 16
+//     FMAs of a thread, so 8 x 8 outputs (16 reads per 256 FMAs) are the least that does not wait for them.  Both operands stay K-major in
+//     shared memory as they lie in global memory (rows padded to 20 floats: conflict-free 16-byte reads along K, no
+//     transposition), 16 columns a stage, two stages a group by cp.async.  After each round of four slices the groups trade: each
+//     keeps the totals of two of a thread's columns and adds the four groups' sums of them in the order of the slices.
+//     The number of rows is the one whose tiles fill the SMs' rounds best.
 // Where K is no multiple of 4 or a pointer is not 16-byte aligned the same kernels load element by element.
 //
-// Measured on one B200 at the 0.5B layer sizes, 24 layers, three prompts of 453 tokens together and four decoded tokens:
-// all products 19.1 ms (a decode step's 0.79 ms, the output head's 300 MB included; the prompts' 15.9 ms, 21 TFLOP/s) against
-// 106 ms with one 64 x 64 tile kernel of scalar loads for every shape, which kept 16 of its 64 rows busy at most in a
-// decode step and summed all of K in one chain (its error against 64 bits was three times as large).
+// Measured on one B200 at the 0.5B layer sizes, 24 layers, prompts of 400, 141 and 50 tokens together and four decoded tokens:
+// all products 16.9 ms (a decode step's 0.79 ms, the output head's 300 MB included; the prompts' 13.6 ms, about half of what the
+// FMA units give; the down product of 591 rows 168 us).  One 64 x 64 tile kernel of scalar loads for every shape took 106 ms, kept
+// 16 of its 64 rows busy at most in a decode step and summed all of K in one chain (its error against 64 bits was three times
+// as large).  Tiles of 64 x 64 with one group of 128 threads, 8 x 4 outputs each, took 15.9 ms for the prompts (the down product
+// 257 us: 160 tiles of one warp a scheduler, 12 shared reads per 128 FMAs).
 #include "common.cuh"
 
 constexpr int kSliceK = 64;
@@ -130,82 +136,113 @@ gemm_f32_few_rows_kernel(const float* __restrict__ A, const float* __restrict__ 
 // ---------------------------------------------------------------------------------------------------------------------
 // more rows
 // ---------------------------------------------------------------------------------------------------------------------
-constexpr int BM = 64, BN = 64, BK = 32, kTilePad = BK + 4, kTileStages = 3, kTileThreads = 128;
-constexpr size_t kTileSmem = (size_t)kTileStages * (BM + BN) * kTilePad * sizeof(float);
+constexpr int BN = 64, BK = 16, kTilePad = BK + 4, kGroups = 4, kGroupThreads = 64, kTileThreads = kGroups * kGroupThreads;
+template <int RI> constexpr int tile_stage_floats() { return (8 * RI + BN) * kTilePad; }
+template <int RI> constexpr size_t tile_smem_bytes() {
+    return (size_t)(kGroups * 2 * tile_stage_floats<RI>() + kGroups * RI * 8 * kGroupThreads) * sizeof(float);
+}
 
-template <bool VEC>
-__global__ void __launch_bounds__(kTileThreads)
+template <bool VEC, int RI>
+__global__ void __launch_bounds__(kTileThreads, 1)
 gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C,
                      int M, int N, int K, int64_t lda, int64_t ldw, int64_t ldc, float alpha) {
     extern __shared__ float tile_smem[];
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;          // outputs (ty + 8 i, tx + 16 j)
+    constexpr int BM = 8 * RI, kStage = tile_stage_floats<RI>(), kSteps = kSliceK / BK, kOwn = 8 / kGroups;
+    const int group = threadIdx.x / kGroupThreads, tid = threadIdx.x % kGroupThreads;
+    const int tx = tid & 7, ty = tid >> 3;                              // outputs (ty + 8 i, tx + 8 j)
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-    const int steps = (K + BK - 1) / BK;
-    auto stage = [&](int s) {
-        float* as = tile_smem + (s % kTileStages) * (BM + BN) * kTilePad;
+    const int slices = (K + kSliceK - 1) / kSliceK, steps = (slices + kGroups - 1) / kGroups * kSteps;
+    float* ring = tile_smem + group * 2 * kStage;
+    float* trade = tile_smem + kGroups * 2 * kStage;                    // [group][RI * 8][64]
+    auto stage = [&](int s) {                                           // columns past K are zeros
+        float* as = ring + (s & 1) * kStage;
         float* bs = as + BM * kTilePad;
-        const int k0 = s * BK;
+        const int k = ((s / kSteps) * kGroups + group) * kSliceK + (s % kSteps) * BK + 4 * (tid & 3);
 #pragma unroll
-        for (int i = 0; i < BM * (BK / 4) / kTileThreads; ++i) {
-            const int e = tid + kTileThreads * i, r = e / (BK / 4), k = 4 * (e % (BK / 4));
-            f32_stage4<VEC>(as + r * kTilePad + k, A + (int64_t)min(m0 + r, M - 1) * lda, k0 + k, K, m0 + r < M);
-            f32_stage4<VEC>(bs + r * kTilePad + k, W + (int64_t)min(n0 + r, N - 1) * ldw, k0 + k, K, n0 + r < N);
+        for (int i = 0; i < BM / 16; ++i) {
+            const int r = (tid >> 2) + 16 * i;
+            f32_stage4<VEC>(as + r * kTilePad + 4 * (tid & 3), A + (int64_t)min(m0 + r, M - 1) * lda, k, K, m0 + r < M);
         }
+#pragma unroll
+        for (int i = 0; i < BN / 16; ++i) {
+            const int r = (tid >> 2) + 16 * i;
+            f32_stage4<VEC>(bs + r * kTilePad + 4 * (tid & 3), W + (int64_t)min(n0 + r, N - 1) * ldw, k, K, n0 + r < N);
+        }
+        f32_cp_commit();
     };
+    stage(0);
+    float total[RI][kOwn], acc[RI][8];
 #pragma unroll
-    for (int s = 0; s < kTileStages - 1; ++s) {
-        if (s < steps) stage(s);
-        f32_cp_commit();
+    for (int i = 0; i < RI; ++i) {
+#pragma unroll
+        for (int j = 0; j < kOwn; ++j) total[i][j] = 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
     }
-    float total[8][4], acc[8][4];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) total[i][j] = acc[i][j] = 0.f;
     for (int s = 0; s < steps; ++s) {
-        f32_cp_wait<kTileStages - 2>();
-        __syncthreads();
-        if (s + kTileStages - 1 < steps) stage(s + kTileStages - 1);
-        f32_cp_commit();
-        const float* as = tile_smem + (s % kTileStages) * (BM + BN) * kTilePad + ty * kTilePad;
-        const float* bs = tile_smem + (s % kTileStages) * (BM + BN) * kTilePad + BM * kTilePad + tx * kTilePad;
+        f32_cp_wait<0>();
+        asm volatile("bar.sync %0, 64;" :: "r"(group + 1) : "memory");      // the stage has arrived; the other one has been used
+        if (s + 1 < steps) stage(s + 1);
+        const float* as = ring + (s & 1) * kStage + ty * kTilePad;
+        const float* bs = ring + (s & 1) * kStage + (BM + tx) * kTilePad;
 #pragma unroll
         for (int k = 0; k < BK; k += 4) {
-            float4 b[4];
+            float4 b[8];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4*>(bs + 16 * j * kTilePad + k);
+            for (int j = 0; j < 8; ++j) b[j] = *reinterpret_cast<const float4*>(bs + 8 * j * kTilePad + k);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
+            for (int i = 0; i < RI; ++i) {
                 const float4 a = *reinterpret_cast<const float4*>(as + 8 * i * kTilePad + k);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    acc[i][j] = fmaf(a.x, b[j].x, acc[i][j]);
-                    acc[i][j] = fmaf(a.y, b[j].y, acc[i][j]);
-                    acc[i][j] = fmaf(a.z, b[j].z, acc[i][j]);
-                    acc[i][j] = fmaf(a.w, b[j].w, acc[i][j]);
-                }
+                for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a.x, b[j].x, acc[i][j]);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a.y, b[j].y, acc[i][j]);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a.z, b[j].z, acc[i][j]);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a.w, b[j].w, acc[i][j]);
             }
         }
-        if ((s + 1) % (kSliceK / BK) == 0 || s + 1 == steps) {           // a slice is complete
+        if ((s + 1) % kSteps != 0) continue;
+        // a round's slices are complete (those past the last are zeros)
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
+        for (int i = 0; i < RI; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    total[i][j] += acc[i][j];
-                    acc[i][j] = 0.f;
-                }
-        }
+            for (int j = 0; j < 8; ++j) {
+                trade[((group * RI + i) * 8 + j) * kGroupThreads + tid] = acc[i][j];
+                acc[i][j] = 0.f;
+            }
+        __syncthreads();
+#pragma unroll
+        for (int g = 0; g < kGroups; ++g)
+#pragma unroll
+            for (int i = 0; i < RI; ++i)
+#pragma unroll
+                for (int j = 0; j < kOwn; ++j) total[i][j] += trade[((g * RI + i) * 8 + group * kOwn + j) * kGroupThreads + tid];
+        __syncthreads();
     }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 0; i < RI; ++i) {
         const int m = m0 + ty + 8 * i;
         if (m >= M) continue;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int n = n0 + tx + 16 * j;
+        for (int j = 0; j < kOwn; ++j) {
+            const int n = n0 + tx + 8 * (group * kOwn + j);
             if (n < N) C[(int64_t)m * ldc + n] = alpha * total[i][j];
         }
     }
+}
+
+template <bool VEC, int RI>
+static int launch_tile(const float* A, const float* W, float* C, int M, int N, int K, int64_t lda, int64_t ldw, int64_t ldc, float alpha,
+                       cudaStream_t stream) {
+    static bool done[kMaxDevices];
+    const int rc = ensure_dynamic_smem(gemm_f32_tile_kernel<VEC, RI>, (int)tile_smem_bytes<RI>(), done);
+    if (rc != CPM_OK) return rc;
+    const dim3 grid((N + BN - 1) / BN, (M + 8 * RI - 1) / (8 * RI));
+    if (grid.y > 65535) return CPM_BAD_ARGUMENT;
+    gemm_f32_tile_kernel<VEC, RI><<<grid, kTileThreads, tile_smem_bytes<RI>(), stream>>>(A, W, C, M, N, K, lda, ldw, ldc, alpha);
+    return launch_status();
 }
 
 template <int MT, bool VEC>
@@ -229,13 +266,17 @@ static int launch_gemm_f32(const float* A, const float* W, float* C, int M, int 
     if (M <= 4) return launch_few_rows<4, VEC>(A, W, C, M, N, K, lda, ldw, ldc, alpha, stream);
     if (M <= 8) return launch_few_rows<8, VEC>(A, W, C, M, N, K, lda, ldw, ldc, alpha, stream);
     if (M <= 16) return launch_few_rows<16, VEC>(A, W, C, M, N, K, lda, ldw, ldc, alpha, stream);
-    static bool done[kMaxDevices];
-    const int rc = ensure_dynamic_smem(gemm_f32_tile_kernel<VEC>, (int)kTileSmem, done);
-    if (rc != CPM_OK) return rc;
-    const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
-    if (grid.y > 65535) return CPM_BAD_ARGUMENT;
-    gemm_f32_tile_kernel<VEC><<<grid, kTileThreads, kTileSmem, stream>>>(A, W, C, M, N, K, lda, ldw, ldc, alpha);
-    return launch_status();
+    // rounds of one block an SM, times the rows of a block
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
+        return CPM_BAD_ARGUMENT;
+    auto cost = [&](int ri) {
+        const int64_t tiles = (int64_t)((M + 8 * ri - 1) / (8 * ri)) * ((N + BN - 1) / BN);
+        return (tiles + sms - 1) / sms * ri;
+    };
+    if (cost(12) < cost(10) && cost(12) < cost(8)) return launch_tile<VEC, 12>(A, W, C, M, N, K, lda, ldw, ldc, alpha, stream);
+    if (cost(10) < cost(8)) return launch_tile<VEC, 10>(A, W, C, M, N, K, lda, ldw, ldc, alpha, stream);
+    return launch_tile<VEC, 8>(A, W, C, M, N, K, lda, ldw, ldc, alpha, stream);
 }
 
 CPM_API int cpm_gemm_f32(const float* A, const float* W, float* C, int M, int N, int K, int64_t lda,

@@ -108,6 +108,20 @@ def test_gemm_f32_rows_agree_across_kernels(K):
     assert torch.equal(ops.linear(a[:5].contiguous(), shifted), whole[:5]) and torch.equal(ops.linear(a, shifted), whole)
 
 
+@pytest.mark.parametrize("M,N", [(640, 1024), (592, 1280), (1100, 1216), (33, 130)])
+@pytest.mark.parametrize("K", [20, 200, 260])
+def test_gemm_f32_heights_of_tiles(M, N, K):
+    """Sizes that take 80, 96 and 64 rows a tile on 148 SMs, ragged at every edge, fewer slices than groups and a round that is not
+    full: the bits of the few-row kernels, and 64-bit products."""
+    ops = _ops("float32")
+    g = torch.Generator().manual_seed(M + K)
+    a, w = torch.randn(M, K, generator=g).cuda(), torch.randn(N, K, generator=g).cuda()
+    whole = ops.linear(a, w)
+    assert _err(whole, (a.double() @ w.double().T).float()) < 1e-5
+    for first in (0, 17, M - 16):
+        assert torch.equal(ops.linear(a[first:first + 16].contiguous(), w), whole[first:first + 16])
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("n_heads,n_kv,d", [(16, 2, 64), (22, 2, 40), (8, 8, 37), (16, 1, 200), (4, 2, 96)])
 def test_attention_generic_shares_of_keys(dtype, n_heads, n_kv, d):
