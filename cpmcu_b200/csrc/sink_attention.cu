@@ -647,8 +647,20 @@ sink_attention_tiles_kernel(const bf16* __restrict__ q, const bf16* __restrict__
 
 // Single tokens (a decode step; also any step without tile lists): a block takes one token, one key-value head and up
 // to 16 of the query heads that share it as the rows of a tile; its warps split the token's keys among them, 32 at a
-// time, and join their maxima, sums and outputs through shared memory.
-constexpr int kSinkTokenWarps = 4;
+// time, and join their maxima, sums and outputs through shared memory.  Bound by latency (1,024 keys of 4 kv heads of 128 are 2 MB): a
+// warp asks for its next two steps' keys and values together, asynchronously, those of all pages but the sequence's last before the
+// kernel ahead is waited for (an earlier step wrote them, as the plain decode attention has it), and the keys go to enough blocks
+// that a warp has a step or two.  Keys, then values, one step after the other and three steps a warp: 20.4 us a launch
+// for one token, 15.4 us for four with 500 to 3,000 keys.
+constexpr int kSinkTokenWarps = 4, kSinkTokenStages = 2;
+template <int D, int DV> struct SinkTokenStage {
+    static constexpr int kKeyChunks = D / 8;                       // 16-byte pieces of a key
+    static constexpr int kKeyBytes = 32 * D * 2, kBytes = kKeyBytes + 32 * DV * 2;
+    static constexpr bool kSwizzleKeys = kKeyChunks % 8 == 0;
+    static constexpr int kJoin = (kSinkTokenWarps - 1) * 16 * (DV + 1) * 4;      // the warps' outputs when they join, in the stages' place
+    static constexpr int kRing = kSinkTokenWarps * kSinkTokenStages * kBytes;
+    static constexpr int kSmem = kRing > kJoin ? kRing : kJoin;
+};
 
 template <int D, int DV>
 __global__ void __launch_bounds__(kSinkTokenWarps * 32)
@@ -657,11 +669,12 @@ sink_attention_token_kernel(const bf16* __restrict__ q, const bf16* __restrict__
                             const int* __restrict__ slots, const int* __restrict__ page_table, int max_pages, int window,
                             int keep_first, int n_heads, int n_kv, float scale, float cap, int sink,
                             const float* __restrict__ sinks, const float* __restrict__ gate, int64_t gate_stride,
-                            float* __restrict__ shares) {
-    __shared__ float part_o[kSinkTokenWarps - 1][16][DV + 1];
+                            float* __restrict__ shares, int one_token) {
+    using S = SinkTokenStage<D, DV>;
+    extern __shared__ __align__(128) unsigned char token_smem[];
+    float (*part_o)[16][DV + 1] = reinterpret_cast<float (*)[16][DV + 1]>(token_smem);
     __shared__ float part_ml[kSinkTokenWarps - 1][16][2];
     pdl_launch_dependents();
-    pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int j = lane & 3, g = lane >> 2;
     const int t = blockIdx.x;
@@ -670,6 +683,47 @@ sink_attention_token_kernel(const bf16* __restrict__ q, const bf16* __restrict__
     const int rows = min(16, (kvh + 1) * group - h0);
     const int p = positions[t];
     const int* pages = page_table + (int64_t)slots[token_seq[t]] * max_pages;
+    const int first = (window > 0 ? max(0, p - window + 1) : 0) & ~31;
+    // the steps of 32 keys that hold kept first tokens before the window come first: step b of the walk begins at key 32 b
+    // while b < kept_steps, then at key first + 32 (b - kept_steps)
+    const int kept_steps = min((keep_first + 31) / 32, first / 32);
+    // the token's steps of 32 keys go to gridDim.z blocks (shares != null when more than one), a block's to its warps
+    const int n_blocks = kept_steps + (p - first) / 32 + 1;
+    const int per_block = (n_blocks + gridDim.z - 1) / gridDim.z;
+    const int blk_begin = blockIdx.z * per_block, blk_end = min(n_blocks, blk_begin + per_block);
+    const int share = (max(0, blk_end - blk_begin) + kSinkTokenWarps - 1) / kSinkTokenWarps;
+    const int b_begin = blk_begin + warp * share, b_end = min(blk_end, b_begin + share);
+    auto first_key = [&](int b) { return b < kept_steps ? 32 * b : first + 32 * (b - kept_steps); };
+    const uint32_t ring = (uint32_t)__cvta_generic_to_shared(token_smem) + warp * kSinkTokenStages * S::kBytes;
+    auto issue = [&](int b) {
+        if (b < b_end) {
+            const int key0 = first_key(b), off = key0 % kPageTokens;
+            const int page = CPM_PAGE(pages, key0 / kPageTokens, max_pages);
+            const bf16* kp = k_cache + page_row_offset(page, kvh, off, n_kv, D);
+            const bf16* vp = v_cache + value_offset(page, kvh, 0, off, n_kv, DV);
+            const uint32_t stage = ring + ((b - b_begin) % kSinkTokenStages) * S::kBytes;
+#pragma unroll 8
+            for (int c = lane; c < 32 * S::kKeyChunks; c += 32) {
+                const int row = c / S::kKeyChunks, col = c % S::kKeyChunks;
+                cp_async16(stage + (row * S::kKeyChunks + (S::kSwizzleKeys ? col ^ ((row & 1) << 2) : col)) * 16, kp + row * D + 8 * col);
+            }
+#pragma unroll 8
+            for (int c = lane; c < 4 * DV; c += 32)
+                cp_async16(stage + S::kKeyBytes + c * 16, vp + (int64_t)(c >> 2) * kPageTokens + 8 * (c & 3));
+        }
+        cp_async_commit();
+    };
+    // the step's own token, the only one of its sequence, lies in the last page: a warp that has that page among its first steps waits
+    // for the kernel ahead first (and every warp does where a sequence brings several tokens)
+    const int last_page = p / kPageTokens;
+    bool early = one_token != 0;
+#pragma unroll
+    for (int b = 0; b < kSinkTokenStages; ++b) early = early && (b_begin + b >= b_end || first_key(b_begin + b) / kPageTokens != last_page);
+    if (early)
+        for (int b = 0; b < kSinkTokenStages; ++b) issue(b_begin + b);
+    pdl_wait();
+    if (!early)
+        for (int b = 0; b < kSinkTokenStages; ++b) issue(b_begin + b);
     uint4 qf[2][D / 32];
     int lo[2], hi[2];
 #pragma unroll
@@ -684,25 +738,23 @@ sink_attention_token_kernel(const bf16* __restrict__ q, const bf16* __restrict__
     }
     SinkTile<DV> st;
     st.init();
-    const int first = (window > 0 ? max(0, p - window + 1) : 0) & ~31;
-    // the steps of 32 keys that hold kept first tokens before the window come first: step b of the walk begins at key 32 b
-    // while b < kept_steps, then at key first + 32 (b - kept_steps)
-    const int kept_steps = min((keep_first + 31) / 32, first / 32);
-    // the token's steps of 32 keys go to gridDim.z blocks (shares != null when more than one), a block's to its warps
-    const int n_blocks = kept_steps + (p - first) / 32 + 1;
-    const int per_block = (n_blocks + gridDim.z - 1) / gridDim.z;
-    const int blk_begin = blockIdx.z * per_block, blk_end = min(n_blocks, blk_begin + per_block);
-    const int share = (max(0, blk_end - blk_begin) + kSinkTokenWarps - 1) / kSinkTokenWarps;
-    const int b_end = min(blk_end, blk_begin + (warp + 1) * share);
-    for (int b = blk_begin + warp * share; b < b_end; ++b) {
-        const int key0 = b < kept_steps ? 32 * b : first + 32 * (b - kept_steps);
-        const int page = CPM_PAGE(pages, key0 / kPageTokens, max_pages), off = key0 % kPageTokens;
-        const bf16* kp = k_cache + page_row_offset(page, kvh, off + 8 * (g >> 1) + (g & 1), n_kv, D) + 8 * j;
-        const bf16* vp = v_cache + value_offset(page, kvh, g, off + 8 * j, n_kv, DV);
-        sink_attend_keys<D, DV>(st, qf, [&](int t, int w) { return ldg16(kp + 2 * t * D + 32 * w); },
-                                [&](int nt) { return ldg16(vp + nt * 8 * kPageTokens); }, key0, lo, hi, keep_first, scale, cap,
-                                lane);
+    const int krow = 8 * (g >> 1) + (g & 1);
+    for (int b = b_begin; b < b_end; ++b) {
+        cp_async_wait<kSinkTokenStages - 1>();
+        __syncwarp();
+        const uint32_t stage = ring + ((b - b_begin) % kSinkTokenStages) * S::kBytes;
+        sink_attend_keys<D, DV>(st, qf,
+                                [&](int t, int w) {
+                                    const int row = krow + 2 * t, col = 4 * w + j;
+                                    return lds16(stage + (row * S::kKeyChunks + (S::kSwizzleKeys ? col ^ ((row & 1) << 2) : col)) * 16);
+                                },
+                                [&](int nt) { return lds16(stage + S::kKeyBytes + ((8 * nt + g) * 4 + j) * 16); },
+                                first_key(b), lo, hi, keep_first, scale, cap, lane);
+        __syncwarp();
+        issue(b + kSinkTokenStages);
     }
+    cp_async_wait<0>();
+    __syncthreads();                                               // the stages have been used: their place is free
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
         st.l[r] += __shfl_xor_sync(0xffffffffu, st.l[r], 1);
@@ -769,6 +821,8 @@ sink_attention_token_kernel(const bf16* __restrict__ q, const bf16* __restrict__
 
 // out[t, h, :] = sum_s o_s 2^(m_s - M) / (sink 2^(b_h - M) + sum_s l_s 2^(m_s - M)), M = max_s m_s, over the shares s of a
 // token's keys (rows of dv + 2 floats: o, m, l), times the head's gate.  One warp per token and head.
+// The statistics and eight shares' outputs are on their way together (one share after the other: 6.6 us a launch for 4 tokens of 16
+// heads of 128 in 11 shares).
 __global__ void sink_combine_shares_kernel(const float* __restrict__ shares, bf16* __restrict__ out, int n_rows, int dv,
                                            int n_splits, int sink, const float* __restrict__ sinks,
                                            const float* __restrict__ gate, int64_t gate_stride, int n_heads) {
@@ -778,27 +832,55 @@ __global__ void sink_combine_shares_kernel(const float* __restrict__ shares, bf1
     if (row >= n_rows) return;
     const int64_t stride = (int64_t)n_rows * (dv + 2);
     const float* mine = shares + (int64_t)row * (dv + 2);
-    float m = -INFINITY;
-    for (int s = 0; s < n_splits; ++s) m = fmaxf(m, mine[s * stride + dv]);
-    const float use = m == -INFINITY ? 0.f : m;
-    float l = 0.f, o[8];                       // channels lane, lane + 32, ... (dv <= 256)
+    float m = -INFINITY, use = 0.f, l = 0.f;
+    float2 o[4];                               // channels 2 lane, 2 lane + 1, 2 lane + 64, ... (dv <= 256, even)
 #pragma unroll
-    for (int i = 0; i < 8; ++i) o[i] = 0.f;
-    for (int s = 0; s < n_splits; ++s) {
-        const float* src = mine + s * stride;
-        const float f = exp2f(src[dv] - use);
-        l = fmaf(src[dv + 1], f, l);
+    for (int i = 0; i < 4; ++i) o[i] = make_float2(0.f, 0.f);
+    for (int s0 = 0; s0 < n_splits; s0 += 32) {
+        const int here = min(32, n_splits - s0);
+        const float2 ml = lane < here ? *reinterpret_cast<const float2*>(mine + (s0 + lane) * stride + dv) : make_float2(-INFINITY, 0.f);
+        float f = 0.f;
+        for (int s = 0; s < here; s += 8) {
+            float2 v[8][4];
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
-            if (lane + 32 * i < dv) o[i] = fmaf(src[lane + 32 * i], f, o[i]);
+            for (int u = 0; u < 8; ++u)
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    v[u][i] = s + u < here && 2 * lane + 64 * i < dv ? *reinterpret_cast<const float2*>(mine + (s0 + s + u) * stride + 2 * lane + 64 * i)
+                                                                   : make_float2(0.f, 0.f);
+            if (s == 0) {                      // these 32 shares' maximum joins the ones before
+                const float mn = fmaxf(m, warp_max(ml.x));
+                use = mn == -INFINITY ? 0.f : mn;
+                const float old = exp2f(m - use);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    o[i].x *= old;
+                    o[i].y *= old;
+                }
+                f = exp2f(ml.x - use);
+                l = l * old + warp_sum(ml.y * f);
+                m = mn;
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const float w = __shfl_sync(0xffffffffu, f, min(s + u, 31));
+                if (s + u < here) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        o[i].x = fmaf(v[u][i].x, w, o[i].x);
+                        o[i].y = fmaf(v[u][i].y, w, o[i].y);
+                    }
+                }
+            }
+        }
     }
     const int h = row % n_heads;
     float inv = sink_join(use, l, sink, sinks != nullptr ? sinks[h] * 1.4426950408889634f : 0.f);
     if (m == -INFINITY) inv = 0.f;
     if (gate != nullptr) inv *= 1.0f / (1.0f + __expf(-gate[(int64_t)(row / n_heads) * gate_stride + h]));
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
-        if (lane + 32 * i < dv) out[(int64_t)row * dv + lane + 32 * i] = __float2bfloat16(o[i] * inv);
+    for (int i = 0; i < 4; ++i)
+        if (2 * lane + 64 * i < dv) *reinterpret_cast<uint32_t*>(out + (int64_t)row * dv + 2 * lane + 64 * i) = pack_bf16(o[i].x * inv, o[i].y * inv);
 }
 
 template <int D, int DV>
@@ -806,7 +888,7 @@ static int launch_sink_bf16(const void* q, const void* k_cache, const void* v_ca
                             const int* tile_row, int n_tiles, const int* cu_q, const int* kv_len, const int* positions,
                             const int* token_seq, const int* slots, const int* page_table, int max_pages, int window,
                             int keep_first, int n_tokens, int n_heads, int n_kv, float scale, float cap, int sink,
-                            const float* sinks, const float* gate, int64_t gate_stride, float* shares, int n_splits,
+                            const float* sinks, const float* gate, int64_t gate_stride, float* shares, int n_splits, int one_token,
                             cudaStream_t stream) {
     if (n_tiles > 0) {
         auto kern = sink_attention_tiles_kernel<D, DV>;
@@ -819,11 +901,15 @@ static int launch_sink_bf16(const void* q, const void* k_cache, const void* v_ca
                    gate_stride);
     } else {
         const int group = n_heads / n_kv;
-        cpm_launch(kLaunchAttention, sink_attention_token_kernel<D, DV>,
-                   dim3(n_tokens, n_kv * ((group + 15) / 16), n_splits), dim3(kSinkTokenWarps * 32), 0, stream, (const bf16*)q,
+        auto kern = sink_attention_token_kernel<D, DV>;
+        constexpr int smem = SinkTokenStage<D, DV>::kSmem;
+        static bool configured[kMaxDevices] = {};            // per kernel and per device
+        if (int st = ensure_dynamic_smem(kern, smem, configured)) return st;
+        cpm_launch(kLaunchAttention, kern,
+                   dim3(n_tokens, n_kv * ((group + 15) / 16), n_splits), dim3(kSinkTokenWarps * 32), smem, stream, (const bf16*)q,
                    (const bf16*)k_cache, (const bf16*)v_cache, (bf16*)out, positions, token_seq, slots, page_table, max_pages,
                    window, keep_first, n_heads, n_kv, scale, cap, sink, sinks, gate, gate_stride,
-                   n_splits > 1 ? shares : (float*)nullptr);
+                   n_splits > 1 ? shares : (float*)nullptr, one_token);
         if (n_splits > 1) {
             const int n_rows = n_tokens * n_heads;
             cpm_launch(kLaunchAttention, sink_combine_shares_kernel, dim3((n_rows + 3) / 4), dim3(128), 0, stream,
@@ -840,13 +926,14 @@ CPM_API int cpm_sink_attention_bf16_sizes(int d, int dv) {
 
 // bf16 q [tokens, heads, d] -> out [tokens, heads * dv].  With n_tiles > 0 the tokens are prompt tokens packed by
 // sequence (cu_q, kv_len, tile lists of 64 rows); else every token is taken alone by its position and sequence, its keys
-// shared out over n_splits blocks (n_splits > 1: shares holds n_splits * tokens * heads * (dv + 2) floats).
+// shared out over n_splits blocks (n_splits > 1: shares holds n_splits * tokens * heads * (dv + 2) floats).  one_token: every sequence
+// brings one token, so that all pages but its last were written before this step.
 CPM_API int cpm_sink_attention_bf16(const void* q, const void* k_cache, const void* v_cache, void* out, const int* tile_seq,
                                     const int* tile_row, int n_tiles, const int* cu_q, const int* kv_len,
                                     const int* positions, const int* token_seq, const int* slots, const int* page_table,
                                     int max_pages, int window, int keep_first, int n_tokens, int n_heads, int n_kv, int d, int dv,
                                     float scale, float cap, int sink, const float* sinks, const float* gate,
-                                    int64_t gate_stride, float* shares, int n_splits, cudaStream_t stream) {
+                                    int64_t gate_stride, float* shares, int n_splits, int one_token, cudaStream_t stream) {
     if (n_tokens <= 0) return CPM_OK;
     if (!cpm_sink_attention_bf16_sizes(d, dv) || n_kv <= 0 || n_heads % n_kv != 0 || window < 0 || keep_first < 0 || n_tiles > 65535 ||
         n_splits < 1 || n_splits > 65535 || (n_splits > 1 && !shares))
@@ -856,7 +943,7 @@ CPM_API int cpm_sink_attention_bf16(const void* q, const void* k_cache, const vo
     if (d == DD && dv == VV)                                                                                               \
         return launch_sink_bf16<DD, VV>(q, k_cache, v_cache, out, tile_seq, tile_row, n_tiles, cu_q, kv_len, positions,    \
                                         token_seq, slots, page_table, max_pages, window, keep_first, n_tokens, n_heads,    \
-                                        n_kv, scale, cap, sink, sinks, gate, gate_stride, shares, n_splits, stream);
+                                        n_kv, scale, cap, sink, sinks, gate, gate_stride, shares, n_splits, one_token, stream);
 #define CPM_SINK_ROW(DD) CPM_SINK_CASE(DD, 32) CPM_SINK_CASE(DD, 64) CPM_SINK_CASE(DD, 96) CPM_SINK_CASE(DD, 128)
     CPM_SINK_ROW(32) CPM_SINK_ROW(64) CPM_SINK_ROW(96) CPM_SINK_ROW(128)
 #undef CPM_SINK_ROW

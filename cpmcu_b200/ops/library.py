@@ -96,7 +96,7 @@ _SIGNATURES = {
     "cpm_sink_attention_generic": [_P, _P, _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float,
                                    c_float, c_int, _P, _P, c_int64, c_int, _P],
     "cpm_sink_attention_bf16": [_P, _P, _P, _P, _P, _P, c_int, _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
-                                c_int, c_float, c_float, c_int, _P, _P, c_int64, _P, c_int, _P],
+                                c_int, c_float, c_float, c_int, _P, _P, c_int64, _P, c_int, c_int, _P],
     "cpm_sink_attention_bf16_sizes": [c_int, c_int],
     "cpm_sink_attention_tcgen05": [_P, _P, _P, _P, _P, _P, c_int, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int,
                                    c_float, c_int, c_float, c_int, c_int, _P, _P, c_int64, _P, c_int, _P],

@@ -1291,12 +1291,12 @@ class Ops:
 
     def sink_attention_splits(self, ctx, n_tokens: int, n_heads: int, n_kv: int, window: int) -> int:
         """Blocks that share the keys of a token taken alone: none while the tokens fill the device; else enough for
-        about two blocks an SM, as long as each of a block's four warps keeps at least two steps of 32 keys."""
+        one block an SM (its stages fill half of the shared memory), as long as each of a block's four warps keeps a step of 32 keys."""
         blocks = n_tokens * n_kv * ((n_heads // n_kv + 15) // 16)
         if blocks * 2 > self.sm_count:
             return 1
         keys = min(window, ctx.max_kv_len) if window else ctx.max_kv_len      # in a recorded step an upper bound
-        return max(1, min(self.SINK_MAX_SPLITS, 2 * self.sm_count // blocks, ((keys + 31) // 32) // 8))
+        return max(1, min(self.SINK_MAX_SPLITS, self.sm_count // blocks, ((keys + 31) // 32) // 4))
 
     SINK_TILE_MIN_ROWS = 8       # shorter portions than this go token by token (a tile of 16 rows would be mostly empty)
 
@@ -1322,7 +1322,7 @@ class Ops:
                                                _ptr(ctx.token_seq), _ptr(ctx.slot_dev), _ptr(lane.page_table),
                                                lane.page_table.shape[1], int(window), keep, n, n_heads, n_kv, d, dv, float(scale),
                                                float(cap), 1 if sink else 0, p_sinks, p_gate, gate_stride, _ptr(shares),
-                                               n_splits, self._stream()),
+                                               n_splits, 1 if ctx.is_decode else 0, self._stream()),
               f"sink attention on tensor cores ({n_heads} heads, {d} / {dv})")
         return out
 
