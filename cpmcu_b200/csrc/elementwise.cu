@@ -1,7 +1,7 @@
 // Row-wise kernels of a step: embedding lookup, residual add + RMS norm, the gated
 // activation, and rotary position encoding fused with the store into the cache.
 // All arithmetic is fp32; only loads and stores touch the storage type.
-#include "common.cuh"
+#include "rownorm.cuh"
 
 int g_cpm_pdl = kDefaultPdlMask;
 
@@ -108,9 +108,46 @@ __global__ void add_rmsnorm_kernel(float* __restrict__ x, const T* __restrict__ 
     }
 }
 
+// Rows of a multiple of four columns up to 8,192 (see rownorm.cuh).
+template <typename T, typename W, int NV>
+__global__ void __launch_bounds__(512)
+add_rmsnorm_rows_kernel(float* __restrict__ x, const T* __restrict__ delta, const T* __restrict__ delta2, float alpha,
+                        const W* __restrict__ w, T* __restrict__ y, const int* __restrict__ rows, int hidden, float eps, int write_back) {
+    __shared__ float scratch[kRowMaxWarps];
+    pdl_launch_dependents();
+    float4 g[NV], v[NV], d[NV], e[NV];
+    row_load(g, w, hidden);
+    pdl_wait();
+    const int64_t src = (rows ? (int64_t)rows[blockIdx.x] : (int64_t)blockIdx.x) * hidden;
+    row_load(v, x + src, hidden);
+    if (delta) {
+        row_load(d, delta + src, hidden);
+        row_load(e, delta2 ? delta2 + src : nullptr, hidden);
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            v[i] = quad_fma(alpha, d[i], v[i]);
+            if (delta2) v[i] = quad_fma(alpha, e[i], v[i]);
+        }
+        if (write_back) row_store(x + src, v, hidden);
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) ss = quad_squares(v[i], ss);
+    const float r = rsqrtf(row_sum(ss, scratch) / (float)hidden + eps);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) v[i] = quad_scaled(v[i], r, g[i]);
+    row_store(y + (int64_t)blockIdx.x * hidden, v, hidden);
+}
+
 template <typename T, typename W>
 static int launch_add_rmsnorm(float* x, const void* delta, const void* delta2, float alpha, const void* w, void* y, const int* rows,
                               int n_rows, int hidden, float eps, int write_back, cudaStream_t stream) {
+    if (const RowShape sh = row_shape(hidden, 4); sh.nv) {
+        auto kern = sh.nv == 1 ? add_rmsnorm_rows_kernel<T, W, 1> : sh.nv == 2 ? add_rmsnorm_rows_kernel<T, W, 2> : add_rmsnorm_rows_kernel<T, W, 4>;
+        cpm_launch(kLaunchNorm, kern, n_rows, sh.threads, 0, stream, x, (const T*)delta, (const T*)delta2, alpha, (const W*)w, (T*)y, rows, hidden,
+                   eps, write_back);
+        return launch_status();
+    }
     const size_t smem = (size_t)(hidden + 33) * sizeof(float);
     if (smem > 227 * 1024) return CPM_BAD_ARGUMENT;
     auto kern = add_rmsnorm_kernel<T, W>;

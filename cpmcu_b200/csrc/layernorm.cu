@@ -11,7 +11,7 @@
 // computed in fp32 (two passes over a row held in shared memory: the mean first, then the deviations); only
 // the loads of ``a`` and the stores of ``y`` touch the storage type.  Weights, biases and mu are fp32; a norm of
 // add_layernorm may have no bias.
-#include "common.cuh"
+#include "rownorm.cuh"
 
 // Four consecutive elements as floats (16-byte or 8-byte aligned loads).
 __device__ __forceinline__ float4 ln_load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
@@ -260,6 +260,115 @@ __global__ void post_norm_add_kernel(float* __restrict__ x, const T* __restrict_
     ln_write_row(y + t * hidden, buf, hidden);
 }
 
+// The three kernels for rows of a multiple of four columns up to 8,192 (token shift: 4,096); see rownorm.cuh.
+template <typename T, int NV>
+__global__ void __launch_bounds__(512)
+add_layernorm_rows_kernel(float* __restrict__ x, const T* __restrict__ a, const T* __restrict__ a2, float alpha, const float* __restrict__ w,
+                          const float* __restrict__ b, T* __restrict__ y, const float* __restrict__ w2, const float* __restrict__ b2,
+                          T* __restrict__ y2, const int* __restrict__ rows, int hidden, float eps, int write_back) {
+    __shared__ float scratch[2 * kRowMaxWarps];
+    pdl_launch_dependents();
+    float4 g[NV], h[NV], v[NV], d[NV], e[NV];
+    row_load(g, w, hidden);
+    row_load(h, b, hidden);
+    pdl_wait();
+    const int64_t src = (rows ? (int64_t)rows[blockIdx.x] : (int64_t)blockIdx.x) * hidden, at = (int64_t)blockIdx.x * hidden;
+    row_load(v, x + src, hidden);
+    if (a) {
+        row_load(d, a + src, hidden);
+        row_load(e, a2 ? a2 + src : nullptr, hidden);
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            v[i] = quad_fma(alpha, d[i], v[i]);
+            if (a2) v[i] = quad_fma(alpha, e[i], v[i]);
+        }
+        if (write_back) row_store(x + src, v, hidden);
+    }
+    if (y2) {                                      // the second norm's weights arrive behind the sums of the first
+        row_load(d, w2, hidden);
+        row_load(e, b2, hidden);
+    }
+    const float r = row_centre(v, hidden, eps, scratch);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        g[i] = quad_scaled(v[i], r, g[i]);
+        if (b) g[i] = quad_add(g[i], h[i]);
+    }
+    row_store(y + at, g, hidden);
+    if (!y2) return;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        d[i] = quad_scaled(v[i], r, d[i]);
+        if (b2) d[i] = quad_add(d[i], e[i]);
+    }
+    row_store(y2 + at, d, hidden);
+}
+
+template <typename T, int NV>
+__global__ void __launch_bounds__(512)
+post_norm_add_rows_kernel(float* __restrict__ x, const T* __restrict__ a, const float* __restrict__ w, const float* __restrict__ b,
+                          const float* __restrict__ w2, const float* __restrict__ b2, T* __restrict__ y, int hidden, float eps) {
+    __shared__ float scratch[4 * kRowMaxWarps];
+    pdl_launch_dependents();
+    float4 g[NV], h[NV], g2[NV], h2[NV], v[NV], old[NV];
+    row_load(g, w, hidden);
+    row_load(h, b, hidden);
+    row_load(g2, w2, hidden);
+    row_load(h2, b2, hidden);
+    pdl_wait();
+    const int64_t at = (int64_t)blockIdx.x * hidden;
+    row_load(v, a + at, hidden);
+    row_load(old, x + at, hidden);
+    float r = row_centre(v, hidden, eps, scratch);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) v[i] = row_col(i) < hidden ? quad_add(old[i], quad_add(quad_scaled(v[i], r, g[i]), h[i])) : make_float4(0.f, 0.f, 0.f, 0.f);
+    row_store(x + at, v, hidden);
+    if (w2 == nullptr) return;
+    r = row_centre(v, hidden, eps, scratch + 2 * kRowMaxWarps);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) v[i] = quad_add(quad_scaled(v[i], r, g2[i]), h2[i]);
+    row_store(y + at, v, hidden);
+}
+
+template <typename T, int NV>
+__global__ void __launch_bounds__(512)
+layernorm_shift_rows_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ b, const float* __restrict__ mu,
+                            float* __restrict__ state, const int* __restrict__ positions, const int* __restrict__ token_seq,
+                            const int* __restrict__ cu_q, const int* __restrict__ slots, T* __restrict__ y, int hidden, float eps) {
+    __shared__ float scratch[6 * kRowMaxWarps];
+    pdl_launch_dependents();
+    float4 g[NV], h[NV], m[NV], v[NV], p[NV];
+    row_load(g, w, hidden);
+    row_load(h, b, hidden);
+    row_load(m, mu, hidden);
+    // (written before this step's kernels began)
+    const int t = blockIdx.x, seq = token_seq[t], begin = cu_q[seq], last = cu_q[seq + 1] - 1, pos = positions[t];
+    const bool first = t == begin;
+    float* st = state + (int64_t)slots[seq] * hidden;
+    pdl_wait();
+    row_load(v, x + (int64_t)t * hidden, hidden);
+    row_load(p, first ? (pos == 0 ? nullptr : st) : x + (int64_t)(t - 1) * hidden, hidden);
+    auto normed = [&](float4 (&row)[NV], float* room) {
+        const float r = row_centre(row, hidden, eps, room);
+#pragma unroll
+        for (int i = 0; i < NV; ++i) row[i] = quad_add(quad_scaled(row[i], r, g[i]), h[i]);
+    };
+    normed(v, scratch);
+    if (!first) normed(p, scratch + 2 * kRowMaxWarps);
+#pragma unroll
+    for (int i = 0; i < NV; ++i)
+        p[i] = make_float4(v[i].x + (p[i].x - v[i].x) * m[i].x, v[i].y + (p[i].y - v[i].y) * m[i].y, v[i].z + (p[i].z - v[i].z) * m[i].z,
+                           v[i].w + (p[i].w - v[i].w) * m[i].w);
+    row_store(y + (int64_t)t * hidden, p, hidden);
+    if (!first) return;
+    // a thread writes the columns of the state that it has read itself
+    if (last != t) {
+        row_load(v, x + (int64_t)last * hidden, hidden);
+        normed(v, scratch + 4 * kRowMaxWarps);
+    }
+    row_store(st, v, hidden);
+}
+
 __global__ void stream_inject_kernel(float* __restrict__ x, const float* __restrict__ saved, const float* __restrict__ vec,
                                      int hidden, int64_t n) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -290,6 +399,14 @@ CPM_API int cpm_add_layernorm(float* x, const void* a, const void* a2, float alp
                               int write_back, int dtype, cudaStream_t stream) {
     if (n_rows <= 0) return CPM_OK;
     if (hidden < 1 || !w || !y || (y2 && !w2) || (a2 && !a)) return CPM_BAD_ARGUMENT;
+    if (const RowShape sh = row_shape(hidden, 4); sh.nv) {
+#define CPM_ADD_LN_ROWS(TT, NV) cpm_launch(kLaunchNorm, add_layernorm_rows_kernel<TT, NV>, n_rows, sh.threads, 0, stream, x, (const TT*)a,     \
+                                           (const TT*)a2, alpha, w, b, (TT*)y, w2, b2, (TT*)y2, rows, hidden, eps, write_back)
+        if (dtype == CPM_BF16) { if (sh.nv == 1) CPM_ADD_LN_ROWS(bf16, 1); else if (sh.nv == 2) CPM_ADD_LN_ROWS(bf16, 2); else CPM_ADD_LN_ROWS(bf16, 4); }
+        else { if (sh.nv == 1) CPM_ADD_LN_ROWS(float, 1); else if (sh.nv == 2) CPM_ADD_LN_ROWS(float, 2); else CPM_ADD_LN_ROWS(float, 4); }
+#undef CPM_ADD_LN_ROWS
+        return launch_status();
+    }
     const size_t smem = (size_t)(hidden + 33) * sizeof(float);
 #define CPM_ADD_LN(TT)                                                                                                      \
     do {                                                                                                                    \
@@ -308,6 +425,14 @@ CPM_API int cpm_layernorm_shift(const float* x, const float* w, const float* b, 
                                 const int* positions, const int* token_seq, const int* cu_q, const int* slots, void* y,
                                 int n_tokens, int hidden, float eps, int dtype, cudaStream_t stream) {
     if (n_tokens <= 0) return CPM_OK;
+    if (const RowShape sh = row_shape(hidden, 2); sh.nv) {
+#define CPM_SHIFT_ROWS(TT, NV) cpm_launch(kLaunchNorm, layernorm_shift_rows_kernel<TT, NV>, n_tokens, sh.threads, 0, stream, x, w, b, mu, state,  \
+                                          positions, token_seq, cu_q, slots, (TT*)y, hidden, eps)
+        if (dtype == CPM_BF16) { if (sh.nv == 1) CPM_SHIFT_ROWS(bf16, 1); else CPM_SHIFT_ROWS(bf16, 2); }
+        else { if (sh.nv == 1) CPM_SHIFT_ROWS(float, 1); else CPM_SHIFT_ROWS(float, 2); }
+#undef CPM_SHIFT_ROWS
+        return launch_status();
+    }
     const size_t smem = (size_t)(2 * hidden + 33) * sizeof(float);
     if (dtype == CPM_BF16) {
         auto kern = layernorm_shift_kernel<bf16>;
@@ -327,6 +452,14 @@ CPM_API int cpm_post_norm_add(float* x, const void* a, const float* w, const flo
                               void* y, int n_tokens, int hidden, float eps, int dtype, cudaStream_t stream) {
     if (n_tokens <= 0) return CPM_OK;
     if ((w2 == nullptr) != (y == nullptr) || (w2 == nullptr) != (b2 == nullptr)) return CPM_BAD_ARGUMENT;
+    if (const RowShape sh = row_shape(hidden, 4); sh.nv) {
+#define CPM_PNA_ROWS(TT, NV) cpm_launch(kLaunchNorm, post_norm_add_rows_kernel<TT, NV>, n_tokens, sh.threads, 0, stream, x, (const TT*)a, w, b, w2,  \
+                                        b2, (TT*)y, hidden, eps)
+        if (dtype == CPM_BF16) { if (sh.nv == 1) CPM_PNA_ROWS(bf16, 1); else if (sh.nv == 2) CPM_PNA_ROWS(bf16, 2); else CPM_PNA_ROWS(bf16, 4); }
+        else { if (sh.nv == 1) CPM_PNA_ROWS(float, 1); else if (sh.nv == 2) CPM_PNA_ROWS(float, 2); else CPM_PNA_ROWS(float, 4); }
+#undef CPM_PNA_ROWS
+        return launch_status();
+    }
     const size_t smem = (size_t)(hidden + 33) * sizeof(float);
     if (dtype == CPM_BF16) {
         auto kern = post_norm_add_kernel<bf16>;

@@ -17,7 +17,7 @@
 // Around it: the short causal convolution over time with SiLU, the unit-length scaling of q and k, the gates of
 // the delta rule, the decay of the gated linear attention, and the per-head RMS norm of the read-out times the
 // output gate.  All of it fp32; only the last kernel's output has the storage type.
-#include "common.cuh"
+#include "rownorm.cuh"
 
 __device__ __forceinline__ float sigmoid_acc(float v) { return 1.0f / (1.0f + expf(-v)); }
 __device__ __forceinline__ float silu_acc(float v) { return v / (1.0f + expf(-v)); }
@@ -618,6 +618,32 @@ __global__ void gated_group_norm_kernel(const float* __restrict__ o, const float
     }
 }
 
+// Groups of a multiple of four channels up to 8,192 in rows of whole 16-byte pieces (see rownorm.cuh).
+template <typename T, int NV>
+__global__ void __launch_bounds__(512)
+gated_group_norm_rows_kernel(const float* __restrict__ o, const float* __restrict__ gate, int64_t gate_stride, const float* __restrict__ weight,
+                             T* __restrict__ out, int groups, int width, int gate_act, float eps) {
+    __shared__ float scratch[kRowMaxWarps];
+    pdl_launch_dependents();
+    float4 g[NV], v[NV], a[NV];
+    row_load(g, weight, width);
+    pdl_wait();
+    const int64_t t = blockIdx.x / groups, at = (int64_t)blockIdx.x * width;
+    row_load(v, o + at, width);
+    row_load(a, gate + t * gate_stride + (int64_t)(blockIdx.x % groups) * width, width);
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) ss = quad_squares(v[i], ss);
+    const float f = rsqrtf(row_sum(ss, scratch) / (float)width + eps);
+    auto act = [&](float x) { return gate_act == 1 ? sigmoid_acc(x) : silu_acc(x); };
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        v[i] = quad_scaled(v[i], f, g[i]);
+        v[i] = make_float4(v[i].x * act(a[i].x), v[i].y * act(a[i].y), v[i].z * act(a[i].z), v[i].w * act(a[i].w));
+    }
+    row_store(out + at, v, width);
+}
+
 CPM_API int cpm_gated_group_norm(const float* o, const float* gate, int64_t gate_stride, const float* weight, void* out,
                                  int n_tokens, int heads, int dv, int group, int gate_act, float eps, int dtype,
                                  cudaStream_t stream) {
@@ -625,6 +651,14 @@ CPM_API int cpm_gated_group_norm(const float* o, const float* gate, int64_t gate
     if (heads < 1 || dv < 1 || group < 1 || heads % group || gate_act < 0 || gate_act > 1) return CPM_BAD_ARGUMENT;
     const int width = group * dv;
     const dim3 grid((unsigned)((int64_t)n_tokens * (heads / group))), block(width >= 2048 ? 256 : 128);
+    if (const RowShape sh = row_shape(width, 4); sh.nv && gate_stride % 4 == 0 && !(((uintptr_t)o | (uintptr_t)gate | (uintptr_t)weight | (uintptr_t)out) & 15)) {
+#define CPM_GROUP_ROWS(TT, NV) cpm_launch(kLaunchNorm, gated_group_norm_rows_kernel<TT, NV>, grid, dim3(sh.threads), 0, stream, o, gate, gate_stride, \
+                                          weight, (TT*)out, heads / group, width, gate_act, eps)
+        if (dtype == CPM_BF16) { if (sh.nv == 1) CPM_GROUP_ROWS(bf16, 1); else if (sh.nv == 2) CPM_GROUP_ROWS(bf16, 2); else CPM_GROUP_ROWS(bf16, 4); }
+        else { if (sh.nv == 1) CPM_GROUP_ROWS(float, 1); else if (sh.nv == 2) CPM_GROUP_ROWS(float, 2); else CPM_GROUP_ROWS(float, 4); }
+#undef CPM_GROUP_ROWS
+        return launch_status();
+    }
     if (dtype == CPM_BF16)
         cpm_launch(kLaunchNorm, gated_group_norm_kernel<bf16>, grid, block, 0, stream, o, gate, gate_stride, weight, (bf16*)out, heads,
                    dv, group, gate_act, eps);

@@ -6,7 +6,7 @@
 //
 // Both leave x in fp32 (the stream) and a copy in the storage type, which is what the next sublayer's products read:
 // with the norm after the sum a sublayer reads the stream itself.  Sums and norms are fp32.
-#include "common.cuh"
+#include "rownorm.cuh"
 
 // Norms the row in ``row_cache`` (hidden floats, ss: this thread's part of the sum of squares; w null: no weight) into x
 // and y (either may be null).
@@ -64,9 +64,42 @@ __global__ void post_norm_kernel(float* __restrict__ x, const T* __restrict__ a,
     norm_row_out<T>(row_cache, ss, row_cache + hidden, w, xr, y ? y + (int64_t)blockIdx.x * hidden : nullptr, hidden, eps, true);
 }
 
+// Rows of a multiple of four columns up to 8,192 (see rownorm.cuh).
+template <typename T, int NV>
+__global__ void __launch_bounds__(512)
+post_norm_rows_kernel(float* __restrict__ x, const T* __restrict__ a, float alpha, const float* __restrict__ scale,
+                      const float* __restrict__ w, T* __restrict__ y, int hidden, float eps) {
+    __shared__ float scratch[kRowMaxWarps];
+    pdl_launch_dependents();
+    float4 g[NV], sc[NV], v[NV], d[NV];
+    row_load(g, w, hidden);
+    row_load(sc, scale, hidden);
+    pdl_wait();
+    const int64_t at = (int64_t)blockIdx.x * hidden;
+    row_load(v, x + at, hidden);
+    row_load(d, a + at, hidden);
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        if (scale) d[i] = make_float4(d[i].x * sc[i].x, d[i].y * sc[i].y, d[i].z * sc[i].z, d[i].w * sc[i].w);
+        v[i] = quad_fma(alpha, v[i], d[i]);
+        ss = quad_squares(v[i], ss);
+    }
+    const float r = 1.0f / sqrtf(row_sum(ss, scratch) / (float)hidden + eps);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) v[i] = quad_scaled(v[i], r, g[i]);
+    row_store(x + at, v, hidden);
+    if (y) row_store(y + at, v, hidden);
+}
+
 template <typename T>
 static int launch_post_norm(float* x, const void* a, float alpha, const float* scale, const float* w, void* y, int n_tokens, int hidden,
                             float eps, cudaStream_t stream) {
+    if (const RowShape sh = row_shape(hidden, 4); sh.nv) {
+        auto kern = sh.nv == 1 ? post_norm_rows_kernel<T, 1> : sh.nv == 2 ? post_norm_rows_kernel<T, 2> : post_norm_rows_kernel<T, 4>;
+        cpm_launch(kLaunchNorm, kern, n_tokens, sh.threads, 0, stream, x, (const T*)a, alpha, scale, w, (T*)y, hidden, eps);
+        return launch_status();
+    }
     const size_t smem = (size_t)(hidden + 36) * sizeof(float);
     if (smem > 227 * 1024) return CPM_BAD_ARGUMENT;
     auto kern = post_norm_kernel<T>;
