@@ -182,6 +182,12 @@ __device__ __forceinline__ int64_t value_offset(int page, int kv_head, int dim, 
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// Asks L2 for ``bytes`` from p on, shared out among the block's threads: weights, or a state that an earlier step left, before the wait.
+__device__ __forceinline__ void prefetch_l2(const void* p, int64_t bytes) {
+    for (int64_t i = (int64_t)threadIdx.x * 128; i < bytes; i += (int64_t)blockDim.x * 128)
+        asm volatile("prefetch.global.L2 [%0];" :: "l"(static_cast<const char*>(p) + i));
+}
+
 // Which kernels are launched with the attribute: a mask over the classes below (bit = 1 << class).  Measured on
 // the 8B decode step (batch 8, 3.64 ms without): norms and products 3.47 ms, with the rotary kernel and the decode
 // attention as well 3.45 ms; the kernel that combines the attention's shares must stay out (with it the gain is

@@ -20,7 +20,7 @@
 //                       every tile of 32 latent rows through shared memory
 //
 // A latent page is [token_in_page][rank] (the key page layout with one key-value head).
-#include "common.cuh"
+#include "rownorm.cuh"
 
 // ---------------------------------------------------------------------------
 // proj rows (fp32, ``stride`` floats) begin [q_rank | rank | rot_dim]: the first two parts are RMS-normed; the third (rot_dim
@@ -34,23 +34,27 @@ __global__ void latent_norm_store_kernel(const float* __restrict__ proj, int64_t
                                          const int* __restrict__ slots, const int* __restrict__ page_table, int max_pages,
                                          int q_rank, int rank, int rot_dim, const float* __restrict__ inv_freq, float magnitude,
                                          int adjacent, float eps) {
-    __shared__ float scratch[33];
+    __shared__ float scratch[2 * kRowMaxWarps];
     pdl_launch_dependents();
+    // what needs the position alone, and the weights' way into L2, comes before the wait for the projections; both sums share a barrier
+    const int t = blockIdx.x, p = positions[t];
+    prefetch_l2(wq, (int64_t)q_rank * 4);
+    if (cache != nullptr) prefetch_l2(wkv, (int64_t)rank * 4);
+    int page = 0;
+    if (cache != nullptr) page = CPM_PAGE(page_table + (int64_t)slots[token_seq[t]] * max_pages, p / kPageTokens, max_pages);
+    float sn0 = 0.f, cs0 = 1.f;                          // this thread's first pair
+    if (threadIdx.x < (rot_dim >> 1) && inv_freq != nullptr) sincosf((float)p * inv_freq[threadIdx.x], &sn0, &cs0);
     pdl_wait();
-    const int t = blockIdx.x;
     const float* row = proj + (int64_t)t * stride;
-    float s = 0.f;
-    for (int c = threadIdx.x; c < q_rank; c += blockDim.x) s = fmaf(row[c], row[c], s);
-    float r = 1.0f / sqrtf(block_sum(s, scratch) / (float)q_rank + eps);
+    float2 s = make_float2(0.f, 0.f);
+    for (int c = threadIdx.x; c < q_rank; c += blockDim.x) s.x = fmaf(row[c], row[c], s.x);
+    for (int c = threadIdx.x; c < rank; c += blockDim.x) s.y = fmaf(row[q_rank + c], row[q_rank + c], s.y);
+    s = row_sum2(s, scratch);
+    float r = 1.0f / sqrtf(s.x / (float)q_rank + eps);
     for (int c = threadIdx.x; c < q_rank; c += blockDim.x) cq[(int64_t)t * q_rank + c] = from_f32<T>(row[c] * r * wq[c]);
     row += q_rank;
-    s = 0.f;
-    for (int c = threadIdx.x; c < rank; c += blockDim.x) s = fmaf(row[c], row[c], s);
-    r = 1.0f / sqrtf(block_sum(s, scratch) / (float)rank + eps);
+    r = 1.0f / sqrtf(s.y / (float)rank + eps);
     if (cache == nullptr) return;
-    const int p = positions[t];
-    const int* pages = page_table + (int64_t)slots[token_seq[t]] * max_pages;
-    const int page = CPM_PAGE(pages, p / kPageTokens, max_pages);
     T* dst = cache + page_row_offset(page, 0, p % kPageTokens, 1, rank + rot_dim);
     for (int c = threadIdx.x; c < rank; c += blockDim.x) dst[c] = from_f32<T>(row[c] * r * wkv[c]);
     row += rank;
@@ -58,8 +62,8 @@ __global__ void latent_norm_store_kernel(const float* __restrict__ proj, int64_t
     const int half = rot_dim >> 1;
     for (int i = threadIdx.x; i < half; i += blockDim.x) {
         const int a = adjacent ? 2 * i : i, b = adjacent ? 2 * i + 1 : i + half;
-        float sn = 0.f, cs = 1.f;
-        if (inv_freq != nullptr) sincosf((float)p * inv_freq[i], &sn, &cs);
+        float sn = sn0, cs = cs0;
+        if (i != (int)threadIdx.x && inv_freq != nullptr) sincosf((float)p * inv_freq[i], &sn, &cs);
         sn *= magnitude;
         cs *= magnitude;
         const float u = row[a], v = row[b];
@@ -146,19 +150,28 @@ __global__ void latent_prepare_kernel(const float* __restrict__ proj, int64_t st
                                       const int* __restrict__ page_table, int max_pages, int n_heads, int dim, int rank, int rot_dim,
                                       const float* __restrict__ inv_freq, float magnitude, int adjacent, float eps) {
     extern __shared__ float lp_smem[];                                   // [half][2] cosine, sine
-    __shared__ float scratch[33];
+    __shared__ float scratch[kRowMaxWarps];
     pdl_launch_dependents();
-    pdl_wait();
+    // (before the wait: see latent_norm_store_kernel)
     const int t = blockIdx.x, half = rot_dim >> 1, dh = dim + rot_dim;
     const int p = positions[t];
+    if (cache != nullptr) prefetch_l2(wkv, (int64_t)rank * 4);
+    int page = 0;
+    if (cache != nullptr) page = CPM_PAGE(page_table + (int64_t)slots[token_seq[t]] * max_pages, p / kPageTokens, max_pages);
     float2* cs = reinterpret_cast<float2*>(lp_smem);
     for (int i = threadIdx.x; i < half; i += blockDim.x) {
         float sn, cn;
         sincosf((float)p * inv_freq[i], &sn, &cn);
         cs[i] = make_float2(cn * magnitude, sn * magnitude);
     }
+    pdl_wait();
     __syncthreads();
     const float* row = proj + (int64_t)t * stride;
+    float s = 0.f;
+    if (cache != nullptr) {
+        const float* lat = row + (int64_t)n_heads * dh;
+        for (int c = threadIdx.x; c < rank; c += blockDim.x) s = fmaf(lat[c], lat[c], s);
+    }
     T* qrow = q + (int64_t)t * n_heads * dh;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n_warps = blockDim.x >> 5;
     const bool vec = ((dim | rot_dim) & 3) == 0 && (stride & 3) == 0;
@@ -176,11 +189,7 @@ __global__ void latent_prepare_kernel(const float* __restrict__ proj, int64_t st
     }
     if (cache == nullptr) return;
     row += (int64_t)n_heads * dh;
-    float s = 0.f;
-    for (int c = threadIdx.x; c < rank; c += blockDim.x) s = fmaf(row[c], row[c], s);
-    const float r = 1.0f / sqrtf(block_sum(s, scratch) / (float)rank + eps);
-    const int* pages = page_table + (int64_t)slots[token_seq[t]] * max_pages;
-    const int page = CPM_PAGE(pages, p / kPageTokens, max_pages);
+    const float r = 1.0f / sqrtf(row_sum(s, scratch) / (float)rank + eps);
     T* dst = cache + page_row_offset(page, 0, p % kPageTokens, 1, rank + rot_dim);
     for (int c = threadIdx.x; c < rank; c += blockDim.x) dst[c] = from_f32<T>(row[c] * r * wkv[c]);
     for (int i = threadIdx.x; i < half; i += blockDim.x) {

@@ -235,10 +235,14 @@ linear_recurrence_step_kernel(const float* __restrict__ q, const float* __restri
     const int h = blockIdx.y, seq = blockIdx.z, g = h / (heads / qk_heads), col = blockIdx.x * 32 + 4 * quad;
     const bool real = col < dv;                                // dv is a multiple of 4
     pdl_launch_dependents();
-    pdl_wait();
-    const int t = cu_q[seq];
+    const int t = cu_q[seq];                                   // written before this step's kernels began
     const bool fresh = positions[t] == 0;
     float* st = state + (((int64_t)slots[seq] * heads + h) * d) * dv + col;
+    if (real && !fresh)                                        // the state's way into L2 (an earlier step left it)
+#pragma unroll
+        for (int i = 0; i < PER; ++i)
+            if (r0 + 32 * i < d) asm volatile("prefetch.global.L2 [%0];" :: "l"(st + (int64_t)(r0 + 32 * i) * dv));
+    pdl_wait();
     float4 S[PER];
     float ck[PER], cq[PER], a[PER];
 #pragma unroll

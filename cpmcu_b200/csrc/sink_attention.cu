@@ -166,20 +166,25 @@ __global__ void qk_norm_prepare_store_kernel(const float* __restrict__ proj, int
     float* cosines = ks + ((k_cols + 3) & ~3);
     float* sines = cosines + half;
     pdl_launch_dependents();
-    pdl_wait();
+    // what needs the position alone, and the weights' way into L2, comes before the wait for the projections (with it behind: 7.7 us a launch
+    // for 4 tokens of 16 + 4 heads of 128, now 7.3)
     const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n_warps = blockDim.x >> 5;
     const int pos = positions[t];
+    prefetch_l2(q_norm, (int64_t)q_cols * 4);
+    if (has_kv) prefetch_l2(k_norm, (int64_t)k_cols * 4);
+    for (int f = threadIdx.x; f < half; f += blockDim.x) sincosf((float)pos * inv_freq[f], sines + f, cosines + f);
+    int page = 0;
+    if (has_kv) page = CPM_PAGE(page_table + (int64_t)slots[token_seq[t]] * max_pages, pos / kPageTokens, max_pages);
+    pdl_wait();
     const float* row = proj + (int64_t)t * stride;
     float2 ss;
     ss.x = row_into_smem(qs, row, q_bias, q_cols);
     ss.y = row_into_smem(ks, row + q_cols, k_bias, k_cols);
-    for (int f = threadIdx.x; f < half; f += blockDim.x) sincosf((float)pos * inv_freq[f], sines + f, cosines + f);
     ss.x = warp_sum(ss.x);
     ss.y = warp_sum(ss.y);
     if (lane == 0) warp_sums[warp] = ss;
     int64_t k_base = 0;
     if (has_kv) {
-        const int page = CPM_PAGE(page_table + (int64_t)slots[token_seq[t]] * max_pages, pos / kPageTokens, max_pages);
         k_base = page_row_offset(page, 0, pos % kPageTokens, n_kv, d);
         T* v_dst = v_cache + value_offset(page, 0, 0, pos % kPageTokens, n_kv, dv);
         const float* src = row + cols;
