@@ -886,4 +886,205 @@ CPM_API int cpm_latent_attention_mma(const float* q, const void* cache, void* ou
                                  n_heads, rank, scale, n_splits, stream);
 }
 
+// ---------------------------------------------------------------------------
+// Prompt tokens: a block takes two neighbouring tokens of a sequence (the query tiles of 64 rows list them) and up to 16 heads, so that
+// a page of 64 latents, brought once into shared memory, serves 32 rows.  Warps 0-3 are the first token's, 4-7 the second's.  A
+// warp forms the scores of 16 of the page's keys over the whole rank (no partial scores to trade: the queries lie in shared memory
+// too), the four warps of a token trade their rows' maxima, leave their weights in shared memory as the next product's operand
+// and then split the latent columns for the weighted sum.  Two blocks an SM: one's page arrives while the other's is worked on.
+// Bound by the operands' way out of shared memory.  The kernel above, one token a block and the rank split over its warps, spent
+// 1,245 instructions a warp and tile on 64 tensor-core ones: 576 us for 2,048 tokens of two prompts, 16 heads, rank 512; this one 317.
+constexpr int kPromptKeys = 64, kPromptTokens = 2;
+
+template <int NT>
+__global__ void __launch_bounds__(256, NT <= 16 ? 2 : 1)
+latent_prompt_mma_kernel(const float* __restrict__ q, const bf16* __restrict__ cache, void* __restrict__ out_any, int out_bf16,
+                         const int* __restrict__ positions, const int* __restrict__ slots, const int* __restrict__ page_table, int max_pages,
+                         const int* __restrict__ tile_seq, const int* __restrict__ tile_row, const int* __restrict__ cu_q, int n_tiles, int window,
+                         int n_heads, int rank, float scale2) {
+    extern __shared__ __align__(16) unsigned char lp_raw[];
+    const int pitch = rank + 8;                                          // bf16 elements per row in shared memory
+    bf16* Ks = reinterpret_cast<bf16*>(lp_raw);                          // [64][pitch]
+    bf16* Qs = Ks + kPromptKeys * pitch;                                 // [2][16][pitch]
+    constexpr int kPPitch = kPromptKeys + 8;
+    __shared__ __align__(16) bf16 Ps[kPromptTokens][16][kPPitch];
+    __shared__ float row_max[kPromptTokens][4][16], row_sums[kPromptTokens][4][16];
+    pdl_launch_dependents();
+    constexpr int kPairs = 64 / kPromptTokens;                           // pairs of a query tile
+    const int tile_no = n_tiles - 1 - blockIdx.x / kPairs;               // later tiles of a sequence have more keys: they go first
+    const int seq = tile_seq[tile_no], row0 = tile_row[tile_no] + kPromptTokens * (blockIdx.x % kPairs);
+    const int q_begin = cu_q[seq], q_len = cu_q[seq + 1] - q_begin;
+    if (row0 >= q_len) return;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tg = lane & 3;
+    const int rt = warp >> 2, cw = warp & 3, h0 = blockIdx.y * kMmaRows;
+    const int t = q_begin + row0 + rt;
+    const bool live = row0 + rt < q_len;                                 // an odd portion's last pair has one token
+    const int first_p = positions[q_begin + row0], last_p = first_p + (row0 + 1 < q_len ? 1 : 0);
+    const int p = live ? first_p + rt : -1;
+    const int lo = window > 0 ? max(0, p - window + 1) : 0;
+    const int page0 = (window > 0 ? max(0, first_p - window + 1) : 0) / kPageTokens, page1 = last_p / kPageTokens;
+    const int* pages = page_table + (int64_t)slots[seq] * max_pages;
+    pdl_wait();
+    // the queries as bf16, rows past the last head or token zeros
+    for (int i = threadIdx.x; i < kPromptTokens * 16 * (rank / 4); i += 256) {
+        const int row = i / (rank / 4), c = 4 * (i % (rank / 4)), tok = row >> 4, h = h0 + (row & 15);
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (h < n_heads && row0 + tok < q_len) v = *reinterpret_cast<const float4*>(q + ((int64_t)(q_begin + row0 + tok) * n_heads + h) * rank + c);
+        store4(Qs + row * pitch + c, v);
+    }
+    const int vec_per_row = rank / 8;
+    auto ldsm = [](uint32_t (&r)[4], uint32_t addr) {
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+    };
+    auto ldsm_t = [](uint32_t (&r)[4], uint32_t addr) {
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+    };
+    auto token_barrier = [&]() { asm volatile("bar.sync %0, 128;" :: "r"(1 + rt) : "memory"); };
+    const uint32_t q_addr = (uint32_t)__cvta_generic_to_shared(Qs + (rt * 16 + (lane & 15)) * pitch + 8 * (lane >> 4));
+    const uint32_t k_addr = (uint32_t)__cvta_generic_to_shared(Ks + (16 * cw + (lane >> 4) * 8 + (lane & 7)) * pitch + 8 * ((lane >> 3) & 1));
+    const uint32_t p_addr = (uint32_t)__cvta_generic_to_shared(&Ps[rt][lane & 15][8 * (lane >> 4)]);
+    const uint32_t v_addr = (uint32_t)__cvta_generic_to_shared(Ks + lane * pitch + 8 * cw);
+    const uint32_t half_page = (uint32_t)(32 * pitch * sizeof(bf16));
+    float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};             // rows g and g + 8; l: this warp's keys only
+    float acc[NT][4];
+#pragma unroll
+    for (int i = 0; i < NT; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+    for (int page = page0; page <= page1; ++page) {
+        const bf16* src = cache + page_row_offset(CPM_PAGE(pages, page, max_pages), 0, 0, 1, rank);
+        for (int r = warp; r < kPromptKeys; r += 8)
+            for (int v = lane; v < vec_per_row; v += 32) cp_async_16(Ks + r * pitch + 8 * v, src + (int64_t)r * rank + 8 * v, true);
+        cp_async_commit();
+        cp_async_wait<0>();
+        __syncthreads();                                                 // the page (and the queries) are there
+        float c[2][4] = {};
+        const int k_steps = rank / 16;
+#pragma unroll 4
+        for (int ks = 0; ks < k_steps; ++ks) {
+            uint32_t a[4], b[4];
+            ldsm(a, q_addr + 32 * ks);
+            ldsm(b, k_addr + 32 * ks);
+            mma_bf16_16816(c[0], a, b[0], b[1]);
+            mma_bf16_16816(c[1], a, b[2], b[3]);
+        }
+        // c[n][e]: row g (e < 2) or g + 8, key 16 cw + 8 n + 2 tg + (e & 1) of the page
+        const int key0 = page * kPageTokens + 16 * cw + 2 * tg;
+        float mx[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int key = key0 + 8 * n + (e & 1);
+                const float x = key <= p && key >= lo ? c[n][e] * scale2 : -INFINITY;
+                c[n][e] = x;
+                mx[e >> 1] = fmaxf(mx[e >> 1], x);
+            }
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 1));
+            mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 2));
+            if (tg == 0) row_max[rt][cw][g + 8 * r] = mx[r];
+        }
+        token_barrier();
+        float corr[2], use[2];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const int row = g + 8 * r;
+            const float mn = fmaxf(fmaxf(m[r], fmaxf(row_max[rt][0][row], row_max[rt][1][row])), fmaxf(row_max[rt][2][row], row_max[rt][3][row]));
+            use[r] = mn == -INFINITY ? 0.f : mn;
+            corr[r] = fast_exp2(m[r] - use[r]);                          // 0 at the first visible key
+            m[r] = mn;
+            l[r] *= corr[r];
+        }
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                c[n][e] = fast_exp2(c[n][e] - use[e >> 1]);
+                l[e >> 1] += c[n][e];
+            }
+            *reinterpret_cast<uint32_t*>(&Ps[rt][g][16 * cw + 8 * n + 2 * tg]) = pack_bf16(c[n][0], c[n][1]);
+            *reinterpret_cast<uint32_t*>(&Ps[rt][g + 8][16 * cw + 8 * n + 2 * tg]) = pack_bf16(c[n][2], c[n][3]);
+        }
+        if (__any_sync(0xffffffffu, corr[0] != 1.f || corr[1] != 1.f)) {
+#pragma unroll
+            for (int i = 0; i < NT; ++i) {
+                acc[i][0] *= corr[0]; acc[i][1] *= corr[0];
+                acc[i][2] *= corr[1]; acc[i][3] *= corr[1];
+            }
+        }
+        token_barrier();                                                 // the token's weights are there
+        uint32_t pa[4][4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) ldsm(pa[k], p_addr + 32 * k);
+#pragma unroll
+        for (int i = 0; i < NT; ++i) {
+            if (8 * (cw + 4 * i) < rank) {
+                uint32_t b[4];
+                ldsm_t(b, v_addr + (uint32_t)(32 * i * sizeof(bf16)));
+                mma_bf16_16816(acc[i], pa[0], b[0], b[1]);
+                mma_bf16_16816(acc[i], pa[1], b[2], b[3]);
+                ldsm_t(b, v_addr + half_page + (uint32_t)(32 * i * sizeof(bf16)));
+                mma_bf16_16816(acc[i], pa[2], b[0], b[1]);
+                mma_bf16_16816(acc[i], pa[3], b[2], b[3]);
+            }
+        }
+        __syncthreads();                                                 // the page has been used
+    }
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        l[r] += __shfl_xor_sync(0xffffffffu, l[r], 1);
+        l[r] += __shfl_xor_sync(0xffffffffu, l[r], 2);
+        if (tg == 0) row_sums[rt][cw][g + 8 * r] = l[r];
+    }
+    token_barrier();
+    if (!live) return;
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        const int row = g + 8 * r, h = h0 + row;
+        if (h >= n_heads) continue;
+        const float sum = (row_sums[rt][0][row] + row_sums[rt][1][row]) + (row_sums[rt][2][row] + row_sums[rt][3][row]);
+        const float inv = sum > 0.f ? 1.f / sum : 0.f;
+        const int64_t o = ((int64_t)t * n_heads + h) * rank;
+#pragma unroll
+        for (int i = 0; i < NT; ++i) {
+            const int col = 8 * (cw + 4 * i) + 2 * tg;
+            if (col >= rank) continue;
+            if (out_bf16) *reinterpret_cast<uint32_t*>(static_cast<bf16*>(out_any) + o + col) = pack_bf16(acc[i][2 * r] * inv, acc[i][2 * r + 1] * inv);
+            else *reinterpret_cast<float2*>(static_cast<float*>(out_any) + o + col) = make_float2(acc[i][2 * r] * inv, acc[i][2 * r + 1] * inv);
+        }
+    }
+}
+
+template <int NT>
+static int launch_latent_prompt(const float* q, const void* cache, void* out, int out_bf16, const int* positions, const int* slots,
+                                const int* page_table, int max_pages, const int* tile_seq, const int* tile_row, const int* cu_q, int n_tiles,
+                                int window, int n_heads, int rank, float scale, cudaStream_t stream) {
+    static bool done[kMaxDevices];
+    const size_t smem = (size_t)(kPromptKeys + 16 * kPromptTokens) * (rank + 8) * sizeof(bf16);
+    auto kern = latent_prompt_mma_kernel<NT>;
+    if (int e = ensure_dynamic_smem(kern, (kPromptKeys + 16 * kPromptTokens) * (32 * NT + 8) * (int)sizeof(bf16), done)) return e;
+    const dim3 grid(n_tiles * (64 / kPromptTokens), (n_heads + kMmaRows - 1) / kMmaRows);
+    cpm_launch(kLaunchAttention, kern, grid, 256, smem, stream, q, (const bf16*)cache, out, out_bf16, positions, slots, page_table, max_pages,
+               tile_seq, tile_row, cu_q, n_tiles, window, n_heads, rank, scale * 1.4426950408889634f);
+    return launch_status();
+}
+
+// The same attention for the tokens of prompts, packed by sequence: cu_q, slots by sequence; tile_seq, tile_row: tiles of 64 rows that cover
+// every sequence's tokens (tiles past a sequence's end hold none); a sequence's tokens have consecutive positions.
+CPM_API int cpm_latent_attention_prompt(const float* q, const void* cache, void* out, int out_bf16, const int* positions, const int* slots,
+                                        const int* page_table, int max_pages, const int* tile_seq, const int* tile_row, const int* cu_q,
+                                        int n_tiles, int window, int n_heads, int rank, float scale, cudaStream_t stream) {
+    if (n_tiles <= 0) return CPM_OK;
+    if (n_heads <= 0 || rank <= 0 || rank > 576 || rank % 16 || window < 0 || n_tiles > (1 << 24) || (n_heads + kMmaRows - 1) / kMmaRows > 65535 ||
+        (((uintptr_t)q | (uintptr_t)cache) & 15))
+        return CPM_BAD_ARGUMENT;
+#define CPM_LATENT_PROMPT(N) return launch_latent_prompt<N>(q, cache, out, out_bf16, positions, slots, page_table, max_pages, tile_seq, tile_row, cu_q, \
+                                                            n_tiles, window, n_heads, rank, scale, stream)
+    if (rank <= 128) CPM_LATENT_PROMPT(4);
+    if (rank <= 256) CPM_LATENT_PROMPT(8);
+    if (rank <= 512) CPM_LATENT_PROMPT(16);
+    CPM_LATENT_PROMPT(18);
+#undef CPM_LATENT_PROMPT
+}
+
 CPM_BOUNDS_TU(latent_attention)

@@ -474,6 +474,12 @@ class Ops:
         keys = min(window, ctx.max_kv_len) if window else ctx.max_kv_len      # in a recorded step an upper bound
         return max(1, min(self.LATENT_MAX_SPLITS, 3 * self.sm_count // blocks, ((keys + 31) // 32) // 2))
 
+    LATENT_PROMPT_MIN_TOKENS = 96      # fewer leave most SMs idle: the kernel of one token a block shares their keys out instead
+
+    def latent_prompt_ok(self, ctx, n_tokens: int) -> bool:
+        """Whether a step's tokens go by pairs of neighbours (the kernel for prompts) instead of one by one."""
+        return not ctx.is_decode and ctx.q_tiles is not None and n_tokens >= self.LATENT_PROMPT_MIN_TOKENS
+
     def latent_attention_on_tensor_cores(self, rank: int) -> bool:
         return self.code == BF16 and rank % 16 == 0 and rank <= 576
 
@@ -492,6 +498,13 @@ class Ops:
         if tensor_cores and not mma_ok:
             raise ValueError("the tensor-core latent attention takes bf16 latents of a rank that is a multiple of 16 up to 576")
         if mma_ok and tensor_cores is not False:
+            if n_splits is None and self.latent_prompt_ok(ctx, n):
+                tile_seq, tile_row, n_tiles = ctx.q_tiles
+                check(self.lib.cpm_latent_attention_prompt(_ptr(q_lat), _ptr(lane.k), _ptr(out), 1 if narrow else 0, _ptr(ctx.positions),
+                                                           _ptr(ctx.slot_dev), _ptr(lane.page_table), lane.page_table.shape[1],
+                                                           _ptr(tile_seq), _ptr(tile_row), _ptr(ctx.cu_q), int(n_tiles), int(window), H, R,
+                                                           float(scale), self._stream()), f"latent attention of prompts (rank {R}, {H} heads)")
+                return out
             if n_splits is None:
                 n_splits = self.latent_attention_splits(ctx, n, H, int(window))
             scratch = None

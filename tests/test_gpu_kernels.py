@@ -1011,3 +1011,36 @@ def test_recurrence_of_one_token_a_sequence(H, G, d, dv, delta, vector):
             S = S + kk[:, None] * u[None]
             want[i, h], after[slots[i], h] = 0.7 * (S.T @ qq), S
     assert _err(got, want) < KTOL["float32"] and _err(st, after) < KTOL["float32"]
+
+
+@pytest.mark.parametrize("rank,heads,window", [(48, 3, 37), (128, 16, 0), (256, 20, 300), (512, 16, 64), (576, 33, 0)])
+def test_latent_attention_of_prompts(rank, heads, window):
+    """Pairs of neighbouring tokens against the fp32 kernel: odd portions, one token, portions that begin inside a page and deep in a
+    history, windows that end inside a page, more heads than a tile's rows, tiles of an empty sequence.  bf16 queries and weights:
+    within 2e-2 of the largest value, as for the kernel of single tokens."""
+    from types import SimpleNamespace
+
+    from cpmcu_b200.cache import Cache
+    from cpmcu_b200.parts.base import CacheNeeds
+
+    ops = _ops("bfloat16")
+    g = torch.Generator().manual_seed(rank + heads)
+    q_lens, starts = [71, 1, 130, 6], [0, 0, 191, 700]
+    cache = Cache([CacheNeeds(kv_heads=1, head_dim=rank, values=False)], max_tokens=64 * 30, dtype=torch.bfloat16, device="cuda:0")
+    slots = cache.open_sequences(4)
+    for s, n, first in zip(slots, q_lens, starts):
+        cache.reserve(s, first + n)
+    cache.sync()
+    lane = cache.lane(0)
+    lane.k.copy_((torch.randn(lane.k.shape, generator=g) * 0.7).bfloat16())
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32).cuda()
+    tiles = [(i, r) for i, n in enumerate(q_lens) for r in range(0, n, 64)] + [(4, 0), (4, 0)]
+    cu = [0, 71, 72, 202, 208, 208]
+    ctx = SimpleNamespace(positions=torch.cat([torch.arange(f, f + n) for f, n in zip(starts, q_lens)]).int().cuda(), cu_q=i32(cu),
+                          token_seq=torch.cat([torch.full((n,), i) for i, n in enumerate(q_lens)]).int().cuda(), slot_dev=i32(slots + [slots[0]]),
+                          n_seqs=5, is_decode=False, q_tiles=(i32([a for a, _ in tiles]), i32([b for _, b in tiles]), len(tiles)), max_kv_len=706)
+    q = torch.randn(208, heads, rank, generator=g).cuda()
+    assert ops.latent_prompt_ok(ctx, 208)
+    want = ops.latent_attention(ctx, q, lane, 0.11, window, tensor_cores=False)
+    assert _err(ops.latent_attention(ctx, q, lane, 0.11, window), want) < 2e-2
+    assert _err(ops.latent_attention(ctx, q, lane, 0.11, window, out_compute_dtype=True), want) < 2e-2
