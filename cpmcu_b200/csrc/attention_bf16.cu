@@ -834,7 +834,7 @@ listed_attention_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_c
                         const int* __restrict__ block_list, int list_cap, int n_heads, int n_kv, int m_tiles,
                         float scale_log2, float* __restrict__ part_o, float* __restrict__ part_ml, int n_splits) {
     // With n_splits > 1 (few tokens: decode) the listed blocks of a token are shared out over
-    // gridDim.z blocks of threads, which write unnormalised partial results for combine_splits_kernel.
+    // gridDim.z blocks of threads, which write unnormalised partial results for combine_shares_kernel.
     using S = DecodeSmem<D>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ float sm_m[DecodeSmem<D>::kWarps][16], sm_l[DecodeSmem<D>::kWarps][16];
