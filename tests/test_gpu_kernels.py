@@ -1044,3 +1044,16 @@ def test_latent_attention_of_prompts(rank, heads, window):
     want = ops.latent_attention(ctx, q, lane, 0.11, window, tensor_cores=False)
     assert _err(ops.latent_attention(ctx, q, lane, 0.11, window), want) < 2e-2
     assert _err(ops.latent_attention(ctx, q, lane, 0.11, window, out_compute_dtype=True), want) < 2e-2
+
+
+@pytest.mark.parametrize("M", [1, 8, 9, 16])
+@pytest.mark.parametrize("N,K", [(17, 2080), (1000, 4096), (1184, 2080), (1185, 2080), (64, 2048)])
+def test_products_of_few_rows_on_few_blocks(M, N, K):
+    """The widest block's sizes (up to 74 blocks of 16 weight rows, K over 2,048), one block more and a shorter row: bf16 and fp32 results against 64
+    bits; fp32 sums of K products in another order, bf16 one rounding."""
+    ops = _ops("bfloat16")
+    g = torch.Generator().manual_seed(M + N + K)
+    x, w = torch.randn(M, K, generator=g).bfloat16().cuda(), (torch.randn(N, K, generator=g) * K ** -0.5).bfloat16().cuda()
+    want = x.double() @ w.double().T
+    assert _err(ops.linear(x, w, out_f32=True), want) < 1e-5
+    assert _err(ops.linear(x, w), want) < 2.0 ** -8
