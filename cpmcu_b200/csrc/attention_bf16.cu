@@ -353,7 +353,7 @@ struct DecodeShare { int seq, index, count, pages; };      // share ``index`` of
 // Where that is not worth its search, a sequence's pages are cut into n_splits shares, less where they do not fill them: at head
 // size 128 with one block an SM and several shares a sequence, the search (about a microsecond where the block cannot start before
 // the kernel ahead ends) ate what it gave (8 sequences of 513 to 4085 tokens: 28.3 ms for eight steps of the 8B sizes against 27.3).
-__host__ __device__ constexpr bool decode_by_size(int d, int n_splits) { return n_splits > 1 && (d == 64 || n_splits <= 2); }
+__host__ __device__ constexpr bool decode_by_size(int d, int n_splits) { return n_splits > 1 && d == 64; }
 __device__ __forceinline__ DecodeShare equal_decode_share(const int* __restrict__ kv_len, int seq, int index, int n_splits) {
     const int pages = max(1, (__ldg(kv_len + seq) + kPageTokens - 1) / kPageTokens), per = (pages + n_splits - 1) / n_splits;
     DecodeShare s{seq, index, (pages + per - 1) / per, per};

@@ -803,13 +803,14 @@ class Ops:
     def decode_splits(self, n_seqs: int, n_heads: int, n_kv: int, d: int = 0) -> int:
         """How many shares a sequence's pages are cut into, on average (the decode attention gives long sequences more): the
         kernel holds one block per SM (its page buffers fill the shared memory; with ``d`` the number the decode kernel
-        holds at that head size), so aim at one wave of blocks, but where one wave is about one share a sequence at
-        two, so that there are shares to give to the long ones."""
+        holds at that head size), so aim at one wave of blocks, but where an SM holds several blocks and one wave is
+        about one share a sequence at two, so that there are shares to give to the long ones (with one block an SM, 64 equal
+        sequences of the 8B sizes lost 7 % to the second share)."""
         m_tiles = (n_heads // n_kv + 15) // 16
         units = max(1, n_seqs * n_kv * m_tiles)
         room = self.sm_count * (self.lib.cpm_decode_attention_blocks_per_sm(d) if d else 1)
         wave = max(1, min(self.MAX_DECODE_SPLITS, room // units))
-        return min(2, 2 * room // units) if d and wave == 1 and 2 * room >= 2 * units else wave
+        return min(2, 2 * room // units) if room > self.sm_count and wave == 1 and room >= units else wave
 
     def _arrivals(self, rows: int, n_heads: int, n_kv: int, d: int) -> Optional[torch.Tensor]:
         """Counters with which the decode attention's blocks find out which of them is the last of its sequence and adds up
