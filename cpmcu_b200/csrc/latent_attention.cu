@@ -21,6 +21,7 @@
 //
 // A latent page is [token_in_page][rank] (the key page layout with one key-value head).
 #include "rownorm.cuh"
+#include <type_traits>
 
 // ---------------------------------------------------------------------------
 // proj rows (fp32, ``stride`` floats) begin [q_rank | rank | rot_dim]: the first two parts are RMS-normed; the third (rot_dim
@@ -892,6 +893,8 @@ CPM_API int cpm_latent_attention_mma(const float* q, const void* cache, void* ou
 // warp forms the scores of 16 of the page's keys over the whole rank (no partial scores to trade: the queries lie in shared memory
 // too), the four warps of a token trade their rows' maxima, leave their weights in shared memory as the next product's operand
 // and then split the latent columns for the weighted sum.  Two blocks an SM: one's page arrives while the other's is worked on.
+// A latent that a token does not see never meets a weight of zero (0 * NaN is NaN): rows that neither token of a pair sees come as zeros, and
+// the row that only the other one sees (the second token itself; behind a window, the first one's first key) is cleared from the operand.
 // Bound by the operands' way out of shared memory.  The kernel above, one token a block and the rank split over its warps, spent
 // 1,245 instructions a warp and tile on 64 tensor-core ones: 576 us for 2,048 tokens of two prompts, 16 heads, rank 512; this one 317.
 constexpr int kPromptKeys = 64, kPromptTokens = 2;
@@ -922,7 +925,10 @@ latent_prompt_mma_kernel(const float* __restrict__ q, const bf16* __restrict__ c
     const int first_p = positions[q_begin + row0], last_p = first_p + (row0 + 1 < q_len ? 1 : 0);
     const int p = live ? first_p + rt : -1;
     const int lo = window > 0 ? max(0, p - window + 1) : 0;
-    const int page0 = (window > 0 ? max(0, first_p - window + 1) : 0) / kPageTokens, page1 = last_p / kPageTokens;
+    const int first_key = window > 0 ? max(0, first_p - window + 1) : 0;
+    const int page0 = first_key / kPageTokens, page1 = last_p / kPageTokens;
+    // the key between first_key and last_p that this warp's token does not see (at most one; -1: none)
+    const int hidden_key = rt == 0 ? (last_p > first_p ? last_p : -1) : (live && lo > first_key ? first_key : -1);
     const int* pages = page_table + (int64_t)slots[seq] * max_pages;
     pdl_wait();
     // the queries as bf16, rows past the last head or token zeros
@@ -952,7 +958,10 @@ latent_prompt_mma_kernel(const float* __restrict__ q, const bf16* __restrict__ c
     for (int page = page0; page <= page1; ++page) {
         const bf16* src = cache + page_row_offset(CPM_PAGE(pages, page, max_pages), 0, 0, 1, rank);
         for (int r = warp; r < kPromptKeys; r += 8)
-            for (int v = lane; v < vec_per_row; v += 32) cp_async_16(Ks + r * pitch + 8 * v, src + (int64_t)r * rank + 8 * v, true);
+            for (int v = lane; v < vec_per_row; v += 32) {
+                const int key = page * kPageTokens + r;
+                cp_async_16(Ks + r * pitch + 8 * v, src + (int64_t)r * rank + 8 * v, key >= first_key && key <= last_p);
+            }
         cp_async_commit();
         cp_async_wait<0>();
         __syncthreads();                                                 // the page (and the queries) are there
@@ -1016,18 +1025,29 @@ latent_prompt_mma_kernel(const float* __restrict__ q, const bf16* __restrict__ c
         uint32_t pa[4][4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) ldsm(pa[k], p_addr + 32 * k);
+        // a register of the values holds keys 8 j + 2 tg and the next: the half of the hidden key, if it lies in this page, is masked
+        const int hidden = hidden_key - page * kPageTokens;
+        uint32_t keep[8];
 #pragma unroll
-        for (int i = 0; i < NT; ++i) {
-            if (8 * (cw + 4 * i) < rank) {
-                uint32_t b[4];
-                ldsm_t(b, v_addr + (uint32_t)(32 * i * sizeof(bf16)));
-                mma_bf16_16816(acc[i], pa[0], b[0], b[1]);
-                mma_bf16_16816(acc[i], pa[1], b[2], b[3]);
-                ldsm_t(b, v_addr + half_page + (uint32_t)(32 * i * sizeof(bf16)));
-                mma_bf16_16816(acc[i], pa[2], b[0], b[1]);
-                mma_bf16_16816(acc[i], pa[3], b[2], b[3]);
+        for (int j = 0; j < 8; ++j) keep[j] = hidden >> 1 != 4 * j + tg ? 0xffffffffu : hidden & 1 ? 0x0000ffffu : 0xffff0000u;
+        auto add_values = [&](auto masked) {
+#pragma unroll
+            for (int i = 0; i < NT; ++i) {
+                if (8 * (cw + 4 * i) < rank) {
+                    uint32_t b[2][4];
+                    ldsm_t(b[0], v_addr + (uint32_t)(32 * i * sizeof(bf16)));
+                    ldsm_t(b[1], v_addr + half_page + (uint32_t)(32 * i * sizeof(bf16)));
+                    if (decltype(masked)::value)
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) b[j >> 2][j & 3] &= keep[j];
+                    mma_bf16_16816(acc[i], pa[0], b[0][0], b[0][1]);
+                    mma_bf16_16816(acc[i], pa[1], b[0][2], b[0][3]);
+                    mma_bf16_16816(acc[i], pa[2], b[1][0], b[1][1]);
+                    mma_bf16_16816(acc[i], pa[3], b[1][2], b[1][3]);
+                }
             }
-        }
+        };
+        if (hidden >= 0 && hidden < kPromptKeys) add_values(std::true_type{}); else add_values(std::false_type{});
         __syncthreads();                                                 // the page has been used
     }
 #pragma unroll

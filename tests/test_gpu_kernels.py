@@ -1046,6 +1046,53 @@ def test_latent_attention_of_prompts(rank, heads, window):
     assert _err(ops.latent_attention(ctx, q, lane, 0.11, window, out_compute_dtype=True), want) < 2e-2
 
 
+@pytest.mark.parametrize("rank,heads,window", [(48, 3, 37), (128, 16, 0), (256, 20, 300), (512, 16, 64), (576, 33, 1)])
+def test_latent_attention_of_prompts_meets_only_the_keys_it_sees(rank, heads, window):
+    """Every cached row that belongs to no token is not a number (what an earlier sequence may leave in a page): the results are
+    finite.  Then one token's own latent is: exactly the queries that see it change, whether it is the first or the second
+    of a pair, and in windows that begin with it or behind it."""
+    from types import SimpleNamespace
+
+    from cpmcu_b200.cache import Cache
+    from cpmcu_b200.parts.base import CacheNeeds
+
+    ops = _ops("bfloat16")
+    g = torch.Generator().manual_seed(rank + heads)
+    q_lens, starts = [71, 1, 130, 6], [0, 0, 191, 700]
+    cache = Cache([CacheNeeds(kv_heads=1, head_dim=rank, values=False)], max_tokens=64 * 30, dtype=torch.bfloat16, device="cuda:0")
+    slots = cache.open_sequences(4)
+    for s, n, first in zip(slots, q_lens, starts):
+        cache.reserve(s, first + n)
+    cache.sync()
+    lane = cache.lane(0)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32).cuda()
+    flat = lane.k.view(-1, rank)
+    row_of = lambda i, key: int(lane.page_table[slots[i], key // 64]) * 64 + key % 64
+    flat.fill_(float("nan"))
+    for i, (n, first) in enumerate(zip(q_lens, starts)):
+        rows = torch.tensor([row_of(i, key) for key in range(first + n)]).cuda()
+        flat[rows] = (torch.randn(first + n, rank, generator=g) * 0.7).bfloat16().cuda()
+    tiles = [(i, r) for i, n in enumerate(q_lens) for r in range(0, n, 64)]
+    ctx = SimpleNamespace(positions=torch.cat([torch.arange(f, f + n) for f, n in zip(starts, q_lens)]).int().cuda(), cu_q=i32([0, 71, 72, 202, 208]),
+                          token_seq=torch.cat([torch.full((n,), i) for i, n in enumerate(q_lens)]).int().cuda(), slot_dev=i32(slots),
+                          n_seqs=4, is_decode=False, q_tiles=(i32([a for a, _ in tiles]), i32([b for _, b in tiles]), len(tiles)), max_kv_len=706)
+    q = torch.randn(208, heads, rank, generator=g).cuda()
+    assert ops.latent_prompt_ok(ctx, 208)
+    base = ops.latent_attention(ctx, q, lane, 0.11, window)
+    assert bool(base.isfinite().all())
+    for key in (191, 192, 250, 251, 255, 256, 319, 320):
+        row = row_of(2, key)
+        kept = flat[row].clone()
+        flat[row] = float("nan")
+        got = ops.latent_attention(ctx, q, lane, 0.11, window)
+        flat[row] = kept
+        sees = torch.zeros(208, dtype=torch.bool)
+        p = torch.arange(191, 321)
+        sees[72:202] = (p >= key) & ((p - key < window) if window else torch.ones(130, dtype=torch.bool))
+        sees = sees.cuda()
+        assert torch.equal(got[~sees], base[~sees]) and not bool(got[sees].isfinite().any()), key
+
+
 @pytest.mark.parametrize("M", [1, 8, 9, 16])
 @pytest.mark.parametrize("N,K", [(17, 2080), (1000, 4096), (1184, 2080), (1185, 2080), (64, 2048)])
 def test_products_of_few_rows_on_few_blocks(M, N, K):
