@@ -744,6 +744,8 @@ static int launch_decode(const void* q, const void* k_cache, const void* v_cache
     if (n_rows > 65535 || n_kv * m_tiles > 65535) return CPM_BAD_ARGUMENT;
     const int64_t shares = (int64_t)n_seqs * n_splits;
     if (shares > 0x7fffffff) return CPM_BAD_ARGUMENT;
+    // the block that adds up a sequence's shares has room for the weights of kMaxShares
+    if (arrivals != nullptr && n_splits > kMaxShares && !decode_by_size(D, n_splits)) return CPM_BAD_ARGUMENT;
     float* part_o = scratch;
     float* part_ml = scratch + shares * runs * n_kv * m_tiles * 16 * D;
     auto kern = decode_attention_kernel<D>;
@@ -761,7 +763,8 @@ static int launch_decode(const void* q, const void* k_cache, const void* v_cache
 }
 
 // q [n_seqs, heads, d] bf16, one token per sequence; out [n_seqs, heads, d] bf16.  arrivals: null, or n_seqs * n_kv * ceil(group / 16) (times
-// the runs) counters that are zero, are zero again when the kernel ends, and belong to no other kernel meanwhile.
+// the runs) counters that are zero, are zero again when the kernel ends, and belong to no other kernel meanwhile (at head sizes other than
+// 64 for up to 32 shares a sequence: without them the shares are added up by a kernel of its own, which takes any number).
 CPM_API int cpm_decode_attention_bf16(const void* q, const void* k_cache, const void* v_cache, void* out,
                                       const int* kv_len, const int* slots, const int* page_table, int max_pages,
                                       float* scratch, int n_seqs, int n_heads, int n_kv, int d, int n_splits,

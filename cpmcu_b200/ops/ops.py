@@ -812,14 +812,15 @@ class Ops:
         wave = max(1, min(self.MAX_DECODE_SPLITS, room // units))
         return min(2, 2 * room // units) if room > self.sm_count and wave == 1 and room >= units else wave
 
-    def _arrivals(self, rows: int, n_heads: int, n_kv: int, d: int) -> Optional[torch.Tensor]:
+    def _arrivals(self, rows: int, n_heads: int, n_kv: int, d: int, n_splits: int) -> Optional[torch.Tensor]:
         """Counters with which the decode attention's blocks find out which of them is the last of its sequence and adds up
         the shares, so that no kernel for that has to follow (it cost 3.4 us a layer at one sequence, 4.5 us at eight).
         Launches that share them must follow one another: they are given only where a workspace is attached, whose memory
         asks for the same; elsewhere, or with more rows than there are counters, the shares are added up by a kernel of its own.
         So they are at head sizes above 64, where a block's three warps take longer for 16 rows of the shares than that kernel
-        (8 sequences of the 8B sizes: 29.3 against 28.3 ms for eight steps)."""
-        if d > 64 or self.workspace is None or self.arrivals is None or rows * n_kv * ((n_heads // n_kv + 15) // 16) > self.arrivals.numel():
+        (8 sequences of the 8B sizes: 29.3 against 28.3 ms for eight steps).  And so are more shares a sequence than the last
+        block has room for the weights of (at head size 64 the kernel keeps to that by itself)."""
+        if d > 64 or (n_splits > 32 and d != 64) or self.workspace is None or self.arrivals is None or rows * n_kv * ((n_heads // n_kv + 15) // 16) > self.arrivals.numel():
             return None
         return self.arrivals
 
@@ -837,7 +838,7 @@ class Ops:
             n_splits = self.decode_splits(rows, n_heads, n_kv, d)
         floats = self.lib.cpm_decode_attention_scratch_floats(rows, n_heads, n_kv, d, n_splits)
         scratch = self.empty(floats, dtype=torch.float32)
-        arrivals = self._arrivals(rows, n_heads, n_kv, d)
+        arrivals = self._arrivals(rows, n_heads, n_kv, d, n_splits)
         if out is None:
             out = self.empty(rows, n_heads * d) if v_runs <= 1 else self.empty(v_runs, n, n_heads * d)
         if v_shift or v_runs > 1:
@@ -887,7 +888,7 @@ class Ops:
         floats = self.lib.cpm_decode_attention_scratch_floats(n, n_heads, n_kv, d, n_splits)
         scratch = self.empty(floats, dtype=torch.float32)
         out = self.empty(n, n_heads * d)
-        arrivals = self._arrivals(n, n_heads, n_kv, d)
+        arrivals = self._arrivals(n, n_heads, n_kv, d, n_splits)
         check(self.lib.cpm_decode_attention_rope_bf16(_ptr(qkv), _ptr(lane.k), _ptr(lane.v), _ptr(out), _ptr(kv_len),
                                                       _ptr(slots), _ptr(lane.page_table), lane.page_table.shape[1],
                                                       _ptr(scratch), n, n_heads, n_kv, d, n_splits, float(scale),

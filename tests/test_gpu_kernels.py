@@ -940,8 +940,11 @@ def test_head_project_of_few_tokens(K, N, n):
 @pytest.mark.parametrize("n_heads,n_kv,d", [(16, 2, 64), (4, 2, 128), (40, 2, 32), (3, 3, 96)])
 @pytest.mark.parametrize("lens", [[1], [3000], [64, 65, 1, 2111, 700, 129], [1 + 17 * i % 900 for i in range(150)], [2500] + [5] * 33])
 def test_decode_attention_shares_of_ragged_batches(n_heads, n_kv, d, lens):
-    """Sequences cut into shares of one size, added up by the last block and by a kernel of its own, against one share a sequence
-    and against fp32 torch on the longest: one sequence, more sequences than a warp, lengths at the edges of a page."""
+    """Sequences cut into shares, added up by the last block and by a kernel of its own (as many shares as the last block has room for, more,
+    and more than that kernel takes at a time), against one share a sequence and against fp32 torch on the longest: one sequence, more
+    sequences than a warp, lengths at the edges of a page."""
+    from types import SimpleNamespace
+
     from cpmcu_b200.cache import Cache
     from cpmcu_b200.parts.base import CacheNeeds
 
@@ -966,10 +969,11 @@ def test_decode_attention_shares_of_ragged_batches(n_heads, n_kv, d, lens):
     own = rows[sum(lens[:i]):sum(lens[:i + 1])].float().view(lens[i], -1, d)
     ref = plain.dense_attention(torch.cat([torch.zeros(lens[i] - 1, n_heads, d), q[i:i + 1].float().cpu()]), own[:, n_heads:n_heads + n_kv],
                                 own[:, n_heads + n_kv:], d ** -0.5)[-1].reshape(-1)
-    for splits in (None, 2, 5):
+    for splits in (None, 2, 5, 33, 64):
         assert _err(run(splits), want) < KTOL["bfloat16"]
-    ops._arrivals = lambda *a: ops.arrivals
-    for splits in (None, 2, 5, None):
+    ops._arrivals = lambda *a, given=ops._arrivals: given(*a) if a[-1] > 32 else ops.arrivals
+    ops.workspace = SimpleNamespace(alloc=lambda shape, dtype: torch.empty(*shape, dtype=dtype, device="cuda"))
+    for splits in (None, 2, 5, 32, 33, 64, None):
         got = run(splits)
         assert _err(got, want) < KTOL["bfloat16"] and _err(got[i], ref) < KTOL["bfloat16"]
         assert not ops.arrivals.any()
