@@ -10,7 +10,7 @@ offsets for ``chunk_length`` tokens (src/model/model.cuh:103-120).
 """
 from __future__ import annotations
 
-from typing import List, Optional, Tuple
+from typing import List, Optional, Sequence, Tuple
 
 import torch
 
@@ -126,29 +126,77 @@ def _meta(n: int) -> torch.Tensor:
     return torch.empty(n, dtype=torch.int32, device="meta")
 
 
-def dry_context(n_tokens: int, n_seqs: int, max_kv_len: int, cache, decode: bool, captured: bool = False) -> StepContext:
-    """A step of ``n_tokens`` tokens shared out evenly over ``n_seqs`` sequences, on tensors without storage."""
-    base, extra = divmod(n_tokens, n_seqs)
-    q_lens = [base + (1 if i < extra else 0) for i in range(n_seqs)]
+def dry_context(q_lens: Sequence[int], max_kv_len: int, cache, decode: bool, captured: bool = False,
+                n_tiles: Optional[int] = None) -> StepContext:
+    """A step that brings ``q_lens`` tokens of its sequences, on tensors without storage.  ``n_tiles``: as many query tiles
+    instead of the portions' own (a recorded step has room for those of any portions, and takes its longest to be all tokens)."""
+    n_tokens, n_seqs = sum(q_lens), len(q_lens)
     ctx = StepContext(
-        n_tokens=n_tokens, n_seqs=n_seqs, is_decode=decode, captured=captured, q_lens=q_lens,
+        n_tokens=n_tokens, n_seqs=n_seqs, is_decode=decode, captured=captured, q_lens=[n_tokens] if captured and not decode else list(q_lens),
         kv_lens=[] if captured else [max_kv_len] * n_seqs, slots=[] if captured else list(range(n_seqs)),
-        max_q_len=max(q_lens), max_kv_len=max_kv_len, token_ids=_meta(n_tokens), positions=_meta(n_tokens),
-        token_seq=_meta(n_tokens), cu_q=_meta(n_seqs + 1), kv_len_dev=_meta(n_seqs), slot_dev=_meta(n_seqs), cache=cache)
-    n_tiles = sum((n + PREFILL_TILE_ROWS - 1) // PREFILL_TILE_ROWS for n in q_lens)
+        max_q_len=n_tokens if captured and not decode else max(q_lens), max_kv_len=max_kv_len, token_ids=_meta(n_tokens),
+        positions=_meta(n_tokens), token_seq=_meta(n_tokens), cu_q=_meta(n_seqs + 1), kv_len_dev=_meta(n_seqs), slot_dev=_meta(n_seqs),
+        cache=cache)
+    if n_tiles is None:
+        n_tiles = sum((n + PREFILL_TILE_ROWS - 1) // PREFILL_TILE_ROWS for n in q_lens)
     ctx.q_tiles = (_meta(n_tiles), _meta(n_tiles), n_tiles)
     ctx.extras["step_begun"] = True
     return ctx
 
 
+def _evenly(n_tokens: int, n_seqs: int) -> List[int]:
+    base, extra = divmod(n_tokens, n_seqs)
+    return [base + (1 if i < extra else 0) for i in range(n_seqs)]
+
+
+def _most_tiles(n_tokens: int, most_seqs: int, longest: int) -> List[int]:
+    """The portions of a step of ``n_tokens`` tokens that need most query tiles while one of them has ``longest`` tokens or more: as many
+    sequences of one token as there may be, and the rest."""
+    ones = max(0, min(most_seqs - 1, n_tokens - longest))
+    return [1] * ones + [n_tokens - ones]
+
+
+def workspace_steps(max_step_tokens: int, max_batch: int, max_seq_tokens: int, packed_pieces: int = 0):
+    """The steps a workspace is measured with: (portions, keys of the longest sequence, decode, captured, query tiles or None).
+
+    Which step needs most room differs from part to part.  Most tensors grow with the step's tokens; the scratch of parts that go
+    by query tiles with their number, which is largest when one portion is long and the others have one token; the scratch of
+    shared-out keys, and the plain copies that narrow products make, are largest just below the number of tokens where a
+    kernel that needs none takes over; block-sparse attention needs other tensors below its threshold than above.
+    ``max_batch`` counts up to the next power of two, as the workspace lets steps through.  ``packed_pieces``: sequences of a recorded
+    chunk of several prompts (0: none is recorded)."""
+    T, b = int(max_step_tokens), 1
+    while b < max_batch:
+        b *= 2
+    steps = []
+    for n in sorted({T, max(1, T // 2)} | {min(T, p) for p in (512, 256, 255, 128, 95, 64, 63)}):
+        if n in (T, max(1, T // 2)):
+            steps.append((_evenly(n, min(n, max_batch)), max_seq_tokens, False, False, None))
+        uneven = {tuple(_most_tiles(n, b, longest)) for longest in (Ops.RETENTION_TILE_MIN_TOKENS, Ops.MINGRU_TILE_MIN_TOKENS)}
+        for portions in sorted(uneven | {(n,)}):
+            for kv in {min(max(max(portions), k), max_seq_tokens) for k in ((0, 4096, 8192) if len(portions) == 1 else (0,))} | {max_seq_tokens}:
+                steps.append((list(portions), kv, False, False, None))
+    steps.append(([T], max_seq_tokens, False, True, None))
+    if packed_pieces and b >= packed_pieces + 1 and T > packed_pieces:
+        steps.append((_evenly(T, packed_pieces + 1), max_seq_tokens, False, True, T // PREFILL_TILE_ROWS + packed_pieces))
+    size = 1
+    while size <= b:                                        # a captured decode step of every bucket; eager ones of as many sequences
+        steps.append(([1] * size, max_seq_tokens, True, True, None))
+        size *= 2
+    for size in sorted({max_batch, b, max(1, b - 1)}):
+        for kv in (1, max_seq_tokens):
+            steps.append(([1] * size, kv, True, False, None))
+    return steps
+
+
 def measure_workspace(spec, dtype: torch.dtype, max_step_tokens: int, max_batch: int, max_seq_tokens: int,
                       sm_count: int = 148) -> Tuple[int, int, List[str]]:
-    """(bytes of the persistent part, bytes of one frame, notes) that the steps of a model need at most: prompts of
-    ``max_step_tokens`` packed tokens (one long sequence, many short ones, short chunks after a long history) and
-    decode steps of ``max_batch`` sequences, each run once on tensors without storage.  A part that cannot run that
-    way (it reads values on the host) is left out of the measurement; what it allocates comes from torch's
-    allocator anyway, and the note says so."""
+    """(bytes of the persistent part, bytes of one frame, notes) that the steps of a model need at most: prompts of up to
+    ``max_step_tokens`` packed tokens and decode steps of up to ``max_batch`` sequences (see ``workspace_steps``), each run once on
+    tensors without storage.  A part that cannot run that way (it reads values on the host) is left out of the
+    measurement; what it allocates comes from torch's allocator anyway, and the note says so."""
     from ..cache import Cache
+    from ..engine.step import MAX_GRAPH_PIECES
     from ..models.model import Model
 
     ops = DryOps(dtype, sm_count)
@@ -158,23 +206,17 @@ def measure_workspace(spec, dtype: torch.dtype, max_step_tokens: int, max_batch:
     per_seq = max(64, int(max_seq_tokens))
     cache = Cache(model.cache_needs(), max_tokens=per_seq, dtype=dtype, device="meta", n_slots=max(2, max_batch + 1),
                   max_seq_tokens=per_seq, max_step_tokens=max_step_tokens)
-    cases = []
-    T = int(max_step_tokens)
-    for n in sorted({T, max(1, T // 2), min(T, 512), min(T, 256), min(T, 128), min(T, 64)}):
-        cases.append((n, 1, per_seq, False, False))
-        cases.append((n, min(n, max_batch), per_seq, False, False))
-    b = 1
-    while b < max_batch:
-        b *= 2
-    cases.append((b, b, per_seq, True, True))               # a captured decode step of the largest bucket
-    cases.append((max_batch, max_batch, per_seq, True, False))
+    recorded = model.recordable_prompt()
     notes: List[str] = []
-    for n_tokens, n_seqs, kv, decode, captured in cases:
+    for q_lens, kv, decode, captured, n_tiles in workspace_steps(max_step_tokens, max_batch, per_seq, MAX_GRAPH_PIECES if recorded else 0):
+        if captured and not decode and not recorded:
+            continue
+        n_tokens = sum(q_lens)
         ops.workspace.begin_step()
         try:
-            ctx = dry_context(n_tokens, n_seqs, kv, cache, decode, captured)
+            ctx = dry_context(q_lens, kv, cache, decode, captured, n_tiles)
             rows = ops.empty(n_tokens, dtype=torch.int32)                  # the step's descriptor: ids, positions, ...
-            ops.empty(8 * n_tokens + 4 * n_seqs + 64, dtype=torch.int32)
+            ops.empty(8 * n_tokens + 4 * len(q_lens) + 64, dtype=torch.int32)
             model.forward(ctx, rows)
         except Exception as e:                                            # a part that needs real values
             note = f"a part could not be measured without a device ({type(e).__name__}: {str(e)[:80]})"

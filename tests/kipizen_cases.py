@@ -98,6 +98,12 @@ def config_d() -> dict:
 CONFIGS = {"a": config_a, "b": config_b, "c": config_c, "d": config_d}
 
 
+def config_wide_state() -> dict:
+    """A state far larger than a token's other tensors: what a step needs beside its tokens' rows goes by its tiles."""
+    return {"architecture": NAME, "vocab": 60, "width": 64, "embedding": {"scale": 1.0}, "norm": {"eps": 1e-5},
+            "layers": [_layer(_lightning(4, 128, 256, [0.5, 0.9, 0.99, 0.999]), None), _layer(_attn(2, 1, 32, 32, 0.2), _moe(5, 2, 32))]}
+
+
 def tensor_shapes(cfg: dict) -> Dict[str, tuple]:
     W, out = cfg["width"], {}
     out["embed"] = (cfg["vocab"], W)

@@ -5,7 +5,7 @@ import torch
 from cpmcu_b200.cache import Cache, CacheFull
 from cpmcu_b200.memory import ALIGN, Arena, PoolExhausted, Workspace, plan_storage
 from cpmcu_b200.parts.base import CacheNeeds
-from tests import configs
+from tests import configs, dinutar_cases, kipizen_cases, reravik_cases
 
 
 def test_regions_are_carved_in_order_and_name_themselves_when_full():
@@ -96,6 +96,67 @@ def test_workspace_is_measured_by_the_models_own_forward_pass():
     assert f32 > sizes[("a", 64)][1]
     # a frame holds at least the widest tensor of a layer: the gate_up product of 64 tokens
     assert sizes[("a", 64)][1] >= 64 * 176 * 2
+
+
+def _need(spec, dtype, portions, max_kv_len, chunk, max_batch):
+    """Bytes (persistent, frame) that one step asks for."""
+    from cpmcu_b200.cache import Cache as AnyCache
+    from cpmcu_b200.models.model import Model
+    from cpmcu_b200.ops.dry import DryOps, dry_context
+
+    ops = DryOps(dtype)
+    model = Model(spec, ops)
+    model.load_weights({name: torch.empty(w.shape, device="meta", dtype=torch.int32 if w.role == "table" else dtype)
+                        for name, w in model.weight_specs().items()})
+    cache = AnyCache(model.cache_needs(), max_tokens=16384, dtype=dtype, device="meta", n_slots=max_batch + 1, max_seq_tokens=16384,
+                     max_step_tokens=chunk)
+    ops.workspace.begin_step()
+    n = sum(portions)
+    ctx = dry_context(portions, max_kv_len, cache, all(q == 1 for q in portions))
+    rows = ops.empty(n, dtype=torch.int32)
+    ops.empty(8 * n + 4 * len(portions) + 64, dtype=torch.int32)
+    model.forward(ctx, rows)
+    return ops.workspace.peaks()
+
+
+@pytest.mark.parametrize("arch_name,config,chunk,max_batch", [
+    ("Kipizen", kipizen_cases.config_wide_state, 300, 64), ("Kipizen", kipizen_cases.config_wide_state, 2048, 64),
+    ("Kipizen", kipizen_cases.config_wide_state, 2048, 5), ("Kipizen", kipizen_cases.config_d, 64, 200),
+    ("Dinutar", dinutar_cases.config_d, 300, 64), ("Dinutar", dinutar_cases.config_a, 2048, 33), ("Reravik", reravik_cases.config_a, 300, 5),
+    ("MiniCPMForCausalLM", configs.tiny_b, 300, 64), ("MiniCPMForCausalLM", configs.tiny_e, 64, 200),
+])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_no_step_needs_more_than_the_workspace_is_measured_for(arch_name, config, chunk, max_batch, dtype):
+    """Steps of portions as uneven as they come, of fewer tokens than a chunk, over short and long histories, and decode steps
+    between the buckets, against what storage gives a frame (the measured bytes, a twentieth and 1 MiB more)."""
+    from cpmcu_b200.ops.dry import measure_workspace
+    from cpmcu_b200.registry import architecture
+
+    arch = architecture(arch_name)
+    spec = arch.model_spec(arch.config_class.from_dict(config()))
+    persistent, frame, notes = measure_workspace(spec, dtype, chunk, max_batch, 16384)
+    assert notes == []
+    given = (int(persistent * 1.05) + (1 << 20), int(frame * 1.05) + (1 << 20))
+    bucket = 1
+    while bucket < max_batch:
+        bucket *= 2
+    steps = []
+    for n in {chunk, chunk - 1, chunk // 2 + 3, min(chunk, 254), min(chunk, 95), min(chunk, 61)}:
+        for seqs in {1, 2, max_batch, bucket, (bucket + 1) // 2}:
+            ones = min(seqs, n) - 1
+            steps.append([1] * ones + [n - ones])                                        # one long portion among single tokens
+            few = min(seqs, n // 8)
+            if few > 1:
+                steps.append([8] * (few - 1) + [n - 8 * (few - 1)])
+            if seqs * 65 <= n:
+                steps.append([65] * (seqs - 1) + [n - 65 * (seqs - 1)])                    # a tile and one token each
+            if seqs <= n:
+                steps.append([n // seqs + (i < n % seqs) for i in range(seqs)])
+    steps += [[1] * n for n in {1, 3, max_batch, bucket, max(1, bucket - 1), (bucket * 3 + 3) // 4}]
+    for portions in steps:
+        for kv in (max(portions), 4000, 16384):
+            need = _need(spec, dtype, portions, max(kv, max(portions)), chunk, bucket)
+            assert need[0] <= given[0] and need[1] <= given[1], (portions[:3], max(portions), len(portions), kv)
 
 
 def test_cache_inside_regions():

@@ -174,6 +174,20 @@ def test_batches_of_unequal_requests(folders, name, dtype):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+def test_one_long_prompt_among_many_short_ones_through_the_arena(tmp_path, dtype):
+    """63 portions of one token and one of 237 in one step: the most query tiles a step of 300 tokens and 64 sequences has."""
+    from cpmcu_b200 import LLM
+
+    cfg = cases.config_wide_state()
+    w = cases.random_weights(cfg, 5)
+    llm = LLM(cases.write_folder(cfg, w, str(tmp_path)), dtype=dtype, max_tokens=64 * 80, chunk_length=300, max_batch=64)
+    llm.init_storage()
+    llm.load_from_hf()
+    reqs = [cases.random_ids(cfg["vocab"], n, 50 + i) for i, n in enumerate([2] * 63 + [237])]
+    run_and_check(llm.stepper, cfg, w, reqs, [[1, 1]] * 63 + [[237]], dtype, "uneven batch")
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("name", ["a", "d"])
 def test_slots_pages_and_state_are_used_again(folders, name, dtype):
     """A cache of two slots and few pages serves nine requests one after another and in pairs: every slot, every page
