@@ -156,11 +156,20 @@ def _most_tiles(n_tokens: int, most_seqs: int, longest: int) -> List[int]:
     return [1] * ones + [n_tokens - ones]
 
 
+def _half_full_tiles(n_tokens: int, most_seqs: int) -> List[int]:
+    """The same while the tiles are half full on average (what ``Ops.recurrence_by_tiles`` asks for)."""
+    ones = 0
+    while ones + 1 < most_seqs and 32 * (ones + 1 + (n_tokens - ones - 1 + PREFILL_TILE_ROWS - 1) // PREFILL_TILE_ROWS) <= n_tokens:
+        ones += 1
+    return [1] * ones + [n_tokens - ones]
+
+
 def workspace_steps(max_step_tokens: int, max_batch: int, max_seq_tokens: int, packed_pieces: int = 0):
     """The steps a workspace is measured with: (portions, keys of the longest sequence, decode, captured, query tiles or None).
 
     Which step needs most room differs from part to part.  Most tensors grow with the step's tokens; the scratch of parts that go
-    by query tiles with their number, which is largest when one portion is long and the others have one token; the scratch of
+    by query tiles with their number, which is largest when one portion is long and the others have one token (as many of these as
+    the part's rule allows); the scratch of
     shared-out keys, and the plain copies that narrow products make, are largest just below the number of tokens where a
     kernel that needs none takes over; block-sparse attention needs other tensors below its threshold than above.
     ``max_batch`` counts up to the next power of two, as the workspace lets steps through.  ``packed_pieces``: sequences of a recorded
@@ -173,6 +182,7 @@ def workspace_steps(max_step_tokens: int, max_batch: int, max_seq_tokens: int, p
         if n in (T, max(1, T // 2)):
             steps.append((_evenly(n, min(n, max_batch)), max_seq_tokens, False, False, None))
         uneven = {tuple(_most_tiles(n, b, longest)) for longest in (Ops.RETENTION_TILE_MIN_TOKENS, Ops.MINGRU_TILE_MIN_TOKENS)}
+        uneven.add(tuple(_half_full_tiles(n, b)))
         for portions in sorted(uneven | {(n,)}):
             for kv in {min(max(max(portions), k), max_seq_tokens) for k in ((0, 4096, 8192) if len(portions) == 1 else (0,))} | {max_seq_tokens}:
                 steps.append((list(portions), kv, False, False, None))

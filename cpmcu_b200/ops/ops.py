@@ -1148,6 +1148,15 @@ class Ops:
         return (not ctx.is_decode and ctx.q_tiles is not None and ctx.max_q_len >= self.RETENTION_TILE_MIN_TOKENS
                 and d <= 256 and dv <= 256)
 
+    def recurrence_by_tiles(self, ctx, d: int, dv: int) -> bool:
+        """Whether a recurrence with a fixed decay goes by the prompt's tiles instead of token by token.  The walk takes as long as the
+        longest portion: 0.2 us a token at 16 heads of 64 x 128 (0.17 at 8 heads, 0.45 at 16 of 128 x 256); the tiles' three kernels 20 to 45 us and 2
+        us a tile (1; 7) however full it is.  So a portion has to be longer than 128 tokens and 10 for each tile of the step: one of
+        128 tokens takes 28 us in the walk and 33 by tiles, one of 512 105 and 46, one of 2,048 411 and 84; 63 of one token
+        beside one of 256 94 and 155, 64 of 16 105 and 148.  And the tiles are half full on average, since each takes a whole state of scratch."""
+        tiles = ctx.q_tiles[2] if ctx.q_tiles is not None else 0
+        return self.retention_tiles_ok(ctx, d, dv) and ctx.max_q_len >= 128 + 10 * tiles and 32 * tiles <= ctx.n_tokens
+
     def retention_tiles(self, ctx, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, gate: Optional[torch.Tensor],
                         powers: torch.Tensor, state: torch.Tensor, heads: int, d: int, dv: int, eps: float = 0.0) -> torch.Tensor:
         """The recurrence S <- a_h S + k v^T, o = S^T q over a prompt's tiles of 64 tokens (``ctx.q_tiles``), in 32-bit:

@@ -262,8 +262,7 @@ class LightningAttention(_MatrixStateMixer):
         ops.silu_columns(proj, 2 * H * d + H * dv)
         q, k = proj[:, :H * d], proj[:, H * d:2 * H * d]
         v, g = proj[:, 2 * H * d:2 * H * d + H * dv], proj[:, 2 * H * d + H * dv:]
-        if self.q_scale == 1.0 and ops.retention_tiles_ok(ctx, d, dv):
-            # a prompt: by tiles of 64 tokens, as the retention's (16 heads of 64 x 128, 2,048 tokens: 359 us token by token)
+        if self.q_scale == 1.0 and ops.recurrence_by_tiles(ctx, d, dv):
             o = ops.retention_tiles(ctx, q, k, v, None, self.powers, lane.state["matrix_state"], H, d, dv)
         else:
             decay = self.decay.unsqueeze(0).expand(ctx.n_tokens, H)         # the same row for every token (stride 0)

@@ -1,0 +1,29 @@
+"""Which kernel a step goes to and how its work is shared out: decisions made on the host, on the CPU."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from cpmcu_b200.ops.dry import DryOps, dry_context
+from cpmcu_b200.ops.ops import Ops
+
+
+@pytest.mark.parametrize("d", [32, 64, 96, 128])
+def test_counters_are_given_only_for_shares_that_the_last_block_can_add_up(d):
+    """At head size 32 a sequence has as many shares as the caller asks for, and the block that adds them up has room for 32."""
+    ops = SimpleNamespace(workspace=object(), arrivals=torch.zeros(16384, dtype=torch.int32))
+    for n_splits in (2, 16, 32, 33, 64, 1000):
+        got = Ops._arrivals(ops, 2, 16, 2, d, n_splits)
+        assert (got is not None) == (d == 64 or (d == 32 and n_splits <= 32)), n_splits
+
+
+@pytest.mark.parametrize("portions,by_tiles", [
+    ([2048], True), ([512], True), ([256], True), ([128], False), ([16], False), ([16] * 64, False), ([32] * 64, False),
+    ([1] * 63 + [256], False), ([1] * 63 + [1985], False), ([65] * 15 + [1073], True), ([512] * 4, True), ([8] * 63 + [1544], False),
+    ([1] * 255 + [45], False), ([1] * 8 + [504], True),
+])
+def test_recurrence_goes_by_tiles_where_they_are_few_and_full(portions, by_tiles):
+    """Few long portions go by tiles; many short ones, each of which would fill a tile of its own, token by token."""
+    ops = DryOps(torch.float32)
+    ctx = dry_context(portions, max(portions), None, all(n == 1 for n in portions))
+    assert ops.recurrence_by_tiles(ctx, 64, 128) == by_tiles
