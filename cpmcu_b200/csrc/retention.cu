@@ -16,6 +16,7 @@
 // A tile's work depends on nothing but its own tokens and the state before it, so tiles run side by side; a portion of any
 // size and a batch of any sequences give the same sums up to their order.
 #include "common.cuh"
+#include <type_traits>
 
 constexpr int kRetTile = 64;         // tokens of a tile (the step's query tiles)
 constexpr int kRetPitch = 68;        // floats of a staged row of 64: 16-byte aligned, neighbouring rows in other banks
@@ -445,9 +446,7 @@ retention_tile_out_kernel(const float* __restrict__ q, const float* __restrict__
             store4(stage + m * kCols + c, j0 + m < tl.n ? row4(vh + (int64_t)(j0 + m) * v_stride, c, dv, vec) : make_float4(0.f, 0.f, 0.f, 0.f));
         }
         __syncthreads();
-        const int count = min(kSlice, 8 * warp + 8 - j0);                  // a warp's rows end at 8 warp + 7
-#pragma unroll 4
-        for (int m = 0; m < count; ++m) {
+        auto add = [&](int m, auto edge) {
             const float4 a = load4(as + (j0 + m) * kRetPitch + 4 * ty);
             const float av[4] = {a.x, a.y, a.z, a.w};
 #pragma unroll
@@ -455,9 +454,23 @@ retention_tile_out_kernel(const float* __restrict__ q, const float* __restrict__
                 const float4 b = load4(stage + m * kCols + 64 * g + 4 * tx);
                 const float bv[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
-                for (int r = 0; r < 4; ++r)
+                for (int r = 0; r < 4; ++r) {
+                    if (decltype(edge)::value && j0 + m > 4 * ty + r) continue;
 #pragma unroll
                     for (int x = 0; x < 4; ++x) o[r][4 * g + x] = fmaf(av[r], bv[x], o[r][4 * g + x]);
+                }
+            }
+        };
+        // the warp's rows are 8 warp to 8 warp + 7: all of them see the keys before these, and of these each sees its own and those before
+        // (a later key is left out, not multiplied by zero: its values may be anything)
+#pragma unroll 1
+        for (int m8 = 0; m8 < kSlice && j0 + m8 <= 8 * warp; m8 += 8) {
+            if (j0 + m8 < 8 * warp) {
+#pragma unroll 4
+                for (int m = m8; m < m8 + 8; ++m) add(m, std::false_type{});
+            } else {
+#pragma unroll 2
+                for (int m = m8; m < m8 + 8; ++m) add(m, std::true_type{});
             }
         }
     }

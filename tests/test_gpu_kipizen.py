@@ -647,6 +647,28 @@ def test_lightning_recurrence_in_one_piece_and_in_pieces(H, d, dv):
             _close(torch.cat(got[i]), want[i], "float32")
 
 
+@pytest.mark.parametrize("H,d,dv", [(3, 20, 24), (2, 64, 128), (1, 128, 130), (2, 32, 200)])
+@pytest.mark.parametrize("at", [0, 1, 6, 63, 64, 70, 127, 149])
+def test_recurrence_by_tiles_does_not_look_ahead(H, d, dv, at):
+    """A token whose key and value are not numbers changes the tokens from itself on: none before it, whether in its tile or
+    not, and no other sequence's."""
+    from cpmcu_b200.ops.ops import Ops
+
+    ops = Ops(torch.float32)
+    g = torch.Generator().manual_seed(d + dv)
+    lens = [150, 37]
+    a = torch.rand(H, generator=g, dtype=torch.float64) * 0.5 + 0.5
+    powers = (a[:, None] ** torch.arange(65, dtype=torch.float64)).float().cuda()
+    q, k, v = (torch.randn(sum(lens), H * w, generator=g).cuda() for w in (d, d, dv))
+    run = lambda kk, vv: ops.retention_tiles(_ctx(lens, [0, 0], [1, 0]), q, kk, vv, None, powers, torch.zeros(2, H, d, dv, device="cuda"), H, d, dv)
+    base = run(k, v)
+    k2, v2 = k.clone(), v.clone()
+    k2[at], v2[at] = float("nan"), float("inf")
+    got = run(k2, v2)
+    assert torch.equal(got[:at], base[:at]) and torch.equal(got[150:], base[150:])
+    assert not bool(got[at:150].isfinite().any())
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("H,dv,group,act", [(6, 64, 6, "sigmoid"), (3, 24, 3, "sigmoid"), (4, 16, 2, "silu"), (1, 130, 1, "sigmoid"), (5, 8, 1, "silu")])
 def test_norm_over_heads_with_gate_and_activations_in_place(dtype, H, dv, group, act):
