@@ -177,8 +177,11 @@ __device__ __forceinline__ int64_t value_offset(int page, int kv_head, int dim, 
 // (or an earlier one) writes before pdl_wait() returns, which is when the preceding kernel
 // has completed and its writes are visible.  pdl_launch_dependents() lets the kernel after
 // this one begin its own launch.  Both are no-ops for a kernel launched the ordinary way.
-// What a kernel does before pdl_wait() here is only ever to prefetch weights, which no
-// kernel writes.
+// Since a kernel may start as soon as the one ahead has been let go, and that one as soon as the one before it, what is read before
+// pdl_wait() has to be older than the step: weights; the step's description (positions, lengths, offsets, slots, page tables); pages and states
+// that earlier steps wrote.  (The one exception, an expert product that reads the choice of experts, says why.)  What keeps
+// this true at the border of two steps is advance_decode_kernel, the last of a decode step: it lets nothing go before it has
+// waited and written the next step's description, whatever the mask below.  Steps from the host begin with copies, which nothing overtakes.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

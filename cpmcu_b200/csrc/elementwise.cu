@@ -462,16 +462,18 @@ CPM_API int cpm_rope_store(const void* qkv, void* q_out, void* k_cache, void* v_
 __global__ void advance_decode_kernel(int* __restrict__ ids, int* __restrict__ positions, int* __restrict__ kv_len,
                                       int* __restrict__ step_key, const int* __restrict__ sampled,
                                       const int* __restrict__ live, int n) {
-    pdl_launch_dependents();
+    // This kernel ends a step: everything of the step is over when it writes, and nothing of the next one, whose kernels read positions
+    // and lengths before they wait, may start before it has written.
     pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (live[i]) {
+    if (i < n && live[i]) {
         ids[i] = sampled[i];
         positions[i] += 1;
         kv_len[i] += 1;
         step_key[i] += 1;
     }
+    __threadfence();
+    pdl_launch_dependents();
 }
 
 CPM_API int cpm_advance_decode(int* ids, int* positions, int* kv_len, int* step_key, const int* sampled,

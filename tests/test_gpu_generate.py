@@ -66,6 +66,29 @@ def test_greedy_batch_tiny_a(model_folders, dtype, graph):
     llm.cache.check_consistent()
 
 
+@pytest.mark.parametrize("graph", [False, True])
+def test_steps_follow_one_another_whatever_is_launched_early(model_folders, graph):
+    """Every kernel class launched with the attribute, the border of two decode steps included: the same tokens and the same logits, to
+    the last bit, as with none.  (The kernel that ends a step writes the next one's positions, which kernels read before they wait.)"""
+    from cpmcu_b200 import LLM
+    from cpmcu_b200.ops import library
+
+    folder = model_folders("tiny_e", configs.tiny_e(), 0, "bfloat16")
+    prompts = [helpers.random_ids(configs.tiny_e()["vocab_size"], n, 17 + n) for n in (5, 62, 130)]
+    lib = library.load()
+    seen = []
+    try:
+        for mask in (0, 0x3f, -1):
+            lib.cpm_set_pdl(mask)
+            llm = LLM(folder, dtype="bfloat16", cuda_graph=graph, max_tokens=64 * 24, chunk_length=64)
+            res = llm.generate_batch(prompts, generation_length=24)
+            seen.append([r.tokens for r in res] + [llm.backend.runner.logits().clone()])
+    finally:
+        lib.cpm_set_pdl(-1)
+    for other in seen[1:]:
+        assert other[:-1] == seen[0][:-1] and torch.equal(other[-1], seen[0][-1])
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_tiny_b_sampling_batch(model_folders, dtype):
     """Tiny B's workload: batch 4 with prompts of 1/40/97/150 tokens, 24 steps at temperature
