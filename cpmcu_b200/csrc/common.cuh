@@ -233,6 +233,19 @@ static inline int ensure_dynamic_smem(Kernel kernel, int bytes, bool* done) {
     return CPM_OK;
 }
 
+// Multiprocessors of the current device (0: it could not be asked).
+static inline int device_sms() {
+    static int known[kMaxDevices] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
+    if (known[dev] == 0) {
+        int n = 0;
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+        known[dev] = n;
+    }
+    return known[dev];
+}
+
 static inline int launch_status() {
     cudaError_t e = cudaPeekAtLastError();
     return e == cudaSuccess ? CPM_OK : (int)e;

@@ -267,9 +267,8 @@ static int launch_gemm_f32(const float* A, const float* W, float* C, int M, int 
     if (M <= 8) return launch_few_rows<8, VEC>(A, W, C, M, N, K, lda, ldw, ldc, alpha, stream);
     if (M <= 16) return launch_few_rows<16, VEC>(A, W, C, M, N, K, lda, ldw, ldc, alpha, stream);
     // rounds of one block an SM, times the rows of a block
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
-        return CPM_BAD_ARGUMENT;
+    const int sms = device_sms();
+    if (sms < 1) return CPM_BAD_ARGUMENT;
     auto cost = [&](int ri) {
         const int64_t tiles = (int64_t)((M + 8 * ri - 1) / (8 * ri)) * ((N + BN - 1) / BN);
         return (tiles + sms - 1) / sms * ri;

@@ -59,11 +59,10 @@ __device__ __forceinline__ uint4 ld_stream16(const void* p) {
 // the other two blocks (24.1 against 24.8 ms for four rows), at 4096 27.7 against 29.8.
 constexpr int kShortK = 1024;
 // Long rows in blocks for at most half of the SMs: sixteen warps a block instead of eight, since no second block comes to keep more of
-// the weights in flight.  One row, 1,024 weight rows of K 4,096 in every layer of the 0.5B sizes: one short turn 15.4 -> 14.9 ms.  Such a
-// block takes an SM's whole register file and cannot be placed before the kernel ahead has left it: at K of 2,048 (an expert router, an output
-// projection) that costs more than it gives, 13.4 against 13.6 ms for a call of such layers.
-constexpr unsigned kFewBlocks = 74;
-constexpr int kFewBlocksK = 2048;
+// the weights in flight.  One row, inputs cold, eight and sixteen warps: 1,024 weight rows of K 4,096 4.4 and 3.7 us, of 8,192 7.5 and 6.4, 256 of
+// 16,384 11.4 and 8.6.  Such a block takes an SM's whole register file and cannot be placed before the kernel ahead has left it, and at K of
+// 2,560 and 3,072 that costs more than it gives: 3.6 and 4.5, 4.9 and 5.3 us.
+constexpr int kManyWarpsK = 4096;
 template <int NT, int EPI, int kSkinnyWarps, bool kShort>
 __global__ void __launch_bounds__(kSkinnyWarps * 32, kShort ? (NT == 1 ? 4 : 3) : (NT == 1 || kSkinnyWarps > 8 ? 1 : 2))
 skinny_gemm_kernel(const bf16* __restrict__ W, const bf16* __restrict__ X, void* __restrict__ out, int M, int N, int K,
@@ -169,7 +168,7 @@ template <int NT, int EPI>
 static int launch_skinny_epi(const void* W, const void* X, void* out, int M, int N, int K, float alpha,
                              const GluClamp& clamp, cudaStream_t stream) {
     const unsigned blocks = (unsigned)((N + 15) / 16);
-    if (blocks <= kFewBlocks && K > kFewBlocksK)
+    if (K >= kManyWarpsK && 2 * blocks <= (unsigned)device_sms())
         cpm_launch(kLaunchProduct, skinny_gemm_kernel<NT, EPI, 16, false>, blocks, 512, 0, stream, (const bf16*)W, (const bf16*)X, out, M, N, K,
                    alpha, g_skinny_prefetch_lines, clamp);
     else if (K <= kShortK)

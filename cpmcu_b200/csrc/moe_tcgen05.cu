@@ -293,18 +293,6 @@ moe_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     }
 }
 
-static int sm_count() {
-    static int known[kMaxDevices] = {};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
-    int n = known[dev];
-    if (n == 0) {
-        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-        known[dev] = n;
-    }
-    return n;
-}
-
 template <int MODE>
 static int launch(const void* A, const void* B0, const void* B1, void* C, const int* offsets, const int* order, int n_pairs,
                   int E, int N, int K, const float* in_scale, const GluClamp& clamp, cudaStream_t stream) {
@@ -317,7 +305,7 @@ static int launch(const void* A, const void* B0, const void* B1, void* C, const 
     auto kern = moe_tcgen05_kernel<MODE>;
     static bool configured[kMaxDevices] = {};
     if (int st = ensure_dynamic_smem(kern, Ring<GATED>::kSmem, configured)) return st;
-    const int sms = sm_count();
+    const int sms = device_sms();
     if (sms < 1) return CPM_BAD_ARGUMENT;
     const int64_t most = ((int64_t)(n_pairs + kMaxPairs - 1) / kMaxPairs + (E < n_pairs ? E : n_pairs)) * ((N + kFeatures - 1) / kFeatures);
     cpm_launch(kLaunchProduct, kern, dim3((unsigned)(most < sms ? most : sms)), dim3(kThreads), (size_t)Ring<GATED>::kSmem, stream,

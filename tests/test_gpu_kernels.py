@@ -1098,9 +1098,9 @@ def test_latent_attention_of_prompts_meets_only_the_keys_it_sees(rank, heads, wi
 
 
 @pytest.mark.parametrize("M", [1, 8, 9, 16])
-@pytest.mark.parametrize("N,K", [(17, 2080), (1000, 4096), (1184, 2080), (1185, 2080), (64, 2048)])
+@pytest.mark.parametrize("N,K", [(17, 4096), (1000, 4128), (1184, 4096), (1185, 4096), (64, 4064)])
 def test_products_of_few_rows_on_few_blocks(M, N, K):
-    """The widest block's sizes (up to 74 blocks of 16 weight rows, K over 2,048), one block more and a shorter row: bf16 and fp32 results against 64
+    """The widest block's sizes (up to 74 blocks of 16 weight rows, K from 4,096 on), one block more and a shorter row: bf16 and fp32 results against 64
     bits; fp32 sums of K products in another order, bf16 one rounding."""
     ops = _ops("bfloat16")
     g = torch.Generator().manual_seed(M + N + K)
