@@ -164,21 +164,21 @@ def _half_full_tiles(n_tokens: int, most_seqs: int) -> List[int]:
     return [1] * ones + [n_tokens - ones]
 
 
-def workspace_steps(max_step_tokens: int, max_batch: int, max_seq_tokens: int, packed_pieces: int = 0):
+def workspace_steps(max_step_tokens: int, max_batch: int, max_seq_tokens: int, packed_pieces: int = 0, sm_count: int = 148):
     """The steps a workspace is measured with: (portions, keys of the longest sequence, decode, captured, query tiles or None).
 
     Which step needs most room differs from part to part.  Most tensors grow with the step's tokens; the scratch of parts that go
     by query tiles with their number, which is largest when one portion is long and the others have one token (as many of these as
     the part's rule allows); the scratch of
     shared-out keys, and the plain copies that narrow products make, are largest just below the number of tokens where a
-    kernel that needs none takes over; block-sparse attention needs other tensors below its threshold than above.
+    kernel that needs none takes over (or the last step down of the number of shares); block-sparse attention needs other tensors below its threshold than above.
     ``max_batch`` counts up to the next power of two, as the workspace lets steps through.  ``packed_pieces``: sequences of a recorded
     chunk of several prompts (0: none is recorded)."""
     T, b = int(max_step_tokens), 1
     while b < max_batch:
         b *= 2
     steps = []
-    for n in sorted({T, max(1, T // 2)} | {min(T, p) for p in (512, 256, 255, 128, 95, 64, 63)}):
+    for n in sorted({T, max(1, T // 2)} | {min(T, p) for p in (512, 256, 255, 3 * sm_count // 2, 128, 95, 64, 63)}):
         if n in (T, max(1, T // 2)):
             steps.append((_evenly(n, min(n, max_batch)), max_seq_tokens, False, False, None))
         uneven = {tuple(_most_tiles(n, b, longest)) for longest in (Ops.RETENTION_TILE_MIN_TOKENS, Ops.MINGRU_TILE_MIN_TOKENS)}
@@ -218,7 +218,7 @@ def measure_workspace(spec, dtype: torch.dtype, max_step_tokens: int, max_batch:
                   max_seq_tokens=per_seq, max_step_tokens=max_step_tokens)
     recorded = model.recordable_prompt()
     notes: List[str] = []
-    for q_lens, kv, decode, captured, n_tiles in workspace_steps(max_step_tokens, max_batch, per_seq, MAX_GRAPH_PIECES if recorded else 0):
+    for q_lens, kv, decode, captured, n_tiles in workspace_steps(max_step_tokens, max_batch, per_seq, MAX_GRAPH_PIECES if recorded else 0, sm_count):
         if captured and not decode and not recorded:
             continue
         n_tokens = sum(q_lens)

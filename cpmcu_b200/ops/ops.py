@@ -474,11 +474,17 @@ class Ops:
         keys = min(window, ctx.max_kv_len) if window else ctx.max_kv_len      # in a recorded step an upper bound
         return max(1, min(self.LATENT_MAX_SPLITS, 3 * self.sm_count // blocks, ((keys + 31) // 32) // 2))
 
-    LATENT_PROMPT_MIN_TOKENS = 96      # fewer leave most SMs idle: the kernel of one token a block shares their keys out instead
+    LATENT_PROMPT_MIN_TOKENS, LATENT_PROMPT_MIN_PORTION, LATENT_PROMPT_MIN_KEYS = 96, 8, 128
 
     def latent_prompt_ok(self, ctx, n_tokens: int) -> bool:
-        """Whether a step's tokens go by pairs of neighbours (the kernel for prompts) instead of one by one."""
-        return not ctx.is_decode and ctx.q_tiles is not None and n_tokens >= self.LATENT_PROMPT_MIN_TOKENS
+        """Whether a step's tokens go by pairs of neighbours (the kernel for prompts) instead of one by one, when they share
+        enough keys to pay for it: fewer than 96 leave most SMs idle (the kernel of one token a block shares their keys out instead); a
+        portion of one token leaves half of a block idle, and a history of a page or two ends before the pair's page pays.  16 heads of
+        rank 512, one by one and by pairs, in us: 128 tokens of one prompt 15.4 and 14.3, behind 1,000 more 109 and 86; 32 portions of 8
+        8.8 and 12.8, behind 1,000 more 118 and 98; 255 portions of one token and one of two 8.8 and 24.6; 32 heads of
+        rank 576, 95 portions of one token and one of two behind 1,000 more 118 and 163."""
+        return (not ctx.is_decode and ctx.q_tiles is not None and n_tokens >= max(self.LATENT_PROMPT_MIN_TOKENS, self.LATENT_PROMPT_MIN_PORTION * ctx.n_seqs)
+                and ctx.max_kv_len >= self.LATENT_PROMPT_MIN_KEYS)
 
     def latent_attention_on_tensor_cores(self, rank: int) -> bool:
         return self.code == BF16 and rank % 16 == 0 and rank <= 576
@@ -498,7 +504,7 @@ class Ops:
         if tensor_cores and not mma_ok:
             raise ValueError("the tensor-core latent attention takes bf16 latents of a rank that is a multiple of 16 up to 576")
         if mma_ok and tensor_cores is not False:
-            if n_splits is None and self.latent_prompt_ok(ctx, n):
+            if n_splits is None and self.latent_prompt_ok(ctx, n) and q_lat.data_ptr() % 16 == 0:      # (its queries come in 16-byte loads)
                 tile_seq, tile_row, n_tiles = ctx.q_tiles
                 check(self.lib.cpm_latent_attention_prompt(_ptr(q_lat), _ptr(lane.k), _ptr(out), 1 if narrow else 0, _ptr(ctx.positions),
                                                            _ptr(ctx.slot_dev), _ptr(lane.page_table), lane.page_table.shape[1],

@@ -27,3 +27,14 @@ def test_recurrence_goes_by_tiles_where_they_are_few_and_full(portions, by_tiles
     ops = DryOps(torch.float32)
     ctx = dry_context(portions, max(portions), None, all(n == 1 for n in portions))
     assert ops.recurrence_by_tiles(ctx, 64, 128) == by_tiles
+
+
+@pytest.mark.parametrize("portions,keys,by_pairs", [
+    ([128], 128, True), ([96], 96, False), ([96], 1096, True), ([95], 4000, False), ([1] * 95 + [2], 1000, False), ([1] * 63 + [1985], 1985, True),
+    ([8] * 32, 8, False), ([8] * 32, 1008, True), ([3] * 40, 1003, False), ([1] * 128, 4000, False),
+])
+def test_latent_attention_goes_by_pairs_where_they_share_keys(portions, keys, by_pairs):
+    """Prompt tokens in portions long enough for both tokens of a pair, over histories long enough for the pages they share."""
+    ops = DryOps(torch.bfloat16)
+    ctx = dry_context(portions, keys, None, all(n == 1 for n in portions))
+    assert ops.latent_prompt_ok(ctx, sum(portions)) == by_pairs
