@@ -923,7 +923,7 @@ def test_expert_products_by_tiles_and_for_few(E, top, W, ff, n, skew, mode):
 
 
 @pytest.mark.parametrize("K,N", [(1, 8), (63, 40), (513, 128), (576, 136), (1151, 24)])
-@pytest.mark.parametrize("n", [1, 2, 3, 8, 9])
+@pytest.mark.parametrize("n", [1, 2, 3, 8, 9, 16, 17])
 def test_head_project_of_few_tokens(K, N, n):
     """The per-head maps of a decode step: sums shorter and longer than what is asked for ahead, ragged columns, every number of
     tokens a block takes, from and to both types; 64-bit products.  fp32 results: sums of K products in another order."""
