@@ -1488,10 +1488,18 @@ class Ops:
               f"moe_route ({n_experts} experts, top {top})")
         return chosen, weights, gate
 
-    # Up to here the chosen experts are streamed without grouping.  Both kernels' products of a layer, inputs cold: 64 experts of
-    # 768 x 2048, 6 choices: 96 pairs 95 against 129 us by tiles, 198 pairs 126 against 137, 384 pairs 191 against 142; 32 of 512 x 1024, 4 choices:
-    # 96 pairs 34 against 46, 192 pairs 50 against 46.
+    # Up to here the chosen experts are streamed without grouping, eight pairs of an expert at a time: up to 12 pairs an expert on average, and no
+    # more than these.  Both kernels' products of a layer, inputs cold, by pair and by tiles: 64 experts of 768 x 2048, 6 choices: 96 pairs
+    # 85 against 121 us, 156 99 against 129, 198 113 against 129, 396 187 against 132; 32 of 512 x 1024, 4 choices: 96 26 against 35, 160 35 against 36; 8 of
+    # 1024 x 2048, 2 choices: 72 39 against 41, 96 48 against 42, 160 76 against 42; 4 of 2048 x 1024: 48 36 against 36, 96 60 against 36; 2 of
+    # 2048 x 2048, 1 choice: 24 31 against 43, 48 54 against 43, 160 159 against 52.
     MOE_PAIRWISE_MAX_PAIRS = int(os.environ.get("CPMCU_MOE_PAIRWISE_MAX", "160"))
+    MOE_PAIRWISE_PER_EXPERT = 12
+
+    def moe_by_pair(self, pairs: int, n_experts: int, hidden: int, ff: int) -> bool:
+        """Whether the products of ``pairs`` (token, choice) pairs go by pair, without grouping."""
+        return (self.code == BF16 and pairs <= min(self.MOE_PAIRWISE_MAX_PAIRS, self.MOE_PAIRWISE_PER_EXPERT * n_experts, 8192)
+                and hidden % 8 == 0 and ff % 8 == 0)
 
     def moe_experts(self, x: torch.Tensor, chosen: torch.Tensor, w_gate: Optional[torch.Tensor], w_up: torch.Tensor,
                     w_down: torch.Tensor, input_scale: Optional[torch.Tensor] = None,
@@ -1520,7 +1528,7 @@ class Ops:
         pairs = n * top
         h = self.empty(pairs, ff)
         y = self.empty(pairs, hidden)
-        if self.code == BF16 and pairs <= min(self.MOE_PAIRWISE_MAX_PAIRS, 8192) and hidden % 8 == 0 and ff % 8 == 0:
+        if self.moe_by_pair(pairs, E, hidden, ff):
             # few pairs (a decode step): every chosen expert's weights are streamed once, no grouping
             check(self.lib.cpm_moe_pair_product(_ptr(x), _ptr(first), _ptr(second), _ptr(h), _ptr(chosen), pairs, top, ff, hidden, mode,
                                                 _ptr(input_scale), *lims, self._stream()), "moe gate/up product by pair")

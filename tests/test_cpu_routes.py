@@ -38,3 +38,10 @@ def test_latent_attention_goes_by_pairs_where_they_share_keys(portions, keys, by
     ops = DryOps(torch.bfloat16)
     ctx = dry_context(portions, keys, None, all(n == 1 for n in portions))
     assert ops.latent_prompt_ok(ctx, sum(portions)) == by_pairs
+
+
+@pytest.mark.parametrize("pairs,experts,by_pair", [(160, 64, True), (161, 64, False), (160, 14, True), (160, 13, False), (24, 2, True), (25, 2, False), (12, 1, True)])
+def test_experts_go_by_pair_for_few_pairs_and_few_an_expert(pairs, experts, by_pair):
+    ops = DryOps(torch.bfloat16)
+    assert ops.moe_by_pair(pairs, experts, 64, 32) == by_pair
+    assert not ops.moe_by_pair(pairs, experts, 64, 20) and not DryOps(torch.float32).moe_by_pair(pairs, experts, 64, 32)

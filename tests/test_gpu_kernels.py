@@ -876,10 +876,12 @@ def test_decode_attention_with_rotation_inside(n_heads, n_kv, d):
     (4, 2, 136, 72, 700, True),        # chunks of more than 256 pairs, a ragged last slice of K, an expert nobody chose
     (512, 3, 64, 136, 65, False),      # the most experts, most of one pair or none
     (3, 1, 8, 12, 600, False),         # a row shorter than a slice, rows that are no whole 16-byte pieces
-    (8, 4, 200, 40, 40, False),        # the most pairs of the kernel for few
-    (8, 4, 200, 40, 41, False),        # more: tiles
+    (16, 4, 200, 40, 40, False),       # the most pairs of the kernel for few
+    (16, 4, 200, 40, 41, False),       # more: tiles
+    (8, 4, 200, 40, 24, False),        # the most pairs an expert of the kernel for few
+    (8, 4, 200, 40, 25, True),         # more: tiles
     (16, 4, 2048, 768, 7, False),      # sums of many slices
-    (2, 1, 72, 264, 33, False),        # more pairs of one expert than the eight columns of an instruction
+    (2, 1, 72, 264, 24, False),        # more pairs of one expert than the eight columns of an instruction
 ])
 @pytest.mark.parametrize("mode", ["silu", "relu2", "bounded"])
 def test_expert_products_by_tiles_and_for_few(E, top, W, ff, n, skew, mode):
