@@ -573,6 +573,17 @@ CPM_API int cpm_moe_group(const int* chosen, int n_pairs, int E, int* offsets, i
     return launch_status();
 }
 
+// Whether a product of many pairs goes to the tensor cores.
+static bool expert_tiles(const void* A, const void* B0, const void* B1, const void* rows, int E, int N, int K, int mode, int dtype) {
+    return dtype == CPM_BF16 && K % 8 == 0 && !(((uintptr_t)A | (uintptr_t)B0 | (uintptr_t)B1) & 15) && E <= 512 && (int64_t)E * N < (1 << 30) &&
+           g_moe_tensor_cores && (mode == 0 || (rows != nullptr && ((uintptr_t)rows & 15) == 0));
+}
+
+// Kernels that cpm_moe_expert_product launches for these arguments.
+CPM_API int cpm_moe_expert_product_kernels(const void* A, const void* B0, const void* B1, const void* rows, int E, int N, int K, int mode, int dtype) {
+    return mode != 0 && expert_tiles(A, B0, B1, rows, E, N, K, mode, dtype) ? 2 : 1;      // the rows in expert order, then the product
+}
+
 // mode 1: A = x [tokens, K], B0 = gate stack [E, N, K], B1 = up stack, C = H [pairs, N] in expert order.
 // mode 3: the same with the gate of two bounded products (limit, slope, offset).
 // mode 2: A = x, B0 = up stack, C = H = relu(in_scale[pair] * product)^2 in expert order (in_scale null: 1).
@@ -585,8 +596,7 @@ CPM_API int cpm_moe_expert_product(const void* A, const void* B0, const void* B1
     if (n_pairs <= 0) return CPM_OK;
     if (E < 1 || top < 1 || N < 1 || K < 1 || mode < 0 || mode > 3) return CPM_BAD_ARGUMENT;
     const GluClamp clamp{limit, slope, offset};
-    if (dtype == CPM_BF16 && K % 8 == 0 && ((uintptr_t)A & 15) == 0 && ((uintptr_t)B0 & 15) == 0 && ((uintptr_t)B1 & 15) == 0 &&
-        E <= 512 && (int64_t)E * N < (1 << 30) && g_moe_tensor_cores && (mode == 0 || (rows != nullptr && ((uintptr_t)rows & 15) == 0))) {
+    if (expert_tiles(A, B0, B1, rows, E, N, K, mode, dtype)) {
         if (mode != 0)
             cpm_launch(kLaunchNorm, moe_gather_kernel, dim3((n_pairs + 7) / 8), dim3(256), 0, stream, (const uint4*)A, order, (uint4*)rows,
                        n_pairs, top, K / 8);

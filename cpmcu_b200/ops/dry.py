@@ -51,6 +51,10 @@ class _NoLibrary:
         return 1
 
     @staticmethod
+    def cpm_moe_expert_product_kernels(*args):
+        return 1
+
+    @staticmethod
     def cpm_sink_attention_bf16_sizes(d, dv):
         return int(d in (32, 64, 96, 128) and dv in (32, 64, 96, 128))
 

@@ -173,6 +173,8 @@ def load() -> ctypes.CDLL:
             lib.cpm_set_decode_early(int(os.environ["CPMCU_DECODE_EARLY"]))
         lib.cpm_gemm_tcgen05_error.argtypes = []
         lib.cpm_gemm_tcgen05_error.restype = c_int
+        lib.cpm_moe_expert_product_kernels.argtypes = [_P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int]
+        lib.cpm_moe_expert_product_kernels.restype = c_int
         lib.cpm_moe_tcgen05_error.argtypes = []
         lib.cpm_moe_tcgen05_error.restype = c_int
         lib.cpm_attention_tcgen05_error.argtypes = []

@@ -1541,8 +1541,7 @@ class Ops:
         # (y holds the tokens' rows in expert order until the down product writes it)
         check(self.lib.cpm_moe_expert_product(_ptr(x), _ptr(first), _ptr(second), _ptr(h), _ptr(offsets), _ptr(order), _ptr(y), pairs, E, top,
                                               ff, hidden, mode, _ptr(input_scale), *lims, self.code, self._stream()), "moe gate/up product")
-        if self.code == BF16 and hidden % 8 == 0 and E <= 512:
-            LAUNCHES_EXTRA[0] += 1       # the launcher starts two kernels: the rows in expert order, then the product
+        LAUNCHES_EXTRA[0] += self.lib.cpm_moe_expert_product_kernels(_ptr(x), _ptr(first), _ptr(second), _ptr(y), E, ff, hidden, mode, self.code) - 1
         check(self.lib.cpm_moe_expert_product(_ptr(h), _ptr(w_down), None, _ptr(y), _ptr(offsets), _ptr(order), None, pairs, E, top,
                                               hidden, ff, 0, None, 0.0, 0.0, 0.0, self.code, self._stream()), "moe down product")
         return y

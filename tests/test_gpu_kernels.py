@@ -924,6 +924,27 @@ def test_expert_products_by_tiles_and_for_few(E, top, W, ff, n, skew, mode):
     assert _err(out, total) < 2.0 ** -8                            # one rounding to bf16
 
 
+def test_launches_of_expert_products_are_counted_as_they_are():
+    """Grouping, rows in expert order, two products; without the tensor cores no rows are laid out; few pairs: two products."""
+    from cpmcu_b200.ops import library
+
+    ops = _ops("bfloat16")
+    w = torch.zeros(4, 16, 16, dtype=torch.bfloat16, device="cuda")
+
+    def launches(n):
+        x, chosen = torch.zeros(n, 16, dtype=torch.bfloat16, device="cuda"), torch.zeros(n, 2, dtype=torch.int32, device="cuda")
+        before = library.LAUNCHES[0]
+        ops.moe_experts(x, chosen, w, w, w)
+        return library.LAUNCHES[0] - before
+
+    assert launches(4) == 2 and launches(200) == 4
+    ops.lib.cpm_set_moe_tensor_cores(0)
+    try:
+        assert launches(200) == 3
+    finally:
+        ops.lib.cpm_set_moe_tensor_cores(1)
+
+
 @pytest.mark.parametrize("K,N", [(1, 8), (63, 40), (513, 128), (576, 136), (1151, 24)])
 @pytest.mark.parametrize("n", [1, 2, 3, 8, 9, 16, 17])
 def test_head_project_of_few_tokens(K, N, n):
