@@ -142,7 +142,7 @@ add_rmsnorm_rows_kernel(float* __restrict__ x, const T* __restrict__ delta, cons
 template <typename T, typename W>
 static int launch_add_rmsnorm(float* x, const void* delta, const void* delta2, float alpha, const void* w, void* y, const int* rows,
                               int n_rows, int hidden, float eps, int write_back, cudaStream_t stream) {
-    if (const RowShape sh = row_shape(n_rows, hidden, 4); sh.nv) {
+    if (const RowShape sh = row_shape(n_rows, hidden, 4, sizeof(T) == 4); sh.nv) {
         auto kern = sh.nv == 1 ? add_rmsnorm_rows_kernel<T, W, 1> : sh.nv == 2 ? add_rmsnorm_rows_kernel<T, W, 2> : add_rmsnorm_rows_kernel<T, W, 4>;
         cpm_launch(kLaunchNorm, kern, n_rows, sh.threads, 0, stream, x, (const T*)delta, (const T*)delta2, alpha, (const W*)w, (T*)y, rows, hidden,
                    eps, write_back);

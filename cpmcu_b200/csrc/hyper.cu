@@ -140,7 +140,7 @@ CPM_API int cpm_hyper_step(float* X, const void* y, const float* mix, const floa
     if (y && (!mix || !out_w)) return CPM_BAD_ARGUMENT;
     if (in_w && (!gain || !h)) return CPM_BAD_ARGUMENT;
     const bool aligned = !(((uintptr_t)X | (uintptr_t)y | (uintptr_t)h | (uintptr_t)total) & 15);
-    if (const RowShape sh = row_shape(n_tokens, W, 1); sh.nv && S <= 4 && aligned) {
+    if (const RowShape sh = row_shape(n_tokens, W, 1, dtype != CPM_BF16); sh.nv && S <= 4 && aligned) {
 #define CPM_HYPER_ROWS(TT, NS) cpm_launch(kLaunchNorm, hyper_step_rows_kernel<TT, NS>, dim3(n_tokens), dim3(sh.threads), 0, stream, X, (const TT*)y, \
                                           mix, out_w, in_w, gain, eps, (TT*)h, total, S, W)
         if (dtype == CPM_BF16) { if (S <= 2) CPM_HYPER_ROWS(bf16, 2); else CPM_HYPER_ROWS(bf16, 4); }

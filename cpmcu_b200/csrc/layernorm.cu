@@ -399,7 +399,7 @@ CPM_API int cpm_add_layernorm(float* x, const void* a, const void* a2, float alp
                               int write_back, int dtype, cudaStream_t stream) {
     if (n_rows <= 0) return CPM_OK;
     if (hidden < 1 || !w || !y || (y2 && !w2) || (a2 && !a)) return CPM_BAD_ARGUMENT;
-    if (const RowShape sh = row_shape(n_rows, hidden, 4); sh.nv) {
+    if (const RowShape sh = row_shape(n_rows, hidden, 4, dtype != CPM_BF16); sh.nv) {
 #define CPM_ADD_LN_ROWS(TT, NV) cpm_launch(kLaunchNorm, add_layernorm_rows_kernel<TT, NV>, n_rows, sh.threads, 0, stream, x, (const TT*)a,     \
                                            (const TT*)a2, alpha, w, b, (TT*)y, w2, b2, (TT*)y2, rows, hidden, eps, write_back)
         if (dtype == CPM_BF16) { if (sh.nv == 1) CPM_ADD_LN_ROWS(bf16, 1); else if (sh.nv == 2) CPM_ADD_LN_ROWS(bf16, 2); else CPM_ADD_LN_ROWS(bf16, 4); }
@@ -425,7 +425,7 @@ CPM_API int cpm_layernorm_shift(const float* x, const float* w, const float* b, 
                                 const int* positions, const int* token_seq, const int* cu_q, const int* slots, void* y,
                                 int n_tokens, int hidden, float eps, int dtype, cudaStream_t stream) {
     if (n_tokens <= 0) return CPM_OK;
-    if (const RowShape sh = row_shape(n_tokens, hidden, 2); sh.nv) {
+    if (const RowShape sh = row_shape(n_tokens, hidden, 2, dtype != CPM_BF16); sh.nv && ((uintptr_t)state & 15) == 0) {
 #define CPM_SHIFT_ROWS(TT, NV) cpm_launch(kLaunchNorm, layernorm_shift_rows_kernel<TT, NV>, n_tokens, sh.threads, 0, stream, x, w, b, mu, state,  \
                                           positions, token_seq, cu_q, slots, (TT*)y, hidden, eps)
         if (dtype == CPM_BF16) { if (sh.nv == 1) CPM_SHIFT_ROWS(bf16, 1); else CPM_SHIFT_ROWS(bf16, 2); }
@@ -452,7 +452,7 @@ CPM_API int cpm_post_norm_add(float* x, const void* a, const float* w, const flo
                               void* y, int n_tokens, int hidden, float eps, int dtype, cudaStream_t stream) {
     if (n_tokens <= 0) return CPM_OK;
     if ((w2 == nullptr) != (y == nullptr) || (w2 == nullptr) != (b2 == nullptr)) return CPM_BAD_ARGUMENT;
-    if (const RowShape sh = row_shape(n_tokens, hidden, 4); sh.nv) {
+    if (const RowShape sh = row_shape(n_tokens, hidden, 4, dtype != CPM_BF16); sh.nv) {
 #define CPM_PNA_ROWS(TT, NV) cpm_launch(kLaunchNorm, post_norm_add_rows_kernel<TT, NV>, n_tokens, sh.threads, 0, stream, x, (const TT*)a, w, b, w2,  \
                                         b2, (TT*)y, hidden, eps)
         if (dtype == CPM_BF16) { if (sh.nv == 1) CPM_PNA_ROWS(bf16, 1); else if (sh.nv == 2) CPM_PNA_ROWS(bf16, 2); else CPM_PNA_ROWS(bf16, 4); }

@@ -95,7 +95,7 @@ post_norm_rows_kernel(float* __restrict__ x, const T* __restrict__ a, float alph
 template <typename T>
 static int launch_post_norm(float* x, const void* a, float alpha, const float* scale, const float* w, void* y, int n_tokens, int hidden,
                             float eps, cudaStream_t stream) {
-    if (const RowShape sh = row_shape(n_tokens, hidden, 4); sh.nv) {
+    if (const RowShape sh = row_shape(n_tokens, hidden, 4, sizeof(T) == 4); sh.nv) {
         auto kern = sh.nv == 1 ? post_norm_rows_kernel<T, 1> : sh.nv == 2 ? post_norm_rows_kernel<T, 2> : post_norm_rows_kernel<T, 4>;
         cpm_launch(kLaunchNorm, kern, n_tokens, sh.threads, 0, stream, x, (const T*)a, alpha, scale, w, (T*)y, hidden, eps);
         return launch_status();

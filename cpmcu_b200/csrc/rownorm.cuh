@@ -9,12 +9,14 @@
 
 constexpr int kRowMaxWarps = 16;
 
-// Threads and groups a thread for ``rows`` rows of ``hidden`` columns; nv 0: not for these kernels.  Many wide rows are bound by memory and want
-// more of them on an SM than the registers of these kernels leave room for (2,048 rows of 4,096: 21.0 against 20.4 us with the
-// row in shared memory, of 2,048 11.7 against 10.9; of 1,024 6.1 against 6.3).
+// Threads and groups a thread for ``rows`` rows of ``hidden`` columns; nv 0: not for these kernels.  In bf16 many wide rows are bound by memory
+// and want more of them on an SM than the registers of these kernels leave room for (2,048 rows of 4,096: 21.0 against 20.4 us
+// with the row in shared memory, of 2,048 11.7 against 10.9; of 1,024 6.1 against 6.3; 512 of 8,192 8.9 against 7.3).  In 32-bit the
+// width alone decides, so that a row's sum runs in one order whatever else is in the step.
 struct RowShape { int threads, nv; };
-static inline RowShape row_shape(int64_t rows, int hidden, int most_nv) {
-    if (hidden < 4 || hidden % 4 || hidden > 4 * 32 * kRowMaxWarps * most_nv || (rows > 512 && hidden >= 2048)) return {0, 0};
+static inline RowShape row_shape(int64_t rows, int hidden, int most_nv, bool f32) {
+    if (hidden < 4 || hidden % 4 || hidden > 4 * 32 * kRowMaxWarps * most_nv) return {0, 0};
+    if (f32 ? hidden > 4096 : (rows > 512 && hidden >= 2048) || (rows > 200 && hidden > 4096)) return {0, 0};
     const int quads = hidden / 4, warps = (quads + 31) / 32, threads = 32 * (warps < kRowMaxWarps ? warps : kRowMaxWarps);
     const int nv = (quads + threads - 1) / threads;
     return {threads, nv == 3 ? 4 : nv};
