@@ -116,7 +116,7 @@ def test_streams_blended_and_normed(dtype, S, W, rows):
 
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
-@pytest.mark.parametrize("tokens,heads,dv,group", [(3, 3, 44, 3), (2, 4, 128, 1), (2, 16, 128, 16), (2, 33, 64, 33), (2, 32, 256, 32), (300, 2, 1024, 1), (200, 3, 1024, 1)])
+@pytest.mark.parametrize("tokens,heads,dv,group", [(3, 3, 44, 3), (3, 2, 64, 1), (2, 4, 128, 1), (2, 16, 128, 16), (2, 33, 64, 33), (2, 32, 256, 32), (300, 2, 1024, 1), (200, 3, 1024, 1)])
 @pytest.mark.parametrize("act", ["sigmoid", "silu"])
 def test_norm_over_heads_with_a_gate_on_whole_loads(dtype, tokens, heads, dv, group, act):
     """The gate is a slice of a wider row that begins on a 16-byte boundary, and (the same numbers) one that does not."""
