@@ -8,7 +8,7 @@
 // row's result therefore does not depend on what else is in the batch.  The slices are what lets the two kernels share the
 // work of an output among threads (few rows) or not (many) and still agree to the last bit.
 //
-// Two kernels, by rows:
+// Two kernels, by rows (and K):
 //   up to 16 rows (decode): bound by streaming the weights; a block owns 8 weight rows, a thread one slice of one of them for
 //     all token rows.  Weight pieces of 1,024 columns come by 16-byte cp.async three stages deep, each slice padded by four
 //     floats so that the 16-byte reads of a quarter warp (8 rows) fall into 8 different bank groups.
@@ -18,7 +18,8 @@
 //     shared memory as they lie in global memory (rows padded to 20 floats: conflict-free 16-byte reads along K, no
 //     transposition), 16 columns a stage, two stages a group by cp.async.  After each round of four slices the groups trade: each
 //     keeps the totals of two of a thread's columns and adds the four groups' sums of them in the order of the slices.
-//     The number of rows is the one whose tiles fill the SMs' rounds best.
+//     The number of rows is the one whose tiles fill the SMs' rounds best.  Where K is one or two slices, from 9 rows on, a block is one such
+//     group and takes 64 or 32 rows.
 // Where K is no multiple of 4 or a pointer is not 16-byte aligned the same kernels load element by element.
 //
 // Measured on one B200 at the 0.5B layer sizes, 24 layers, prompts of 400, 141 and 50 tokens together and four decoded tokens:
@@ -136,41 +137,46 @@ gemm_f32_few_rows_kernel(const float* __restrict__ A, const float* __restrict__ 
 // ---------------------------------------------------------------------------------------------------------------------
 // more rows
 // ---------------------------------------------------------------------------------------------------------------------
-constexpr int BN = 64, BK = 16, kTilePad = BK + 4, kGroups = 4, kGroupThreads = 64, kTileThreads = kGroups * kGroupThreads;
+constexpr int BN = 64, BK = 16, kTilePad = BK + 4, kGroups = 4, kGroupThreads = 64;
 template <int RI> constexpr int tile_stage_floats() { return (8 * RI + BN) * kTilePad; }
-template <int RI> constexpr size_t tile_smem_bytes() {
-    return (size_t)(kGroups * 2 * tile_stage_floats<RI>() + kGroups * RI * 8 * kGroupThreads) * sizeof(float);
+template <int NG> constexpr int tile_stages() { return NG == 1 ? 4 : 2; }
+template <int RI, int NG> constexpr size_t tile_smem_bytes() {
+    return (size_t)(NG * tile_stages<NG>() * tile_stage_floats<RI>() + (NG == 1 ? 0 : NG * RI * 8 * kGroupThreads)) * sizeof(float);
 }
 
-template <bool VEC, int RI>
-__global__ void __launch_bounds__(kTileThreads, 1)
+template <bool VEC, int RI, int NG>
+__global__ void __launch_bounds__(NG * kGroupThreads, 1)
 gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C,
                      int M, int N, int K, int64_t lda, int64_t ldw, int64_t ldc, float alpha) {
     extern __shared__ float tile_smem[];
-    constexpr int BM = 8 * RI, kStage = tile_stage_floats<RI>(), kSteps = kSliceK / BK, kOwn = 8 / kGroups;
+    constexpr int BM = 8 * RI, kStage = tile_stage_floats<RI>(), kStages = tile_stages<NG>(), kSteps = kSliceK / BK, kOwn = 8 / NG;
     const int group = threadIdx.x / kGroupThreads, tid = threadIdx.x % kGroupThreads;
     const int tx = tid & 7, ty = tid >> 3;                              // outputs (ty + 8 i, tx + 8 j)
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-    const int slices = (K + kSliceK - 1) / kSliceK, steps = (slices + kGroups - 1) / kGroups * kSteps;
-    float* ring = tile_smem + group * 2 * kStage;
-    float* trade = tile_smem + kGroups * 2 * kStage;                    // [group][RI * 8][64]
+    // (a group alone need not go on to the end of the last slice: what follows K is zeros)
+    const int slices = (K + kSliceK - 1) / kSliceK, steps = NG == 1 ? (K + BK - 1) / BK : (slices + NG - 1) / NG * kSteps;
+    float* ring = tile_smem + group * kStages * kStage;
+    float* trade = tile_smem + NG * kStages * kStage;                   // [group][RI * 8][64]
     auto stage = [&](int s) {                                           // columns past K are zeros
-        float* as = ring + (s & 1) * kStage;
-        float* bs = as + BM * kTilePad;
-        const int k = ((s / kSteps) * kGroups + group) * kSliceK + (s % kSteps) * BK + 4 * (tid & 3);
+        if (s < steps) {
+            float* as = ring + (s % kStages) * kStage;
+            float* bs = as + BM * kTilePad;
+            const int k = ((s / kSteps) * NG + group) * kSliceK + (s % kSteps) * BK + 4 * (tid & 3);
 #pragma unroll
-        for (int i = 0; i < BM / 16; ++i) {
-            const int r = (tid >> 2) + 16 * i;
-            f32_stage4<VEC>(as + r * kTilePad + 4 * (tid & 3), A + (int64_t)min(m0 + r, M - 1) * lda, k, K, m0 + r < M);
-        }
+            for (int i = 0; i < BM / 16; ++i) {
+                const int r = (tid >> 2) + 16 * i;
+                f32_stage4<VEC>(as + r * kTilePad + 4 * (tid & 3), A + (int64_t)min(m0 + r, M - 1) * lda, k, K, m0 + r < M);
+            }
 #pragma unroll
-        for (int i = 0; i < BN / 16; ++i) {
-            const int r = (tid >> 2) + 16 * i;
-            f32_stage4<VEC>(bs + r * kTilePad + 4 * (tid & 3), W + (int64_t)min(n0 + r, N - 1) * ldw, k, K, n0 + r < N);
+            for (int i = 0; i < BN / 16; ++i) {
+                const int r = (tid >> 2) + 16 * i;
+                f32_stage4<VEC>(bs + r * kTilePad + 4 * (tid & 3), W + (int64_t)min(n0 + r, N - 1) * ldw, k, K, n0 + r < N);
+            }
         }
         f32_cp_commit();
     };
-    stage(0);
+#pragma unroll
+    for (int s = 0; s < kStages - 1; ++s) stage(s);
     float total[RI][kOwn], acc[RI][8];
 #pragma unroll
     for (int i = 0; i < RI; ++i) {
@@ -180,11 +186,11 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, f
         for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
     }
     for (int s = 0; s < steps; ++s) {
-        f32_cp_wait<0>();
-        asm volatile("bar.sync %0, 64;" :: "r"(group + 1) : "memory");      // the stage has arrived; the other one has been used
-        if (s + 1 < steps) stage(s + 1);
-        const float* as = ring + (s & 1) * kStage + ty * kTilePad;
-        const float* bs = ring + (s & 1) * kStage + (BM + tx) * kTilePad;
+        f32_cp_wait<kStages - 2>();
+        asm volatile("bar.sync %0, 64;" :: "r"(group + 1) : "memory");      // the stage has arrived; the one before it has been used
+        stage(s + kStages - 1);
+        const float* as = ring + (s % kStages) * kStage + ty * kTilePad;
+        const float* bs = ring + (s % kStages) * kStage + (BM + tx) * kTilePad;
 #pragma unroll
         for (int k = 0; k < BK; k += 4) {
             float4 b[8];
@@ -203,23 +209,33 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, f
                 for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a.w, b[j].w, acc[i][j]);
             }
         }
-        if ((s + 1) % kSteps != 0) continue;
+        if ((s + 1) % kSteps != 0 && (NG > 1 || s + 1 < steps)) continue;
         // a round's slices are complete (those past the last are zeros)
-#pragma unroll
-        for (int i = 0; i < RI; ++i)
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                trade[((group * RI + i) * 8 + j) * kGroupThreads + tid] = acc[i][j];
-                acc[i][j] = 0.f;
-            }
-        __syncthreads();
-#pragma unroll
-        for (int g = 0; g < kGroups; ++g)
+        if constexpr (NG == 1) {
 #pragma unroll
             for (int i = 0; i < RI; ++i)
 #pragma unroll
-                for (int j = 0; j < kOwn; ++j) total[i][j] += trade[((g * RI + i) * 8 + group * kOwn + j) * kGroupThreads + tid];
-        __syncthreads();
+                for (int j = 0; j < 8; ++j) {
+                    total[i][j] += acc[i][j];
+                    acc[i][j] = 0.f;
+                }
+        } else {
+#pragma unroll
+            for (int i = 0; i < RI; ++i)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    trade[((group * RI + i) * 8 + j) * kGroupThreads + tid] = acc[i][j];
+                    acc[i][j] = 0.f;
+                }
+            __syncthreads();
+#pragma unroll
+            for (int g = 0; g < NG; ++g)
+#pragma unroll
+                for (int i = 0; i < RI; ++i)
+#pragma unroll
+                    for (int j = 0; j < kOwn; ++j) total[i][j] += trade[((g * RI + i) * 8 + group * kOwn + j) * kGroupThreads + tid];
+            __syncthreads();
+        }
     }
 #pragma unroll
     for (int i = 0; i < RI; ++i) {
@@ -233,15 +249,15 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, f
     }
 }
 
-template <bool VEC, int RI>
+template <bool VEC, int RI, int NG = kGroups>
 static int launch_tile(const float* A, const float* W, float* C, int M, int N, int K, int64_t lda, int64_t ldw, int64_t ldc, float alpha,
                        cudaStream_t stream) {
     static bool done[kMaxDevices];
-    const int rc = ensure_dynamic_smem(gemm_f32_tile_kernel<VEC, RI>, (int)tile_smem_bytes<RI>(), done);
+    const int rc = ensure_dynamic_smem(gemm_f32_tile_kernel<VEC, RI, NG>, (int)tile_smem_bytes<RI, NG>(), done);
     if (rc != CPM_OK) return rc;
     const dim3 grid((N + BN - 1) / BN, (M + 8 * RI - 1) / (8 * RI));
     if (grid.y > 65535) return CPM_BAD_ARGUMENT;
-    gemm_f32_tile_kernel<VEC, RI><<<grid, kTileThreads, tile_smem_bytes<RI>(), stream>>>(A, W, C, M, N, K, lda, ldw, ldc, alpha);
+    gemm_f32_tile_kernel<VEC, RI, NG><<<grid, NG * kGroupThreads, tile_smem_bytes<RI, NG>(), stream>>>(A, W, C, M, N, K, lda, ldw, ldc, alpha);
     return launch_status();
 }
 
@@ -265,10 +281,16 @@ static int launch_gemm_f32(const float* A, const float* W, float* C, int M, int 
     if (M <= 2) return launch_few_rows<2, VEC>(A, W, C, M, N, K, lda, ldw, ldc, alpha, stream);
     if (M <= 4) return launch_few_rows<4, VEC>(A, W, C, M, N, K, lda, ldw, ldc, alpha, stream);
     if (M <= 8) return launch_few_rows<8, VEC>(A, W, C, M, N, K, lda, ldw, ldc, alpha, stream);
-    if (M <= 16) return launch_few_rows<16, VEC>(A, W, C, M, N, K, lda, ldw, ldc, alpha, stream);
-    // rounds of one block an SM, times the rows of a block
+    const bool short_k = K <= 2 * kSliceK;               // (of which the kernel for few rows has little to share among its threads)
+    if (M <= 16 && !short_k) return launch_few_rows<16, VEC>(A, W, C, M, N, K, lda, ldw, ldc, alpha, stream);
     const int sms = device_sms();
     if (sms < 1) return CPM_BAD_ARGUMENT;
+    // One or two slices leave three or two of four groups idle (N 1,000, K 64: 17 rows 10.0 us, 2,048 rows 33.0): a group alone sums them,
+    // several blocks an SM, of half the rows where there are not two of them for every SM (4.5 and 12.2).
+    if (short_k)
+        return (int64_t)((M + 63) / 64) * ((N + BN - 1) / BN) >= 2 * sms ? launch_tile<VEC, 8, 1>(A, W, C, M, N, K, lda, ldw, ldc, alpha, stream)
+                                                                       : launch_tile<VEC, 4, 1>(A, W, C, M, N, K, lda, ldw, ldc, alpha, stream);
+    // rounds of one block an SM, times the rows of a block
     auto cost = [&](int ri) {
         const int64_t tiles = (int64_t)((M + 8 * ri - 1) / (8 * ri)) * ((N + BN - 1) / BN);
         return (tiles + sms - 1) / sms * ri;

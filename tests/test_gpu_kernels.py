@@ -92,7 +92,7 @@ def test_gemm_f32(M, N, K):
     assert torch.equal(one[0], got[0])
 
 
-@pytest.mark.parametrize("K", [63, 64, 65, 1023, 1024, 1028, 3100])
+@pytest.mark.parametrize("K", [63, 64, 65, 127, 128, 129, 1023, 1024, 1028, 3100])
 def test_gemm_f32_rows_agree_across_kernels(K):
     """The few-row kernels (1, 2, 4, 8 and 16 rows), the tile kernel (more) and both ways of loading sum in one order: a row
     is the same to the last bit whatever the batch.  Bound: K FMAs in slices of 64, so below K/64 + 64 roundings of 2^-24
@@ -109,7 +109,7 @@ def test_gemm_f32_rows_agree_across_kernels(K):
 
 
 @pytest.mark.parametrize("M,N", [(640, 1024), (592, 1280), (1100, 1216), (33, 130)])
-@pytest.mark.parametrize("K", [20, 200, 260])
+@pytest.mark.parametrize("K", [20, 64, 68, 128, 132, 200, 260])
 def test_gemm_f32_heights_of_tiles(M, N, K):
     """Sizes that take 80, 96 and 64 rows a tile on 148 SMs, ragged at every edge, fewer slices than groups and a round that is not
     full: the bits of the few-row kernels, and 64-bit products."""
@@ -943,6 +943,21 @@ def test_launches_of_expert_products_are_counted_as_they_are():
         assert launches(200) == 3
     finally:
         ops.lib.cpm_set_moe_tensor_cores(1)
+
+
+@pytest.mark.parametrize("vocab", [1000, 4095, 4096, 4099, 32767, 32772, 73449])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_greedy_choice_is_the_first_of_equals(vocab, shift):
+    """Rows below and above the length from which they come in 16-byte loads, that begin on such a boundary and that do not, the largest
+    number twice: in the same load, in neighbouring ones, a whole turn of the block apart, in what is left at the end."""
+    ops = _ops("bfloat16")
+    g = torch.Generator().manual_seed(vocab)
+    pairs = [(0, 1), (3, 4), (5, vocab - 1), (vocab - 2, vocab - 1), (vocab // 2, vocab // 2 + 7), (2, min(vocab - 1, 32770)), (511, vocab - 3)]
+    z = torch.randn(len(pairs), vocab, generator=g)
+    for row, (a, b) in enumerate(pairs):
+        z[row, [a, b]] = 9.0
+    dev = torch.empty(z.numel() + shift, device="cuda")[shift:].view(z.shape).copy_(z)
+    assert ops.sample(dev).tolist() == [min(p) for p in pairs]
 
 
 @pytest.mark.parametrize("K,N", [(1, 8), (63, 40), (513, 128), (576, 136), (1151, 24)])
