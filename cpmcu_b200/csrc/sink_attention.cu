@@ -656,18 +656,21 @@ sink_attention_tiles_kernel(const bf16* __restrict__ q, const bf16* __restrict__
 // warp asks for its next two steps' keys and values together, asynchronously, those of all pages but the sequence's last before the
 // kernel ahead is waited for (an earlier step wrote them, as the plain decode attention has it), and the keys go to enough blocks
 // that a warp has a step or two.  Keys, then values, one step after the other and three steps a warp: 20.4 us a launch
-// for one token, 15.4 us for four with 500 to 3,000 keys.
-constexpr int kSinkTokenWarps = 4, kSinkTokenStages = 2;
-template <int D, int DV> struct SinkTokenStage {
+// for one token, 15.4 us for four with 500 to 3,000 keys.  Where a batch has more blocks than the SMs hold with two steps a warp in shared
+// memory (one an SM at head size 128), one step a warp and more blocks hide the latency better: 128 tokens of 100 keys, 4 kv
+// heads of 128, 11.5 us against 19.0 (13.3 with loads into registers), of 1,000 keys 58 and 74; 64 tokens of 1,000 keys, heads of 64, fit
+// with two (16.8 us, 19.0 with one).
+constexpr int kSinkTokenWarps = 4;
+template <int D, int DV, int STAGES> struct SinkTokenStage {
     static constexpr int kKeyChunks = D / 8;                       // 16-byte pieces of a key
     static constexpr int kKeyBytes = 32 * D * 2, kBytes = kKeyBytes + 32 * DV * 2;
     static constexpr bool kSwizzleKeys = kKeyChunks % 8 == 0;
     static constexpr int kJoin = (kSinkTokenWarps - 1) * 16 * (DV + 1) * 4;      // the warps' outputs when they join, in the stages' place
-    static constexpr int kRing = kSinkTokenWarps * kSinkTokenStages * kBytes;
+    static constexpr int kRing = kSinkTokenWarps * STAGES * kBytes;
     static constexpr int kSmem = kRing > kJoin ? kRing : kJoin;
 };
 
-template <int D, int DV>
+template <int D, int DV, int STAGES>
 __global__ void __launch_bounds__(kSinkTokenWarps * 32)
 sink_attention_token_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_cache, const bf16* __restrict__ v_cache,
                             bf16* __restrict__ out, const int* __restrict__ positions, const int* __restrict__ token_seq,
@@ -675,7 +678,7 @@ sink_attention_token_kernel(const bf16* __restrict__ q, const bf16* __restrict__
                             int keep_first, int n_heads, int n_kv, float scale, float cap, int sink,
                             const float* __restrict__ sinks, const float* __restrict__ gate, int64_t gate_stride,
                             float* __restrict__ shares, int one_token) {
-    using S = SinkTokenStage<D, DV>;
+    using S = SinkTokenStage<D, DV, STAGES>;
     extern __shared__ __align__(128) unsigned char token_smem[];
     float (*part_o)[16][DV + 1] = reinterpret_cast<float (*)[16][DV + 1]>(token_smem);
     __shared__ float part_ml[kSinkTokenWarps - 1][16][2];
@@ -699,14 +702,14 @@ sink_attention_token_kernel(const bf16* __restrict__ q, const bf16* __restrict__
     const int share = (max(0, blk_end - blk_begin) + kSinkTokenWarps - 1) / kSinkTokenWarps;
     const int b_begin = blk_begin + warp * share, b_end = min(blk_end, b_begin + share);
     auto first_key = [&](int b) { return b < kept_steps ? 32 * b : first + 32 * (b - kept_steps); };
-    const uint32_t ring = (uint32_t)__cvta_generic_to_shared(token_smem) + warp * kSinkTokenStages * S::kBytes;
+    const uint32_t ring = (uint32_t)__cvta_generic_to_shared(token_smem) + warp * STAGES * S::kBytes;
     auto issue = [&](int b) {
         if (b < b_end) {
             const int key0 = first_key(b), off = key0 % kPageTokens;
             const int page = CPM_PAGE(pages, key0 / kPageTokens, max_pages);
             const bf16* kp = k_cache + page_row_offset(page, kvh, off, n_kv, D);
             const bf16* vp = v_cache + value_offset(page, kvh, 0, off, n_kv, DV);
-            const uint32_t stage = ring + ((b - b_begin) % kSinkTokenStages) * S::kBytes;
+            const uint32_t stage = ring + ((b - b_begin) % STAGES) * S::kBytes;
 #pragma unroll 8
             for (int c = lane; c < 32 * S::kKeyChunks; c += 32) {
                 const int row = c / S::kKeyChunks, col = c % S::kKeyChunks;
@@ -723,12 +726,12 @@ sink_attention_token_kernel(const bf16* __restrict__ q, const bf16* __restrict__
     const int last_page = p / kPageTokens;
     bool early = one_token != 0;
 #pragma unroll
-    for (int b = 0; b < kSinkTokenStages; ++b) early = early && (b_begin + b >= b_end || first_key(b_begin + b) / kPageTokens != last_page);
+    for (int b = 0; b < STAGES; ++b) early = early && (b_begin + b >= b_end || first_key(b_begin + b) / kPageTokens != last_page);
     if (early)
-        for (int b = 0; b < kSinkTokenStages; ++b) issue(b_begin + b);
+        for (int b = 0; b < STAGES; ++b) issue(b_begin + b);
     pdl_wait();
     if (!early)
-        for (int b = 0; b < kSinkTokenStages; ++b) issue(b_begin + b);
+        for (int b = 0; b < STAGES; ++b) issue(b_begin + b);
     uint4 qf[2][D / 32];
     int lo[2], hi[2];
 #pragma unroll
@@ -745,9 +748,9 @@ sink_attention_token_kernel(const bf16* __restrict__ q, const bf16* __restrict__
     st.init();
     const int krow = 8 * (g >> 1) + (g & 1);
     for (int b = b_begin; b < b_end; ++b) {
-        cp_async_wait<kSinkTokenStages - 1>();
+        cp_async_wait<STAGES - 1>();
         __syncwarp();
-        const uint32_t stage = ring + ((b - b_begin) % kSinkTokenStages) * S::kBytes;
+        const uint32_t stage = ring + ((b - b_begin) % STAGES) * S::kBytes;
         sink_attend_keys<D, DV>(st, qf,
                                 [&](int t, int w) {
                                     const int row = krow + 2 * t, col = 4 * w + j;
@@ -756,7 +759,7 @@ sink_attention_token_kernel(const bf16* __restrict__ q, const bf16* __restrict__
                                 [&](int nt) { return lds16(stage + S::kKeyBytes + ((8 * nt + g) * 4 + j) * 16); },
                                 first_key(b), lo, hi, keep_first, scale, cap, lane);
         __syncwarp();
-        issue(b + kSinkTokenStages);
+        issue(b + STAGES);
     }
     cp_async_wait<0>();
     __syncthreads();                                               // the stages have been used: their place is free
@@ -906,15 +909,22 @@ static int launch_sink_bf16(const void* q, const void* k_cache, const void* v_ca
                    gate_stride);
     } else {
         const int group = n_heads / n_kv;
-        auto kern = sink_attention_token_kernel<D, DV>;
-        constexpr int smem = SinkTokenStage<D, DV>::kSmem;
-        static bool configured[kMaxDevices] = {};            // per kernel and per device
-        if (int st = ensure_dynamic_smem(kern, smem, configured)) return st;
-        cpm_launch(kLaunchAttention, kern,
-                   dim3(n_tokens, n_kv * ((group + 15) / 16), n_splits), dim3(kSinkTokenWarps * 32), smem, stream, (const bf16*)q,
-                   (const bf16*)k_cache, (const bf16*)v_cache, (bf16*)out, positions, token_seq, slots, page_table, max_pages,
-                   window, keep_first, n_heads, n_kv, scale, cap, sink, sinks, gate, gate_stride,
-                   n_splits > 1 ? shares : (float*)nullptr, one_token);
+        const dim3 grid(n_tokens, n_kv * ((group + 15) / 16), n_splits);
+        auto start = [&](auto kern, int smem, bool* configured) -> int {
+            if (int st = ensure_dynamic_smem(kern, smem, configured)) return st;
+            cpm_launch(kLaunchAttention, kern, grid, dim3(kSinkTokenWarps * 32), smem, stream, (const bf16*)q, (const bf16*)k_cache,
+                       (const bf16*)v_cache, (bf16*)out, positions, token_seq, slots, page_table, max_pages, window, keep_first, n_heads,
+                       n_kv, scale, cap, sink, sinks, gate, gate_stride, n_splits > 1 ? shares : (float*)nullptr, one_token);
+            return CPM_OK;
+        };
+        static bool configured[2][kMaxDevices] = {};         // per kernel and per device
+        // two steps ahead where all blocks fit the SMs at once with room for two, else one ahead and twice the blocks an SM (see above)
+        using Two = SinkTokenStage<D, DV, 2>;
+        using One = SinkTokenStage<D, DV, 1>;
+        const bool at_once = (int64_t)grid.x * grid.y * grid.z <= (int64_t)(227 * 1024 / Two::kSmem) * device_sms();
+        if (int st = at_once ? start(sink_attention_token_kernel<D, DV, 2>, Two::kSmem, configured[0])
+                             : start(sink_attention_token_kernel<D, DV, 1>, One::kSmem, configured[1]))
+            return st;
         if (n_splits > 1) {
             const int n_rows = n_tokens * n_heads;
             cpm_launch(kLaunchAttention, sink_combine_shares_kernel, dim3((n_rows + 3) / 4), dim3(128), 0, stream,

@@ -960,6 +960,43 @@ def test_greedy_choice_is_the_first_of_equals(vocab, shift):
     assert ops.sample(dev).tolist() == [min(p) for p in pairs]
 
 
+@pytest.mark.parametrize("H,G,d,dv", [(8, 4, 128, 128), (8, 4, 64, 64), (16, 8, 32, 32), (4, 4, 96, 32)])
+@pytest.mark.parametrize("window", [0, 200])
+def test_sink_attention_of_large_batches(H, G, d, dv, window):
+    """More single tokens than the SMs hold blocks with two steps in shared memory (300 sequences), of 1 to 700 keys: the bits of
+    small batches, which take the kernel with two, and the kernel of every size on a part of them."""
+    from cpmcu_b200.cache import Cache
+    from cpmcu_b200.parts.base import CacheNeeds, StepContext
+
+    ops = _ops("bfloat16")
+    g = torch.Generator().manual_seed(d + dv)
+    lens = [1 + (37 * i) % 700 for i in range(300)]
+    n = len(lens)
+    cache = Cache([CacheNeeds(kv_heads=G, head_dim=d, value_dim=dv if dv != d else 0)], max_tokens=sum(64 * ((m + 63) // 64) for m in lens), dtype=torch.bfloat16,
+                  device="cuda:0", n_slots=n)
+    slots = cache.open_sequences(n)
+    for s, m in zip(slots, lens):
+        cache.reserve(s, m)
+    cache.sync()
+    lane = cache.lane(0)
+    lane.k.copy_(torch.randn(lane.k.shape, generator=g).bfloat16())
+    lane.v.copy_(torch.randn(lane.v.shape, generator=g).bfloat16())
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32).cuda()
+    q = torch.randn(n, H, d, generator=g).bfloat16().cuda()
+
+    def run(lo, hi, fn):
+        ctx = StepContext(n_tokens=hi - lo, n_seqs=hi - lo, is_decode=True, captured=False, q_lens=[1] * (hi - lo), kv_lens=lens[lo:hi], slots=slots[lo:hi],
+                          max_q_len=1, max_kv_len=max(lens[lo:hi]), token_ids=i32([0] * (hi - lo)), positions=i32([m - 1 for m in lens[lo:hi]]),
+                          token_seq=i32(list(range(hi - lo))), cu_q=i32(list(range(hi - lo + 1))), kv_len_dev=i32(lens[lo:hi]), slot_dev=i32(slots[lo:hi]), cache=cache)
+        return fn(ctx, q[lo:hi].contiguous(), lane, G, dv, d ** -0.5, window, 20.0, True, 16 if window else 0, None, None)
+
+    ops.sink_attention_splits = lambda *a: 1
+    whole = run(0, n, ops.sink_attention_bf16)
+    for lo in (0, 100, 295):
+        assert torch.equal(run(lo, lo + 5, ops.sink_attention_bf16), whole[lo:lo + 5])
+        assert _err(run(lo, lo + 5, ops.sink_attention_generic), whole[lo:lo + 5]) < KTOL["bfloat16"]
+
+
 @pytest.mark.parametrize("K,N", [(1, 8), (63, 40), (513, 128), (576, 136), (1151, 24)])
 @pytest.mark.parametrize("n", [1, 2, 3, 8, 9, 16, 17])
 def test_head_project_of_few_tokens(K, N, n):
