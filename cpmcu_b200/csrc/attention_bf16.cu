@@ -342,92 +342,31 @@ __device__ __forceinline__ void put_new_token(unsigned char* stage, const bf16* 
     }
 }
 
-// How a decode step's pages are shared out.  The sequences of a batch differ in length, and a step ends with its slowest block, so
-// they are cut into shares of one size: the smallest ``pages`` a share (from ``least`` on) with which all sequences together
-// need at most ``budget`` shares, each sequence at most kMaxShares.  Every block works that out from the lengths, before it
-// waits for the kernel ahead.  (An equal number of shares a sequence: 64 sequences of 500 to 8000 tokens, 2 kv heads of 64, took 29.9 us
-// a layer, as long as one SM needs for the longest sequence; 8 of 513 to 4085 tokens, 2 kv heads of 128, 8.5 us.)
-constexpr int kMaxShares = 32;
-struct DecodeShare { int seq, index, count, pages; };      // share ``index`` of the ``count`` of sequence ``seq``; seq -1: none
-
-// Where that is not worth its search, a sequence's pages are cut into n_splits shares, less where they do not fill them: at head
-// size 128 with one block an SM and several shares a sequence, the search (about a microsecond where the block cannot start before
-// the kernel ahead ends) ate what it gave (8 sequences of 513 to 4085 tokens: 28.3 ms for eight steps of the 8B sizes against 27.3).
-__host__ __device__ constexpr bool decode_by_size(int d, int n_splits) { return n_splits > 1 && d == 64; }
-__device__ __forceinline__ DecodeShare equal_decode_share(const int* __restrict__ kv_len, int seq, int index, int n_splits) {
-    const int pages = max(1, (__ldg(kv_len + seq) + kPageTokens - 1) / kPageTokens), per = (pages + n_splits - 1) / n_splits;
-    DecodeShare s{seq, index, (pages + per - 1) / per, per};
-    if (index >= s.count) s.seq = -1;
-    return s;
-}
-
-__device__ __forceinline__ int pages_of_sequence(const int* __restrict__ kv_len, int b) {
-    return max(1, (__ldg(kv_len + b) + kPageTokens - 1) / kPageTokens);
-}
-
-// Pages a share; a warp's work.
-__device__ __forceinline__ int decode_share_pages(const int* __restrict__ kv_len, int n, int budget, int least, int lane) {
-    auto pages_of = [&](int b) { return pages_of_sequence(kv_len, b); };
-    int total = 0, longest = 0;
-    for (int b = lane; b < n; b += 32) {
-        const int p = pages_of(b);
-        total += p;
-        longest = max(longest, p);
-    }
-    total = __reduce_add_sync(0xffffffffu, total);
-    longest = __reduce_max_sync(0xffffffffu, longest);
-    auto shares = [&](int pages) {
-        int c = 0;
-        for (int b = lane; b < n; b += 32) c += (pages_of(b) + pages - 1) / pages;
-        return __reduce_add_sync(0xffffffffu, c);
-    };
-    int lo = max(least, max((total + budget - 1) / budget, (longest + kMaxShares - 1) / kMaxShares));
-    if (shares(lo) > budget) {                             // (one share a sequence always fits: budget >= n)
-        int hi = budget > n ? min(longest, (total + budget - n - 1) / (budget - n)) : longest;
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (shares(mid) > budget) lo = mid; else hi = mid;
-        }
-        lo = hi;
-    }
-    return lo;
-}
-
-__device__ __forceinline__ DecodeShare find_decode_share(const int* __restrict__ kv_len, int n, int budget, int least, int x, int lane) {
-    const int lo = decode_share_pages(kv_len, n, budget, least, lane);
-    DecodeShare s{-1, 0, 0, lo};
-    int before = 0;
-    for (int b0 = 0; b0 < n; b0 += 32) {
-        const int b = b0 + lane, own = b < n ? (pages_of_sequence(kv_len, b) + lo - 1) / lo : 0;
-        int upto = own;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, upto, o);
-            if (lane >= o) upto += v;
-        }
-        const unsigned past = __ballot_sync(0xffffffffu, x < before + upto);
-        if (past) {
-            const int src = __ffs(past) - 1;
-            s.seq = b0 + src;
-            s.count = __shfl_sync(0xffffffffu, own, src);
-            s.index = x - (before + __shfl_sync(0xffffffffu, upto, src) - s.count);
-            return s;
-        }
-        before += __shfl_sync(0xffffffffu, upto, 31);
-    }
-    return s;
-}
-
-// Warps of a decode block: three fill an SM's shared memory at head size 128; at head size 64 they fill half of it, and two blocks
-// an SM overlap one's start and merge with the other's pages.
-template <int D> struct DecodeBlock {
-    static constexpr int kWarps = D == 64 ? 3 : DecodeSmem<D>::kWarps;
-    static constexpr int kPerSm = D == 64 ? 2 : 1;
-    static constexpr int kSmem = kWarps * kDecodeStages * DecodeSmem<D>::kStageBytes;
-};
-
+// How a decode step's pages are shared out: a sequence's pages in ``n_splits`` shares of one size, fewer where a share would have less than
+// kLeastPages.  At head size 64 that is nine, three for each of a block's warps: adding up shares costs a block about 3 us, as long as ten pages
+// take (a step of 24 layers, one sequence of 300, 500, 1,000 and 4,000 tokens: 589, 608, 684 and 702 us; with six pages 589, 657, 673, 683; with
+// three 648, 648, 666, 692; eight sequences of 500: 675, 701, 705).  Equal numbers of shares, not equal sizes over the whole batch: cutting all
+// sequences into shares of one size, found on the device from their lengths, gained 1 % where 64 sequences have 500 to 8,000 tokens and lost
+// up to 12 % on batches of equal or short ones (64 of 500: 1,122 us a step against 1,009), and made a row's bits depend on its
+// neighbours' lengths.
+constexpr int kMaxShares = 32;                             // what the last of a sequence's blocks has room to add up
+template <int D> constexpr int kLeastPages = D == 64 ? 9 : 1;
+struct DecodeShare { int pages, count; };                  // pages a share, and the shares that hold any
 template <int D>
-__global__ void __launch_bounds__(DecodeBlock<D>::kWarps * 32, DecodeBlock<D>::kPerSm)
+__device__ __forceinline__ DecodeShare decode_share(int kv_len, int n_splits) {
+    const int pages = max(1, (kv_len + kPageTokens - 1) / kPageTokens), per = max(kLeastPages<D>, (pages + n_splits - 1) / n_splits);
+    return DecodeShare{per, (pages + per - 1) / per};
+}
+
+// Warps of a decode block: at head size 128 three fill an SM's shared memory, at 96 four, at 32 eight.  At head size 64 three fill half of it,
+// and two blocks an SM overlap one's start and merge with the other's pages; six, one block an SM, where every block has a whole
+// sequence and there is at most one for an SM (64 sequences of 4,000 tokens, 2 kv heads: 22 us a layer, against 26 as two shares of three
+// warps each).
+template <int D> constexpr int kDecodeWarps = D == 64 ? 3 : DecodeSmem<D>::kWarps;
+template <int D, int W> constexpr int kDecodePerSm = D == 64 && W == 3 ? 2 : 1;
+
+template <int D, int kWarps>
+__global__ void __launch_bounds__(kWarps * 32, kDecodePerSm<D, kWarps>)
 decode_attention_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_cache, const bf16* __restrict__ v_cache,
                         const int* __restrict__ kv_len, const int* __restrict__ slots,
                         const int* __restrict__ page_table, int max_pages, float* __restrict__ part_o,
@@ -437,7 +376,6 @@ decode_attention_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_c
     // share and merge their results in shared memory before anything is written.  Where a sequence is one share
     // the block writes the final result to ``out`` itself; else, with ``arrivals`` (a zeroed counter per sequence and head tile,
     // left zeroed), the block that finishes last adds up the shares, and without, a kernel behind this one.
-    constexpr int kWarps = DecodeBlock<D>::kWarps;
     using S = DecodeSmem<D>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ float sm_m[kWarps][16], sm_l[kWarps][16];
@@ -452,15 +390,13 @@ decode_attention_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_c
     // Lengths, slots, page numbers and every page but the sequence's last were written by earlier steps (or by the
     // host before this one): they are read, and the first pages asked for, before this kernel waits for the
     // one ahead of it, which writes only the step's own token (into the last page) and q.
-    const DecodeShare share = decode_by_size(D, n_splits) ? find_decode_share(kv_len, n_seqs, n_seqs * n_splits, kWarps, blockIdx.x, lane)
-                                                          : equal_decode_share(kv_len, blockIdx.x / n_splits, blockIdx.x % n_splits, n_splits);
-    const int b = share.seq;
-    if (b < 0) return;
-    const int bv = blockIdx.z * n_seqs + b;
+    const int b = blockIdx.x / n_splits, index = blockIdx.x % n_splits;
     const int len = kv_len[b];
+    const DecodeShare share = decode_share<D>(len, n_splits);
+    if (index >= share.count) return;
+    const int bv = blockIdx.z * n_seqs + b;
     const int n_pages = (len + kPageTokens - 1) / kPageTokens;
-    const int per = share.pages;
-    const int p0 = share.index * per, p1 = min(n_pages, p0 + per);
+    const int p0 = index * share.pages, p1 = min(n_pages, p0 + share.pages);
     const int* pages = page_table + (int64_t)slots[b] * max_pages;
     const uint32_t my_stages = (uint32_t)__cvta_generic_to_shared(smem_raw) + warp * kDecodeStages * S::kStageBytes;
     const int64_t page_elems = (int64_t)n_kv * kPageTokens * D;
@@ -593,53 +529,72 @@ decode_attention_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_c
         }
     }
     if (share.count == 1 || arrivals == nullptr) return;
-    // ---- the last of a sequence's blocks adds up the shares ----
-    __threadfence();
+    // ---- the last of a sequence's blocks adds up the shares: statistics and the first eight shares' sums are asked for together ----
+    // (one thread's fence stands for the block: the barrier orders the block's writes before it, and the other reads behind it)
     __syncthreads();
     int* last = reinterpret_cast<int*>(sm_l);                          // (its sums have been used)
     if (threadIdx.x == 0) {
         int* counter = arrivals + ((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * n_seqs + b;
+        __threadfence();
         const bool mine = atomicAdd(counter, 1) == share.count - 1;
         if (mine) *counter = 0;
         *last = mine;
+        __threadfence();
     }
     __syncthreads();
     if (!*last) return;
-    __threadfence();
-    float* weight = reinterpret_cast<float*>(smem_raw);                // [count][16]: a share's part in a row's result
-    float* ml = weight + kMaxShares * 16;                              // [count][32]
-    const int64_t first = unit - share.index;
-    const int rows = min(16, group - mt * 16);
-    for (int i = threadIdx.x; i < share.count * 32; i += kWarps * 32) ml[i] = __ldcg(part_ml + first * 32 + i);
-    __syncthreads();
-    for (int i = threadIdx.x; i < share.count * 16; i += kWarps * 32) {
-        const int row = i & 15, s = i >> 4;
-        float mx = -INFINITY, l = 0.f;
-        for (int k = 0; k < share.count; ++k) mx = fmaxf(mx, ml[k * 32 + 2 * row]);
-        const float use = mx == -INFINITY ? 0.f : mx;
-        for (int k = 0; k < share.count; ++k) l = fmaf(ml[k * 32 + 2 * row + 1], exp2f(ml[k * 32 + 2 * row] - use), l);
-        weight[i] = l > 0.f ? exp2f(ml[s * 32 + 2 * row] - use) / l : 0.f;
+    constexpr int kRows = (16 + kWarps - 1) / kWarps, kQuads = D / 4;
+    float* weight = reinterpret_cast<float*>(smem_raw);                // [row][kMaxShares]: a share's part in a row's result
+    const int64_t first = unit - index;
+    const int rows = min(16, group - mt * 16), items = rows * kQuads;
+    float2 ml[kRows];                                                  // a lane holds a share's statistics of the warp's rows
+#pragma unroll
+    for (int u = 0; u < kRows; ++u) {
+        const int row = warp + u * kWarps;
+        ml[u] = row < rows && lane < share.count ? __ldcg(reinterpret_cast<const float2*>(part_ml + (first + lane) * 32 + 2 * row)) : make_float2(-INFINITY, 0.f);
+    }
+    const float* sums = part_o + first * 16 * D;
+    auto fetch = [&](float4 (&o)[8], int item, int s0) {               // row item / kQuads, columns from 4 (item % kQuads) on
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            o[u] = item < items && s0 + u < share.count ? __ldcg(reinterpret_cast<const float4*>(sums + (int64_t)(s0 + u) * 16 * D + item * 4))
+                                                        : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    float4 o[2][8];                                                    // two items at a time
+    fetch(o[0], threadIdx.x, 0);
+    fetch(o[1], threadIdx.x + kWarps * 32, 0);
+#pragma unroll
+    for (int u = 0; u < kRows; ++u) {
+        const int row = warp + u * kWarps;
+        const float mx = warp_max(ml[u].x), w = exp2f(ml[u].x - (mx == -INFINITY ? 0.f : mx)), l = warp_sum(ml[u].y * w);
+        if (row < rows) weight[row * kMaxShares + lane] = l > 0.f ? w / l : 0.f;
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < rows * (D / 4); i += kWarps * 32) {
-        const int row = i / (D / 4), c = (i % (D / 4)) * 4;
-        const float* src = part_o + (first * 16 + row) * D + c;
-        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int s0 = 0; s0 < share.count; s0 += 8) {                  // eight shares in flight
-            float4 o[8];
+    for (int i0 = threadIdx.x; i0 < items; i0 += 2 * kWarps * 32) {
+        float4 acc[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
+        for (int s0 = 0; s0 < share.count; s0 += 8) {
+            if (i0 != (int)threadIdx.x || s0) {
+                fetch(o[0], i0, s0);
+                fetch(o[1], i0 + kWarps * 32, s0);
+            }
 #pragma unroll
-            for (int u = 0; u < 8; ++u)
-                o[u] = s0 + u < share.count ? __ldcg(reinterpret_cast<const float4*>(src + (s0 + u) * 16 * D)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int h = 0; h < 2; ++h) {
+                const float* wr = weight + min(i0 + h * kWarps * 32, items - 1) / kQuads * kMaxShares + s0;
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const float w = s0 + u < share.count ? weight[(s0 + u) * 16 + row] : 0.f;
-                acc.x = fmaf(o[u].x, w, acc.x);
-                acc.y = fmaf(o[u].y, w, acc.y);
-                acc.z = fmaf(o[u].z, w, acc.z);
-                acc.w = fmaf(o[u].w, w, acc.w);
+                for (int u = 0; u < 8; ++u) {
+                    const float w = s0 + u < share.count ? wr[u] : 0.f;
+                    acc[h].x = fmaf(o[h][u].x, w, acc[h].x);
+                    acc[h].y = fmaf(o[h][u].y, w, acc[h].y);
+                    acc[h].z = fmaf(o[h][u].z, w, acc[h].z);
+                    acc[h].w = fmaf(o[h][u].w, w, acc[h].w);
+                }
             }
         }
-        store4(out + ((int64_t)bv * n_heads + kvh * group + mt * 16 + row) * D + c, acc);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int i = i0 + h * kWarps * 32;
+            if (i < items) store4(out + ((int64_t)bv * n_heads + kvh * group + mt * 16) * D + i * 4, acc[h]);
+        }
     }
 }
 
@@ -660,18 +615,9 @@ combine_shares_kernel(const float* __restrict__ part_o, const float* __restrict_
     int count = n_splits;
     int64_t first = ((int64_t)row * units + unit) * n_splits;
     if (kv_len != nullptr) {
-        int before = b * n_splits;
-        if (decode_by_size(D, n_splits)) {
-            const int pages = decode_share_pages(kv_len, n_seqs, n_seqs * n_splits, DecodeBlock<D>::kWarps, lane);
-            count = (pages_of_sequence(kv_len, b) + pages - 1) / pages;
-            before = 0;
-            for (int i = lane; i < b; i += 32) before += (pages_of_sequence(kv_len, i) + pages - 1) / pages;
-            before = __reduce_add_sync(0xffffffffu, before);
-        } else {
-            count = equal_decode_share(kv_len, b, 0, n_splits).count;
-        }
+        count = decode_share<D>(kv_len[b], n_splits).count;
         if (count == 1) return;
-        first = ((int64_t)(row / n_seqs) * units + unit) * n_seqs * n_splits + before;
+        first = ((int64_t)(row / n_seqs) * units + unit) * n_seqs * n_splits + (int64_t)b * n_splits;
     }
     const float* ml = part_ml + first * 32 + 2 * r;
     const int c = (lane % kCols) * 4, sub = lane / kCols;
@@ -731,7 +677,7 @@ CPM_API int64_t cpm_decode_attention_scratch_floats(int n_seqs, int n_heads, int
 }
 
 // Blocks of the decode kernel an SM holds.
-CPM_API int cpm_decode_attention_blocks_per_sm(int d) { return d == 64 ? DecodeBlock<64>::kPerSm : 1; }
+CPM_API int cpm_decode_attention_blocks_per_sm(int d) { return d == 64 ? kDecodePerSm<64, kDecodeWarps<64>> : 1; }
 
 template <int D>
 static int launch_decode(const void* q, const void* k_cache, const void* v_cache, void* out, const int* kv_len,
@@ -745,17 +691,25 @@ static int launch_decode(const void* q, const void* k_cache, const void* v_cache
     const int64_t shares = (int64_t)n_seqs * n_splits;
     if (shares > 0x7fffffff) return CPM_BAD_ARGUMENT;
     // the block that adds up a sequence's shares has room for the weights of kMaxShares
-    if (arrivals != nullptr && n_splits > kMaxShares && !decode_by_size(D, n_splits)) return CPM_BAD_ARGUMENT;
+    if (arrivals != nullptr && n_splits > kMaxShares) return CPM_BAD_ARGUMENT;
     float* part_o = scratch;
     float* part_ml = scratch + shares * runs * n_kv * m_tiles * 16 * D;
-    auto kern = decode_attention_kernel<D>;
     rope.early = g_decode_early;
-    constexpr int smem = DecodeBlock<D>::kSmem;
-    static bool configured[kMaxDevices] = {};            // per kernel and per device
-    if (int st = ensure_dynamic_smem(kern, smem, configured)) return st;
-    cpm_launch(kLaunchAttention, kern, dim3((unsigned)shares, n_kv * m_tiles, runs), DecodeBlock<D>::kWarps * 32, smem, stream, (const bf16*)q,
-               (const bf16*)k_cache, (const bf16*)v_cache, kv_len, slots, page_table, max_pages, part_o, part_ml, arrivals, (bf16*)out,
-               n_seqs, n_heads, n_kv, m_tiles, n_splits, scale * 1.4426950408889634f, rope, v_shift, runs);
+    auto start = [&](auto kern, int warps, bool* configured) -> int {      // configured: per kernel and per device
+        const int smem = warps * kDecodeStages * DecodeSmem<D>::kStageBytes;
+        if (int st = ensure_dynamic_smem(kern, smem, configured)) return st;
+        cpm_launch(kLaunchAttention, kern, dim3((unsigned)shares, n_kv * m_tiles, runs), warps * 32, smem, stream, (const bf16*)q, (const bf16*)k_cache,
+                   (const bf16*)v_cache, kv_len, slots, page_table, max_pages, part_o, part_ml, arrivals, (bf16*)out, n_seqs, n_heads, n_kv,
+                   m_tiles, n_splits, scale * 1.4426950408889634f, rope, v_shift, runs);
+        return CPM_OK;
+    };
+    static bool configured[2][kMaxDevices] = {};
+    int st;
+    if (D == 64 && n_splits == 1 && (int64_t)n_rows * n_kv * m_tiles <= device_sms())
+        st = start(decode_attention_kernel<D, DecodeSmem<D>::kWarps>, DecodeSmem<D>::kWarps, configured[1]);
+    else
+        st = start(decode_attention_kernel<D, kDecodeWarps<D>>, kDecodeWarps<D>, configured[0]);
+    if (st != CPM_OK) return st;
     if (n_splits > 1 && arrivals == nullptr)
         cpm_launch(kLaunchCombine, combine_shares_kernel<D>, dim3((n_heads + 3) / 4, n_rows), 128, 0, stream, (const float*)part_o,
                    (const float*)part_ml, kv_len, (bf16*)out, n_seqs, n_heads, n_kv, m_tiles, n_splits);
@@ -763,8 +717,8 @@ static int launch_decode(const void* q, const void* k_cache, const void* v_cache
 }
 
 // q [n_seqs, heads, d] bf16, one token per sequence; out [n_seqs, heads, d] bf16.  arrivals: null, or n_seqs * n_kv * ceil(group / 16) (times
-// the runs) counters that are zero, are zero again when the kernel ends, and belong to no other kernel meanwhile (at head sizes other than
-// 64 for up to 32 shares a sequence: without them the shares are added up by a kernel of its own, which takes any number).
+// the runs) counters that are zero, are zero again when the kernel ends, and belong to no other kernel meanwhile (for up to 32 shares a
+// sequence: without them the shares are added up by a kernel of its own, which takes any number).
 CPM_API int cpm_decode_attention_bf16(const void* q, const void* k_cache, const void* v_cache, void* out,
                                       const int* kv_len, const int* slots, const int* page_table, int max_pages,
                                       float* scratch, int n_seqs, int n_heads, int n_kv, int d, int n_splits,

@@ -807,26 +807,28 @@ class Ops:
 
     # ---- bf16 tensor-core attention ----
     def decode_splits(self, n_seqs: int, n_heads: int, n_kv: int, d: int = 0) -> int:
-        """How many shares a sequence's pages are cut into, on average (the decode attention gives long sequences more): the
-        kernel holds one block per SM (its page buffers fill the shared memory; with ``d`` the number the decode kernel
-        holds at that head size), so aim at one wave of blocks, but where an SM holds several blocks and one wave is
-        about one share a sequence at two, so that there are shares to give to the long ones (with one block an SM, 64 equal
-        sequences of the 8B sizes lost 7 % to the second share)."""
+        """How many shares a sequence's pages are cut into (fewer where it has few): one wave of blocks.  The kernel holds one
+        block per SM (its page buffers fill the shared memory), the decode kernel at head size ``d`` 64 two of half the size; but a
+        sequence that would be one share of a block that fills an SM stays one there too (64 sequences of 4,000 tokens, 2 kv heads:
+        1,465 us a step of 24 layers, 1,543 as two shares)."""
         m_tiles = (n_heads // n_kv + 15) // 16
         units = max(1, n_seqs * n_kv * m_tiles)
-        room = self.sm_count * (self.lib.cpm_decode_attention_blocks_per_sm(d) if d else 1)
-        wave = max(1, min(self.MAX_DECODE_SPLITS, room // units))
-        return min(2, 2 * room // units) if room > self.sm_count and wave == 1 and room >= units else wave
+        per_sm = self.lib.cpm_decode_attention_blocks_per_sm(d) if d else 1
+        if self.sm_count // units == 1:
+            per_sm = 1
+        return max(1, min(self.MAX_DECODE_SPLITS, self.sm_count * per_sm // units))
+
+    MAX_JOINED_SHARES = 32      # what the last of a sequence's blocks has room to add up
 
     def _arrivals(self, rows: int, n_heads: int, n_kv: int, d: int, n_splits: int) -> Optional[torch.Tensor]:
         """Counters with which the decode attention's blocks find out which of them is the last of its sequence and adds up
-        the shares, so that no kernel for that has to follow (it cost 3.4 us a layer at one sequence, 4.5 us at eight).
-        Launches that share them must follow one another: they are given only where a workspace is attached, whose memory
-        asks for the same; elsewhere, or with more rows than there are counters, the shares are added up by a kernel of its own.
+        the shares, so that no kernel for that has to follow.  Launches that share them must follow one another: they are given only
+        where a workspace is attached, whose memory asks for the same; elsewhere, with more rows than there are counters, or with more
+        shares than the last block has room for, the shares are added up by a kernel of its own.
         So they are at head sizes above 64, where a block's three warps take longer for 16 rows of the shares than that kernel
-        (8 sequences of the 8B sizes: 29.3 against 28.3 ms for eight steps).  And so are more shares a sequence than the last
-        block has room for the weights of (at head size 64 the kernel keeps to that by itself)."""
-        if d > 64 or (n_splits > 32 and d != 64) or self.workspace is None or self.arrivals is None or rows * n_kv * ((n_heads // n_kv + 15) // 16) > self.arrivals.numel():
+        (8 sequences of the 8B sizes: 29.3 against 28.3 ms for eight steps)."""
+        if (d > 64 or n_splits > self.MAX_JOINED_SHARES or self.workspace is None or self.arrivals is None
+                or rows * n_kv * ((n_heads // n_kv + 15) // 16) > self.arrivals.numel()):
             return None
         return self.arrivals
 
