@@ -1054,6 +1054,42 @@ def test_decode_attention_shares_of_ragged_batches(n_heads, n_kv, d, lens):
         assert not ops.arrivals.any()
 
 
+@pytest.mark.parametrize("n_heads,n_kv,d", [(16, 2, 64), (6, 3, 64), (40, 2, 64), (8, 2, 32)])
+def test_last_block_adds_up_shares_behind_rotation_and_with_shifted_values(n_heads, n_kv, d):
+    """The entries that turn the queries themselves, that take another head's values and that do several runs at once: shares added up by
+    the last block of a sequence (a workspace is attached) against a kernel of its own (none is), with as many sequences of one share."""
+    from types import SimpleNamespace
+
+    from cpmcu_b200.cache import Cache
+    from cpmcu_b200.parts.base import CacheNeeds
+
+    ops = _ops("bfloat16")
+    lens = [1, 577, 1300, 64, 3000, 640]
+    n, g = len(lens), torch.Generator().manual_seed(n_heads + d)
+    c = Cache([CacheNeeds(kv_heads=n_kv, head_dim=d)], max_tokens=64 * 100, dtype=torch.bfloat16, device="cuda:0", n_slots=n)
+    slots = c.open_sequences(n)
+    for s, m in zip(slots, lens):
+        c.reserve(s, m)
+    c.sync()
+    lane = c.lane(0)
+    lane.k.copy_(torch.randn(lane.k.shape, generator=g).bfloat16())
+    lane.v.copy_(torch.randn(lane.v.shape, generator=g).bfloat16())
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32).cuda()
+    q = torch.randn(n, n_heads, d, generator=g).bfloat16().cuda()
+    qkv = torch.randn(n, (n_heads + 2 * n_kv) * d, generator=g).bfloat16().cuda()
+    inv_freq = (1.0 / (10000.0 ** (torch.arange(0, d, 2, dtype=torch.float32) / d))).cuda()
+    args = (lane.k, lane.v, i32(lens), i32(slots), lane.page_table, n_kv, d ** -0.5)
+    entries = [lambda: ops.decode_attention(q, *args, n_splits=16, v_shift=1), lambda: ops.decode_attention(q, *args, n_splits=16, v_runs=n_kv)]
+    if d == 64:
+        entries.append(lambda: ops.decode_attention_rope(qkv, lane, i32(lens), i32(slots), n_heads, n_kv, d, d ** -0.5, inv_freq, 1.1, False, n_splits=16))
+    want = [f().clone() for f in entries]
+    ops.workspace = SimpleNamespace(alloc=lambda shape, dtype: torch.empty(*shape, dtype=dtype, device="cuda"))
+    for _ in range(2):
+        for f, w in zip(entries, want):
+            assert _err(f(), w) < 2.0 ** -8                # the same shares, added up in another order, rounded once
+            assert not ops.arrivals.any()
+
+
 @pytest.mark.parametrize("H,G,d,dv", [(1, 1, 1, 4), (6, 3, 31, 36), (4, 4, 64, 128), (2, 1, 100, 64), (3, 3, 256, 8), (2, 2, 128, 6)])
 @pytest.mark.parametrize("delta,vector", [(False, False), (False, True), (True, False), (True, True)])
 def test_recurrence_of_one_token_a_sequence(H, G, d, dv, delta, vector):
