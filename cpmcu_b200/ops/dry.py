@@ -182,24 +182,25 @@ def workspace_steps(max_step_tokens: int, max_batch: int, max_seq_tokens: int, p
     while b < max_batch:
         b *= 2
     steps = []
-    for n in sorted({T, max(1, T // 2)} | {min(T, p) for p in (512, 256, 255, 3 * sm_count // 2, 128, 95, 64, 63)}):
+    # (a step of an eighth of the tokens fits wherever the full one does, whatever its scratch)
+    for n in sorted({T, max(1, T // 2)} | {p for p in (512, 256, 255, 3 * sm_count // 2, 128, 95, 64, 63) if T > p > T // 8}):
         if n in (T, max(1, T // 2)):
             steps.append((_evenly(n, min(n, max_batch)), max_seq_tokens, False, False, None))
         uneven = {tuple(_most_tiles(n, b, longest)) for longest in (Ops.RETENTION_TILE_MIN_TOKENS, Ops.MINGRU_TILE_MIN_TOKENS)}
         uneven.add(tuple(_half_full_tiles(n, b)))
-        for portions in sorted(uneven | {(n,)}):
-            for kv in {min(max(max(portions), k), max_seq_tokens) for k in ((0, 4096, 8192) if len(portions) == 1 else (0,))} | {max_seq_tokens}:
-                steps.append((list(portions), kv, False, False, None))
-    steps.append(([T], max_seq_tokens, False, True, None))
-    if packed_pieces and b >= packed_pieces + 1 and T > packed_pieces:
-        steps.append((_evenly(T, packed_pieces + 1), max_seq_tokens, False, True, T // PREFILL_TILE_ROWS + packed_pieces))
-    size = 1
-    while size <= b:                                        # a captured decode step of every bucket; eager ones of as many sequences
+        for portions in sorted(uneven - {(n,)}):
+            steps.append((list(portions), max_seq_tokens, False, False, None))
+        for kv in {min(max(n, k), max_seq_tokens) for k in (0, 8192)} | {max_seq_tokens}:
+            steps.append(([n], kv, False, False, None))
+    if packed_pieces:
+        steps.append(([T], max_seq_tokens, False, True, None))
+        if b >= packed_pieces + 1 and T > packed_pieces:
+            steps.append((_evenly(T, packed_pieces + 1), max_seq_tokens, False, True, T // PREFILL_TILE_ROWS + packed_pieces))
+    for size in sorted({b, max(1, b // 2), max(1, b // 4), min(b, 8), 1}):      # captured decode steps; eager ones of as many sequences
         steps.append(([1] * size, max_seq_tokens, True, True, None))
-        size *= 2
+    steps.append(([1] * max(1, b - 1), 1, True, False, None))
     for size in sorted({max_batch, b, max(1, b - 1)}):
-        for kv in (1, max_seq_tokens):
-            steps.append(([1] * size, kv, True, False, None))
+        steps.append(([1] * size, max_seq_tokens, True, False, None))
     return steps
 
 
@@ -223,8 +224,6 @@ def measure_workspace(spec, dtype: torch.dtype, max_step_tokens: int, max_batch:
     recorded = model.recordable_prompt()
     notes: List[str] = []
     for q_lens, kv, decode, captured, n_tiles in workspace_steps(max_step_tokens, max_batch, per_seq, MAX_GRAPH_PIECES if recorded else 0, sm_count):
-        if captured and not decode and not recorded:
-            continue
         n_tokens = sum(q_lens)
         ops.workspace.begin_step()
         try:
