@@ -1086,7 +1086,9 @@ def test_last_block_adds_up_shares_behind_rotation_and_with_shifted_values(n_hea
     ops.workspace = SimpleNamespace(alloc=lambda shape, dtype: torch.empty(*shape, dtype=dtype, device="cuda"))
     for _ in range(2):
         for f, w in zip(entries, want):
-            assert _err(f(), w) < 2.0 ** -8                # the same shares, added up in another order, rounded once
+            # the same shares added up in another order: sums that differ by a rounding of 2^-24 may fall on two sides of a bf16 border, one
+            # unit in the last place apart, which is at most 2^-7 of the number
+            assert _err(f(), w) <= 2.0 ** -7
             assert not ops.arrivals.any()
 
 
