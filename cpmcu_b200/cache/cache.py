@@ -24,6 +24,7 @@ from typing import Dict, List, Optional, Sequence
 
 import torch
 
+from ..memory import Staging
 from ..parts.base import PAGE_TOKENS, CacheNeeds
 from .allocator import CacheFull, FreeList, HandleError
 
@@ -119,16 +120,19 @@ class CacheGroup:
         self.first_live[slot] = dead
         return dead - first
 
-    def sync(self) -> None:
-        """Brings the device's page table up to date (pageable staging: no later host
-        write can reach a copy that is still queued)."""
+    def sync(self, staging: Staging) -> None:
+        """Brings the device's page table up to date, behind what is queued on the current stream.  The rows are staged together;
+        the host does not wait (a decode step that takes a page did, for everything queued before it)."""
+        rows, values = [], []
         for slot, first in self._dirty.items():
             pages = self.pages_of_slot[slot]
             first = max(first, self.first_live.get(slot, 0)) if first >= self.kept_pages else first
             if first >= len(pages):
                 continue
-            row = torch.tensor([max(p, 0) for p in pages[first:]], dtype=torch.int32)      # a released page: no kernel follows it
-            self.page_table[slot, first:len(pages)].copy_(row)
+            rows.append((slot, first, len(pages)))
+            values.extend(max(p, 0) for p in pages[first:])                                # a released page: no kernel follows it
+        if rows:
+            staging.copy(torch.tensor(values, dtype=torch.int32), [self.page_table[slot, first:end] for slot, first, end in rows])
         self._dirty.clear()
 
 
@@ -170,6 +174,7 @@ class Cache:
         state_region / page_region: regions of an arena (cpmcu_b200.memory) that hold the page tables and the
         per-sequence state, and the pages; without them the tensors come from torch's allocator."""
         self.device = torch.device(device)
+        self.staging = Staging(self.device)           # by which the host's numbers reach the device: page tables, and a step's description
         make = None
         if state_region is not None or page_region is not None:
             def make(kind, shape, dt, zero):
@@ -212,17 +217,25 @@ class Cache:
 
     # ---- sequences ----
     def open_sequence(self) -> int:
-        slot = self.slots.take(1)[0]
-        self.lengths[slot] = 0
-        for lane in self.lanes:
-            for t in lane.state.values():
-                t[slot].zero_()
-        return slot
+        return self.open_sequences(1)[0]
 
     def open_sequences(self, n: int) -> List[int]:
         if n > self.slots.n_free:
             raise CacheFull(f"{n} sequences wanted, {self.slots.n_free} of {self.n_slots} slots free")
-        return [self.open_sequence() for _ in range(n)]
+        slots = self.slots.take(n)
+        for slot in slots:
+            self.lengths[slot] = 0
+        runs = []                                          # of neighbouring slots, which are cleared together: [first, end)
+        for slot in slots:
+            if runs and runs[-1][1] == slot:
+                runs[-1][1] = slot + 1
+            else:
+                runs.append([slot, slot + 1])
+        for lane in self.lanes:
+            for t in lane.state.values():
+                for first, end in runs:
+                    t[first:end].zero_()
+        return slots
 
     def reserve(self, slot: int, new_length: int) -> None:
         """Makes room for the sequence to hold ``new_length`` tokens (all or nothing)."""
@@ -299,7 +312,7 @@ class Cache:
 
     def sync(self) -> None:
         for g in self.groups:
-            g.sync()
+            g.sync(self.staging)
 
     def lane(self, i: int) -> Lane:
         return self.lanes[i]

@@ -15,6 +15,7 @@ from __future__ import annotations
 
 from typing import Dict, List, Optional, Sequence
 
+import numpy as np
 import torch
 
 from ..parts.base import StepContext
@@ -33,18 +34,15 @@ class _Bucket:
     def __init__(self, size: int, device: torch.device):
         i32 = dict(dtype=torch.int32, device=device)
         self.size = size
-        self.ids = torch.zeros(size, **i32)
-        self.positions = torch.zeros(size, **i32)
-        self.kv_len = torch.ones(size, **i32)
-        self.slot = torch.zeros(size, **i32)
+        # what a batch begins with lies in the rows of one tensor (each on a 16-byte boundary), so that one copy brings it
+        self.block = torch.zeros(9, (size + 3) // 4 * 4, **i32)
+        self.ids, self.positions, self.kv_len, self.slot, self.live, self.seq_key, self.step_key = (row[:size] for row in self.block[:7])
+        self.temperature, self.top_p = (row[:size] for row in self.block[7:].view(torch.float32))
+        self.kv_len.fill_(1)
+        self.top_p.fill_(1.0)
         self.token_seq = torch.arange(size, **i32)
         self.cu_q = torch.arange(size + 1, **i32)
         self.want_rows = torch.arange(size, **i32)
-        self.live = torch.zeros(size, **i32)
-        self.seq_key = torch.zeros(size, **i32)
-        self.step_key = torch.zeros(size, **i32)
-        self.temperature = torch.zeros(size, dtype=torch.float32, device=device)
-        self.top_p = torch.ones(size, dtype=torch.float32, device=device)
         self.sampled = torch.zeros(size, **i32)
         self.logits: Optional[torch.Tensor] = None
         self.graph: Optional[torch.cuda.CUDAGraph] = None
@@ -145,17 +143,20 @@ class DecodeRunner:
         n = len(slots)
         b = self._bucket(n)
         self._prepare(b)
-        pad = b.size - n
         lengths = [self.cache.length(s) for s in slots]
-        host = torch.tensor(
-            list(last_tokens) + [0] * pad + lengths + [0] * pad + [l + 1 for l in lengths] + [1] * pad
-            + list(slots) + [self.pad_slot] * pad + [1] * n + [0] * pad + list(seq_keys) + [0] * pad
-            + list(step_keys) + [0] * pad, dtype=torch.int32).view(7, b.size).to(self.ops.device)
-        b.ids.copy_(host[0]); b.positions.copy_(host[1]); b.kv_len.copy_(host[2]); b.slot.copy_(host[3])
-        b.live.copy_(host[4]); b.seq_key.copy_(host[5]); b.step_key.copy_(host[6])
-        fl = torch.tensor([p.temperature for p in sampling] + [0.0] * pad + [p.top_p for p in sampling] + [1.0] * pad,
-                          dtype=torch.float32).view(2, b.size).to(self.ops.device)
-        b.temperature.copy_(fl[0]); b.top_p.copy_(fl[1])
+        if any(len(v) != n for v in (last_tokens, seq_keys, step_keys, sampling)):
+            raise ValueError(f"a batch of {n} sequences needs as many tokens, keys and sampling parameters")
+        host = np.zeros(tuple(b.block.shape), dtype=np.int32)          # padding: token 0, position 0, not live
+        host[2] = 1                                                    # one key
+        host[3] = self.pad_slot
+        for row, values in ((0, last_tokens), (1, lengths), (2, [length + 1 for length in lengths]), (3, slots), (4, 1),
+                            (5, seq_keys), (6, step_keys)):
+            host[row, :n] = values
+        real = host[7:].view(np.float32)
+        real[1] = 1.0
+        real[0, :n] = [p.temperature for p in sampling]
+        real[1, :n] = [p.top_p for p in sampling]
+        self.cache.staging.copy(torch.from_numpy(host).view(-1), [b.block.view(-1)])
         self.current = b
         self.slots = list(slots)
 

@@ -181,7 +181,7 @@ class Stepper:
         g = self.prompt_graphs[(n, len(want_rows), self._length_bound(start + n), False)]
         host = np.concatenate([tokens, np.arange(start, start + n, dtype=np.int32),
                                np.asarray([start + n, slot] + list(want_rows), dtype=np.int32)])
-        g.inputs.copy_(torch.from_numpy(host))
+        self.cache.staging.copy(torch.from_numpy(host), [g.inputs])
         g.graph.replay()
         return None if g.logits is None else g.logits.clone()
 
@@ -329,7 +329,7 @@ class Stepper:
                              ("tile_seq", ts), ("tile_row", tr)):
             o, length = lay[name]
             host[o:o + length] = values
-        g.inputs.copy_(torch.from_numpy(host))
+        self.cache.staging.copy(torch.from_numpy(host), [g.inputs])
         g.graph.replay()
         return None if g.logits is None else g.logits.clone()
 
@@ -365,7 +365,7 @@ class Stepper:
             np.asarray(kv_lens, dtype=np.int32), np.asarray(slots, dtype=np.int32), np.asarray(want_rows, dtype=np.int32),
             tile_seq, tile_row.astype(np.int32)]).astype(np.int32, copy=False))
         dev = self.ops.empty(packed.numel(), dtype=torch.int32)
-        dev.copy_(packed)                     # pageable staging: the copy is over when this returns
+        self.cache.staging.copy(packed, [dev])      # the host goes on: this chunk's launches meet the last one's work
         o = 0
 
         def cut(n: int) -> torch.Tensor:

@@ -32,7 +32,7 @@ def nbytes_of(shape: Sequence[int], dtype: torch.dtype) -> int:
     n = 1
     for s in shape:
         n *= int(s)
-    return n * torch.empty((), dtype=dtype).element_size()
+    return n * dtype.itemsize
 
 
 class PoolExhausted(MemoryError):
@@ -99,6 +99,7 @@ class Arena:
             self.buffer = raw[skip:skip + self.total]
         self.regions: Dict[str, Region] = {}
         self.carved = 0
+        self._typed: Dict[torch.dtype, torch.Tensor] = {}      # the buffer's whole elements of each type a tensor was asked of
 
     def carve(self, name: str, nbytes: Optional[int]) -> Region:
         """The next region, ``nbytes`` long (None: unbounded, in a counting arena only)."""
@@ -135,7 +136,17 @@ class Arena:
     def view(self, at: int, nbytes: int, shape: Tuple[int, ...], dtype: torch.dtype, zero: bool) -> torch.Tensor:
         if self.buffer is None:
             return torch.empty(shape, dtype=dtype, device="meta")
-        t = self.buffer[at:at + nbytes].view(dtype).view(shape)
+        base = self._typed.get(dtype)
+        if base is None:
+            size = dtype.itemsize
+            base = self._typed[dtype] = self.buffer[:self.buffer.numel() // size * size].view(dtype)
+        if at % dtype.itemsize:
+            raise RuntimeError(f"byte {at} of the arena is no place for {dtype}")
+        strides, n = [], 1
+        for s in reversed(shape):
+            strides.append(n)
+            n *= max(s, 1)
+        t = base.as_strided(shape, strides[::-1], base.storage_offset() + at // dtype.itemsize)       # one call of torch's, not three
         if zero:
             t.zero_()
         return t

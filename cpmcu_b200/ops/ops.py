@@ -33,13 +33,14 @@ def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_current_device = getattr(torch._C, "_cuda_getDevice", torch.cuda.current_device)       # (an Ops exists only where CUDA is initialised)
 
 
 def _current_stream() -> int:
     """Handle of the stream torch would launch on now (the raw query is an order of magnitude cheaper than
     building a Stream object for every kernel launch)."""
     if _raw_stream is not None:
-        return _raw_stream(torch.cuda.current_device())
+        return _raw_stream(_current_device())
     return torch.cuda.current_stream().cuda_stream
 
 

@@ -195,3 +195,16 @@ def test_guard_words_show_which_region_was_overrun():
     arena.buffer[a.offset + a.size + 3] = 0                 # one byte past frame0's end
     with pytest.raises(RuntimeError, match="behind region 'frame0'.*byte 3"):
         arena.check_guards()
+
+
+def test_opened_slots_are_cleared_together_and_others_left():
+    """Neighbouring and scattered slots: their state is zeros, the rest of the state as it was."""
+    c = Cache([CacheNeeds(state={"s": ((3,), torch.float32)})], max_tokens=64 * 8, dtype=torch.float32, device="cpu", n_slots=7)
+    first = c.open_sequences(6)
+    assert first == [0, 1, 2, 3, 4, 5]
+    state = c.lanes[0].state["s"]
+    state.fill_(5.0)
+    for s in (1, 3, 4):
+        c.close_sequence(s)
+    assert c.open_sequences(3) == [1, 3, 4]
+    assert [float(r.sum()) for r in state] == [15.0, 0.0, 15.0, 0.0, 0.0, 15.0, 15.0]

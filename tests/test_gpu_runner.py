@@ -70,3 +70,23 @@ def test_runner_logits_bucket_of_64(model_folders, dtype, graph):
     assert helpers.runner_parity(st, seqs, lens, check, graph) == 6
     assert count[0] == 64 + sum(extra)
     st.cache.check_consistent()
+
+
+@pytest.mark.parametrize("sizes", [[5, 0, 7], [8192, 1], [70_000, 3, 20_000]])
+def test_staged_copies_arrive_whole_behind_a_busy_stream(sizes):
+    """Three times round the ring of pinned buffers while the stream is busy: every copy holds what the host array held when it was
+    queued, in arrays smaller than a buffer, as large and larger."""
+    from cpmcu_b200.memory import Staging
+
+    staging, n = Staging(torch.device("cuda:0")), sum(sizes)
+    a = torch.randn(4096, 4096, device="cuda:0")
+    outs = []
+    for i in range(3 * Staging.BUFFERS + 1):
+        a = torch.tanh(a @ a)                                  # milliseconds of work in front of each copy
+        host = torch.arange(n, dtype=torch.int32) * (i + 1)
+        parts = [torch.zeros(s, dtype=torch.int32, device="cuda:0") for s in sizes]
+        staging.copy(host, parts)
+        host.zero_()                                           # the caller's array is its own again
+        outs.append(parts)
+    for i, parts in enumerate(outs):
+        assert torch.equal(torch.cat(parts).cpu(), torch.arange(n, dtype=torch.int32) * (i + 1)), i
