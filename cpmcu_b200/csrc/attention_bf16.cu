@@ -306,41 +306,62 @@ __device__ __forceinline__ void rotate8(uint4& lo, uint4& hi, const float (&cs)[
     hi = make_uint4(b[0], b[1], b[2], b[3]);
 }
 
-// The new token's key (rotated) and value into the stage that holds its page (so that this block attends to
-// it) and, if ``to_cache``, into the cache pages for later steps.  One warp; row = the token's place in its page.
+// The step's own token in a warp's registers: lane c holds dims c + 32 i of the key's first half and the same of its second, and
+// dims c + 32 i of the value.  Angles need the position alone and are worked out before the wait, the rows are asked for right behind it.
 template <int D>
-__device__ __forceinline__ void put_new_token(unsigned char* stage, const bf16* __restrict__ k_raw,
-                                              const bf16* __restrict__ v_raw, const float* __restrict__ inv_freq,
-                                              float magnitude, int pos, int row, bf16* __restrict__ k_page,
-                                              bf16* __restrict__ v_page, bool to_cache, int lane) {
-    using S = DecodeSmem<D>;
-    constexpr int kHalf = D / 2;
-    const int swz = S::kSwizzleKeys ? ((row & 1) << 2) : 0;
-    bf16* k_row = reinterpret_cast<bf16*>(stage);
-    for (int c = lane; c < kHalf; c += 32) {
-        float cs = 1.f, sn = 0.f;
-        if (inv_freq) {
-            sincosf((float)pos * inv_freq[c], &sn, &cs);
-            cs *= magnitude;
-            sn *= magnitude;
-        }
-        const float x = __bfloat162float(k_raw[c]), y = __bfloat162float(k_raw[c + kHalf]);
-        const bf16 xr = __float2bfloat16_rn(x * cs - y * sn), yr = __float2bfloat16_rn(x * sn + y * cs);
-        const int c2 = c + kHalf;
-        k_row[(row * S::kChunksPerKeyRow + ((c >> 3) ^ swz)) * 8 + (c & 7)] = xr;
-        k_row[(row * S::kChunksPerKeyRow + ((c2 >> 3) ^ swz)) * 8 + (c2 & 7)] = yr;
-        if (to_cache) {
-            k_page[row * D + c] = xr;
-            k_page[row * D + c2] = yr;
+struct NewToken {
+    static constexpr int kPairs = D >= 64 ? D / 64 : 1;
+    float cs[kPairs], sn[kPairs];
+    bf16 x[kPairs], y[kPairs], v[2 * kPairs];
+    __device__ __forceinline__ void angles(const float* __restrict__ inv_freq, float magnitude, int pos, int lane) {
+#pragma unroll
+        for (int i = 0; i < kPairs; ++i) {
+            cs[i] = 1.f;
+            sn[i] = 0.f;
+            if (inv_freq) {
+                sincosf((float)pos * inv_freq[lane + 32 * i], &sn[i], &cs[i]);
+                cs[i] *= magnitude;
+                sn[i] *= magnitude;
+            }
         }
     }
-    bf16* v_rows = reinterpret_cast<bf16*>(stage + S::kKeyBytes);
-    for (int dd = lane; dd < D; dd += 32) {
-        const bf16 v = v_raw[dd];
-        v_rows[(dd * 8 + ((row >> 3) ^ ((dd & 1) << 2))) * 8 + (row & 7)] = v;
-        if (to_cache) v_page[dd * kPageTokens + row] = v;
+    __device__ __forceinline__ void load(const bf16* __restrict__ k_raw, const bf16* __restrict__ v_raw, int lane) {
+#pragma unroll
+        for (int i = 0; i < kPairs; ++i) {
+            x[i] = k_raw[lane + 32 * i];
+            y[i] = k_raw[lane + 32 * i + D / 2];
+            v[2 * i] = v_raw[lane + 64 * i];
+            v[2 * i + 1] = v_raw[lane + 64 * i + 32];
+        }
     }
-}
+    // The key (rotated) and the value into the stage that holds their page, so that this block attends to them, and, if ``to_cache``, into
+    // the cache pages for later steps; row = the token's place in its page.
+    __device__ __forceinline__ void put(unsigned char* stage, int row, bf16* __restrict__ k_page, bf16* __restrict__ v_page, bool to_cache,
+                                        int lane) const {
+        using S = DecodeSmem<D>;
+        const int swz = S::kSwizzleKeys ? ((row & 1) << 2) : 0;
+        bf16* k_row = reinterpret_cast<bf16*>(stage);
+        bf16* v_rows = reinterpret_cast<bf16*>(stage + S::kKeyBytes);
+#pragma unroll
+        for (int i = 0; i < kPairs; ++i) {
+            const int c = lane + 32 * i, c2 = c + D / 2;
+            const float xf = __bfloat162float(x[i]), yf = __bfloat162float(y[i]);
+            const bf16 xr = __float2bfloat16_rn(xf * cs[i] - yf * sn[i]), yr = __float2bfloat16_rn(xf * sn[i] + yf * cs[i]);
+            k_row[(row * S::kChunksPerKeyRow + ((c >> 3) ^ swz)) * 8 + (c & 7)] = xr;
+            k_row[(row * S::kChunksPerKeyRow + ((c2 >> 3) ^ swz)) * 8 + (c2 & 7)] = yr;
+            if (to_cache) {
+                k_page[row * D + c] = xr;
+                k_page[row * D + c2] = yr;
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int dd = lane + 64 * i + 32 * h;
+                v_rows[(dd * 8 + ((row >> 3) ^ ((dd & 1) << 2))) * 8 + (row & 7)] = v[2 * i + h];
+                if (to_cache) v_page[dd * kPageTokens + row] = v[2 * i + h];
+            }
+        }
+    }
+};
 
 // How a decode step's pages are shared out: a sequence's pages in ``n_splits`` shares of one size, fewer where a share would have less than
 // kLeastPages.  At head size 64 that is nine, three for each of a block's warps: adding up shares costs a block about 3 us, as long as ten pages
@@ -411,8 +432,10 @@ decode_attention_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_c
         }
         cp_async_commit();
     };
-    // the warp whose first two pages include the last page waits first (its copies must stay in order)
-    const bool early = rope.early && p0 + warp != n_pages - 1 && p0 + warp + kWarps != n_pages - 1;
+    // the warp whose first two pages include the last page waits first (its copies must stay in order), but where this kernel itself puts
+    // the step's token there: the page's other rows are older than the step
+    const bool writes = rope.qkv && rope.write_cache;
+    const bool early = rope.early && (writes || (p0 + warp != n_pages - 1 && p0 + warp + kWarps != n_pages - 1));
     if (early) {
         issue(0);
         issue(1);
@@ -433,6 +456,10 @@ decode_attention_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_c
                 }
         }
     }
+    const bool owner = writes && p1 == n_pages && (n_pages - 1 - p0) % kWarps == warp;       // this warp's pages include the step's token's
+    NewToken<D> fresh;
+    if constexpr (D == 64 || D == 128)
+        if (owner) fresh.angles(rope.inv_freq, rope.magnitude, len - 1, lane);
     pdl_wait();
     if (!early) {
         issue(0);
@@ -460,18 +487,19 @@ decode_attention_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_c
             }
         }
     }
+    if constexpr (D == 64 || D == 128) {
+        const bf16* raw = rope.qkv + (int64_t)b * q_row_stride + (int64_t)(n_heads + kvh) * D;
+        if (owner) fresh.load(raw, raw + (int64_t)n_kv * D, lane);
+    }
     for (int k = 0; p0 + warp + k * kWarps < p1; ++k) {
         cp_async_wait<kDecodeStages - 1>();
         __syncwarp();
         const int p = p0 + warp + k * kWarps;
         if constexpr (D == 64 || D == 128) {
-            if (rope.qkv && rope.write_cache && p == n_pages - 1) {
-                // the step's own token is not in the cache yet: this warp holds its page and puts it there
-                const bf16* raw = rope.qkv + (int64_t)b * q_row_stride + (int64_t)(n_heads + kvh) * D;
+            if (owner && p == n_pages - 1) {
                 const int64_t base = (int64_t)CPM_PAGE(pages, p, max_pages) * page_elems + (int64_t)kvh * kPageTokens * D;
-                put_new_token<D>(smem_raw + (warp * kDecodeStages + (k % kDecodeStages)) * S::kStageBytes, raw,
-                                 raw + (int64_t)n_kv * D, rope.inv_freq, rope.magnitude, len - 1, (len - 1) % kPageTokens,
-                                 rope.k_out + base, rope.v_out + base, mt == 0, lane);
+                fresh.put(smem_raw + (warp * kDecodeStages + (k % kDecodeStages)) * S::kStageBytes, (len - 1) % kPageTokens, rope.k_out + base,
+                          rope.v_out + base, mt == 0, lane);
                 __syncwarp();
             }
         }

@@ -41,7 +41,7 @@ __device__ __forceinline__ void mma_16816_s(float (&c)[4], uint32_t a0, uint32_t
 // weights are used once: keep them out of L1
 __device__ __forceinline__ uint4 ld_stream16(const void* p) {
     uint4 v;
-    asm("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];\n"
+    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];\n"
                  : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
     return v;
 }
@@ -63,15 +63,22 @@ constexpr int kShortK = 1024;
 // 16,384 11.4 and 8.6.  Such a block takes an SM's whole register file and cannot be placed before the kernel ahead has left it, and at K of
 // 2,560 and 3,072 that costs more than it gives: 3.6 and 4.5, 4.9 and 5.3 us.
 constexpr int kManyWarpsK = 4096;
+// In a decode step's chain a product of a few MB lives for little more than latencies: of its launch, of its weights, of its activations.  So
+// the first kFlight steps' weights (all of them up to K 1,024 and, with eight steps, 2,048) are on their way into registers before the kernel
+// ahead has ended, and a grid whose blocks the SMs hold all at once (``let_go``) lets the next kernel's blocks in at its start, so that
+// these do the same; a grid of several waves would lose slots on the SMs to blocks that do nothing but wait, and lets them in
+// after its main loop.  us of a recorded decode step before, with let_go alone, with both: 0.5B one row 585, 577, 549, 16 rows
+// 862, 821, 787; 8B eight rows 3,305, 3,259, 3,244; Mufevik 1k 16 rows 647, 620, 597; Rabadra 2k four rows 707, 684, 671.
 template <int NT, int EPI, int kSkinnyWarps, bool kShort>
 __global__ void __launch_bounds__(kSkinnyWarps * 32, kShort ? (NT == 1 ? 4 : 3) : (NT == 1 || kSkinnyWarps > 8 ? 1 : 2))
 skinny_gemm_kernel(const bf16* __restrict__ W, const bf16* __restrict__ X, void* __restrict__ out, int M, int N, int K,
-                   float alpha, int prefetch_lines, GluClamp clamp) {
+                   float alpha, int prefetch_lines, int let_go, GluClamp clamp) {
     constexpr int MT = NT * 8;                          // token columns
     __shared__ float red[kSkinnyWarps][16][MT + 1];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, j = lane & 3;
     const int n0 = blockIdx.x * 16;
+    if (let_go) pdl_launch_dependents();
     // Before the kernel ahead of this one in the stream has finished, this block already asks for its
     // 16 weight rows to be brought into L2: weights are never written, and the tail of one product then
     // overlaps with the start of the next.
@@ -83,34 +90,62 @@ skinny_gemm_kernel(const bf16* __restrict__ W, const bf16* __restrict__ X, void*
             asm volatile("prefetch.global.L2 [%0];" :: "l"(p));
         }
     }
-    pdl_wait();
     // Rows beyond N and token columns beyond M read a valid row instead and their results are never
     // stored: rows of the product are independent, so no load needs a predicate.
     const bf16* w0 = W + (int64_t)min(n0 + g, N - 1) * K + 8 * j;
     const bf16* w1 = W + (int64_t)min(n0 + g + 8, N - 1) * K + 8 * j;
+    const int steps = K / 32;
+    constexpr int kFlight = kShort ? 4 : 8;                // K steps whose loads are in flight
+    // the first steps' weights are on their way into registers before the wait
+    uint4 lo[kFlight], hi[kFlight];
+#pragma unroll
+    for (int i = 0; i < kFlight; ++i) {
+        const int s = min(warp + i * kSkinnyWarps, steps - 1);
+        lo[i] = ld_stream16(w0 + 32 * s);
+        hi[i] = ld_stream16(w1 + 32 * s);
+    }
+    pdl_wait();
     const bf16* xp[NT];
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) xp[nt] = X + (int64_t)min(nt * 8 + g, M - 1) * K + 8 * j;
     float acc[NT][4];
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
-
-    const int steps = K / 32;
-    constexpr int kFlight = kShort ? 4 : 8;                // K steps whose loads are in flight
-#pragma unroll kFlight
-    for (int s = warp; s < steps; s += kSkinnyWarps) {
-        const uint4 lo = ld_stream16(w0 + 32 * s);
-        const uint4 hi = ld_stream16(w1 + 32 * s);
+    constexpr int kAtOnce = NT == 1 || kShort ? kFlight : kFlight / 2;       // steps whose activations are asked for together
 #pragma unroll
-        for (int nt = 0; nt < NT; ++nt) {
-            const uint4 b = __ldg(reinterpret_cast<const uint4*>(xp[nt] + 32 * s));
-            mma_16816_s(acc[nt], lo.x, hi.x, lo.y, hi.y, b.x, b.y);
-            mma_16816_s(acc[nt], lo.z, hi.z, lo.w, hi.w, b.z, b.w);
+    for (int i0 = 0; i0 < kFlight; i0 += kAtOnce) {
+        uint4 b[kAtOnce][NT];
+#pragma unroll
+        for (int i = 0; i < kAtOnce; ++i)
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt)
+                b[i][nt] = __ldg(reinterpret_cast<const uint4*>(xp[nt] + 32 * min(warp + (i0 + i) * kSkinnyWarps, steps - 1)));
+#pragma unroll
+        for (int i = 0; i < kAtOnce; ++i) {
+            const uint4 l = lo[i0 + i], h = hi[i0 + i];
+            if (warp + (i0 + i) * kSkinnyWarps < steps) {
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt) {
+                    mma_16816_s(acc[nt], l.x, h.x, l.y, h.y, b[i][nt].x, b[i][nt].y);
+                    mma_16816_s(acc[nt], l.z, h.z, l.w, h.w, b[i][nt].z, b[i][nt].w);
+                }
+            }
         }
     }
-    // Only now may the next kernel's blocks be placed: a grid of many waves would otherwise lose slots on the
-    // SMs to blocks that do nothing but wait.
-    pdl_launch_dependents();
+    if constexpr (!kShort) {
+#pragma unroll kFlight
+        for (int s = warp + kFlight * kSkinnyWarps; s < steps; s += kSkinnyWarps) {
+            const uint4 l = ld_stream16(w0 + 32 * s);
+            const uint4 h = ld_stream16(w1 + 32 * s);
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) {
+                const uint4 b = __ldg(reinterpret_cast<const uint4*>(xp[nt] + 32 * s));
+                mma_16816_s(acc[nt], l.x, h.x, l.y, h.y, b.x, b.y);
+                mma_16816_s(acc[nt], l.z, h.z, l.w, h.w, b.z, b.w);
+            }
+        }
+    }
+    if (!let_go) pdl_launch_dependents();
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
         red[warp][g][nt * 8 + 2 * j] = acc[nt][0];
@@ -167,16 +202,17 @@ skinny_gemm_kernel(const bf16* __restrict__ W, const bf16* __restrict__ X, void*
 template <int NT, int EPI>
 static int launch_skinny_epi(const void* W, const void* X, void* out, int M, int N, int K, float alpha,
                              const GluClamp& clamp, cudaStream_t stream) {
-    const unsigned blocks = (unsigned)((N + 15) / 16);
-    if (K >= kManyWarpsK && 2 * blocks <= (unsigned)device_sms())
-        cpm_launch(kLaunchProduct, skinny_gemm_kernel<NT, EPI, 16, false>, blocks, 512, 0, stream, (const bf16*)W, (const bf16*)X, out, M, N, K,
-                   alpha, g_skinny_prefetch_lines, clamp);
+    const unsigned blocks = (unsigned)((N + 15) / 16), sms = (unsigned)device_sms();
+    auto start = [&](auto kern, int warps, unsigned per_sm) {
+        cpm_launch(kLaunchProduct, kern, blocks, warps * 32, 0, stream, (const bf16*)W, (const bf16*)X, out, M, N, K, alpha,
+                   g_skinny_prefetch_lines, (int)(blocks <= per_sm * sms), clamp);       // per_sm: blocks an SM holds by their registers
+    };
+    if (K >= kManyWarpsK && 2 * blocks <= sms)
+        start(skinny_gemm_kernel<NT, EPI, 16, false>, 16, 1u);
     else if (K <= kShortK)
-        cpm_launch(kLaunchProduct, skinny_gemm_kernel<NT, EPI, 8, true>, blocks, 256, 0, stream, (const bf16*)W, (const bf16*)X, out, M, N, K,
-                   alpha, g_skinny_prefetch_lines, clamp);
+        start(skinny_gemm_kernel<NT, EPI, 8, true>, 8, NT == 1 ? 4u : 3u);
     else
-        cpm_launch(kLaunchProduct, skinny_gemm_kernel<NT, EPI, 8, false>, blocks, 256, 0, stream, (const bf16*)W, (const bf16*)X, out, M, N, K,
-                   alpha, g_skinny_prefetch_lines, clamp);
+        start(skinny_gemm_kernel<NT, EPI, 8, false>, 8, 2u);
     return launch_status();
 }
 

@@ -865,16 +865,18 @@ class Ops:
             LAUNCHES_EXTRA[0] += 1       # the launcher starts two kernels: the shares, then their combination
         return out
 
+    FUSED_ROPE_ROWS = 32
     FUSED_ROPE_HEAD_DIMS = (64, 128)      # head sizes whose rotary pairs lie in one thread's fragments of the decode kernel
 
     def fused_decode_ok(self, ctx, d: int, rot_dim: int, window: int, sparse) -> bool:
         """Whether a decode step's rotation and cache store are done by the attention kernel itself.  It saves a
-        launch, which counts where launches are what a step waits for (steps that are not recorded into a graph).
-        Inside a graph the separate rotary kernel overlaps with its neighbours and the fused kernel is 0.7 % slower
-        on the 8B decode step (3.537 against 3.501 ms at batch 8), so recorded steps keep the two kernels.
+        launch, which always counts in steps that are not recorded into a graph.  In recorded ones it does at head size 64 for up to
+        FUSED_ROPE_ROWS sequences (us a step of the 0.5B sizes, two kernels and one: 1 sequence 549 and 510, 8 750 and 718, 16 787 and
+        753, 32 1,243 and 1,218, 64 1,599 and 1,632).  At head size 128 a block's pages fill an SM beside the product ahead,
+        the separate kernel's launch hides behind that, and the fused one is slower (8B, batch 8: 3,268 against 3,244).
         CPMCU_FUSED_ROPE=1 / 0 forces the choice."""
         forced = os.environ.get("CPMCU_FUSED_ROPE")
-        want = (forced != "0") if forced is not None else not ctx.captured
+        want = (forced != "0") if forced is not None else not ctx.captured or (d == 64 and ctx.n_seqs <= self.FUSED_ROPE_ROWS)
         return (want and self.code == BF16 and ctx.is_decode and not window and sparse is None
                 and d in self.FUSED_ROPE_HEAD_DIMS and rot_dim in (0, d))
 

@@ -378,6 +378,30 @@ def test_skinny_gemm(M, N, K):
     assert torch.equal(one[0], got32[0])
 
 
+@pytest.mark.parametrize("M", [1, 8, 16])
+@pytest.mark.parametrize("N,K", [(64, 992), (40, 1056), (2384, 2016), (4720, 2080), (17, 4128), (9488, 1024), (1200, 6112)])
+def test_skinny_gemm_with_steps_asked_for_before_the_wait(M, N, K):
+    """One after the other in a chain of products (each reads what the one before wrote): K at the edges of what a warp asks for before it
+    waits (fewer steps than it has room for, one step more, several rounds), grids that let the next kernel in at once and grids of
+    more blocks than the SMs hold.  fp32 sums of K products in another order."""
+    ops = _ops("bfloat16")
+    ops.SKINNY_MAX_ROWS = 16
+    g = torch.Generator().manual_seed(K + M)
+    a = (torch.randn(M, K, generator=g) * 0.5).bfloat16().cuda()
+    w = (torch.randn(N, K, generator=g) * 0.05).bfloat16().cuda()
+    back = (torch.randn(K, N - N % 32, generator=g) * 0.05).bfloat16().cuda()
+    x = a
+    for _ in range(4):
+        h = ops.linear(x, w)
+        y = ops.linear(h[:, :N - N % 32].contiguous(), back, out_f32=True) if N >= 32 else None
+        want = (x.float() @ w.float().T)
+        assert _err(h, want) < KTOL["bfloat16"]
+        if y is None:
+            break
+        assert _err(y, h[:, :N - N % 32].float() @ back.float().T) < 2e-5
+        x = (y / y.abs().max()).bfloat16()
+
+
 def test_which_products_of_9_to_16_rows_take_the_weight_streaming_kernel():
     """At 9 to 16 rows the engine keeps a product on the weight-streaming kernel while the bytes its blocks read of
     the activations stay small: the QKV, O and down products of the 8B sizes, not gate_up, the head or 17 rows."""
