@@ -364,14 +364,20 @@ struct NewToken {
 };
 
 // How a decode step's pages are shared out: a sequence's pages in ``n_splits`` shares of one size, fewer where a share would have less than
-// kLeastPages.  At head size 64 that is nine, three for each of a block's warps: adding up shares costs a block about 3 us, as long as ten pages
-// take (a step of 24 layers, one sequence of 300, 500, 1,000 and 4,000 tokens: 589, 608, 684 and 702 us; with six pages 589, 657, 673, 683; with
-// three 648, 648, 666, 692; eight sequences of 500: 675, 701, 705).  Equal numbers of shares, not equal sizes over the whole batch: cutting all
+// kLeastPages.  At head size 64 that is three, one for each of a block's warps: a sequence's blocks are a cluster there, and adding up its
+// shares out of each other's shared memory takes about 1 us (through global memory, by the block that finishes last, 3 us; shares
+// had nine pages at least then).  us a step of 24 layers, last block and cluster: one sequence of 400, 1,000, 8,000 and 32,000 tokens 616 and
+// 542, 728 and 524, 758 and 616, 952 and 854; eight of 100 to 400 649 and 590, of 200 to 2,000 731 and 609; sixteen of 200 to
+// 3,000 862 and 711; with four pages at least one sequence of 1,000 551, with two eight of 100 to 400 591 against 587.  At head size 128 a
+// block fills an SM, a cluster finds its SMs later, and the kernel that adds up the shares is as fast (8B, batch 8: 3,247 and 3,257).
+// Equal numbers of shares, not equal sizes over the whole batch: cutting all
 // sequences into shares of one size, found on the device from their lengths, gained 1 % where 64 sequences have 500 to 8,000 tokens and lost
 // up to 12 % on batches of equal or short ones (64 of 500: 1,122 us a step against 1,009), and made a row's bits depend on its
-// neighbours' lengths.
+// neighbours' lengths.  (64 sequences as clusters of four: 500 to 8,000 tokens 1,595 -> 1,453, but 2,000 each 1,217 -> 1,362 and 60 to 500
+// 1,000 -> 1,046: they stay one block each.)
 constexpr int kMaxShares = 32;                             // what the last of a sequence's blocks has room to add up
-template <int D> constexpr int kLeastPages = D == 64 ? 9 : 1;
+constexpr int kClusterShares = 16;                         // the blocks of the largest cluster
+template <int D> constexpr int kLeastPages = D == 64 ? 3 : 1;
 struct DecodeShare { int pages, count; };                  // pages a share, and the shares that hold any
 template <int D>
 __device__ __forceinline__ DecodeShare decode_share(int kv_len, int n_splits) {
@@ -386,7 +392,7 @@ __device__ __forceinline__ DecodeShare decode_share(int kv_len, int n_splits) {
 template <int D> constexpr int kDecodeWarps = D == 64 ? 3 : DecodeSmem<D>::kWarps;
 template <int D, int W> constexpr int kDecodePerSm = D == 64 && W == 3 ? 2 : 1;
 
-template <int D, int kWarps>
+template <int D, int kWarps, bool kCluster>
 __global__ void __launch_bounds__(kWarps * 32, kDecodePerSm<D, kWarps>)
 decode_attention_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_cache, const bf16* __restrict__ v_cache,
                         const int* __restrict__ kv_len, const int* __restrict__ slots,
@@ -395,8 +401,9 @@ decode_attention_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_c
                         int n_kv, int m_tiles, int n_splits, float scale_log2, DecodeRope rope, int v_shift, int v_runs) {
     // A block takes one share of a sequence's pages (n_splits 1: all of them); its warps take every kWarps-th page of the
     // share and merge their results in shared memory before anything is written.  Where a sequence is one share
-    // the block writes the final result to ``out`` itself; else, with ``arrivals`` (a zeroed counter per sequence and head tile,
-    // left zeroed), the block that finishes last adds up the shares, and without, a kernel behind this one.
+    // the block writes the final result to ``out`` itself; else, with kCluster, a sequence's blocks are a cluster and each adds up a part of
+    // the result out of the others' shared memory; with ``arrivals`` (a zeroed counter per sequence and head tile, left zeroed) the block
+    // that finishes last adds up the shares, and with neither a kernel behind this one.
     using S = DecodeSmem<D>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ float sm_m[kWarps][16], sm_l[kWarps][16];
@@ -530,7 +537,9 @@ decode_attention_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_c
     }
     __syncthreads();
     const int64_t unit = ((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-    float* po = part_o + unit * 16 * D;
+    float* own = sm_o + kWarps * 16 * kLd;                 // [16][D], behind the warps' results
+    __shared__ float2 own_ml[16];
+    float* po = kCluster ? own : part_o + unit * 16 * D;
     for (int i = threadIdx.x; i < 16 * D; i += kWarps * 32) {
         const int row = i / D, c = i - row * D;
         float mx = -INFINITY;
@@ -551,12 +560,51 @@ decode_attention_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_c
             continue;
         }
         po[i] = o;
-        if (c == 0) {
+        if (kCluster) {
+            if (c == 0) own_ml[row] = make_float2(mx, l);
+        } else if (c == 0) {
             part_ml[unit * 32 + 2 * row] = mx;
             part_ml[unit * 32 + 2 * row + 1] = l;
         }
     }
-    if (share.count == 1 || arrivals == nullptr) return;
+    if (share.count == 1) return;
+    if constexpr (kCluster) {
+        // blocks beyond the sequence's shares have exited and are not waited for; an item is four columns of a row
+        cluster_sync();
+        const int items = min(16, group - mt * 16) * (D / 4);
+        for (int i = index * kWarps * 32 + (int)threadIdx.x; i < items; i += share.count * kWarps * 32) {
+            float2 ml[kClusterShares];
+            float4 part[kClusterShares];
+#pragma unroll
+            for (int s = 0; s < kClusterShares; ++s) {
+                ml[s] = make_float2(-INFINITY, 0.f);
+                part[s] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (s < share.count) {
+                    ml[s] = cluster_load2(cluster_address(own_ml + i / (D / 4), s));
+                    part[s] = cluster_load4(cluster_address(own + 4 * i, s));
+                }
+            }
+            float mx = -INFINITY, l = 0.f;
+#pragma unroll
+            for (int s = 0; s < kClusterShares; ++s) mx = fmaxf(mx, ml[s].x);
+            const float use = mx == -INFINITY ? 0.f : mx;
+            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int s = 0; s < kClusterShares; ++s) {
+                const float w = exp2f(ml[s].x - use);
+                l = fmaf(ml[s].y, w, l);
+                acc.x = fmaf(part[s].x, w, acc.x);
+                acc.y = fmaf(part[s].y, w, acc.y);
+                acc.z = fmaf(part[s].z, w, acc.z);
+                acc.w = fmaf(part[s].w, w, acc.w);
+            }
+            const float inv = l > 0.f ? 1.f / l : 0.f;
+            store4(out + ((int64_t)bv * n_heads + kvh * group + mt * 16) * D + 4 * i, make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv));
+        }
+        cluster_sync();                                    // no block leaves while another still reads its sums
+        return;
+    }
+    if (arrivals == nullptr) return;
     // ---- the last of a sequence's blocks adds up the shares: statistics and the first eight shares' sums are asked for together ----
     // (one thread's fence stands for the block: the barrier orders the block's writes before it, and the other reads behind it)
     __syncthreads();
@@ -723,22 +771,27 @@ static int launch_decode(const void* q, const void* k_cache, const void* v_cache
     float* part_o = scratch;
     float* part_ml = scratch + shares * runs * n_kv * m_tiles * 16 * D;
     rope.early = g_decode_early;
-    auto start = [&](auto kern, int warps, bool* configured) -> int {      // configured: per kernel and per device
+    auto start = [&](auto kern, int warps, bool* configured, int cluster) -> int {      // configured: per kernel and per device
         const int smem = warps * kDecodeStages * DecodeSmem<D>::kStageBytes;
         if (int st = ensure_dynamic_smem(kern, smem, configured)) return st;
-        cpm_launch(kLaunchAttention, kern, dim3((unsigned)shares, n_kv * m_tiles, runs), warps * 32, smem, stream, (const bf16*)q, (const bf16*)k_cache,
-                   (const bf16*)v_cache, kv_len, slots, page_table, max_pages, part_o, part_ml, arrivals, (bf16*)out, n_seqs, n_heads, n_kv,
-                   m_tiles, n_splits, scale * 1.4426950408889634f, rope, v_shift, runs);
+        if (cluster > 8)                                                   // more than a portable cluster has
+            if (cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) return (int)e;
+        cpm_launch_cluster(kLaunchAttention, kern, dim3((unsigned)shares, n_kv * m_tiles, runs), warps * 32, smem, stream, cluster, (const bf16*)q,
+                           (const bf16*)k_cache, (const bf16*)v_cache, kv_len, slots, page_table, max_pages, part_o, part_ml, arrivals, (bf16*)out,
+                           n_seqs, n_heads, n_kv, m_tiles, n_splits, scale * 1.4426950408889634f, rope, v_shift, runs);
         return CPM_OK;
     };
-    static bool configured[2][kMaxDevices] = {};
+    static bool configured[3][kMaxDevices] = {};
     int st;
-    if (D == 64 && n_splits == 1 && (int64_t)n_rows * n_kv * m_tiles <= device_sms())
-        st = start(decode_attention_kernel<D, DecodeSmem<D>::kWarps>, DecodeSmem<D>::kWarps, configured[1]);
+    const bool cluster = D == 64 && n_splits > 1 && n_splits <= kClusterShares;
+    if (cluster)
+        st = start(decode_attention_kernel<D, kDecodeWarps<D>, D == 64>, kDecodeWarps<D>, configured[2], n_splits);
+    else if (D == 64 && n_splits == 1 && (int64_t)n_rows * n_kv * m_tiles <= device_sms())
+        st = start(decode_attention_kernel<D, DecodeSmem<D>::kWarps, false>, DecodeSmem<D>::kWarps, configured[1], 1);
     else
-        st = start(decode_attention_kernel<D, kDecodeWarps<D>>, kDecodeWarps<D>, configured[0]);
+        st = start(decode_attention_kernel<D, kDecodeWarps<D>, false>, kDecodeWarps<D>, configured[0], 1);
     if (st != CPM_OK) return st;
-    if (n_splits > 1 && arrivals == nullptr)
+    if (n_splits > 1 && !cluster && arrivals == nullptr)
         cpm_launch(kLaunchCombine, combine_shares_kernel<D>, dim3((n_heads + 3) / 4, n_rows), 128, 0, stream, (const float*)part_o,
                    (const float*)part_ml, kv_len, (bf16*)out, n_seqs, n_heads, n_kv, m_tiles, n_splits);
     return launch_status();

@@ -807,18 +807,25 @@ class Ops:
                                           _ptr(live), ids.numel(), self._stream()), "advance_decode")
 
     # ---- bf16 tensor-core attention ----
-    def decode_splits(self, n_seqs: int, n_heads: int, n_kv: int, d: int = 0) -> int:
+    def decode_splits(self, n_seqs: int, n_heads: int, n_kv: int, d: int = 0, longest: int = 0) -> int:
         """How many shares a sequence's pages are cut into (fewer where it has few): one wave of blocks.  The kernel holds one
         block per SM (its page buffers fill the shared memory), the decode kernel at head size ``d`` 64 two of half the size; but a
         sequence that would be one share of a block that fills an SM stays one there too (64 sequences of 4,000 tokens, 2 kv heads:
-        1,465 us a step of 24 layers, 1,543 as two shares)."""
+        1,465 us a step of 24 layers, 1,543 as two shares).  At head size 64 the shares of a sequence are a cluster of blocks, and eight are
+        better than sixteen as long as they have few pages each: where the page table ends at ``longest`` <= SHORT_TOKENS tokens (one
+        sequence of 1,000 tokens: 524 and 553 us a step; of 8,000: 659 and 616)."""
         m_tiles = (n_heads // n_kv + 15) // 16
         units = max(1, n_seqs * n_kv * m_tiles)
         per_sm = self.lib.cpm_decode_attention_blocks_per_sm(d) if d else 1
         if self.sm_count // units == 1:
             per_sm = 1
-        return max(1, min(self.MAX_DECODE_SPLITS, self.sm_count * per_sm // units))
+        most = self.MAX_DECODE_SPLITS
+        if d == self.CLUSTER_HEAD_DIM and 0 < longest <= self.SHORT_TOKENS:
+            most = min(most, self.SHORT_SHARES)
+        return max(1, min(most, self.sm_count * per_sm // units))
 
+    CLUSTER_SHARES, CLUSTER_HEAD_DIM = 16, 64    # up to so many a sequence's blocks are a cluster and add up the shares among themselves
+    SHORT_SHARES, SHORT_TOKENS = 8, 5120         # blocks of a cluster where no sequence can be longer
     MAX_JOINED_SHARES = 32      # what the last of a sequence's blocks has room to add up
 
     def _arrivals(self, rows: int, n_heads: int, n_kv: int, d: int, n_splits: int) -> Optional[torch.Tensor]:
@@ -827,7 +834,7 @@ class Ops:
         where a workspace is attached, whose memory asks for the same; elsewhere, with more rows than there are counters, or with more
         shares than the last block has room for, the shares are added up by a kernel of its own.
         So they are at head sizes above 64, where a block's three warps take longer for 16 rows of the shares than that kernel
-        (8 sequences of the 8B sizes: 29.3 against 28.3 ms for eight steps)."""
+        (8 sequences of the 8B sizes: 29.3 against 28.3 ms for eight steps).  (At head size 64 they are used beyond CLUSTER_SHARES only.)"""
         if (d > 64 or n_splits > self.MAX_JOINED_SHARES or self.workspace is None or self.arrivals is None
                 or rows * n_kv * ((n_heads // n_kv + 15) // 16) > self.arrivals.numel()):
             return None
@@ -844,7 +851,7 @@ class Ops:
         n, n_heads, d = q.shape
         rows = n * max(1, int(v_runs))
         if n_splits is None:
-            n_splits = self.decode_splits(rows, n_heads, n_kv, d)
+            n_splits = self.decode_splits(rows, n_heads, n_kv, d, page_table.shape[1] * PAGE_TOKENS)
         floats = self.lib.cpm_decode_attention_scratch_floats(rows, n_heads, n_kv, d, n_splits)
         scratch = self.empty(floats, dtype=torch.float32)
         arrivals = self._arrivals(rows, n_heads, n_kv, d, n_splits)
@@ -861,19 +868,20 @@ class Ops:
                                                      _ptr(slots), _ptr(page_table), page_table.shape[1], _ptr(scratch),
                                                      n, n_heads, n_kv, d, n_splits, float(scale), _ptr(arrivals), self._stream()),
                   f"decode attention (head_dim {d})")
-        if n_splits > 1 and arrivals is None:
+        if n_splits > (self.CLUSTER_SHARES if d == self.CLUSTER_HEAD_DIM else 1) and arrivals is None:
             LAUNCHES_EXTRA[0] += 1       # the launcher starts two kernels: the shares, then their combination
         return out
 
-    FUSED_ROPE_ROWS = 32
+    FUSED_ROPE_ROWS = 16
     FUSED_ROPE_HEAD_DIMS = (64, 128)      # head sizes whose rotary pairs lie in one thread's fragments of the decode kernel
 
     def fused_decode_ok(self, ctx, d: int, rot_dim: int, window: int, sparse) -> bool:
         """Whether a decode step's rotation and cache store are done by the attention kernel itself.  It saves a
         launch, which always counts in steps that are not recorded into a graph.  In recorded ones it does at head size 64 for up to
-        FUSED_ROPE_ROWS sequences (us a step of the 0.5B sizes, two kernels and one: 1 sequence 549 and 510, 8 750 and 718, 16 787 and
-        753, 32 1,243 and 1,218, 64 1,599 and 1,632).  At head size 128 a block's pages fill an SM beside the product ahead,
-        the separate kernel's launch hides behind that, and the fused one is slower (8B, batch 8: 3,268 against 3,244).
+        FUSED_ROPE_ROWS sequences, whose products let this kernel's blocks in before they end (us a step of the 0.5B sizes, two kernels and
+        one: 1 sequence 549 and 510, 8 750 and 718, 16 787 and 753; 32 of 3,000 tokens 1,120 and 1,193).  At head size 128 a block's pages
+        fill an SM beside the product ahead, the separate kernel's launch hides behind that, and the fused one is slower (8B,
+        batch 8: 3,268 against 3,244).
         CPMCU_FUSED_ROPE=1 / 0 forces the choice."""
         forced = os.environ.get("CPMCU_FUSED_ROPE")
         want = (forced != "0") if forced is not None else not ctx.captured or (d == 64 and ctx.n_seqs <= self.FUSED_ROPE_ROWS)
@@ -895,7 +903,7 @@ class Ops:
             if inv_freq.numel() != d // 2:
                 raise ValueError("inv_freq needs head_dim/2 entries")
         if n_splits is None:
-            n_splits = self.decode_splits(n, n_heads, n_kv, d)
+            n_splits = self.decode_splits(n, n_heads, n_kv, d, lane.page_table.shape[1] * PAGE_TOKENS)
         floats = self.lib.cpm_decode_attention_scratch_floats(n, n_heads, n_kv, d, n_splits)
         scratch = self.empty(floats, dtype=torch.float32)
         out = self.empty(n, n_heads * d)
@@ -905,7 +913,7 @@ class Ops:
                                                       _ptr(scratch), n, n_heads, n_kv, d, n_splits, float(scale),
                                                       _ptr(inv_freq), float(magnitude), 1 if write_cache else 0,
                                                       _ptr(arrivals), self._stream()), f"decode attention with rotation (head_dim {d})")
-        if n_splits > 1 and arrivals is None:
+        if n_splits > (self.CLUSTER_SHARES if d == self.CLUSTER_HEAD_DIM else 1) and arrivals is None:
             LAUNCHES_EXTRA[0] += 1
         return out
 

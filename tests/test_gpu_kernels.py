@@ -1078,6 +1078,34 @@ def test_decode_attention_shares_of_ragged_batches(n_heads, n_kv, d, lens):
         assert not ops.arrivals.any()
 
 
+@pytest.mark.parametrize("n_heads,n_kv", [(16, 2), (6, 3), (40, 2), (7, 1)])
+@pytest.mark.parametrize("splits", [2, 3, 7, 8, 9, 16])
+def test_clusters_add_up_shares(n_heads, n_kv, splits):
+    """Head size 64, a sequence's blocks as a cluster: lengths around the border of one share and two (three pages), of two and
+    three, sequences of every share and of one, each against one block a sequence.  Weights and sums in another order: two roundings to bf16."""
+    from cpmcu_b200.cache import Cache
+    from cpmcu_b200.parts.base import CacheNeeds
+
+    ops, d = _ops("bfloat16"), 64
+    lens = [1, 64, 191, 192, 193, 384, 385, 64 * 3 * splits, 64 * 3 * splits + 1, 4000]
+    n, g = len(lens), torch.Generator().manual_seed(splits)
+    c = Cache([CacheNeeds(kv_heads=n_kv, head_dim=d)], max_tokens=sum(64 * ((m + 63) // 64) for m in lens), dtype=torch.bfloat16,
+              device="cuda:0", n_slots=n)
+    slots = c.open_sequences(n)
+    for s, m in zip(slots, lens):
+        c.reserve(s, m)
+    c.sync()
+    lane = c.lane(0)
+    lane.k.copy_(torch.randn(lane.k.shape, generator=g).bfloat16())
+    lane.v.copy_(torch.randn(lane.v.shape, generator=g).bfloat16())
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32).cuda()
+    q = torch.randn(n, n_heads, d, generator=g).bfloat16().cuda()
+    run = lambda k: ops.decode_attention(q, lane.k, lane.v, i32(lens), i32(slots), lane.page_table, n_kv, d ** -0.5, n_splits=k)
+    want = run(1)
+    for _ in range(3):
+        assert _err(run(splits), want) <= 2.0 ** -7
+
+
 @pytest.mark.parametrize("n_heads,n_kv,d", [(16, 2, 64), (6, 3, 64), (40, 2, 64), (8, 2, 32)])
 def test_last_block_adds_up_shares_behind_rotation_and_with_shifted_values(n_heads, n_kv, d):
     """The entries that turn the queries themselves, that take another head's values and that do several runs at once: shares added up by
