@@ -760,9 +760,10 @@ class Ops:
                                               lane.page_table, n_kv, scale)
         if (self.code == BF16 and block_list is not None and block_size == PAGE_TOKENS and not window
                 and d in FAST_HEAD_DIMS):
-            return self.listed_attention(q, lane.k, lane.v, ctx.positions, ctx.token_seq, ctx.slot_dev,
-                                         lane.page_table, block_list, n_kv, scale,
-                                         tiles=not ctx.is_decode and n >= self.LISTED_TILE_MIN_TOKENS)
+            prompt = not ctx.is_decode and n >= self.LISTED_TILE_MIN_TOKENS
+            alone = prompt and self.listed_token_by_token(n, n_heads, n_kv, d, lane.page_table.shape[1])
+            return self.listed_attention(q, lane.k, lane.v, ctx.positions, ctx.token_seq, ctx.slot_dev, lane.page_table, block_list, n_kv,
+                                         scale, tiles=prompt and not alone, n_splits=1 if prompt else None)
         return self.attention_generic(q, lane.k, lane.v, ctx.positions, ctx.token_seq, ctx.slot_dev,
                                       lane.page_table, n_kv, scale, window, block_list, block_size)
 
@@ -1588,18 +1589,31 @@ class Ops:
                 raise RuntimeError(f"checked build: a kernel of {name}.cu met {what}: index {rec[1]}, value {rec[2]}, "
                                    f"limit {rec[3]}; it used page 0 instead, the step's results are not valid")
 
+    def _listed_tcgen05_ok(self, n_heads: int, n_kv: int, d: int, max_pages: int) -> bool:
+        return (self.use_tcgen05_attention and self.use_tcgen05_listed and d == 128 and n_heads == 16 * n_kv
+                and max_pages <= self.lib.cpm_listed_attention_tcgen05_max_pages())
+
+    def listed_token_by_token(self, n: int, n_heads: int, n_kv: int, d: int, max_pages: int) -> bool:
+        """Whether a prompt chunk of few tokens goes token by token, as decoded ones do: a tile walks all blocks that its tokens' lists
+        name, one after the other, which takes as long for 40 tokens as for 600, while a token's own list takes a wave of blocks of
+        one an SM.  Lists of 98 blocks of 12,300 keys, 32 heads on 2 of 128 channels, tokens with equal lists and with lists of their own: 57
+        tokens 119 and 216 us in tiles, 68 alone; 100 tokens 118 and 215, 129 alone.  16 heads on 2 of 64: 200 tokens 144 and 181, 95 alone; 296
+        tokens 144 and 185, 126 alone.  So: one wave against the tcgen05 tiles, two against the others."""
+        waves = 1 if self._listed_tcgen05_ok(n_heads, n_kv, d, max_pages) else 2
+        return n * n_kv * ((n_heads // n_kv + 15) // 16) <= waves * self.sm_count
+
     def listed_attention(self, q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, positions: torch.Tensor,
                          token_seq: torch.Tensor, slots: torch.Tensor, page_table: torch.Tensor,
-                         block_list: torch.Tensor, n_kv: int, scale: float, tiles: bool = False) -> torch.Tensor:
+                         block_list: torch.Tensor, n_kv: int, scale: float, tiles: bool = False,
+                         n_splits: Optional[int] = None) -> torch.Tensor:
         """Attention of every token over the 64-token key blocks its list names (block-sparse).  ``tiles``: the
         tokens are those of prompts (consecutive tokens mostly of one sequence); eight of them then share the
-        blocks they bring from the cache."""
+        blocks they bring from the cache.  Without, a token's blocks are cut into ``n_splits`` shares (None: one wave of them)."""
         self._act(q, "q")
         self._i32(block_list, "block list")
         n, n_heads, d = q.shape
         out = self.empty(n, n_heads * d)
-        if (tiles and self.use_tcgen05_attention and self.use_tcgen05_listed and d == 128 and n_heads == 16 * n_kv
-                and page_table.shape[1] <= self.lib.cpm_listed_attention_tcgen05_max_pages()):
+        if tiles and self._listed_tcgen05_ok(n_heads, n_kv, d, page_table.shape[1]):
             # prompt tokens of the long-context shape: eight tokens x sixteen heads are one tensor-core tile
             check(self.lib.cpm_listed_attention_tcgen05(_ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(out), _ptr(positions),
                                                         _ptr(token_seq), _ptr(slots), _ptr(page_table), page_table.shape[1],
@@ -1607,7 +1621,8 @@ class Ops:
                                                         n_kv, d, float(scale), self._stream()),
                   "block-list attention on tcgen05")
             return out
-        n_splits = 1 if tiles else self.decode_splits(n, n_heads, n_kv)      # few tokens (decode): share a token's blocks out
+        if tiles or n_splits is None:
+            n_splits = 1 if tiles else self.decode_splits(n, n_heads, n_kv)  # few tokens (decode): share a token's blocks out
         scratch = None
         if n_splits > 1:
             scratch = self.empty(self.lib.cpm_decode_attention_scratch_floats(n, n_heads, n_kv, d, n_splits),

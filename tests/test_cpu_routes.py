@@ -17,6 +17,13 @@ def test_counters_are_given_only_for_shares_that_the_last_block_can_add_up(d):
         assert (got is not None) == (d <= 64 and n_splits <= 32), n_splits
 
 
+@pytest.mark.parametrize("n,n_heads,n_kv,d,alone", [(57, 32, 2, 128, True), (74, 32, 2, 128, True), (75, 32, 2, 128, False), (2048, 32, 2, 128, False),
+                                                    (148, 16, 2, 64, True), (149, 16, 2, 64, False), (40, 80, 2, 64, True), (50, 80, 2, 64, False)])
+def test_prompt_chunks_of_few_tokens_take_their_block_lists_token_by_token(n, n_heads, n_kv, d, alone):
+    ops = DryOps(torch.bfloat16)
+    assert ops.sm_count == 148 and ops.listed_token_by_token(n, n_heads, n_kv, d, 500) == alone
+
+
 @pytest.mark.parametrize("portions,by_tiles", [
     ([2048], True), ([512], True), ([256], True), ([128], False), ([16], False), ([16] * 64, False), ([32] * 64, False),
     ([1] * 63 + [256], False), ([1] * 63 + [1985], False), ([65] * 15 + [1073], True), ([512] * 4, True), ([8] * 63 + [1544], False),
