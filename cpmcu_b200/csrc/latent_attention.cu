@@ -558,12 +558,17 @@ template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile(
 // partial 16 x 32 score tile in shared memory), every warp adds the four partials and keeps the softmax statistics, and
 // the warps split the latent columns for the weighted sum.  Tiles arrive by cp.async one tile ahead, in two buffers.
 // scratch per (token, head group, share): 16 * (rank + 2) floats.
+// Blocks without keys leave at once.  one_token: no sequence brings more than one token, so that all cached rows but its own are older than the
+// step, and pages and the first tiles without that row are asked for before the wait (a recorded decode step of Reravik 2k, four
+// sequences of 90 to 1,900 tokens, 698 -> 677 us, of Dinutar 2k, eight of 100 to 700, 391 -> 381, of Lukelorn 2k 527 -> 520).  The blocks of a
+// token as a cluster that adds up its shares out of shared memory instead of a kernel that follows: 728, 459 and 519 (a share is
+// 33 KB here, which blocks read out of each other slower than out of L2).
 template <int NT>
 __global__ void __launch_bounds__(128)
 latent_attention_mma_kernel(const float* __restrict__ q, const bf16* __restrict__ cache, void* __restrict__ out_any, int out_bf16,
                             float* __restrict__ scratch, const int* __restrict__ positions, const int* __restrict__ token_seq,
                             const int* __restrict__ slots, const int* __restrict__ page_table, int max_pages, int window,
-                            int n_heads, int rank, float scale, int n_splits) {
+                            int n_heads, int rank, float scale, int n_splits, int one_token) {
     constexpr int KS = NT / 2;                                           // 16-wide steps of the rank per warp, at most
     extern __shared__ __align__(16) unsigned char lm_smem[];
     __shared__ int page_s[kPageSlots];
@@ -571,34 +576,20 @@ latent_attention_mma_kernel(const float* __restrict__ q, const bf16* __restrict_
     bf16* Ks = reinterpret_cast<bf16*>(lm_smem);                         // [2][32][pitch]
     float* Ss = reinterpret_cast<float*>(Ks + 2 * kMmaKeys * pitch);     // [4 warps][16 values][32 lanes]
     pdl_launch_dependents();
-    pdl_wait();
+    // (positions, slots and page tables were written before this step's kernels began)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tg = lane & 3;
     const int t = blockIdx.x, h0 = blockIdx.y * kMmaRows, split = blockIdx.z;
     const int p = positions[t];
     const int* pages = page_table + (int64_t)slots[token_seq[t]] * max_pages;
     const int lo = window > 0 ? max(0, p - window + 1) : 0;
     const int tiles_total = (p + 1 - lo + kMmaKeys - 1) / kMmaKeys;
-    const int per = (tiles_total + n_splits - 1) / n_splits;
+    const int per = (tiles_total + n_splits - 1) / n_splits, used = (tiles_total + per - 1) / per;
     const int tile0 = split * per, tile1 = min(tiles_total, tile0 + per);
+    if (split >= used) return;                                           // (the merge reads the shares that had keys alone)
     const int k_steps = rank / 16;
-
-    // this warp's part of the queries, as A fragments: 16-wide steps warp, warp + 4, ... of the rank
-    uint32_t qa[KS][4];
-#pragma unroll
-    for (int i = 0; i < KS; ++i) {
-        const int ks = warp + 4 * i;
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int h = h0 + g + 8 * (e & 1);
-            const int c = ks * 16 + 2 * tg + 8 * (e >> 1);
-            float2 v = make_float2(0.f, 0.f);
-            if (ks < k_steps && h < n_heads) v = *reinterpret_cast<const float2*>(q + ((int64_t)t * n_heads + h) * rank + c);
-            qa[i][e] = pack_bf16(v.x, v.y);
-        }
-    }
     const int first_page = (lo + tile0 * kMmaKeys) / kPageTokens;
     const int last_key = min(p, lo + tile1 * kMmaKeys - 1);
-    const int n_block_pages = tile1 > tile0 ? last_key / kPageTokens - first_page + 1 : 0;
+    const int n_block_pages = last_key / kPageTokens - first_page + 1;
     const bool pages_in_smem = n_block_pages <= kPageSlots;
     if (pages_in_smem)
         for (int i = threadIdx.x; i < n_block_pages; i += blockDim.x) page_s[i] = CPM_PAGE(pages, first_page + i, max_pages);
@@ -606,9 +597,9 @@ latent_attention_mma_kernel(const float* __restrict__ q, const bf16* __restrict_
 
     const int vec_per_row = rank / 8;                                    // 16-byte pieces of a latent row
     // a warp brings every fourth row of a tile (the row's address worked out once), its lanes the row's 16-byte pieces
-    auto fetch = [&](int tile, int buf) {
+    auto fetch = [&](int tile) {
         const int j0 = lo + tile * kMmaKeys;
-        bf16* dst = Ks + buf * kMmaKeys * pitch;
+        bf16* dst = Ks + ((tile - tile0) & 1) * kMmaKeys * pitch;
 #pragma unroll
         for (int rr = 0; rr < kMmaKeys / 4; ++rr) {
             const int r = warp + 4 * rr;
@@ -624,7 +615,26 @@ latent_attention_mma_kernel(const float* __restrict__ q, const bf16* __restrict_
         }
         cp_async_commit();
     };
+    int asked = tile0;                                                   // the next tile to ask for
+    if (one_token)
+        while (asked < min(tile0 + 2, tile1) && asked != tiles_total - 1) fetch(asked++);      // (the last tile has the token's own row)
+    pdl_wait();
+    if (asked == tile0) fetch(asked++);
 
+    // this warp's part of the queries, as A fragments: 16-wide steps warp, warp + 4, ... of the rank
+    uint32_t qa[KS][4];
+#pragma unroll
+    for (int i = 0; i < KS; ++i) {
+        const int ks = warp + 4 * i;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int h = h0 + g + 8 * (e & 1);
+            const int c = ks * 16 + 2 * tg + 8 * (e >> 1);
+            float2 v = make_float2(0.f, 0.f);
+            if (ks < k_steps && h < n_heads) v = *reinterpret_cast<const float2*>(q + ((int64_t)t * n_heads + h) * rank + c);
+            qa[i][e] = pack_bf16(v.x, v.y);
+        }
+    }
     // softmax statistics in the base-2 domain: scores are multiplied by scale * log2(e) and weights are exp2
     float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};             // rows g and g + 8
     float acc[NT][4];
@@ -638,12 +648,11 @@ latent_attention_mma_kernel(const float* __restrict__ q, const bf16* __restrict_
     const int v_off = lane * pitch + 8 * warp;
     float* mine = Ss + warp * 16 * 32;                                   // [16 values][32 lanes] of this warp's partial scores
 
-    if (tile0 < tile1) fetch(tile0, 0);
     for (int tile = tile0; tile < tile1; ++tile) {
         const int buf = (tile - tile0) & 1;
         const int j0 = lo + tile * kMmaKeys;
         if (tile + 1 < tile1) {
-            fetch(tile + 1, buf ^ 1);
+            if (asked == tile + 1) fetch(asked++);
             cp_async_wait<1>();
         } else {
             cp_async_wait<0>();
@@ -849,7 +858,7 @@ CPM_API int64_t cpm_latent_attention_scratch_floats(int n_tokens, int n_heads, i
 template <int NT>
 static int launch_latent_mma(const float* q, const void* cache, void* out, int out_bf16, float* scratch, const int* positions,
                              const int* token_seq, const int* slots, const int* page_table, int max_pages, int window,
-                             int n_tokens, int n_heads, int rank, float scale, int n_splits, cudaStream_t stream) {
+                             int n_tokens, int n_heads, int rank, float scale, int n_splits, int one_token, cudaStream_t stream) {
     static bool smem_done[kMaxDevices];
     const size_t smem = (size_t)2 * kMmaKeys * (rank + 8) * sizeof(bf16) + (size_t)4 * 16 * 32 * sizeof(float);
     auto kern = latent_attention_mma_kernel<NT>;
@@ -857,36 +866,38 @@ static int launch_latent_mma(const float* q, const void* cache, void* out, int o
         int dev = 0;
         cudaGetDevice(&dev);
         const bool first = dev >= 0 && dev < kMaxDevices && !smem_done[dev];
-        if (int e = ensure_dynamic_smem(kern, (int)smem, smem_done)) return e;
+        // (of the template's largest rank: the attribute is set once, whatever rank comes first)
+        if (int e = ensure_dynamic_smem(kern, (int)(2 * kMmaKeys * (32 * NT + 8) * sizeof(bf16) + 4 * 16 * 32 * sizeof(float)), smem_done)) return e;
         // all of the SM's unified memory as shared memory: three blocks of the rank-512 kernel then fit one SM
         if (first) cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     }
     const int groups = (n_heads + kMmaRows - 1) / kMmaRows;
     dim3 grid(n_tokens, groups, n_splits);
     cpm_launch(kLaunchAttention, kern, grid, 128, smem, stream, q, (const bf16*)cache, out, out_bf16, scratch, positions, token_seq, slots,
-               page_table, max_pages, window, n_heads, rank, scale, n_splits);
+               page_table, max_pages, window, n_heads, rank, scale, n_splits, one_token);
     if (n_splits > 1)
         cpm_launch(kLaunchCombine, latent_attention_merge_kernel, dim3(n_tokens, groups, kMmaRows), rank > 512 ? 288 : rank > 256 ? 256 : 128, 0, stream,
                    (const float*)scratch, out, out_bf16, positions, window, n_heads, rank, n_splits);
     return launch_status();
 }
 
-// bf16 latents, rank a multiple of 16 up to 576; ``out`` fp32, or bf16 with ``out_bf16``; ``scratch``: cpm_latent_attention_scratch_floats floats when n_splits > 1.
+// bf16 latents, rank a multiple of 16 up to 576; ``out`` fp32, or bf16 with ``out_bf16``; ``scratch``: cpm_latent_attention_scratch_floats floats
+// when n_splits > 1.  ``one_token``: no sequence brings more than one token.
 CPM_API int cpm_latent_attention_mma(const float* q, const void* cache, void* out, int out_bf16, float* scratch, const int* positions,
                                      const int* token_seq, const int* slots, const int* page_table, int max_pages, int window,
-                                     int n_tokens, int n_heads, int rank, float scale, int n_splits, cudaStream_t stream) {
+                                     int n_tokens, int n_heads, int rank, float scale, int n_splits, int one_token, cudaStream_t stream) {
     if (n_tokens <= 0) return CPM_OK;
     if (n_heads <= 0 || rank <= 0 || rank > 576 || rank % 16 || window < 0 || n_splits < 1 || n_splits > 64) return CPM_BAD_ARGUMENT;
     if (n_splits > 1 && scratch == nullptr) return CPM_BAD_ARGUMENT;
     if ((n_heads + kMmaRows - 1) / kMmaRows > 65535) return CPM_BAD_ARGUMENT;
     if (rank <= 128) return launch_latent_mma<4>(q, cache, out, out_bf16, scratch, positions, token_seq, slots, page_table, max_pages, window,
-                                                  n_tokens, n_heads, rank, scale, n_splits, stream);
+                                                  n_tokens, n_heads, rank, scale, n_splits, one_token, stream);
     if (rank <= 256) return launch_latent_mma<8>(q, cache, out, out_bf16, scratch, positions, token_seq, slots, page_table, max_pages, window,
-                                                  n_tokens, n_heads, rank, scale, n_splits, stream);
+                                                  n_tokens, n_heads, rank, scale, n_splits, one_token, stream);
     if (rank <= 512) return launch_latent_mma<16>(q, cache, out, out_bf16, scratch, positions, token_seq, slots, page_table, max_pages, window,
-                                                  n_tokens, n_heads, rank, scale, n_splits, stream);
+                                                  n_tokens, n_heads, rank, scale, n_splits, one_token, stream);
     return launch_latent_mma<18>(q, cache, out, out_bf16, scratch, positions, token_seq, slots, page_table, max_pages, window, n_tokens,
-                                 n_heads, rank, scale, n_splits, stream);
+                                 n_heads, rank, scale, n_splits, one_token, stream);
 }
 
 // ---------------------------------------------------------------------------

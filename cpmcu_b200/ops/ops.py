@@ -520,7 +520,7 @@ class Ops:
             check(self.lib.cpm_latent_attention_mma(_ptr(q_lat), _ptr(lane.k), _ptr(out), 1 if narrow else 0, _ptr(scratch), _ptr(ctx.positions),
                                                     _ptr(ctx.token_seq), _ptr(ctx.slot_dev), _ptr(lane.page_table),
                                                     lane.page_table.shape[1], int(window), n, H, R, float(scale), n_splits,
-                                                    self._stream()), f"latent attention on tensor cores (rank {R}, {H} heads)")
+                                                    1 if ctx.max_q_len == 1 else 0, self._stream()), f"latent attention on tensor cores (rank {R}, {H} heads)")
             if n_splits > 1:
                 LAUNCHES_EXTRA[0] += 1
             return out
