@@ -490,6 +490,31 @@ def test_convolution_reads_the_state_and_leaves_the_last_inputs(K):
                 _close(torch.cat([piece[j] for piece in got[i]]), want[i][j], "float32", tol32=2e-5)
 
 
+@pytest.mark.parametrize("H,G,d,dv,gates", [(2, 1, 20, 44, True), (4, 2, 64, 64, False), (2, 2, 128, 256, True), (6, 3, 132, 8, False)])
+def test_short_convolution_by_quads_of_channels(H, G, d, dv, gates):
+    """Four taps, rows on 16-byte boundaries: a lane takes four channels.  Against the kernel of single channels, which rows one float longer
+    take: sequences that start, go on inside the taps' reach and behind it, in steps of several and of one token.  The
+    convolution's sums run in one order; the sum of squares of up to 132 channels in another."""
+    from cpmcu_b200.ops.ops import Ops
+
+    ops = Ops(torch.float32)
+    g = torch.Generator().manual_seed(d + dv)
+    C = 2 * G * d + H * dv
+    N = (C + 2 * H + 3) // 4 * 4
+    taps, a_log, dt_bias = torch.randn(C, 4, generator=g).cuda(), torch.randn(H, generator=g).cuda(), torch.randn(H, generator=g).cuda()
+    extra = (a_log, dt_bias) if gates else (None, None)
+    for lens, starts in (([5, 1, 2, 30], [0, 0, 1, 40]), ([1, 1, 1, 1], [0, 1, 2, 9])):
+        proj = torch.randn(sum(lens), N + 1, generator=g).cuda()
+        state = torch.randn(6, 3, C, generator=g).cuda()
+        outs = []
+        ctx = _ctx(lens, starts, [5, 0, 2, 3])
+        for p in (proj[:, :N].contiguous(), proj):
+            st = state.clone()
+            outs.append([*ops.conv_prepare(ctx, p, taps, st, *extra, C, C + H, H, G, d, dv, 1e-6, head_decay=gates), st])
+        for a, b in zip(*outs):
+            assert (a is None and b is None) or float((a - b).abs().max()) <= 1e-6 * max(1.0, float(b.abs().max()))
+
+
 @pytest.mark.parametrize("E,top,groups,keep", [(10, 3, 2, 1), (8, 2, 4, 2), (9, 4, 3, 2), (6, 6, 1, 1), (64, 6, 8, 3), (300, 8, 1, 1)])
 def test_routing_follows_the_rule(E, top, groups, keep):
     from cpmcu_b200.ops.ops import Ops
