@@ -102,6 +102,9 @@ class DryOps(Ops):
     def set_page_limit(self, n_pages):
         pass
 
+    def _library_bmm(self, a, w, c):          # (the fp32 form has no kernel for tensors without storage)
+        pass
+
     kept_bytes = 0      # what the parts asked to keep for good, each tensor rounded up to the arena's alignment
 
     def keep(self, t):

@@ -454,9 +454,7 @@ class Ops:
             raise ValueError("head_project: the input must be fp32 or the compute dtype")
         out = self.empty(n_tok, H, N, dtype=torch.float32 if out_f32 else self.dtype)
         if self.head_project_by_library(n_tok) and not in_f32:
-            by_head = torch.bmm(x.view(n_tok, H, K).transpose(0, 1), w, out_dtype=out.dtype) if out_f32 else \
-                torch.bmm(x.view(n_tok, H, K).transpose(0, 1), w)
-            out.copy_(by_head.transpose(0, 1))
+            self._library_bmm(x.view(n_tok, H, K).transpose(0, 1), w, out.transpose(0, 1))       # (into place: no tensor and no copy between)
             return out
         check(self.lib.cpm_head_project(_ptr(x), _ptr(w), _ptr(out), n_tok, H, K, N, 1 if in_f32 else 0,
                                         1 if out_f32 else 0, self.code, self._stream()), f"head_project ({K} -> {N})")
@@ -591,6 +589,13 @@ class Ops:
         self._f32(x, "values to cap")
         check(self.lib.cpm_softcap(_ptr(x), x.numel(), float(cap), self._stream()), "softcap")
         return x
+
+    def _library_bmm(self, a: torch.Tensor, w: torch.Tensor, c: torch.Tensor) -> None:
+        """c[h] = a[h] @ w[h] by the library; c may be a view whose matrices lie between each other's rows."""
+        if c.dtype == a.dtype:
+            torch.bmm(a, w, out=c)
+        else:
+            torch.bmm(a, w, out_dtype=c.dtype, out=c)
 
     def _library_mm(self, a: torch.Tensor, w: torch.Tensor, c: torch.Tensor) -> None:
         """c = a @ w^T by the library (cuBLAS through torch), into a tensor of this library's own."""
@@ -1075,6 +1080,8 @@ class Ops:
         C, K = taps.shape
         if C != 2 * qk_heads * d + heads * dv or tuple(conv_state.shape[1:]) != (max(K - 1, 1), C):
             raise ValueError("conv_prepare: taps [channels, K] and state [slots, K-1, channels] do not match the head sizes")
+        if head_decay and (a_log is None or dt_bias is None):
+            raise ValueError("conv_prepare: a decay per head needs a_log and dt_bias")
         qo = self.empty(n, qk_heads * d, dtype=torch.float32)
         ko = self.empty(n, qk_heads * d, dtype=torch.float32)
         vo = self.empty(n, heads * dv, dtype=torch.float32)
