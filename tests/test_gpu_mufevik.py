@@ -493,8 +493,7 @@ def test_convolution_reads_the_state_and_leaves_the_last_inputs(K):
 @pytest.mark.parametrize("H,G,d,dv,gates", [(2, 1, 20, 44, True), (4, 2, 64, 64, False), (2, 2, 128, 256, True), (6, 3, 132, 8, False)])
 def test_short_convolution_by_quads_of_channels(H, G, d, dv, gates):
     """Four taps, rows on 16-byte boundaries: a lane takes four channels.  Against the kernel of single channels, which rows one float longer
-    take: sequences that start, go on inside the taps' reach and behind it, in steps of several and of one token.  The
-    convolution's sums run in one order; the sum of squares of up to 132 channels in another."""
+    take: sequences that start, go on inside the taps' reach and behind it, in steps of several and of one token."""
     from cpmcu_b200.ops.ops import Ops
 
     ops = Ops(torch.float32)
@@ -513,6 +512,27 @@ def test_short_convolution_by_quads_of_channels(H, G, d, dv, gates):
             outs.append([*ops.conv_prepare(ctx, p, taps, st, *extra, C, C + H, H, G, d, dv, 1e-6, head_decay=gates), st])
         for a, b in zip(*outs):
             assert (a is None and b is None) or float((a - b).abs().max()) <= 1e-6 * max(1.0, float(b.abs().max()))
+
+
+@pytest.mark.parametrize("H,G,d,dv", [(1, 1, 4, 4), (4, 2, 32, 36), (2, 1, 64, 64), (3, 3, 100, 20), (2, 2, 128, 128), (2, 1, 132, 8), (1, 1, 256, 256)])
+def test_short_convolution_by_quads_gives_the_bits_of_single_channels(H, G, d, dv):
+    """Rows one float longer take the kernel of single channels: every sum of the two runs in the same order, over the widths at which a
+    lane has one quad, part of one, two, and none."""
+    from cpmcu_b200.ops.ops import Ops
+
+    ops, g = Ops(torch.float32), torch.Generator().manual_seed(d)
+    C = 2 * G * d + H * dv
+    N = (C + 2 * H + 3) // 4 * 4
+    taps, a_log, dt_bias = torch.randn(C, 4, generator=g).cuda(), torch.randn(H, generator=g).cuda(), torch.randn(H, generator=g).cuda()
+    for lens, starts in (([40, 1, 3, 200], [0, 0, 1, 40]), ([1, 1, 1, 1], [0, 1, 2, 9])):
+        proj = torch.randn(sum(lens), N + 1, generator=g).cuda()
+        state = torch.randn(6, 3, C, generator=g).cuda()
+        ctx, outs = _ctx(lens, starts, [5, 0, 2, 3]), []
+        for p in (proj[:, :N].contiguous(), proj):
+            st = state.clone()
+            outs.append([*ops.conv_prepare(ctx, p, taps, st, a_log, dt_bias, C, C + H, H, G, d, dv, 1e-6), st])
+        for a, b in zip(*outs):
+            assert torch.equal(a, b)
 
 
 @pytest.mark.parametrize("E,top,groups,keep", [(10, 3, 2, 1), (8, 2, 4, 2), (9, 4, 3, 2), (6, 6, 1, 1), (64, 6, 8, 3), (300, 8, 1, 1)])
