@@ -71,6 +71,12 @@ __device__ __forceinline__ int take_largest(uint32_t (&key)[PER], int lane) {
 
 // One warp per token.  logits rows of ``ld`` floats: the first E are the router's, column ``gate_col`` (if >= 0) is the
 // shared expert's raw gate.
+// The next kernel is let in behind the wait, not before it: the products ahead let this one in at their start, and the experts' blocks
+// (by pair: hundreds, four an SM, which hold their place while they wait) would be placed around the blocks of up to four kernels that
+// still run, unevenly over the SMs.  Rabadra 1k, four tokens: the first product 13.4 us behind the kernel ahead of it, 6.6 so.  us of a
+// recorded decode step before and now: Rabadra 1k one, four, eight, 16 tokens 310, 404,
+// 431, 502 and 308, 343, 384, 471; Kipizen 1k 252, 312, 349, 423 and 250, 282, 321, 405; Lukelorn 1k 275, 304, 350,
+// 416 and 274, 295, 322, 391.
 template <int PER>
 __global__ void moe_route_kernel(const float* __restrict__ logits, int ld, const float* __restrict__ correction,
                                  int* __restrict__ chosen, float* __restrict__ weights, float* __restrict__ shared_gate,
@@ -78,8 +84,8 @@ __global__ void moe_route_kernel(const float* __restrict__ logits, int ld, const
                                  const float* __restrict__ bias, int top_first, int group_top2, int normalize,
                                  float route_scale) {
     extern __shared__ float route_smem[];
-    pdl_launch_dependents();
     pdl_wait();
+    pdl_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t = blockIdx.x * (blockDim.x >> 5) + warp;
     if (t >= n_tokens) return;
