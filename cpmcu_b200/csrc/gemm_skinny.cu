@@ -65,10 +65,13 @@ constexpr int kShortK = 1024;
 constexpr int kManyWarpsK = 4096;
 // In a decode step's chain a product of a few MB lives for little more than latencies: of its launch, of its weights, of its activations.  So
 // the first kFlight steps' weights (all of them up to K 1,024 and, with eight steps, 2,048) are on their way into registers before the kernel
-// ahead has ended, and a grid whose blocks the SMs hold all at once (``let_go``) lets the next kernel's blocks in at its start, so that
+// ahead has ended (kAhead), and a grid whose blocks the SMs hold all at once (``let_go``) lets the next kernel's blocks in at its start, so that
 // these do the same; a grid of several waves would lose slots on the SMs to blocks that do nothing but wait, and lets them in
 // after its main loop.  us of a recorded decode step before, with let_go alone, with both: 0.5B one row 585, 577, 549, 16 rows
 // 862, 821, 787; 8B eight rows 3,305, 3,259, 3,244; Mufevik 1k 16 rows 647, 620, 597; Rabadra 2k four rows 707, 684, 671.
+// With two tiles of columns and K over kShortK the registers do not hold a step's activations beside eight steps' weights: the loop that asks
+// for both step by step is faster (us of a recorded step of 16 rows with the weights ahead and without: Dinutar 2k 444 and 428, Kipizen
+// 2k 908 and 892, Lukelorn 2k 743 and 728, Rabadra 2k 1,010 and 991, Reravik 2k 822 and 808, the 8B sizes 3,708 and 3,707).
 template <int NT, int EPI, int kSkinnyWarps, bool kShort>
 __global__ void __launch_bounds__(kSkinnyWarps * 32, kShort ? (NT == 1 ? 4 : 3) : (NT == 1 || kSkinnyWarps > 8 ? 1 : 2))
 skinny_gemm_kernel(const bf16* __restrict__ W, const bf16* __restrict__ X, void* __restrict__ out, int M, int N, int K,
@@ -97,12 +100,15 @@ skinny_gemm_kernel(const bf16* __restrict__ W, const bf16* __restrict__ X, void*
     const int steps = K / 32;
     constexpr int kFlight = kShort ? 4 : 8;                // K steps whose loads are in flight
     // the first steps' weights are on their way into registers before the wait
+    constexpr bool kAhead = NT == 1 || kShort;
     uint4 lo[kFlight], hi[kFlight];
+    if constexpr (kAhead) {
 #pragma unroll
-    for (int i = 0; i < kFlight; ++i) {
-        const int s = min(warp + i * kSkinnyWarps, steps - 1);
-        lo[i] = ld_stream16(w0 + 32 * s);
-        hi[i] = ld_stream16(w1 + 32 * s);
+        for (int i = 0; i < kFlight; ++i) {
+            const int s = min(warp + i * kSkinnyWarps, steps - 1);
+            lo[i] = ld_stream16(w0 + 32 * s);
+            hi[i] = ld_stream16(w1 + 32 * s);
+        }
     }
     pdl_wait();
     const bf16* xp[NT];
@@ -111,30 +117,25 @@ skinny_gemm_kernel(const bf16* __restrict__ W, const bf16* __restrict__ X, void*
     float acc[NT][4];
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
-    constexpr int kAtOnce = NT == 1 || kShort ? kFlight : kFlight / 2;       // steps whose activations are asked for together
+    if constexpr (kAhead) {
+        uint4 b[kFlight][NT];
 #pragma unroll
-    for (int i0 = 0; i0 < kFlight; i0 += kAtOnce) {
-        uint4 b[kAtOnce][NT];
+        for (int i = 0; i < kFlight; ++i)
 #pragma unroll
-        for (int i = 0; i < kAtOnce; ++i)
+            for (int nt = 0; nt < NT; ++nt) b[i][nt] = __ldg(reinterpret_cast<const uint4*>(xp[nt] + 32 * min(warp + i * kSkinnyWarps, steps - 1)));
 #pragma unroll
-            for (int nt = 0; nt < NT; ++nt)
-                b[i][nt] = __ldg(reinterpret_cast<const uint4*>(xp[nt] + 32 * min(warp + (i0 + i) * kSkinnyWarps, steps - 1)));
-#pragma unroll
-        for (int i = 0; i < kAtOnce; ++i) {
-            const uint4 l = lo[i0 + i], h = hi[i0 + i];
-            if (warp + (i0 + i) * kSkinnyWarps < steps) {
+        for (int i = 0; i < kFlight; ++i)
+            if (warp + i * kSkinnyWarps < steps) {
 #pragma unroll
                 for (int nt = 0; nt < NT; ++nt) {
-                    mma_16816_s(acc[nt], l.x, h.x, l.y, h.y, b[i][nt].x, b[i][nt].y);
-                    mma_16816_s(acc[nt], l.z, h.z, l.w, h.w, b[i][nt].z, b[i][nt].w);
+                    mma_16816_s(acc[nt], lo[i].x, hi[i].x, lo[i].y, hi[i].y, b[i][nt].x, b[i][nt].y);
+                    mma_16816_s(acc[nt], lo[i].z, hi[i].z, lo[i].w, hi[i].w, b[i][nt].z, b[i][nt].w);
                 }
             }
-        }
     }
     if constexpr (!kShort) {
 #pragma unroll kFlight
-        for (int s = warp + kFlight * kSkinnyWarps; s < steps; s += kSkinnyWarps) {
+        for (int s = warp + (kAhead ? kFlight * kSkinnyWarps : 0); s < steps; s += kSkinnyWarps) {
             const uint4 l = ld_stream16(w0 + 32 * s);
             const uint4 h = ld_stream16(w1 + 32 * s);
 #pragma unroll
@@ -205,7 +206,7 @@ static int launch_skinny_epi(const void* W, const void* X, void* out, int M, int
     const unsigned blocks = (unsigned)((N + 15) / 16), sms = (unsigned)device_sms();
     auto start = [&](auto kern, int warps, unsigned per_sm) {
         cpm_launch(kLaunchProduct, kern, blocks, warps * 32, 0, stream, (const bf16*)W, (const bf16*)X, out, M, N, K, alpha,
-                   g_skinny_prefetch_lines, (int)(blocks <= per_sm * sms), clamp);       // per_sm: blocks an SM holds by their registers
+                   g_skinny_prefetch_lines, (int)(blocks <= per_sm * sms), clamp);       // per_sm: blocks an SM holds by their registers (128, kShort 64 and 80)
     };
     if (K >= kManyWarpsK && 2 * blocks <= sms)
         start(skinny_gemm_kernel<NT, EPI, 16, false>, 16, 1u);
