@@ -15,7 +15,6 @@ from __future__ import annotations
 
 from typing import Dict, List, Optional, Sequence
 
-import numpy as np
 import torch
 
 from ..parts.base import StepContext
@@ -144,19 +143,15 @@ class DecodeRunner:
         b = self._bucket(n)
         self._prepare(b)
         lengths = [self.cache.length(s) for s in slots]
+        last_tokens, seq_keys, step_keys = list(last_tokens), list(seq_keys), list(step_keys)
         if any(len(v) != n for v in (last_tokens, seq_keys, step_keys, sampling)):
-            raise ValueError(f"a batch of {n} sequences needs as many tokens, keys and sampling parameters")
-        host = np.zeros(tuple(b.block.shape), dtype=np.int32)          # padding: token 0, position 0, not live
-        host[2] = 1                                                    # one key
-        host[3] = self.pad_slot
-        for row, values in ((0, last_tokens), (1, lengths), (2, [length + 1 for length in lengths]), (3, slots), (4, 1),
-                            (5, seq_keys), (6, step_keys)):
-            host[row, :n] = values
-        real = host[7:].view(np.float32)
-        real[1] = 1.0
-        real[0, :n] = [p.temperature for p in sampling]
-        real[1, :n] = [p.top_p for p in sampling]
-        self.cache.staging.copy(torch.from_numpy(host).view(-1), [b.block.view(-1)])
+            raise RuntimeError(f"a batch of {n} sequences needs as many tokens, keys and sampling parameters")
+        pad = b.block.shape[1] - n         # padding: token 0, position 0, one key, not live
+        ints = torch.tensor(               # (of lists: a number that 32 bits do not hold is refused, whatever it comes in)
+            last_tokens + [0] * pad + lengths + [0] * pad + [length + 1 for length in lengths] + [1] * pad
+            + list(slots) + [self.pad_slot] * pad + [1] * n + [0] * pad + seq_keys + [0] * pad + step_keys + [0] * pad, dtype=torch.int32)
+        reals = torch.tensor([p.temperature for p in sampling] + [0.0] * pad + [p.top_p for p in sampling] + [1.0] * pad, dtype=torch.float32)
+        self.cache.staging.copy(torch.cat((ints, reals.view(torch.int32))), [b.block.view(-1)])
         self.current = b
         self.slots = list(slots)
 
