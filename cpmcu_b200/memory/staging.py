@@ -27,7 +27,10 @@ class Staging:
         self._next = 0
 
     def copy(self, values: torch.Tensor, parts: Sequence[torch.Tensor]) -> None:
-        """Copies the flat host tensor ``values`` into ``parts`` one after the other, in the order of the current stream."""
+        """Copies the flat host tensor ``values`` into ``parts`` one after the other, in the order of the current stream.
+        The parts hold together as many numbers as there are values."""
+        if sum(part.numel() for part in parts) != values.numel():
+            raise RuntimeError(f"{values.numel()} numbers for parts of {[part.numel() for part in parts]}")
         if self.device.type != "cuda":
             at = 0
             for part in parts:

@@ -3,7 +3,7 @@ import pytest
 import torch
 
 from cpmcu_b200.cache import Cache, CacheFull
-from cpmcu_b200.memory import ALIGN, Arena, PoolExhausted, Workspace, plan_storage
+from cpmcu_b200.memory import ALIGN, Arena, PoolExhausted, Staging, Workspace, plan_storage
 from cpmcu_b200.parts.base import CacheNeeds
 from tests import configs, dinutar_cases, kipizen_cases, reravik_cases
 
@@ -208,3 +208,12 @@ def test_opened_slots_are_cleared_together_and_others_left():
         c.close_sequence(s)
     assert c.open_sequences(3) == [1, 3, 4]
     assert [float(r.sum()) for r in state] == [15.0, 0.0, 15.0, 0.0, 0.0, 15.0, 15.0]
+
+
+@pytest.mark.parametrize("n,sizes", [(5, [3]), (5, [2, 2]), (3, [5]), (0, [1]), (4, []), (6, [2, 0, 5])])
+def test_staged_copies_need_parts_of_the_sources_size(n, sizes):
+    """Refused before anything is copied, as a plain copy between unequal shapes is."""
+    parts = [torch.full((m,), 7, dtype=torch.int32) for m in sizes]
+    with pytest.raises(RuntimeError, match=f"{n} numbers"):
+        Staging(torch.device("cpu")).copy(torch.arange(n, dtype=torch.int32), parts)
+    assert all(p.tolist() == [7] * p.numel() for p in parts)
