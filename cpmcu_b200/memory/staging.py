@@ -54,7 +54,9 @@ class Staging:
             host = self._buffers[i][:size].view(values.dtype)
             host.copy_(values)
             at = 0
-            for part in parts:
-                part.copy_(host[at:at + part.numel()], non_blocking=True)
-                at += part.numel()
-            self._done[i].record(torch.cuda.current_stream(self.device))
+            try:
+                for part in parts:
+                    part.copy_(host[at:at + part.numel()], non_blocking=True)
+                    at += part.numel()
+            finally:                       # also where a part has refused its numbers: those before it are on their way
+                self._done[i].record(torch.cuda.current_stream(self.device))

@@ -90,3 +90,22 @@ def test_staged_copies_arrive_whole_behind_a_busy_stream(sizes):
         outs.append(parts)
     for i, parts in enumerate(outs):
         assert torch.equal(torch.cat(parts).cpu(), torch.arange(n, dtype=torch.int32) * (i + 1)), i
+
+
+def test_a_staged_copy_that_fails_leaves_its_buffer_to_the_copies_before_it():
+    """The second of two parts has another shape and is refused: the first part's copy is queued by then, and its buffer
+    is not written again before that copy is over."""
+    from cpmcu_b200.memory import Staging
+
+    staging, n = Staging(torch.device("cuda:0")), 4096
+    staging.copy(torch.zeros(1, dtype=torch.int32), [torch.empty(1, dtype=torch.int32, device="cuda:0")])
+    torch.cuda.synchronize()
+    a = torch.randn(8192, 8192, device="cuda:0")
+    for _ in range(8):
+        a = torch.tanh(a @ a)                                  # tens of milliseconds of work in front of the copies
+    first = torch.zeros(n, dtype=torch.int32, device="cuda:0")
+    with pytest.raises(RuntimeError):
+        staging.copy(torch.arange(n + 6, dtype=torch.int32), [first, torch.empty(2, 3, dtype=torch.int32, device="cuda:0")])
+    for _ in range(Staging.BUFFERS):                           # once round the ring, over the same buffer
+        staging.copy(torch.full((n,), -1, dtype=torch.int32), [torch.empty(n, dtype=torch.int32, device="cuda:0")])
+    assert torch.equal(first.cpu(), torch.arange(n, dtype=torch.int32))
