@@ -146,6 +146,8 @@ class Arena:
         for s in reversed(shape):
             strides.append(n)
             n *= max(s, 1)
+        if (0 if 0 in shape else n) * dtype.itemsize != nbytes or at + nbytes > self.total:       # (as_strided asks neither)
+            raise RuntimeError(f"{nbytes} bytes from byte {at} of an arena of {self.total} are no tensor {shape} of {dtype}")
         t = base.as_strided(shape, strides[::-1], base.storage_offset() + at // dtype.itemsize)       # one call of torch's, not three
         if zero:
             t.zero_()

@@ -217,3 +217,12 @@ def test_staged_copies_need_parts_of_the_sources_size(n, sizes):
     with pytest.raises(RuntimeError, match=f"{n} numbers"):
         Staging(torch.device("cpu")).copy(torch.arange(n, dtype=torch.int32), parts)
     assert all(p.tolist() == [7] * p.numel() for p in parts)
+
+
+@pytest.mark.parametrize("at,nbytes,shape", [(0, 16, (100,)), (0, 400, (99,)), (3600, 512, (128,)), (4096, 4, (1,)), (3840, 256, (65,))])
+def test_a_view_lies_inside_the_arena_and_is_as_long_as_its_shape(at, nbytes, shape):
+    arena = Arena(4096, "cpu")
+    with pytest.raises(RuntimeError):
+        arena.view(at, nbytes, shape, torch.float32, False)
+    assert arena.view(3840, 256, (64,), torch.float32, True).tolist() == [0.0] * 64           # the last bytes
+    assert arena.view(4096, 0, (0, 3), torch.bfloat16, True).shape == (0, 3)
