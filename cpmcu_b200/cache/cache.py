@@ -120,7 +120,7 @@ class CacheGroup:
         self.first_live[slot] = dead
         return dead - first
 
-    def sync(self, staging: Staging) -> None:
+    def sync(self, staging: Optional[Staging] = None) -> None:
         """Brings the device's page table up to date, behind what is queued on the current stream.  The rows are staged together;
         the host does not wait (a decode step that takes a page did, for everything queued before it)."""
         rows, values = [], []
@@ -132,6 +132,7 @@ class CacheGroup:
             rows.append((slot, first, len(pages)))
             values.extend(max(p, 0) for p in pages[first:])                                # a released page: no kernel follows it
         if rows:
+            staging = staging or Staging(self.page_table.device)
             staging.copy(torch.tensor(values, dtype=torch.int32), [self.page_table[slot, first:end] for slot, first, end in rows])
         self._dirty.clear()
 

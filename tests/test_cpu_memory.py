@@ -226,3 +226,12 @@ def test_a_view_lies_inside_the_arena_and_is_as_long_as_its_shape(at, nbytes, sh
         arena.view(at, nbytes, shape, torch.float32, False)
     assert arena.view(3840, 256, (64,), torch.float32, True).tolist() == [0.0] * 64           # the last bytes
     assert arena.view(4096, 0, (0, 3), torch.bfloat16, True).shape == (0, 3)
+
+
+def test_a_groups_page_table_is_brought_up_to_date_by_itself():
+    """A group may be asked without the cache around it, as ever."""
+    c = Cache([CacheNeeds(kv_heads=1, head_dim=4)], max_tokens=64 * 8, dtype=torch.float32, device="cpu", n_slots=2)
+    for slot, tokens in zip(c.open_sequences(2), (130, 64)):
+        c.reserve(slot, tokens)
+    c.groups[0].sync()
+    assert [row.tolist()[:3] for row in c.groups[0].page_table] == [c.groups[0].pages_of_slot[0], c.groups[0].pages_of_slot[1] + [0, 0]]
