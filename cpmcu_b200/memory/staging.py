@@ -37,6 +37,8 @@ class Staging:
                 part.copy_(values[at:at + part.numel()])
                 at += part.numel()
             return
+        if torch.cuda.is_current_stream_capturing():       # (a graph would read the buffer again after other copies have written it)
+            raise RuntimeError("the host's numbers cannot be copied to the device while the current stream is captured")
         size = values.numel() * values.element_size()
         with self._lock:
             if not self._buffers:

@@ -109,3 +109,17 @@ def test_a_staged_copy_that_fails_leaves_its_buffer_to_the_copies_before_it():
     for _ in range(Staging.BUFFERS):                           # once round the ring, over the same buffer
         staging.copy(torch.full((n,), -1, dtype=torch.int32), [torch.empty(n, dtype=torch.int32, device="cuda:0")])
     assert torch.equal(first.cpu(), torch.arange(n, dtype=torch.int32))
+
+
+def test_a_staged_copy_is_refused_under_capture():
+    """As a copy out of ordinary memory is: a replay would read a buffer that holds other copies' numbers by then.  The ring goes on."""
+    from cpmcu_b200.memory import Staging
+
+    staging, part = Staging(torch.device("cuda:0")), torch.zeros(5, dtype=torch.int32, device="cuda:0")
+    for i in range(3):
+        staging.copy(torch.full((5,), i, dtype=torch.int32), [part])
+        with pytest.raises(RuntimeError, match="captured"):
+            with torch.cuda.graph(torch.cuda.CUDAGraph()):
+                part.add_(0)
+                staging.copy(torch.full((5,), 9, dtype=torch.int32), [part])
+        assert part.tolist() == [i] * 5
