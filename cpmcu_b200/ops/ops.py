@@ -766,7 +766,10 @@ class Ops:
         if (self.code == BF16 and block_list is not None and block_size == PAGE_TOKENS and not window
                 and d in FAST_HEAD_DIMS):
             prompt = not ctx.is_decode and n >= self.LISTED_TILE_MIN_TOKENS
-            alone = prompt and self.listed_token_by_token(n, n_heads, n_kv, d, lane.page_table.shape[1])
+            # (against the tcgen05 tiles the walk token by token is the faster one too, but where many keys weigh alike its error is the larger)
+            max_pages = lane.page_table.shape[1]
+            alone = (prompt and not self._listed_tcgen05_ok(n_heads, n_kv, d, max_pages)
+                     and self.listed_token_by_token(n, n_heads, n_kv, d, max_pages))
             return self.listed_attention(q, lane.k, lane.v, ctx.positions, ctx.token_seq, ctx.slot_dev, lane.page_table, block_list, n_kv,
                                          scale, tiles=prompt and not alone, n_splits=1 if prompt else None)
         return self.attention_generic(q, lane.k, lane.v, ctx.positions, ctx.token_seq, ctx.slot_dev,
@@ -1601,11 +1604,14 @@ class Ops:
                 and max_pages <= self.lib.cpm_listed_attention_tcgen05_max_pages())
 
     def listed_token_by_token(self, n: int, n_heads: int, n_kv: int, d: int, max_pages: int) -> bool:
-        """Whether a prompt chunk of few tokens goes token by token, as decoded ones do: a tile walks all blocks that its tokens' lists
+        """Whether a prompt chunk of few tokens is faster token by token, as decoded ones go: a tile walks all blocks that its tokens' lists
         name, one after the other, which takes as long for 40 tokens as for 600, while a token's own list takes a wave of blocks of
         one an SM.  Lists of 98 blocks of 12,300 keys, 32 heads on 2 of 128 channels, tokens with equal lists and with lists of their own: 57
         tokens 119 and 216 us in tiles, 68 alone; 100 tokens 118 and 215, 129 alone.  16 heads on 2 of 64: 200 tokens 144 and 181, 95 alone; 296
-        tokens 144 and 185, 126 alone.  So: one wave against the tcgen05 tiles, two against the others."""
+        tokens 144 and 185, 126 alone.  So: one wave against the tcgen05 tiles, two against the others.  Error against 64 bits of 57 tokens
+        on 98 blocks, tiles and alone, queries and keys of spread 0.4, 1 and 2: 32 heads on 2 of 128 channels (tcgen05 tiles) 0.00233 and
+        0.00240, 0.00235 and 0.00225, 0.00207 and 0.00170, so that ``attention`` leaves these to the tiles; 16 on 2 of 64 0.00240 and
+        0.00237, 0.00228 and 0.00221, 0.00173 and 0.00168; 8 on 2 of 128 0.00239 and 0.00237, 0.00228 and 0.00224, 0.00175 and 0.00171."""
         waves = 1 if self._listed_tcgen05_ok(n_heads, n_kv, d, max_pages) else 2
         return n * n_kv * ((n_heads // n_kv + 15) // 16) <= waves * self.sm_count
 

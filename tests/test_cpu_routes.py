@@ -24,6 +24,18 @@ def test_prompt_chunks_of_few_tokens_take_their_block_lists_token_by_token(n, n_
     assert ops.sm_count == 148 and ops.listed_token_by_token(n, n_heads, n_kv, d, 500) == alone
 
 
+@pytest.mark.parametrize("n,n_heads,n_kv,d,tiles,n_splits", [
+    (31, 32, 2, 128, False, None), (32, 32, 2, 128, True, 1), (57, 32, 2, 128, True, 1), (74, 32, 2, 128, True, 1), (75, 32, 2, 128, True, 1),
+    (57, 8, 2, 128, False, 1), (31, 16, 2, 64, False, None), (148, 16, 2, 64, False, 1), (149, 16, 2, 64, True, 1)])
+def test_the_long_context_shapes_prompts_take_their_block_lists_in_tiles(n, n_heads, n_kv, d, tiles, n_splits):
+    """However few their tokens: where many keys weigh alike, a token's own walk has the larger error there."""
+    ops, lane, asked = DryOps(torch.bfloat16), SimpleNamespace(k=None, v=None, page_table=torch.empty(1, 500, device="meta")), {}
+    ops.listed_attention = lambda *a, **kw: asked.update(kw)
+    ctx = SimpleNamespace(is_decode=False, positions=None, token_seq=None, slot_dev=None)
+    ops.attention(ctx, torch.empty(n, n_heads, d, device="meta"), lane, n_kv, 1.0, block_list=torch.empty(0), block_size=64)
+    assert asked == {"tiles": tiles, "n_splits": n_splits}
+
+
 @pytest.mark.parametrize("portions,by_tiles", [
     ([2048], True), ([512], True), ([256], True), ([128], False), ([16], False), ([16] * 64, False), ([32] * 64, False),
     ([1] * 63 + [256], False), ([1] * 63 + [1985], False), ([65] * 15 + [1073], True), ([512] * 4, True), ([8] * 63 + [1544], False),
