@@ -38,6 +38,13 @@ __device__ __forceinline__ void mma_16816_s(float (&c)[4], uint32_t a0, uint32_t
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+// What the kernel ahead has written.  Not __ldg: memory that this kernel's lifetime sees written is not read-only, and the compiler may move
+// such a load in front of the wait.
+__device__ __forceinline__ uint4 ld_written16(const void* p) {
+    uint4 v;
+    asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+    return v;
+}
 // weights are used once: keep them out of L1
 __device__ __forceinline__ uint4 ld_stream16(const void* p) {
     uint4 v;
@@ -122,7 +129,7 @@ skinny_gemm_kernel(const bf16* __restrict__ W, const bf16* __restrict__ X, void*
 #pragma unroll
         for (int i = 0; i < kFlight; ++i)
 #pragma unroll
-            for (int nt = 0; nt < NT; ++nt) b[i][nt] = __ldg(reinterpret_cast<const uint4*>(xp[nt] + 32 * min(warp + i * kSkinnyWarps, steps - 1)));
+            for (int nt = 0; nt < NT; ++nt) b[i][nt] = ld_written16(xp[nt] + 32 * min(warp + i * kSkinnyWarps, steps - 1));
 #pragma unroll
         for (int i = 0; i < kFlight; ++i)
             if (warp + i * kSkinnyWarps < steps) {
@@ -140,7 +147,7 @@ skinny_gemm_kernel(const bf16* __restrict__ W, const bf16* __restrict__ X, void*
             const uint4 h = ld_stream16(w1 + 32 * s);
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt) {
-                const uint4 b = __ldg(reinterpret_cast<const uint4*>(xp[nt] + 32 * s));
+                const uint4 b = ld_written16(xp[nt] + 32 * s);
                 mma_16816_s(acc[nt], l.x, h.x, l.y, h.y, b.x, b.y);
                 mma_16816_s(acc[nt], l.z, h.z, l.w, h.w, b.z, b.w);
             }

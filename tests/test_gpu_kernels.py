@@ -402,6 +402,45 @@ def test_skinny_gemm_with_steps_asked_for_before_the_wait(M, N, K):
         x = (y / y.abs().max()).bfloat16()
 
 
+@pytest.mark.parametrize("M", [1, 4, 8, 9, 16])
+@pytest.mark.parametrize("mid", [32, 64, 256, 512, 1024, 2048])
+def test_products_in_a_row_read_what_the_one_ahead_has_written(M, mid):
+    """A recorded chain of pairs of products, the second of each started long before the first has written; pairs take turns in the
+    same two buffers, so that what lies there before is another pair's.  fp32 results against 64 bits of what the first wrote."""
+    ops = _ops("bfloat16")
+    ops.SKINNY_MAX_ROWS = 16
+    g = torch.Generator().manual_seed(mid + M)
+    W, N, pairs = 1024, 512, 6
+    a = [(torch.randn(M, W, generator=g) * (1 + i)).bfloat16().cuda() for i in range(pairs)]
+    down, up = (torch.randn(mid, W, generator=g) * 0.03).bfloat16().cuda(), torch.randn(N, mid, generator=g).bfloat16().cuda()
+    buffers, taken = [torch.zeros(M, mid, dtype=torch.bfloat16, device="cuda"), torch.zeros(M, mid, dtype=torch.bfloat16, device="cuda")], []
+    hs = [torch.empty(M, mid, dtype=torch.bfloat16, device="cuda") for _ in range(pairs)]
+    ys = [torch.empty(M, N, dtype=torch.float32, device="cuda") for _ in range(pairs)]
+    ops.empty = lambda *shape, dtype=None: taken.pop(0)
+
+    def chain():
+        for i in range(pairs):
+            taken[:] = [buffers[i % 2], ys[i]]
+            h = ops.linear(a[i], down)
+            ops.linear(h, up, out_f32=True)
+            hs[i].copy_(h)
+
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        chain()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        chain()
+    for _ in range(3):
+        graph.replay()
+    for i in range(pairs):
+        first = a[i].double() @ down.double().T
+        assert _err(hs[i], first) < 2.0 ** -7
+        room = hs[i].double().abs() @ up.double().abs().T
+        assert bool(((ys[i].double() - hs[i].double() @ up.double().T).abs() <= mid * 2.0 ** -23 * room).all())
+
+
 def test_which_products_of_9_to_16_rows_take_the_weight_streaming_kernel():
     """At 9 to 16 rows the engine keeps a product on the weight-streaming kernel while the bytes its blocks read of
     the activations stay small: the QKV, O and down products of the 8B sizes, not gate_up, the head or 17 rows."""
