@@ -60,10 +60,14 @@ __device__ __forceinline__ uint4 ld_stream16(const void* p) {
 // instead of 59 us on the gate_up shape, which is what cuBLAS with the activation kernel takes).  Every block
 // reads all the activations from L1 and L2, so the engine hands it 9 to 16 rows only for the products whose
 // blocks * rows * K stays small (QKV, O and down of the 8B sizes, not gate_up or the head).
-// kShort (K up to kShortK): a warp has at most four steps, whose loads take few registers, and a block lives for little more than
-// their latency; four blocks an SM (three with two tiles of columns) hide one's start and sums behind the others' loads.  Whole calls with K
+// kShort (K up to kShortK): a warp has at most four steps (kFlight: one up to K 256, two up to 512), whose loads take few registers, and a
+// block lives for little more than their latency; four blocks an SM (three with two tiles of columns) hide one's start and sums behind the others' loads.  Whole calls with K
 // of 1024 in most products: 17.6 -> 15.5 to 16.4 ms (one row), 29.4 -> 27.6 (16 rows).  At 2048 eight steps in flight are worth more than
 // the other two blocks (24.1 against 24.8 ms for four rows), at 4096 27.7 against 29.8.
+// A block asks for kFlight steps a warp whether K has them or not (steps beyond the last are its again), so the number follows K: with four
+// for all of these, a product of K 64 to 256 took up to twice as long.  us a product in a row of independent ones, four steps and as it is, eight
+// rows: 2,048 x 64 2.90 and 1.24, 4,096 x 128 3.16 and 1.35, 6,144 x 256 3.33 and 1.66, 2,048 x 512 2.82 and 2.03; sixteen rows of 2,048 x 128 3.24 and
+// 1.39.  (Steps left out by a branch, four for all: 1.79, 2.09, 2.47, 2.30, 2.26, and 1,024 x 1,024 2.64 instead of 2.43.)
 constexpr int kShortK = 1024;
 // Long rows in blocks for at most half of the SMs: sixteen warps a block instead of eight, since no second block comes to keep more of
 // the weights in flight.  One row, inputs cold, eight and sixteen warps: 1,024 weight rows of K 4,096 4.4 and 3.7 us, of 8,192 7.5 and 6.4, 256 of
@@ -79,8 +83,8 @@ constexpr int kManyWarpsK = 4096;
 // With two tiles of columns and K over kShortK the registers do not hold a step's activations beside eight steps' weights: the loop that asks
 // for both step by step is faster (us of a recorded step of 16 rows with the weights ahead and without: Dinutar 2k 444 and 428, Kipizen
 // 2k 908 and 892, Lukelorn 2k 743 and 728, Rabadra 2k 1,010 and 991, Reravik 2k 822 and 808, the 8B sizes 3,708 and 3,707).
-template <int NT, int EPI, int kSkinnyWarps, bool kShort>
-__global__ void __launch_bounds__(kSkinnyWarps * 32, kShort ? (NT == 1 ? 4 : 3) : (NT == 1 || kSkinnyWarps > 8 ? 1 : 2))
+template <int NT, int EPI, int kSkinnyWarps, int kFlight>
+__global__ void __launch_bounds__(kSkinnyWarps * 32, kFlight < 8 ? (NT == 1 ? 4 : 3) : (NT == 1 || kSkinnyWarps > 8 ? 1 : 2))
 skinny_gemm_kernel(const bf16* __restrict__ W, const bf16* __restrict__ X, void* __restrict__ out, int M, int N, int K,
                    float alpha, int prefetch_lines, int let_go, GluClamp clamp) {
     constexpr int MT = NT * 8;                          // token columns
@@ -105,14 +109,16 @@ skinny_gemm_kernel(const bf16* __restrict__ W, const bf16* __restrict__ X, void*
     const bf16* w0 = W + (int64_t)min(n0 + g, N - 1) * K + 8 * j;
     const bf16* w1 = W + (int64_t)min(n0 + g + 8, N - 1) * K + 8 * j;
     const int steps = K / 32;
-    constexpr int kFlight = kShort ? 4 : 8;                // K steps whose loads are in flight
     // the first steps' weights are on their way into registers before the wait
-    constexpr bool kAhead = NT == 1 || kShort;
+    constexpr bool kShort = kFlight < 8, kAhead = NT == 1 || kShort;
+    const bool any = kFlight > 1 || warp < steps;
+    auto step_of = [&](int i) { return min(warp + i * kSkinnyWarps, steps - 1); };
     uint4 lo[kFlight], hi[kFlight];
     if constexpr (kAhead) {
 #pragma unroll
         for (int i = 0; i < kFlight; ++i) {
-            const int s = min(warp + i * kSkinnyWarps, steps - 1);
+            const int s = step_of(i);
+            if (!any) break;
             lo[i] = ld_stream16(w0 + 32 * s);
             hi[i] = ld_stream16(w1 + 32 * s);
         }
@@ -129,7 +135,8 @@ skinny_gemm_kernel(const bf16* __restrict__ W, const bf16* __restrict__ X, void*
 #pragma unroll
         for (int i = 0; i < kFlight; ++i)
 #pragma unroll
-            for (int nt = 0; nt < NT; ++nt) b[i][nt] = ld_written16(xp[nt] + 32 * min(warp + i * kSkinnyWarps, steps - 1));
+            for (int nt = 0; nt < NT; ++nt)
+                if (any) b[i][nt] = ld_written16(xp[nt] + 32 * step_of(i));
 #pragma unroll
         for (int i = 0; i < kFlight; ++i)
             if (warp + i * kSkinnyWarps < steps) {
@@ -211,16 +218,21 @@ template <int NT, int EPI>
 static int launch_skinny_epi(const void* W, const void* X, void* out, int M, int N, int K, float alpha,
                              const GluClamp& clamp, cudaStream_t stream) {
     const unsigned blocks = (unsigned)((N + 15) / 16), sms = (unsigned)device_sms();
+    // per_sm: blocks an SM holds by their registers (128 a thread beyond K 1,024, 64 and 80 with four steps)
     auto start = [&](auto kern, int warps, unsigned per_sm) {
         cpm_launch(kLaunchProduct, kern, blocks, warps * 32, 0, stream, (const bf16*)W, (const bf16*)X, out, M, N, K, alpha,
-                   g_skinny_prefetch_lines, (int)(blocks <= per_sm * sms), clamp);       // per_sm: blocks an SM holds by their registers (128, kShort 64 and 80)
+                   g_skinny_prefetch_lines, (int)(blocks <= per_sm * sms), clamp);
     };
     if (K >= kManyWarpsK && 2 * blocks <= sms)
-        start(skinny_gemm_kernel<NT, EPI, 16, false>, 16, 1u);
+        start(skinny_gemm_kernel<NT, EPI, 16, 8>, 16, 1u);
+    else if (K <= kShortK / 4)
+        start(skinny_gemm_kernel<NT, EPI, 8, 1>, 8, NT == 1 ? 4u : 3u);
+    else if (K <= kShortK / 2)
+        start(skinny_gemm_kernel<NT, EPI, 8, 2>, 8, NT == 1 ? 4u : 3u);
     else if (K <= kShortK)
-        start(skinny_gemm_kernel<NT, EPI, 8, true>, 8, NT == 1 ? 4u : 3u);
+        start(skinny_gemm_kernel<NT, EPI, 8, 4>, 8, NT == 1 ? 4u : 3u);
     else
-        start(skinny_gemm_kernel<NT, EPI, 8, false>, 8, 2u);
+        start(skinny_gemm_kernel<NT, EPI, 8, 8>, 8, 2u);
     return launch_status();
 }
 

@@ -402,6 +402,22 @@ def test_skinny_gemm_with_steps_asked_for_before_the_wait(M, N, K):
         x = (y / y.abs().max()).bfloat16()
 
 
+@pytest.mark.parametrize("M", [1, 8, 9, 16])
+@pytest.mark.parametrize("K", [32, 224, 256, 288, 480, 512, 544, 992, 1024, 1056])
+@pytest.mark.parametrize("N", [30, 2416, 6160])
+def test_skinny_gemm_at_the_borders_of_the_steps_a_warp_asks_for(M, N, K):
+    """One, two, four or eight steps a warp by K: at each border, below it and above it, one wave of blocks and several.  fp32 results: K
+    exact products, each of whose sums rounds or truncates by 2^-23 of what it has at most."""
+    ops = _ops("bfloat16")
+    ops.SKINNY_MAX_ROWS = 16
+    g = torch.Generator().manual_seed(K + N + M)
+    a, w = torch.randn(M, K, generator=g).bfloat16().cuda(), torch.randn(N, K, generator=g).bfloat16().cuda()
+    want, room = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
+    for _ in range(2):
+        assert bool(((ops.linear(a, w, out_f32=True).double() - want).abs() <= K * 2.0 ** -23 * room).all())
+    assert bool(((ops.linear(a, w).double() - want).abs() <= 2.0 ** -8 * want.abs() + K * 2.0 ** -23 * room).all())
+
+
 @pytest.mark.parametrize("M", [1, 4, 8, 9, 16])
 @pytest.mark.parametrize("mid", [32, 64, 256, 512, 1024, 2048])
 def test_products_in_a_row_read_what_the_one_ahead_has_written(M, mid):
