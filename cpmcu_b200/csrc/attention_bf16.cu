@@ -299,8 +299,9 @@ __device__ __forceinline__ void rotate8(uint4& lo, uint4& hi, const float (&cs)[
     for (int i = 0; i < 4; ++i) {
         const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&a[i]));
         const float2 y = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&b[i]));
-        a[i] = pack_bf16(x.x * cs[2 * i] - y.x * sn[2 * i], x.y * cs[2 * i + 1] - y.y * sn[2 * i + 1]);
-        b[i] = pack_bf16(x.x * sn[2 * i] + y.x * cs[2 * i], x.y * sn[2 * i + 1] + y.y * cs[2 * i + 1]);
+        const float2 p0 = turn_pair(x.x, y.x, cs[2 * i], sn[2 * i]), p1 = turn_pair(x.y, y.y, cs[2 * i + 1], sn[2 * i + 1]);
+        a[i] = pack_bf16(p0.x, p1.x);
+        b[i] = pack_bf16(p0.y, p1.y);
     }
     lo = make_uint4(a[0], a[1], a[2], a[3]);
     hi = make_uint4(b[0], b[1], b[2], b[3]);
@@ -345,8 +346,8 @@ struct NewToken {
 #pragma unroll
         for (int i = 0; i < kPairs; ++i) {
             const int c = lane + 32 * i, c2 = c + D / 2;
-            const float xf = __bfloat162float(x[i]), yf = __bfloat162float(y[i]);
-            const bf16 xr = __float2bfloat16_rn(xf * cs[i] - yf * sn[i]), yr = __float2bfloat16_rn(xf * sn[i] + yf * cs[i]);
+            const float2 turned = turn_pair(__bfloat162float(x[i]), __bfloat162float(y[i]), cs[i], sn[i]);
+            const bf16 xr = __float2bfloat16_rn(turned.x), yr = __float2bfloat16_rn(turned.y);
             k_row[(row * S::kChunksPerKeyRow + ((c >> 3) ^ swz)) * 8 + (c & 7)] = xr;
             k_row[(row * S::kChunksPerKeyRow + ((c2 >> 3) ^ swz)) * 8 + (c2 & 7)] = yr;
             if (to_cache) {

@@ -172,6 +172,13 @@ __device__ __forceinline__ int64_t value_offset(int page, int kv_head, int dim, 
     return (((int64_t)page * n_kv + kv_head) * d + dim) * (int64_t)kPageTokens + in_page;
 }
 
+// A rotary pair (x, y) turned by the angle of (cs, sn), in fp32.  Which product is rounded before it is added is written out, so that a pair has
+// the same bits wherever it is turned: left to the compiler, the rotary kernel and the decode attention that turns
+// its own token differed in one of 30,000 bf16 results.
+__device__ __forceinline__ float2 turn_pair(float x, float y, float cs, float sn) {
+    return make_float2(__fmaf_rn(x, cs, -__fmul_rn(y, sn)), __fmaf_rn(y, cs, __fmul_rn(x, sn)));
+}
+
 // Programmatic dependent launch.  A kernel launched with the attribute may start while the
 // kernel before it in the stream is still running; it must not touch anything that kernel
 // (or an earlier one) writes before pdl_wait() returns, which is when the preceding kernel

@@ -404,8 +404,9 @@ __global__ void rope_store_vec_kernel(const bf16* __restrict__ qkv, bf16* __rest
             const float2 a = __bfloat1622float2(lo2[e]), b = __bfloat1622float2(hi2[e]);
             const float c0 = cs_table[c + 2 * e], s0 = cs_table[half + c + 2 * e];
             const float c1 = cs_table[c + 2 * e + 1], s1 = cs_table[half + c + 2 * e + 1];
-            ol[e] = __floats2bfloat162_rn(a.x * c0 - b.x * s0, a.y * c1 - b.y * s1);
-            oh[e] = __floats2bfloat162_rn(a.x * s0 + b.x * c0, a.y * s1 + b.y * c1);
+            const float2 p0 = turn_pair(a.x, b.x, c0, s0), p1 = turn_pair(a.y, b.y, c1, s1);
+            ol[e] = __floats2bfloat162_rn(p0.x, p1.x);
+            oh[e] = __floats2bfloat162_rn(p0.y, p1.y);
         }
         *reinterpret_cast<uint4*>(dst + c) = out_lo;
         *reinterpret_cast<uint4*>(dst + c + half) = out_hi;

@@ -1133,6 +1133,37 @@ def test_decode_attention_shares_of_ragged_batches(n_heads, n_kv, d, lens):
         assert not ops.arrivals.any()
 
 
+@pytest.mark.parametrize("n_heads,n_kv,d", [(16, 2, 64), (6, 3, 64), (16, 2, 128)])
+def test_rotation_inside_decode_attention_gives_the_rotary_kernels_bits(n_heads, n_kv, d):
+    """Queries and keys turned by the attention kernel and by the rotary kernel in front of it: one rounding, so one answer, over enough
+    values to meet those that lie next to a border of bf16."""
+    from cpmcu_b200.cache import Cache
+    from cpmcu_b200.parts.base import CacheNeeds
+
+    ops, n = _ops("bfloat16"), 256
+    g = torch.Generator(device="cuda").manual_seed(n_heads + d)
+    lens = [1 + i % 64 for i in range(n)]
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32).cuda()
+    caches = [Cache([CacheNeeds(kv_heads=n_kv, head_dim=d)], max_tokens=64 * n, dtype=torch.bfloat16, device="cuda:0", n_slots=n) for _ in range(2)]
+    slots = [c.open_sequences(n) for c in caches]
+    for c in caches:
+        for s, m in zip(slots[0], lens):
+            c.reserve(s, m)
+        c.sync()
+    (a, b), slots = [c.lane(0) for c in caches], i32(slots[0])
+    a.k.copy_(torch.randn(a.k.shape, generator=g, device="cuda"))
+    a.v.copy_(torch.randn(a.v.shape, generator=g, device="cuda"))
+    b.k.copy_(a.k), b.v.copy_(a.v)
+    inv_freq = (1.0 / (10000.0 ** (torch.arange(0, d, 2, dtype=torch.float32) / d))).cuda()
+    pos, kv_len, seq = i32([m - 1 for m in lens]), i32(lens), torch.arange(n, dtype=torch.int32).cuda()
+    for i in range(40):
+        qkv, magnitude = torch.randn(n, (n_heads + 2 * n_kv) * d, generator=g, device="cuda").bfloat16(), 1.0 + 0.01 * i
+        q = ops.rope_store(qkv, n_heads, n_kv, d, pos, seq, slots, a.page_table, a.k, a.v, inv_freq, magnitude, d)
+        want = ops.decode_attention(q, a.k, a.v, kv_len, slots, a.page_table, n_kv, d ** -0.5)
+        got = ops.decode_attention_rope(qkv, b, kv_len, slots, n_heads, n_kv, d, d ** -0.5, inv_freq, magnitude, True)
+        assert torch.equal(b.k, a.k) and torch.equal(b.v, a.v) and torch.equal(got, want), i
+
+
 @pytest.mark.parametrize("n_heads,n_kv", [(16, 2), (6, 3), (40, 2), (7, 1)])
 @pytest.mark.parametrize("splits", [2, 3, 7, 8, 9, 16])
 def test_clusters_add_up_shares(n_heads, n_kv, splits):
