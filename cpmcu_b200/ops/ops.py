@@ -592,7 +592,9 @@ class Ops:
 
     def _library_bmm(self, a: torch.Tensor, w: torch.Tensor, c: torch.Tensor) -> None:
         """c[h] = a[h] @ w[h] by the library; c may be a view whose matrices lie between each other's rows."""
-        if c.dtype == a.dtype:
+        if torch.is_grad_enabled() and (a.requires_grad or w.requires_grad):       # (torch has no derivative of a product into place)
+            c.copy_(torch.bmm(a, w) if c.dtype == a.dtype else torch.bmm(a, w, out_dtype=c.dtype))
+        elif c.dtype == a.dtype:
             torch.bmm(a, w, out=c)
         else:
             torch.bmm(a, w, out_dtype=c.dtype, out=c)

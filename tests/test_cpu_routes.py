@@ -36,6 +36,22 @@ def test_the_long_context_shapes_prompts_take_their_block_lists_in_tiles(n, n_he
     assert asked == {"tiles": tiles, "n_splits": n_splits}
 
 
+@pytest.mark.parametrize("which", ["none", "a", "w"])
+def test_the_librarys_per_head_product_takes_operands_that_want_a_gradient(which):
+    """Into a view whose matrices lie between each other's rows, as torch's product takes them: the results, and the gradient if one is wanted."""
+    g = torch.Generator().manual_seed(3)
+    a, w, out = torch.randn(5, 2, 12, generator=g), torch.randn(2, 12, 7, generator=g), torch.zeros(5, 2, 7)
+    want = torch.einsum("thk,hkn->thn", a, w)
+    for name, t in (("a", a), ("w", w)):
+        t.requires_grad_(name == which)
+    Ops._library_bmm(SimpleNamespace(), a.transpose(0, 1), w, out.transpose(0, 1))
+    assert torch.allclose(out, want, atol=1e-5) and out.requires_grad == (which != "none")
+    if which != "none":
+        out.sum().backward()
+        grad = {"a": w.sum(2).expand(5, 2, 12), "w": a.sum(0)[:, :, None].expand(2, 12, 7)}[which]
+        assert torch.allclose({"a": a, "w": w}[which].grad, grad, atol=1e-4)
+
+
 @pytest.mark.parametrize("portions,by_tiles", [
     ([2048], True), ([512], True), ([256], True), ([128], False), ([16], False), ([16] * 64, False), ([32] * 64, False),
     ([1] * 63 + [256], False), ([1] * 63 + [1985], False), ([65] * 15 + [1073], True), ([512] * 4, True), ([8] * 63 + [1544], False),
