@@ -1091,6 +1091,23 @@ def test_head_project_of_few_tokens(K, N, n):
         assert _err(ops.head_project(x, w, H, out_f32=False), want) < 2.0 ** -8
 
 
+@pytest.mark.parametrize("H,K,N", [(1, 64, 128), (3, 72, 20), (16, 192, 136), (2, 100, 1), (5, 8, 257)])
+@pytest.mark.parametrize("n", [63, 64, 65, 333])
+def test_head_project_of_many_tokens(H, K, N, n):
+    """From 64 tokens of bf16 on by the library, into rows that hold every head's results: ragged sizes, one head and several, both
+    results, against 64 bits place by place.  K exact products, whose sums round or truncate by 2^-23 of what they have at most (by 2^-8
+    where a bf16 result is added up from bf16 parts)."""
+    ops = _ops("bfloat16")
+    g = torch.Generator().manual_seed(K * 31 + N + n)
+    w, x = torch.randn(H, K, N, generator=g).bfloat16().cuda(), torch.randn(n, H, K, generator=g).bfloat16().cuda()
+    assert ops.head_project_by_library(n) == (n >= 64)
+    want, room = torch.einsum("thk,hkn->thn", x.double(), w.double()), torch.einsum("thk,hkn->thn", x.double().abs(), w.double().abs())
+    for out_f32, unit in ((True, K * 2.0 ** -23), (False, 2.0 ** -8 + K * 2.0 ** -23)):
+        got = ops.head_project(x, w, H, out_f32=out_f32)
+        assert got.is_contiguous() and got.shape == (n, H, N) and got.dtype == (torch.float32 if out_f32 else torch.bfloat16)
+        assert bool(((got.double() - want).abs() <= unit * room).all())
+
+
 @pytest.mark.parametrize("n_heads,n_kv,d", [(16, 2, 64), (4, 2, 128), (40, 2, 32), (3, 3, 96)])
 @pytest.mark.parametrize("lens", [[1], [3000], [64, 65, 1, 2111, 700, 129], [1 + 17 * i % 900 for i in range(150)], [2500] + [5] * 33])
 def test_decode_attention_shares_of_ragged_batches(n_heads, n_kv, d, lens):
@@ -1190,6 +1207,48 @@ def test_clusters_add_up_shares(n_heads, n_kv, splits):
     want = run(1)
     for _ in range(3):
         assert _err(run(splits), want) <= 2.0 ** -7
+
+
+@pytest.mark.parametrize("n_heads,n_kv", [(16, 2), (6, 3), (40, 2)])
+@pytest.mark.parametrize("splits", [2, 8, 9, 16, 17, 32])
+def test_shares_behind_rotation_and_with_shifted_values_against_one_block_a_sequence(n_heads, n_kv, splits):
+    """Head size 64: clusters (up to 16 shares) and the last block of a sequence (a workspace is attached), in the entries that turn queries
+    and the new key, that take another head's values and that do several runs at once.  Each against one block a sequence,
+    and values of another head against the plain entry on caches whose values lie there.  Sums in another order: two roundings to bf16."""
+    from types import SimpleNamespace
+
+    from cpmcu_b200.cache import Cache
+    from cpmcu_b200.parts.base import CacheNeeds
+
+    ops, d = _ops("bfloat16"), 64
+    ops.workspace = SimpleNamespace(alloc=lambda shape, dtype: torch.empty(*shape, dtype=dtype, device="cuda"))
+    lens = [1, 64, 191, 192, 193, 385, 64 * 3 * splits, 64 * 3 * splits + 1, 3000]
+    n, g = len(lens), torch.Generator().manual_seed(splits + n_heads)
+    c = Cache([CacheNeeds(kv_heads=n_kv, head_dim=d)], max_tokens=sum(64 * ((m + 63) // 64) for m in lens), dtype=torch.bfloat16,
+              device="cuda:0", n_slots=n)
+    slots = c.open_sequences(n)
+    for s, m in zip(slots, lens):
+        c.reserve(s, m)
+    c.sync()
+    lane = c.lane(0)
+    lane.k.copy_(torch.randn(lane.k.shape, generator=g).bfloat16())
+    lane.v.copy_(torch.randn(lane.v.shape, generator=g).bfloat16())
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32).cuda()
+    q = torch.randn(n, n_heads, d, generator=g).bfloat16().cuda()
+    qkv = torch.randn(n, (n_heads + 2 * n_kv) * d, generator=g).bfloat16().cuda()
+    inv_freq = (1.0 / (10000.0 ** (torch.arange(0, d, 2, dtype=torch.float32) / d))).cuda()
+    args = (lane.k, lane.v, i32(lens), i32(slots), lane.page_table, n_kv, d ** -0.5)
+    entries = [lambda k: ops.decode_attention(q, *args, n_splits=k, v_shift=1), lambda k: ops.decode_attention(q, *args, n_splits=k, v_runs=n_kv)]
+    entries += [lambda k, w=w: ops.decode_attention_rope(qkv, lane, i32(lens), i32(slots), n_heads, n_kv, d, d ** -0.5, inv_freq, 1.1, w, n_splits=k)
+                for w in (False, True)]
+    for f in entries:
+        want = f(1).clone()
+        for _ in range(2):
+            assert _err(f(splits), want) <= 2.0 ** -7
+    assert not ops.arrivals.any()
+    turned = lane.v.view(lane.v.shape[0], n_kv, -1).roll(-1, dims=1).reshape(lane.v.shape).contiguous()      # head h's place holds head h + 1
+    want = ops.decode_attention(q, lane.k, turned, *args[2:], n_splits=1)
+    assert _err(entries[0](splits), want) <= 2.0 ** -7
 
 
 @pytest.mark.parametrize("n_heads,n_kv,d", [(16, 2, 64), (6, 3, 64), (40, 2, 64), (8, 2, 32)])
