@@ -80,10 +80,12 @@ constexpr int kManyWarpsK = 4096;
 // these do the same; a grid of several waves would lose slots on the SMs to blocks that do nothing but wait, and lets them in
 // after its main loop.  us of a recorded decode step before, with let_go alone, with both: 0.5B one row 585, 577, 549, 16 rows
 // 862, 821, 787; 8B eight rows 3,305, 3,259, 3,244; Mufevik 1k 16 rows 647, 620, 597; Rabadra 2k four rows 707, 684, 671.
-// With two tiles of columns and K over kShortK the registers do not hold a step's activations beside eight steps' weights: the loop that asks
+// With two tiles of columns and K from 2,048 on the registers do not hold a step's activations beside eight steps' weights: the loop that asks
 // for both step by step is faster (us of a recorded step of 16 rows with the weights ahead and without: Dinutar 2k 444 and 428, Kipizen
 // 2k 908 and 892, Lukelorn 2k 743 and 728, Rabadra 2k 1,010 and 991, Reravik 2k 822 and 808, the 8B sizes 3,708 and 3,707).
-template <int NT, int EPI, int kSkinnyWarps, int kFlight>
+// Below 2,048 that loop has less than a round of eight steps a warp and asks for one after the other: 16 rows of 2,048 x 1,536 4.61 us with the weights
+// ahead and 5.55 without, 2,048 x 1,056 4.01 and 4.3.
+template <int NT, int EPI, int kSkinnyWarps, int kFlight, bool kAhead>
 __global__ void __launch_bounds__(kSkinnyWarps * 32, kFlight < 8 ? (NT == 1 ? 4 : 3) : (NT == 1 || kSkinnyWarps > 8 ? 1 : 2))
 skinny_gemm_kernel(const bf16* __restrict__ W, const bf16* __restrict__ X, void* __restrict__ out, int M, int N, int K,
                    float alpha, int prefetch_lines, int let_go, GluClamp clamp) {
@@ -110,7 +112,7 @@ skinny_gemm_kernel(const bf16* __restrict__ W, const bf16* __restrict__ X, void*
     const bf16* w1 = W + (int64_t)min(n0 + g + 8, N - 1) * K + 8 * j;
     const int steps = K / 32;
     // the first steps' weights are on their way into registers before the wait
-    constexpr bool kShort = kFlight < 8, kAhead = NT == 1 || kShort;
+    constexpr bool kShort = kFlight < 8;
     const bool any = kFlight > 1 || warp < steps;
     auto step_of = [&](int i) { return min(warp + i * kSkinnyWarps, steps - 1); };
     uint4 lo[kFlight], hi[kFlight];
@@ -131,21 +133,26 @@ skinny_gemm_kernel(const bf16* __restrict__ W, const bf16* __restrict__ X, void*
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
     if constexpr (kAhead) {
-        uint4 b[kFlight][NT];
+        constexpr int kAtOnce = NT == 1 || kShort ? kFlight : kFlight / 2;       // steps whose activations are asked for together
 #pragma unroll
-        for (int i = 0; i < kFlight; ++i)
+        for (int i0 = 0; i0 < kFlight; i0 += kAtOnce) {
+            uint4 b[kAtOnce][NT];
 #pragma unroll
-            for (int nt = 0; nt < NT; ++nt)
-                if (any) b[i][nt] = ld_written16(xp[nt] + 32 * step_of(i));
+            for (int i = 0; i < kAtOnce; ++i)
 #pragma unroll
-        for (int i = 0; i < kFlight; ++i)
-            if (warp + i * kSkinnyWarps < steps) {
+                for (int nt = 0; nt < NT; ++nt)
+                    if (any) b[i][nt] = ld_written16(xp[nt] + 32 * step_of(i0 + i));
 #pragma unroll
-                for (int nt = 0; nt < NT; ++nt) {
-                    mma_16816_s(acc[nt], lo[i].x, hi[i].x, lo[i].y, hi[i].y, b[i][nt].x, b[i][nt].y);
-                    mma_16816_s(acc[nt], lo[i].z, hi[i].z, lo[i].w, hi[i].w, b[i][nt].z, b[i][nt].w);
+            for (int i = 0; i < kAtOnce; ++i)
+                if (warp + (i0 + i) * kSkinnyWarps < steps) {
+                    const uint4 l = lo[i0 + i], h = hi[i0 + i];
+#pragma unroll
+                    for (int nt = 0; nt < NT; ++nt) {
+                        mma_16816_s(acc[nt], l.x, h.x, l.y, h.y, b[i][nt].x, b[i][nt].y);
+                        mma_16816_s(acc[nt], l.z, h.z, l.w, h.w, b[i][nt].z, b[i][nt].w);
+                    }
                 }
-            }
+        }
     }
     if constexpr (!kShort) {
 #pragma unroll kFlight
@@ -224,15 +231,15 @@ static int launch_skinny_epi(const void* W, const void* X, void* out, int M, int
                    g_skinny_prefetch_lines, (int)(blocks <= per_sm * sms), clamp);
     };
     if (K >= kManyWarpsK && 2 * blocks <= sms)
-        start(skinny_gemm_kernel<NT, EPI, 16, 8>, 16, 1u);
+        start(skinny_gemm_kernel<NT, EPI, 16, 8, NT == 1>, 16, 1u);
     else if (K <= kShortK / 4)
-        start(skinny_gemm_kernel<NT, EPI, 8, 1>, 8, NT == 1 ? 4u : 3u);
+        start(skinny_gemm_kernel<NT, EPI, 8, 1, true>, 8, NT == 1 ? 4u : 3u);
     else if (K <= kShortK / 2)
-        start(skinny_gemm_kernel<NT, EPI, 8, 2>, 8, NT == 1 ? 4u : 3u);
+        start(skinny_gemm_kernel<NT, EPI, 8, 2, true>, 8, NT == 1 ? 4u : 3u);
     else if (K <= kShortK)
-        start(skinny_gemm_kernel<NT, EPI, 8, 4>, 8, NT == 1 ? 4u : 3u);
+        start(skinny_gemm_kernel<NT, EPI, 8, 4, true>, 8, NT == 1 ? 4u : 3u);
     else
-        start(skinny_gemm_kernel<NT, EPI, 8, 8>, 8, 2u);
+        start(NT == 1 || K < 2 * kShortK ? skinny_gemm_kernel<NT, EPI, 8, 8, true> : skinny_gemm_kernel<NT, EPI, 8, 8, NT == 1>, 8, 2u);
     return launch_status();
 }
 
