@@ -800,7 +800,8 @@ static int launch_decode(const void* q, const void* k_cache, const void* v_cache
 
 // q [n_seqs, heads, d] bf16, one token per sequence; out [n_seqs, heads, d] bf16.  arrivals: null, or n_seqs * n_kv * ceil(group / 16) (times
 // the runs) counters that are zero, are zero again when the kernel ends, and belong to no other kernel meanwhile (for up to 32 shares a
-// sequence: without them the shares are added up by a kernel of its own, which takes any number).
+// sequence: without them the shares are added up by a kernel of its own, which takes any number).  At head size 64 up to 16 shares
+// are added up by a sequence's blocks as a cluster, which touches neither counters nor scratch.
 CPM_API int cpm_decode_attention_bf16(const void* q, const void* k_cache, const void* v_cache, void* out,
                                       const int* kv_len, const int* slots, const int* page_table, int max_pages,
                                       float* scratch, int n_seqs, int n_heads, int n_kv, int d, int n_splits,

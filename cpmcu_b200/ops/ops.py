@@ -823,8 +823,11 @@ class Ops:
         block per SM (its page buffers fill the shared memory), the decode kernel at head size ``d`` 64 two of half the size; but a
         sequence that would be one share of a block that fills an SM stays one there too (64 sequences of 4,000 tokens, 2 kv heads:
         1,465 us a step of 24 layers, 1,543 as two shares).  At head size 64 the shares of a sequence are a cluster of blocks, and eight are
-        better than sixteen as long as they have few pages each: where the page table ends at ``longest`` <= SHORT_TOKENS tokens (one
-        sequence of 1,000 tokens: 524 and 553 us a step; of 8,000: 659 and 616)."""
+        better than sixteen as long as they have few pages each.  A recorded step does not know the sequences' lengths, so what
+        counts is what the cache allows: where the page table ends at ``longest`` <= SHORT_TOKENS tokens.  us a layer, attention and O
+        product, with eight and sixteen, one sequence of 1,000 tokens 7.9 and 9.0, 2,500 7.9 and 9.2, 4,000 9.1 and 8.2, 8,000 12.0 and 9.8, 32,000
+        26.9 and 17.7; four of 1,000 9.2 and 9.5, 4,000 10.5 and 9.9.  A cache that allows more than SHORT_TOKENS therefore
+        takes 5 % longer a step for short sequences than one that does not (one of 1,000: 553 us against 524)."""
         m_tiles = (n_heads // n_kv + 15) // 16
         units = max(1, n_seqs * n_kv * m_tiles)
         per_sm = self.lib.cpm_decode_attention_blocks_per_sm(d) if d else 1
