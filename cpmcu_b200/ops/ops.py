@@ -836,7 +836,16 @@ class Ops:
         most = self.MAX_DECODE_SPLITS
         if d == self.CLUSTER_HEAD_DIM and 0 < longest <= self.SHORT_TOKENS:
             most = min(most, self.SHORT_SHARES)
-        return max(1, min(most, self.sm_count * per_sm // units))
+        shares = max(1, min(most, self.sm_count * per_sm // units))
+        if d == self.CLUSTER_HEAD_DIM and shares <= self.CLUSTER_SHARES:
+            # a cluster's blocks lie within one group of SMs, so larger clusters leave places empty, and where a batch's do not run at the same
+            # time the last start when the first have ended: more than four blocks have room on 3/2, more than six on 4/3 of the SMs.  us a
+            # layer, attention and O product, with a share for every place and as it is: eight sequences of 1,000, 2,500 and 6,000 tokens
+            # 16.8, 17.1, 19.2 (16 shares) and 10.0, 12.2, 13.2 (12), twelve 10.7, 19.2, 22.4 (12) and 10.1, 11.5, 14.6 (8), sixteen 11.9, 18.5,
+            # 24.4 (9) and 10.3, 12.8, 17.0 (6), twenty 14.3, 24.5, 32.1 (7) and 15.1, 17.9, 22.7 (5)
+            while shares > 4 and units * shares * 6 > self.sm_count * (8 if shares > 6 else 9):
+                shares -= 1
+        return shares
 
     CLUSTER_SHARES, CLUSTER_HEAD_DIM = 16, 64    # up to so many a sequence's blocks are a cluster and add up the shares among themselves
     SHORT_SHARES, SHORT_TOKENS = 8, 5120         # blocks of a cluster where no sequence can be longer

@@ -52,6 +52,15 @@ def test_the_librarys_per_head_product_takes_operands_that_want_a_gradient(which
         assert torch.allclose({"a": a, "w": w}[which].grad, grad, atol=1e-4)
 
 
+@pytest.mark.parametrize("rows,longest,shares", [(1, 32000, 16), (6, 32000, 16), (7, 32000, 14), (8, 32000, 12), (9, 32000, 10), (10, 32000, 9),
+                                                 (12, 32000, 8), (16, 32000, 6), (20, 32000, 5), (24, 32000, 4), (32, 32000, 4), (8, 4096, 8),
+                                                 (16, 4096, 6), (37, 4096, 4), (40, 4096, 1), (75, 4096, 1)])
+def test_head_size_64_has_as_many_shares_as_clusters_run_at_once(rows, longest, shares):
+    ops = DryOps(torch.bfloat16)
+    ops.lib = SimpleNamespace(cpm_decode_attention_blocks_per_sm=lambda d: 2)
+    assert ops.decode_splits(rows, 16, 2, 64, longest) == shares
+
+
 @pytest.mark.parametrize("portions,by_tiles", [
     ([2048], True), ([512], True), ([256], True), ([128], False), ([16], False), ([16] * 64, False), ([32] * 64, False),
     ([1] * 63 + [256], False), ([1] * 63 + [1985], False), ([65] * 15 + [1073], True), ([512] * 4, True), ([8] * 63 + [1544], False),
